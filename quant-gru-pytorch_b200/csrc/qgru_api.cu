@@ -138,7 +138,8 @@ void qgru_destroy(qgru_handle *h) {
     if (h->h_flags) cudaFreeHost(h->h_flags);
     cudaFree(h->d_bar);
     for (DevBuf *b : {&h->x8, &h->ih, &h->h8, &h->x32, &h->ih32, &h->hh32, &h->hq32, &h->stage_in,
-                      &h->stage_h0, &h->stage_out, &h->f_wx, &h->f_h, &h->f_v, &h->f_acc, &h->f_acc2})
+                      &h->stage_h0, &h->stage_out, &h->f_wx, &h->f_h, &h->f_v, &h->f_acc, &h->f_acc2, &h->vq32, &h->bwd_dp,
+                      &h->bwd_dq, &h->bwd_bias, &h->bwd_pm, &h->f_split, &h->fs_ch})
         cudaFree(b->p);
     cudaGetLastError();
     delete h;

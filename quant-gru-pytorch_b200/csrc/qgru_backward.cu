@@ -3,69 +3,38 @@
 // (src/gru_interface.cc:246-290, src/gru_backward_gpu_quant.cu).  One implementation: the float
 // backward is the masked one with every mask absent.
 //
-// Per timestep, last to first: the pointwise kernel turns dh into the gradients of the two
-// linear layers' outputs (dp for W*x + bw, dq for R*h + br) and the part of dh that flows
-// through the update gate; dh += dq * R^T.  After the loop: dbw / dbr as column sums of dp / dq
-// (the reference adds them with atomics, in arbitrary order; here the sum is a fixed-order tree,
-// so results repeat), then dx = dp * W^T, dR += h^T * dq, dW += x^T * dp.
-// Not a hot path: plain fp32 SIMT GEMMs (the reference calls cuBLAS SGEMM, fp32 without
-// tensor-op math in this pass).
+// Per timestep, last to first: dh becomes the gradients of the two linear layers' outputs (dp for
+// W*x + bw, dq for R*h + br) and the part of dh that flows through the update gate; dh += dq * R^T.
+// All steps in one launch (k_bwd_chain, qgru_rec_f32.cu), which also sums dp and dq over the rows for
+// the bias gradients in a fixed order (the reference adds them with atomics, in arbitrary order).
+// Then dx = dp * W^T, dR += h^T * dq, dW += x^T * dp (k_gemm_f32; the reference calls cuBLAS SGEMM,
+// fp32 without tensor-op math in this pass).
+#include "qgru_gemm_f32.cuh"
 #include "qgru_handle.h"
+#include "qgru_rec_f32.cuh"
 
 using namespace qgru;
 
 namespace {
 
-// C[n][j] (+)= sum_k A(n, k) * B[k][j].  A is [N][K] row-major, or with ATrans stored as [K][N].
-// B is [K][M] row-major, C [N][M].  64x64 tile, 4x4 outputs per thread.
-template <bool ATrans, bool Accum>
-__global__ void __launch_bounds__(256)
-k_bwd_sgemm(const float *__restrict__ A, const float *__restrict__ Bm, float *__restrict__ C,
-            long long N, long long K, int M) {
-    __shared__ float as[16][64 + 1];
-    __shared__ float bs[16][64];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const long long n0 = (long long)blockIdx.x * 64;
-    const int c0 = blockIdx.y * 64;
-    float acc[4][4] = {};
-    for (long long k0 = 0; k0 < K; k0 += 16) {
-        for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-            if (ATrans) {
-                const int kk = i >> 6, r = i & 63;      // consecutive threads walk n: coalesced
-                as[kk][r] = (n0 + r < N && k0 + kk < K) ? A[(k0 + kk) * N + n0 + r] : 0.f;
-            } else {
-                const int r = i >> 4, kk = i & 15;
-                as[kk][r] = (n0 + r < N && k0 + kk < K) ? A[(n0 + r) * K + k0 + kk] : 0.f;
-            }
-            const int kr = i >> 6, cc = i & 63;
-            bs[kr][cc] = (k0 + kr < K && c0 + cc < M) ? Bm[(k0 + kr) * M + c0 + cc] : 0.f;
+// The clamp masks of a step's cells in one word each (PM_* bits): the recurrence reads two bytes per cell
+// and step instead of ten or thirteen.  Absent masks keep everything.
+__global__ void k_bwd_pack_masks(uint16_t *__restrict__ pm, long long N, int H, const uint8_t *__restrict__ ih,
+                                 const uint8_t *__restrict__ hh, const uint8_t *__restrict__ gin,
+                                 const uint8_t *__restrict__ gout, const uint8_t *__restrict__ hm) {
+    const long long total = N * H;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const long long n = i / H;
+        const long long at = n * 3 * H + (i - n * H);
+        unsigned m = 0;
+#pragma unroll
+        for (int g = 0; g < 3; ++g) {
+            const long long k = at + (long long)g * H;
+            m |= (unsigned)(!ih || ih[k]) << (PM_IH + g) | (unsigned)(!hh || hh[k]) << (PM_HH + g) |
+                 (unsigned)(!gin || gin[k]) << (PM_IN + g) | (unsigned)(!gout || gout[k]) << (PM_OUT + g);
         }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = as[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = bs[kk][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const long long n = n0 + ty * 4 + i;
-        if (n >= N) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = c0 + tx + 16 * j;
-            if (c >= M) continue;
-            if (Accum) C[n * M + c] += acc[i][j];
-            else C[n * M + c] = acc[i][j];
-        }
+        m |= (unsigned)(!hm || hm[i]) << PM_H;
+        pm[i] = (uint16_t)m;
     }
 }
 
@@ -73,19 +42,19 @@ k_bwd_sgemm(const float *__restrict__ A, const float *__restrict__ Bm, float *__
 // with masks kernel::PointwiseOperationsQuant, src/gru_backward_gpu_quant.cu:72-250, zoneout
 // off).  h: h_{t-1} [B][H]; v: (z, r, g, R*h_g + br_g) [B][4H]; dh_new: gradient arriving at
 // h_t from outside; dh: in: gradient arriving from step t+1, out: its part through the update
-// gate (the R^T part is added by the GEMM that follows).  Masks: 1 keeps the gradient, 0 (the
-// forward clamped there) drops it; any may be null.
+// gate (the R^T part is added by the GEMM that follows).  pm: packed masks of the step or null; 1 keeps
+// the gradient, 0 (the forward clamped there) drops it.
 __global__ void __launch_bounds__(256)
 k_bwd_pointwise(int B, int H, const float *__restrict__ h, const float *__restrict__ v,
                 const float *__restrict__ dh_new, float *__restrict__ dh, float *__restrict__ dp,
-                float *__restrict__ dq, const uint8_t *__restrict__ m_hh, const uint8_t *__restrict__ m_gin,
-                const uint8_t *__restrict__ m_gout, const uint8_t *__restrict__ m_h) {
+                float *__restrict__ dq, const uint16_t *__restrict__ pm) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int b = blockIdx.y;
     if (j >= H || b >= B) return;
     const size_t base = (size_t)b * H + j;
     float dh_total = dh_new[base] + dh[base];
-    if (m_h) dh_total *= (float)m_h[base];
+    const unsigned m = pm ? pm[base] : 0xffffu;
+    if (!(m >> PM_H & 1)) dh_total *= 0.f;
     const float *vb = v + (size_t)b * 4 * H + j;
     const float z = vb[0], r = vb[H], g = vb[2 * H], q_g = vb[3 * H];
     dh[base] = z * dh_total;
@@ -102,9 +71,10 @@ k_bwd_pointwise(int B, int H, const float *__restrict__ h, const float *__restri
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const size_t at = idx + (size_t)k * H;
-        if (m_gout) { const float m = (float)m_gout[at]; p[k] *= m; q[k] *= m; }
-        if (m_gin) { const float m = (float)m_gin[at]; p[k] *= m; q[k] *= m; }
-        if (m_hh) q[k] *= (float)m_hh[at];
+        const float keep = (m >> (PM_OUT + k) & 1) && (m >> (PM_IN + k) & 1) ? 1.f : 0.f;
+        p[k] *= keep;
+        q[k] *= keep;
+        if (!(m >> (PM_HH + k) & 1)) q[k] *= 0.f;
         dp[at] = p[k];
         dq[at] = q[k];
     }
@@ -139,10 +109,16 @@ __global__ void k_bwd_apply_mask(float *__restrict__ data, const uint8_t *__rest
         data[i] *= (float)mask[i];
 }
 
-template <bool ATrans, bool Accum>
-void sgemm(const float *A, const float *Bm, float *C, long long N, long long K, int M, cudaStream_t st) {
-    dim3 grid((unsigned)((N + 63) / 64), (unsigned)((M + 63) / 64));
-    k_bwd_sgemm<ATrans, Accum><<<grid, 256, 0, st>>>(A, Bm, C, N, K, M);
+// The bias gradients from the sums the recurrence leaves per group of batch rows: part [G][6][H] (z, r, n of
+// dp, then of dq), added in group order.
+__global__ void k_bwd_bias(const float *__restrict__ part, int G, int H, const uint8_t *__restrict__ m_bw,
+                           const uint8_t *__restrict__ m_br, float *__restrict__ dbw, float *__restrict__ dbr) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, C = 3 * H;
+    if (c >= 2 * C) return;
+    float s = 0.f;
+    for (int g = 0; g < G; ++g) s += part[(size_t)g * 2 * C + c];
+    if (c < C) dbw[c] += m_bw ? s * (float)m_bw[c] : s;
+    else dbr[c - C] += m_br ? s * (float)m_br[c - C] : s;
 }
 
 }  // namespace
@@ -166,34 +142,49 @@ int qgru_backward(qgru_handle *h, int T, int B, const float *W_t, const float *R
     float *dp = (float *)h->bwd_dp.p, *dq = (float *)h->bwd_dq.p;
     const qgru_bwd_masks none{};
     const qgru_bwd_masks &m = mk ? *mk : none;
-
-    const dim3 pw_grid((H + 255) / 256, B);
-    for (int i = T - 1; i >= 0; --i) {
-        k_bwd_pointwise<<<pw_grid, 256, 0, st>>>(
-            B, H, h_all + (size_t)i * NH, v + (size_t)i * NH * 4, dh_new + (size_t)(i + 1) * NH, dh,
-            dp + (size_t)i * NH3, dq + (size_t)i * NH3, m.hh_linear ? m.hh_linear + (size_t)i * NH3 : nullptr,
-            m.gate_input ? m.gate_input + (size_t)i * NH3 : nullptr,
-            m.gate_output ? m.gate_output + (size_t)i * NH3 : nullptr, m.h ? m.h + (size_t)i * NH : nullptr);
-        // dh[b][k] += sum_m dq[b][m] * R_t[m][k]
-        sgemm<false, true>(dq + (size_t)i * NH3, R_t, dh, B, C, H, st);
+    uint16_t *pm = nullptr;
+    if (m.ih_linear || m.hh_linear || m.gate_input || m.gate_output || m.h) {
+        if ((rc = ensure(h, h->bwd_pm, (size_t)N * H * sizeof(uint16_t) + 4))) return rc;
+        pm = (uint16_t *)h->bwd_pm.p;
+        k_bwd_pack_masks<<<grid_for(N * H, 256, h->sm_count), 256, 0, st>>>(pm, N, H, m.ih_linear, m.hh_linear, m.gate_input,
+                                                                            m.gate_output, m.h);
+        h->launches++;
     }
-    h->launches += 2ull * T;
-    // bias gradients: column sums of dp / dq before the W*x + bw mask is applied to dp
-    k_bwd_colsum<<<(C + 31) / 32, 256, 0, st>>>(dp, N, C, m.bw, dbw);
-    k_bwd_colsum<<<(C + 31) / 32, 256, 0, st>>>(dq, N, C, m.br, dbr);
-    if (m.ih_linear)
-        k_bwd_apply_mask<<<grid_for(N * C, 256, h->sm_count), 256, 0, st>>>(dp, m.ih_linear, N * C);
+
+    int G = 0;
+    if (bwd_chain_fits(h, B, &G)) {
+        if ((rc = ensure(h, h->bwd_bias, (size_t)G * 2 * C * sizeof(float)))) return rc;
+        float *part = (float *)h->bwd_bias.p;
+        if ((rc = bwd_chain_launch(h, BwdChainArgs{T, B, H, R_t, 1, h_all, v, dh_new, dh, pm, dp, dq, part}, st)))
+            return rc;
+        k_bwd_bias<<<(2 * C + 127) / 128, 128, 0, st>>>(part, G, H, m.bw, m.br, dbw, dbr);
+        h->launches++;
+    } else {
+        // wide layers, step by step: the pointwise part, then dh[b][k] += sum_m dq[b][m] * R_t[m][k]
+        const dim3 pw_grid((H + 255) / 256, B);
+        for (int i = T - 1; i >= 0; --i) {
+            k_bwd_pointwise<<<pw_grid, 256, 0, st>>>(
+                B, H, h_all + (size_t)i * NH, v + (size_t)i * NH * 4, dh_new + (size_t)(i + 1) * NH, dh,
+                dp + (size_t)i * NH3, dq + (size_t)i * NH3, pm ? pm + (size_t)i * NH : nullptr);
+            if ((rc = gemm_f32(h, GemmF32{dq + (size_t)i * NH3, false, R_t, false, dh, B, C, H, true}, st))) return rc;
+        }
+        // bias gradients: column sums of dp / dq before the W*x + bw mask is applied to dp
+        k_bwd_colsum<<<(C + 31) / 32, 256, 0, st>>>(dp, N, C, m.bw, dbw);
+        k_bwd_colsum<<<(C + 31) / 32, 256, 0, st>>>(dq, N, C, m.br, dbr);
+        if (m.ih_linear)
+            k_bwd_apply_mask<<<grid_for(N * C, 256, h->sm_count), 256, 0, st>>>(dp, m.ih_linear, N * C);
+        h->launches += T + 2 + (m.ih_linear ? 1 : 0);
+    }
     // dx[n][i] = sum_m dp[n][m] * W_t[m][i]
-    sgemm<false, false>(dp, W_t, dx, N, C, I, st);
-    if (m.x) k_bwd_apply_mask<<<grid_for(N * I, 256, h->sm_count), 256, 0, st>>>(dx, m.x, N * I);
+    if ((rc = gemm_f32(h, GemmF32{dp, false, W_t, false, dx, N, C, I, false, m.x}, st))) return rc;
     // dR[k][m] += sum_n h[n][k] * dq[n][m]   (h_all's first T slots: h_{t-1} of every step)
-    sgemm<true, true>(h_all, dq, dR, H, N, C, st);
-    if (m.R) k_bwd_apply_mask<<<grid_for((long long)H * C, 256, h->sm_count), 256, 0, st>>>(dR, m.R, (long long)H * C);
+    if ((rc = gemm_f32(h, GemmF32{h_all, true, dq, false, dR, H, N, C, true, m.R}, st))) return rc;
     // dW[i][m] += sum_n x_t[i][n] * dp[n][m]
-    sgemm<false, true>(x_t, dp, dW, I, N, C, st);
-    if (m.W) k_bwd_apply_mask<<<grid_for((long long)I * C, 256, h->sm_count), 256, 0, st>>>(dW, m.W, (long long)I * C);
-    if (m.h0) k_bwd_apply_mask<<<grid_for((long long)NH, 256, h->sm_count), 256, 0, st>>>(dh, m.h0, (long long)NH);
-    h->launches += 9;
+    if ((rc = gemm_f32(h, GemmF32{x_t, false, dp, false, dW, I, N, C, true, m.W}, st))) return rc;
+    if (m.h0) {
+        k_bwd_apply_mask<<<grid_for((long long)NH, 256, h->sm_count), 256, 0, st>>>(dh, m.h0, (long long)NH);
+        h->launches++;
+    }
     CK(cudaGetLastError());
     return QGRU_OK;
 }

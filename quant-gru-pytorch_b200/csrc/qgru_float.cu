@@ -1,15 +1,17 @@
 // qgru_float.cu - the unquantized fp32 GRU ("float mode") and the MinMax calibration pass.
 //
 // Float mode follows hasteGRUForward / ForwardPass<float> of the reference
-// (src/gru_interface.cc:173-207, src/gru_forward_gpu.cu:23-125, 342-414): one GEMM for W*x
-// over all timesteps, then per step R*h and the pointwise gate kernel; here the per-step
-// GEMV and the gates are one kernel.  Calibration runs the same forward and folds the
-// min/max of every operator while the values are still in registers - the reference
+// (src/gru_interface.cc:173-207, src/gru_forward_gpu.cu:23-125, 342-414): one product for W*x
+// over all timesteps, then the recurrence in one launch (qgru_rec_f32.cu; wider layers than its
+// registers hold run step by step).  Calibration runs the same forward with the gate buffer kept and
+// folds the min/max of every operator in one pass over it - the reference
 // materialises five capture tensors and seven temporaries of T*B*H floats and reduces each in
 // its own pass (src/calibration_gpu.cu:1776-1953).
 #include <cfloat>
 
+#include "qgru_gemm_f32.cuh"
 #include "qgru_handle.h"
+#include "qgru_rec_f32.cuh"
 
 using namespace qgru;
 
@@ -51,115 +53,68 @@ __device__ __forceinline__ void warp_fold(MinMax m, unsigned *acc_min, unsigned 
     }
 }
 
-// ---- C[n][c] = sum_k x[n][k] * W[k][c]   (fp32, 64x64 tile, 4x4 per thread)
-__global__ void __launch_bounds__(256)
-k_sgemm_xw(const float *__restrict__ x, const float *__restrict__ W, float *__restrict__ out,
-           long long N, int K, int Cn) {
-    __shared__ float xs[16][64 + 1];
-    __shared__ float ws[16][64];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const long long n0 = (long long)blockIdx.x * 64;
-    const int c0 = blockIdx.y * 64;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        for (int i = threadIdx.x; i < 64 * 16; i += 256) {
-            const int r = i >> 4, kk = i & 15;
-            xs[kk][r] = (n0 + r < N && k0 + kk < K) ? x[(n0 + r) * K + k0 + kk] : 0.f;
-            const int kr = i >> 6, cc = i & 63;
-            ws[kr][cc] = (k0 + kr < K && c0 + cc < Cn) ? W[(size_t)(k0 + kr) * Cn + c0 + cc] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = xs[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = ws[kk][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const long long n = n0 + ty * 4 + i;
-        if (n >= N) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = c0 + tx + 16 * j;
-            if (c < Cn) out[n * Cn + c] = acc[i][j];
-        }
-    }
-}
-
-// ---- one timestep after R*h has been multiplied (k_sgemm_xw on h_{t-1}): the float gates of
+// ---- one timestep after R*h has been multiplied (wide layers): the float gates of
 // src/gru_forward_gpu.cu:23-125 for (b, j).  rh [B][3H] holds R*h without its bias.
-template <bool Calib>
 __global__ void __launch_bounds__(256)
 k_float_step(const float *__restrict__ wx, const float *__restrict__ rh, const float *__restrict__ bw,
              const float *__restrict__ br, const float *__restrict__ h_in, float *__restrict__ h_out,
-             float *__restrict__ v, int v_stride, int B, int H, unsigned *acc_min, unsigned *acc_max) {
+             float *__restrict__ v, int v_stride, int B, int H) {
     const int j = blockIdx.x * 128 + (threadIdx.x & 127);
     const int b = blockIdx.y * 2 + (threadIdx.x >> 7);
-    const bool ok = j < H && b < B;
+    if (j >= H || b >= B) return;
     const int Cn = 3 * H;
-    MinMax m_h, m_ih, m_hh, m_zin, m_rin, m_nin, m_z, m_r, m_n, m_rh, m_new, m_old;
-    if (Calib) {
-        m_h.init(); m_ih.init(); m_hh.init(); m_zin.init(); m_rin.init(); m_nin.init();
-        m_z.init(); m_r.init(); m_n.init(); m_rh.init(); m_new.init(); m_old.init();
+    const float *rhr = rh + (size_t)b * Cn + j;
+    const float *wxr = wx + (size_t)b * Cn + j;
+    const float rz = rhr[0] + br[j], rr = rhr[H] + br[H + j], rg = rhr[2 * H] + br[2 * H + j];
+    const float z = 1.0f / (1.0f + expf(-((wxr[0] + bw[j]) + rz)));
+    const float r = 1.0f / (1.0f + expf(-((wxr[H] + bw[H + j]) + rr)));
+    const float g = tanhf((wxr[2 * H] + bw[2 * H + j]) + r * rg);
+    h_out[(size_t)b * H + j] = z * h_in[(size_t)b * H + j] + (1.0f - z) * g;
+    if (v) {
+        // 4 slots per row: the reference's training buffer (z, r, n, Rh_n + br_n); 6 slots:
+        // all three R*h + br rows as well (z, r, n, Rh_z+br_z, Rh_r+br_r, Rh_n+br_n)
+        float *vb = v + (size_t)b * v_stride * H + j;
+        vb[0] = z; vb[H] = r; vb[2 * H] = g;
+        if (v_stride == 6) { vb[3 * H] = rz; vb[4 * H] = rr; vb[5 * H] = rg; }
+        else vb[3 * H] = rg;
     }
-    if (ok) {
-        const float *rhr = rh + (size_t)b * Cn + j;
-        const float az = rhr[0], ar = rhr[H], an = rhr[2 * H];
-        const float *wxr = wx + (size_t)b * Cn + j;
-        const float wz = wxr[0] + bw[j], rz = az + br[j];
-        const float z_pre = wz + rz;
-        const float z = 1.0f / (1.0f + expf(-z_pre));
-        const float wr = wxr[H] + bw[H + j], rr_ = ar + br[H + j];
-        const float r_pre = wr + rr_;
-        const float r = 1.0f / (1.0f + expf(-r_pre));
-        const float wg = wxr[2 * H] + bw[2 * H + j], rg = an + br[2 * H + j];
-        const float g_pre = wg + r * rg;
-        const float g = tanhf(g_pre);
-        const float h_old = h_in[(size_t)b * H + j];
-        const float old_c = z * h_old;
-        const float new_c = (1.0f - z) * g;
-        const float hn = old_c + new_c;
-        h_out[(size_t)b * H + j] = hn;
-        if (v) {
-            // 4 slots per row: the reference's training buffer (z, r, n, Rh_n + br_n); 6 slots:
-            // all three R*h + br rows as well (z, r, n, Rh_z+br_z, Rh_r+br_r, Rh_n+br_n)
-            float *vb = v + (size_t)b * v_stride * H + j;
-            vb[0] = z; vb[H] = r; vb[2 * H] = g;
-            if (v_stride == 6) { vb[3 * H] = rz; vb[4 * H] = rr_; vb[5 * H] = rg; }
-            else vb[3 * H] = rg;
+}
+
+// ---- min/max of the twelve operators of the cell over a whole sequence, from the forward's buffers: wx
+// (W*x) [N][3H], v with six slots, h [N + B][H].  One pass at memory speed (ten reads per cell) instead of
+// reductions inside the recurrence, whose registers hold R.  A thread walks rows of one unit.
+__global__ void __launch_bounds__(128)
+k_minmax_cell(const float *__restrict__ wx, const float *__restrict__ v, const float *__restrict__ h,
+              const float *__restrict__ bw, long long N, int B, int H, unsigned *acc_min, unsigned *acc_max) {
+    const int j = blockIdx.x * 128 + threadIdx.x;
+    constexpr int OPS[12] = {QGRU_OP_H, QGRU_OP_IH_LINEAR, QGRU_OP_HH_LINEAR, QGRU_OP_UPDATE_IN, QGRU_OP_RESET_IN, QGRU_OP_NEW_IN,
+                             QGRU_OP_UPDATE_OUT, QGRU_OP_RESET_OUT, QGRU_OP_NEW_OUT, QGRU_OP_MUL_RESET_HIDDEN,
+                             QGRU_OP_MUL_NEW_CONTRIB, QGRU_OP_MUL_OLD_CONTRIB};
+    MinMax m[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) m[k].init();
+    if (j < H) {
+        const float bz = bw[j], brr = bw[H + j], bg = bw[2 * H + j];
+#pragma unroll 2
+        for (long long n = blockIdx.y; n < N; n += gridDim.y) {
+            const float *w = wx + n * 3 * H + j, *q = v + n * 6 * H + j;
+            const float wz = w[0] + bz, wr = w[H] + brr, wg = w[2 * H] + bg;
+            const float z = q[0], r = q[H], g = q[2 * H], rz = q[3 * H], rr = q[4 * H], rg = q[5 * H];
+            const float h_old = h[n * H + j], hn = h[(n + B) * H + j];
+            m[0].add(hn);
+            m[1].add(wz); m[1].add(wr); m[1].add(wg);
+            m[2].add(rz); m[2].add(rr); m[2].add(rg);
+            m[3].add(wz + rz);
+            m[4].add(wr + rr);
+            m[5].add(wg + r * rg);
+            m[6].add(z); m[7].add(r); m[8].add(g);
+            m[9].add(r * rg);
+            m[10].add((1.0f - z) * g);
+            m[11].add(z * h_old);
         }
-        if (Calib) {
-            m_h.add(hn);
-            m_ih.add(wz); m_ih.add(wr); m_ih.add(wg);
-            m_hh.add(rz); m_hh.add(rr_); m_hh.add(rg);
-            m_zin.add(z_pre); m_rin.add(r_pre); m_nin.add(g_pre);
-            m_z.add(z); m_r.add(r); m_n.add(g);
-            m_rh.add(r * rg); m_new.add(new_c); m_old.add(old_c);
-        }
     }
-    if (Calib) {
-        warp_fold(m_h, acc_min, acc_max, QGRU_OP_H, true);
-        warp_fold(m_ih, acc_min, acc_max, QGRU_OP_IH_LINEAR, true);
-        warp_fold(m_hh, acc_min, acc_max, QGRU_OP_HH_LINEAR, true);
-        warp_fold(m_zin, acc_min, acc_max, QGRU_OP_UPDATE_IN, true);
-        warp_fold(m_rin, acc_min, acc_max, QGRU_OP_RESET_IN, true);
-        warp_fold(m_nin, acc_min, acc_max, QGRU_OP_NEW_IN, true);
-        warp_fold(m_z, acc_min, acc_max, QGRU_OP_UPDATE_OUT, true);
-        warp_fold(m_r, acc_min, acc_max, QGRU_OP_RESET_OUT, true);
-        warp_fold(m_n, acc_min, acc_max, QGRU_OP_NEW_OUT, true);
-        warp_fold(m_rh, acc_min, acc_max, QGRU_OP_MUL_RESET_HIDDEN, true);
-        warp_fold(m_new, acc_min, acc_max, QGRU_OP_MUL_NEW_CONTRIB, true);
-        warp_fold(m_old, acc_min, acc_max, QGRU_OP_MUL_OLD_CONTRIB, true);
-    }
+#pragma unroll
+    for (int k = 0; k < 12; ++k) warp_fold(m[k], acc_min, acc_max, OPS[k], true);
 }
 
 // min/max of a whole tensor into slot `slot` (warp shuffles, one atomic pair per warp)
@@ -206,7 +161,7 @@ namespace qgru {
 
 int float_forward(qgru_handle *h, int T, int B, const float *W, const float *R, const float *bw,
                   const float *br, const float *x, const float *h0, float *h_out, float *v_out,
-                  int v_stride, unsigned *acc_min, unsigned *acc_max, cudaStream_t st) {
+                  int v_stride, cudaStream_t st) {
     const int H = h->H, Cn = h->C, I = h->I;
     const long long N = (long long)T * B;
     int rc;
@@ -214,24 +169,21 @@ int float_forward(qgru_handle *h, int T, int B, const float *W, const float *R, 
     float *wx = (float *)h->f_wx.p;
     const long long NH = (long long)B * H;
     k_init_h_float<<<(unsigned)((NH + 255) / 256), 256, 0, st>>>(h0, h_out, NH);
-    dim3 gg((unsigned)((N + 63) / 64), (unsigned)((Cn + 63) / 64));
-    k_sgemm_xw<<<gg, 256, 0, st>>>(x, W, wx, N, I, Cn);
-    h->launches += 2;
-    // per step: R*h as a tiled fp32 GEMM ([B][H] x [H][3H], the kernel of the input projection),
-    // then the pointwise gates
+    h->launches++;
+    if ((rc = gemm_f32(h, GemmF32{x, false, W, false, wx, N, I, Cn}, st))) return rc;
+    if (float_chain_fits(h, B))
+        return float_chain_launch(h, FloatFwdArgs{T, B, H, R, wx, bw, br, h_out, v_out, v_stride}, st);
+    // wide layers, step by step: R*h as a tiled product, then the pointwise gates
     if ((rc = ensure(h, h->f_acc2, (size_t)B * Cn * 4))) return rc;
     float *rh = (float *)h->f_acc2.p;
-    dim3 grid((H + 127) / 128, (B + 1) / 2), gr((unsigned)((B + 63) / 64), (unsigned)((Cn + 63) / 64));
+    dim3 grid((H + 127) / 128, (B + 1) / 2);
     for (int t = 0; t < T; ++t) {
         const float *hin = h_out + (size_t)t * NH;
         float *hout = h_out + (size_t)(t + 1) * NH;
         float *vt = v_out ? v_out + (size_t)t * B * v_stride * H : nullptr;
-        k_sgemm_xw<<<gr, 256, 0, st>>>(hin, R, rh, B, H, Cn);
-        if (acc_min)
-            k_float_step<true><<<grid, 256, 0, st>>>(wx + (size_t)t * B * Cn, rh, bw, br, hin, hout, vt, v_stride, B, H, acc_min, acc_max);
-        else
-            k_float_step<false><<<grid, 256, 0, st>>>(wx + (size_t)t * B * Cn, rh, bw, br, hin, hout, vt, v_stride, B, H, nullptr, nullptr);
-        h->launches += 2;
+        if ((rc = gemm_f32(h, GemmF32{hin, false, R, false, rh, B, H, Cn}, st))) return rc;
+        k_float_step<<<grid, 256, 0, st>>>(wx + (size_t)t * B * Cn, rh, bw, br, hin, hout, vt, v_stride, B, H);
+        h->launches++;
     }
     CK(cudaGetLastError());
     return QGRU_OK;
@@ -247,7 +199,7 @@ int qgru_forward_float(qgru_handle *h, int T, int B, const float *W, const float
     if (!h || !W || !R || !bw || !br || !x || !h_out) return QGRU_ERR_BAD_ARG;
     if (T <= 0 || B <= 0) return fail(h, QGRU_ERR_BAD_ARG, "T and B must be positive");
     CK(cudaSetDevice(h->device));
-    return float_forward(h, T, B, W, R, bw, br, x, h0, h_out, v_out, 4, nullptr, nullptr, (cudaStream_t)stream);
+    return float_forward(h, T, B, W, R, bw, br, x, h0, h_out, v_out, 4, (cudaStream_t)stream);
 }
 
 int qgru_calibrate_minmax(qgru_handle *h, int T, int B, const float *W, const float *R,
@@ -283,7 +235,13 @@ int qgru_calibrate_minmax(qgru_handle *h, int T, int B, const float *W, const fl
     for (int k = 0; k < 4; ++k)
         k_minmax_channels<<<(Cn + 127) / 128, 128, 0, st>>>(mats[k], rows[k], Cn, ch + (2 * k) * Cn, ch + (2 * k + 1) * Cn);
     h->launches += 7;
-    if ((rc = float_forward(h, T, B, W, R, bw, br, x, h0, hbuf, nullptr, 4, acc_min, acc_max, st))) return rc;
+    const long long N = (long long)T * B;
+    if ((rc = ensure(h, h->f_v, (size_t)N * 6 * H * 4))) return rc;
+    if ((rc = float_forward(h, T, B, W, R, bw, br, x, h0, hbuf, (float *)h->f_v.p, 6, st))) return rc;
+    const dim3 mg((H + 127) / 128, (unsigned)std::min<long long>(N, std::max(1, 8 * h->sm_count / ((H + 127) / 128))));
+    k_minmax_cell<<<mg, 128, 0, st>>>((const float *)h->f_wx.p, (const float *)h->f_v.p, hbuf, bw, N, B, H, acc_min, acc_max);
+    h->launches++;
+    CK(cudaGetLastError());
     std::vector<unsigned> host(n_acc);
     CK(cudaMemcpyAsync(host.data(), acc, (size_t)n_acc * 4, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));

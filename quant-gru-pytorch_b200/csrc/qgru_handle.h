@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "qgru_gemm_tc.cuh"
+#include "qgru_rec_f32.cuh"
 #include "qgru_rec_mma.cuh"
 #include "qgru_internal.h"
 
@@ -84,6 +85,9 @@ struct qgru_handle {
     DevBuf f_wx, f_h, f_v, f_acc, f_acc2;  // float mode / calibration (f_acc2: R*h of one step)
     DevBuf vq32;                           // integer training forward: gate buffer before dequantization
     DevBuf bwd_dp, bwd_dq;                 // backward pass: gradients of W*x + bw and R*h + br, [T*B][3H] each
+    DevBuf bwd_bias, bwd_pm;               // backward pass: bias sums per batch group, packed clamp masks
+    DevBuf f_split;                        // fp32 matrix product: partial tiles where K is split
+    qgru::F32RecPlan plan_fwd, plan_bwd;   // fp32 recurrences: the plan of the last batch size
     DevBuf fs_ch;                          // float-storage forward: 4 x 3H per-channel scale ratios
     bool fs_ready = false;                 // fs_ch matches the current parameters
     static constexpr int kRing = 64;

@@ -31,7 +31,7 @@ using namespace qgru;
 namespace qgru {
 int float_forward(qgru_handle *h, int T, int B, const float *W, const float *R, const float *bw,
                   const float *br, const float *x, const float *h0, float *h_out, float *v_out,
-                  int v_stride, unsigned *acc_min, unsigned *acc_max, cudaStream_t st);
+                  int v_stride, cudaStream_t st);
 int calibrate_histogram_op(const float *counts, int bins, float min_val, float max_val, long long total,
                            bool pot2, bool use_percentile, float percentile, qgru_op *op);
 }  // namespace qgru
@@ -508,7 +508,7 @@ int qgru_calibrate_hist(qgru_handle *h, qgru_hist *hs, int T, int B, const float
     if ((rc = ensure(h, h->f_h, (size_t)(T + 1) * B * H * 4))) return rc;
     if ((rc = ensure(h, h->f_v, (size_t)N * 6 * H * 4))) return rc;
     float *hbuf = (float *)h->f_h.p, *v = (float *)h->f_v.p;
-    if ((rc = float_forward(h, T, B, W, R, bw, br, x, h0, hbuf, v, 6, nullptr, nullptr, st))) return rc;
+    if ((rc = float_forward(h, T, B, W, R, bw, br, x, h0, hbuf, v, 6, st))) return rc;
     const float *wx = (const float *)h->f_wx.p;
 
     auto run = [&](int idx, Gen g) -> int {

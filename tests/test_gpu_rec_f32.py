@@ -1,0 +1,41 @@
+"""GPU tests of the fp32 recurrences and of the fp32 matrix product behind them, at the sizes where their
+plans change: one CTA per row group, clusters of 2 to 16, layers wider than the registers of a
+cluster hold, ragged rows and units, split and unsplit K."""
+import importlib
+
+import numpy as np
+import pytest
+
+from __graft_entry__ import PKG_NAME
+from oracle.backward_np import gru_backward
+from tests.cases import gen_weights, gen_x
+
+gru_ops = importlib.import_module(PKG_NAME + ".gru_ops")
+pytestmark = pytest.mark.gpu
+
+
+def _t(a, dev):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+
+
+@pytest.mark.parametrize("T,B,I,H", [(3, 1, 1, 1), (5, 3, 7, 31), (4, 2, 64, 32), (7, 40, 5, 33), (6, 9, 129, 128), (3, 17, 3, 129),
+                                     (40, 65, 12, 160), (3, 5, 20, 200), (3, 150, 66, 262), (2, 33, 16, 385), (3, 70, 8, 512),
+                                     (2, 3, 8, 513)])
+def test_float_forward_and_backward(oracle, cuda_device, T, B, I, H):
+    rng = np.random.default_rng(100 * H + B)
+    W, R, bw, br = gen_weights(rng, I, H)
+    x = gen_x(rng, T, B, I)
+    h0 = (rng.standard_normal((B, H)) * 0.3).astype(np.float32)
+    want_h, want_v = oracle.forward_float(T, B, I, H, W, R, bw, br, x, h0, want_v=True)
+    dh_new = rng.standard_normal((T + 1, B, H)).astype(np.float32)
+    with gru_ops.Handle(I, H, device=0) as hd:
+        d = [_t(a, cuda_device) for a in (W, R, bw, br, x)]
+        h, v = hd.forward_float(*d, h0=_t(h0, cuda_device), want_v=True)
+        assert np.abs(h.cpu().numpy() - want_h).max() <= 1e-5
+        assert np.abs(v.cpu().numpy() - want_v).max() <= 1e-5 * max(1.0, np.abs(want_v).max())
+        got = hd.backward(d[0], d[1], d[4], _t(dh_new, cuda_device), _t(want_h, cuda_device), _t(want_v, cuda_device))
+    want = gru_backward(W, R, x, dh_new, want_h, want_v)
+    for g, w in zip(got, want):
+        g = g.cpu().numpy().reshape(w.shape)
+        assert np.abs(g - w).max() <= 2e-5 * max(np.abs(w).max(), 1e-30)
