@@ -352,6 +352,22 @@ QGRU_API int qgru_forward_f32_host(qgru_handle *h, int T, int B, const float *x,
                                    const float *h0, float *h_out, unsigned flags,
                                    void *stream);
 
+/* The forward of a whole layer, as QuantGRU.forward / forward_quantized call it
+ * (pytorch/quant_gru.py:2095-2380): one direction (rev = NULL) or both (rev: the reverse direction's
+ * handle, same device and sizes; it runs beside the forward one on a stream of its own and `stream`
+ * waits for it).  Element (t, b, i) of x lies at t * x_ts + b * x_bs + i; element (t, b, d * H + j) of the
+ * output at t * out_ts + b * out_bs + d * H + j.  h0 and h_n: [D][B][H], h0 may be NULL.  float_storage:
+ * qgru_forward_fstorage's arithmetic instead of qgru_forward_f32's.  Asynchronous.  A device-side wait
+ * expiry of an EARLIER layer forward that nobody has asked about is returned here (QGRU_ERR_TIMEOUT). */
+QGRU_API int qgru_layer_forward(qgru_handle *h, qgru_handle *rev, int float_storage, int T, int B,
+                                const float *x, long long x_ts, long long x_bs, const float *h0,
+                                float *out, long long out_ts, long long out_bs, float *h_n,
+                                void *stream);
+QGRU_API int qgru_layer_forward_i32(qgru_handle *h, qgru_handle *rev, int T, int B, const int32_t *x_q,
+                                    long long x_ts, long long x_bs, const int32_t *h0_q,
+                                    int32_t *out_q, long long out_ts, long long out_bs,
+                                    int32_t *h_n_q, void *stream);
+
 /* Blocks until the work queued on `stream` by this handle is done and reports a device-side
  * bounded-wait expiry (QGRU_ERR_TIMEOUT) or CUDA error, as the reference's
  * cudaDeviceSynchronize + cudaGetLastError + throw does (src/gru_interface.cc:594-602).

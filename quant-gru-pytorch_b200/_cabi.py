@@ -96,6 +96,10 @@ SYMBOLS = {
     "qgru_forward_f32_q8": (C.c_int, [_P, C.c_int, C.c_int, _P, _P, _P, C.c_uint, _P]),
     "qgru_forward_i32_host": (C.c_int, [_P, C.c_int, C.c_int, _P, _P, _P, C.c_uint, _P]),
     "qgru_forward_f32_host": (C.c_int, [_P, C.c_int, C.c_int, _P, _P, _P, C.c_uint, _P]),
+    "qgru_layer_forward": (C.c_int, [_P, _P, C.c_int, C.c_int, C.c_int, _P, C.c_longlong, C.c_longlong, _P, _P, C.c_longlong,
+                                     C.c_longlong, _P, _P]),
+    "qgru_layer_forward_i32": (C.c_int, [_P, _P, C.c_int, C.c_int, _P, C.c_longlong, C.c_longlong, _P, _P, C.c_longlong,
+                                         C.c_longlong, _P, _P]),
     "qgru_synchronize": (C.c_int, [_P, _P]),
     "qgru_last_timing": (C.c_int, [_P, _F, _F, _F]),
     "qgru_timing_window": (C.c_int, [_P, C.POINTER(C.c_int), _F, _F, _F]),

@@ -93,7 +93,7 @@ int qgru_create(qgru_handle **out, int device, int input_size, int hidden_size) 
     ok = ok && cudaDeviceGetAttribute(&h->coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess;
     ok = ok && cudaMalloc(&h->d_flags, 2 * sizeof(int)) == cudaSuccess;
     ok = ok && cudaMemset(h->d_flags, 0, 2 * sizeof(int)) == cudaSuccess;
-    ok = ok && cudaMallocHost(&h->h_flags, 2 * sizeof(int)) == cudaSuccess;
+    ok = ok && cudaHostAlloc(&h->h_flags, 4 * sizeof(int), cudaHostAllocMapped) == cudaSuccess;
     for (int r = 0; r < qgru_handle::kRing && ok; ++r)
         for (int i = 0; i < 4 && ok; ++i) ok = cudaEventCreate(&h->ring[r][i]) == cudaSuccess;
     if (!ok) {
@@ -101,7 +101,7 @@ int qgru_create(qgru_handle **out, int device, int input_size, int hidden_size) 
         qgru_destroy(h);
         return QGRU_ERR_CUDA;
     }
-    h->h_flags[0] = h->h_flags[1] = 0;
+    h->h_flags[0] = h->h_flags[1] = h->h_flags[2] = 0;
     *out = h;
     return QGRU_OK;
 }
@@ -134,6 +134,9 @@ void qgru_destroy(qgru_handle *h) {
     }
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
     if (h->aux) cudaStreamDestroy(h->aux);
+    if (h->ev_split) cudaEventDestroy(h->ev_split);
+    if (h->ev_join) cudaEventDestroy(h->ev_join);
+    if (h->side) cudaStreamDestroy(h->side);
     cudaFree(h->d_flags);
     if (h->h_flags) cudaFreeHost(h->h_flags);
     cudaFree(h->d_bar);
@@ -656,9 +659,67 @@ int launch_gemv(qgru_handle *h, RecArgs &a, bool fused, cudaStream_t st) {
     return QGRU_OK;
 }
 
-// Shared tail of the two device entry points, 8-bit path: x8 and the initial state are ready.
-int run_fast(qgru_handle *h, int T, int B, int32_t *hq_out, float *hf_out, unsigned flags,
-             cudaStream_t st, uint8_t *h8_out = nullptr) {
+// One forward's inputs: row (t, b) of x at x + t * ts + b * bs (elements), initial state rows dense.
+// mode: PrologueArgs (0 fp32, 1 fp32 for the float-storage path, 2 int32 containers).
+struct FwdInput {
+    int mode;
+    const void *x;
+    long long ts, bs;
+    const void *h0;
+    void *xq = nullptr;              // optional dense copy of the quantized x
+    uint8_t *x_keep = nullptr, *h0_keep = nullptr;
+};
+
+// The first launch of a forward (k_prologue); x8: null where another handle has quantized the same x.
+int launch_prologue(qgru_handle *h, int T, int B, const FwdInput &in, uint8_t *x8, uint8_t *h8, const OutView &slot, cudaStream_t st) {
+    const qgru_op &xo = h->p.op[QGRU_OP_X], &ho = h->p.op[QGRU_OP_H];
+    PrologueArgs a{};
+    a.x = x8 ? in.x : nullptr;
+    a.x_ts = in.ts;
+    a.x_bs = in.bs;
+    a.N = (long long)T * B;
+    a.B = B;
+    a.K = h->I;
+    a.Kpad = h->Ipad;
+    a.x8 = x8;
+    a.xq = in.xq;
+    a.keep = in.x_keep;
+    a.x_scale = h->x_scale;
+    a.x_zp = xo.zero_point;
+    a.x_lo = op_qmin(xo);
+    a.x_hi = op_qmax(xo);
+    a.h0 = in.h0;
+    a.h8 = h8;
+    a.H = h->H;
+    a.Hpad = h->Hpad;
+    a.slot = slot;
+    a.h_scale = h->h_scale;
+    a.h_zp = ho.zero_point;
+    a.h_lo = op_qmin(ho);
+    a.h_hi = op_qmax(ho);
+    a.h0_keep = in.h0_keep;
+    a.flags = h->d_flags;
+    a.sticky = in.mode == 2 ? nullptr : h->h_flags + 2;
+    if (in.mode == 2) CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
+    a.q_blocks = x8 ? grid_for(a.N * (h->Ipad / 16), 256, h->sm_count) : 0;
+    const int blocks = a.q_blocks + grid_for((long long)B * h->Hpad, 256, h->sm_count);
+    const bool vec = h->I % 4 == 0 && in.ts % 4 == 0 && in.bs % 4 == 0 && (reinterpret_cast<uintptr_t>(in.x) & 15u) == 0;
+    if (in.mode == 0) {
+        if (vec) k_prologue<0, true><<<blocks, 256, 0, st>>>(a);
+        else k_prologue<0, false><<<blocks, 256, 0, st>>>(a);
+    } else if (in.mode == 1) {
+        if (vec) k_prologue<1, true><<<blocks, 256, 0, st>>>(a);
+        else k_prologue<1, false><<<blocks, 256, 0, st>>>(a);
+    } else {
+        k_prologue<2, false><<<blocks, 256, 0, st>>>(a);
+    }
+    CK(cudaGetLastError());
+    h->launches++;
+    return QGRU_OK;
+}
+
+// Shared tail of the device entry points, 8-bit path: x8 and the initial state are ready.
+int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out, unsigned flags, cudaStream_t st) {
     const long long N = (long long)T * B;
     const int C = h->C;
     int rc;
@@ -764,7 +825,7 @@ int run_fast(qgru_handle *h, int T, int B, int32_t *hq_out, float *hf_out, unsig
         // (the launcher also looks at how the second rescale is applied: table or shift-free scale)
         const bool gemm_fast = lcx.fits32 && h->rs_fast[0] && h->opt_cell != 2;
         const long long Nk = (long long)chunk_T(k) * B;
-        const int r = tc_gemm_launch(h->tc, (const uint8_t *)h->x8.p, (N + 127) / 128 * 128, h->d_w8[0], h->w8_rows[0],
+        const int r = tc_gemm_launch(h->tc, x8, (N + 127) / 128 * 128, h->d_w8[0], h->w8_rows[0],
                                      chunk_ih(k), Nk, C, h->Ipad, h->x_uns, ih_bytes, lcx, ps, gemm_fast,
                                      h->lin_notie[0] && h->opt_tie != 1, h->d_flags + 1, sms, gs, &h->err,
                                      (long long)chunk_t0(k) * B);
@@ -785,7 +846,6 @@ int run_fast(qgru_handle *h, int T, int B, int32_t *hq_out, float *hf_out, unsig
     }
     if (!used_tc) {
         dim3 grid((unsigned)((N + 63) / 64), (unsigned)((C + 63) / 64));
-        const uint8_t *x8 = (const uint8_t *)h->x8.p;
         if (h->ih_bytes == 1) {
             if (h->x_uns) k_gemm_wx_simt<true, int8_t><<<grid, 256, 0, st>>>(x8, h->d_w8[0], (int8_t *)h->ih.p, N, C, h->Ipad, lcx);
             else k_gemm_wx_simt<false, int8_t><<<grid, 256, 0, st>>>(x8, h->d_w8[0], (int8_t *)h->ih.p, N, C, h->Ipad, lcx);
@@ -803,7 +863,9 @@ int run_fast(qgru_handle *h, int T, int B, int32_t *hq_out, float *hf_out, unsig
         if ((rc = alloc_dev(h, &h->d_bar, (size_t)groups * 32))) return rc;
         h->bar_groups = groups;
     }
-    CK(cudaMemsetAsync(h->d_bar, 0, (size_t)groups * 32 * sizeof(unsigned), st));
+    // counters of the forms whose CTAs meet at one in global memory
+    if ((use_mma && !use_cluster) || (!use_mma && !use_gemv && pl.P > 1))
+        CK(cudaMemsetAsync(h->d_bar, 0, (size_t)groups * 32 * sizeof(unsigned), st));
     char buf[400];
     if (use_mma) {
         RecMmaArgs a;
@@ -813,9 +875,7 @@ int run_fast(qgru_handle *h, int T, int B, int32_t *hq_out, float *hf_out, unsig
         a.tmem_cols = (uint32_t)mp.tmem_cols;
         a.ih = h->ih.p;
         a.h8 = (uint8_t *)h->h8.p;
-        a.hq_out = hq_out;
-        a.hf_out = hf_out;
-        a.h8_out = h8_out;
+        a.out = out;
         a.lc = linear_consts(h, 1);
         a.tables = fused ? h->d_ftables : h->d_tables;
         a.n_table = fused ? h->gc_host.ft_ih_off : h->n_table;   // the GEMM-side table stays out of smem
@@ -837,7 +897,6 @@ int run_fast(qgru_handle *h, int T, int B, int32_t *hq_out, float *hf_out, unsig
             rc = rec_c64_launch(h->rec_c64, mp, a, h->gc_host, h->d_w8[1], h->w8_rows[1], (long long)2 * B + 256, h->h_uns,
                                 ih_bytes, cell_notie, st, &h->err);
         else if (use_cluster) {
-            const size_t BHs = (size_t)B * h->H;
             for (int k = 0; k < n_chunks && rc == QGRU_OK; ++k) {
                 if (n_chunks > 1) {
                     // the next chunk's GEMM goes to the second stream first: its buffer is free once the
@@ -848,12 +907,10 @@ int run_fast(qgru_handle *h, int T, int B, int32_t *hq_out, float *hf_out, unsig
                         CK(cudaEventRecord(h->ev_g[(k + 1) & 1], h->aux));
                     }
                     if (k >= 1) CK(cudaStreamWaitEvent(st, h->ev_g[k & 1], 0));
-                    const size_t slot0 = (size_t)chunk_t0(k) * BHs;   // first output slot of the chunk (both directions)
                     a.T = chunk_T(k);
                     a.ih = chunk_ih(k);
-                    a.hq_out = hq_out ? hq_out + slot0 : nullptr;
-                    a.hf_out = hf_out ? hf_out + slot0 : nullptr;
-                    a.h8_out = h8_out ? h8_out + slot0 : nullptr;
+                    a.out = out.shifted((size_t)chunk_t0(k));   // first output slot of the chunk (both directions)
+                    if (k + 1 < n_chunks) a.out.hn_f = nullptr, a.out.hn_q = nullptr;
                     a.write_final = k + 1 < n_chunks ? 1 : 0;
                 }
                 rc = rec_cluster_launch(h->rec_cl, mp, a, h->gc_host, h->d_w8[1], h->w8_rows[1], (long long)2 * B + 256,
@@ -880,9 +937,7 @@ int run_fast(qgru_handle *h, int T, int B, int32_t *hq_out, float *hf_out, unsig
         a.r8 = h->d_w8[1];
         a.ih = h->ih.p;
         a.h8 = (uint8_t *)h->h8.p;
-        a.hq_out = hq_out;
-        a.hf_out = hf_out;
-        a.h8_out = h8_out;
+        a.out = out;
         a.lc = linear_consts(h, 1);
         a.gc = h->d_gc;
         a.tables = h->d_tables;
@@ -973,6 +1028,77 @@ int check_forward_args(qgru_handle *h, int T, int B) {
     return QGRU_OK;
 }
 
+OutView dense_view(const qgru_handle *h, int B) {
+    OutView o;
+    o.ts = (size_t)B * h->H;
+    o.bs = (size_t)h->H;
+    return o;
+}
+
+// One direction of an integer forward: everything after the argument checks.  with_slot0: the view has T + 1
+// slots and the initial state goes to the first one too (slot T in reverse).  x8_shared: the quantized
+// rows of the same x in another handle's workspace.
+int forward_dir(qgru_handle *h, int T, int B, const FwdInput &in, const OutView &out, bool with_slot0, unsigned flags,
+                cudaStream_t st, const uint8_t *x8_shared = nullptr, cudaEvent_t after_prologue = nullptr) {
+    const long long N = (long long)T * B;
+    const bool rev = (flags & QGRU_FLAG_REVERSE) != 0;
+    const size_t init_slot = rev ? (size_t)T : 0;
+    int rc;
+    h->ev = h->ring[h->calls % qgru_handle::kRing];
+    h->calls++;
+    CK(cudaEventRecord(h->ev[0], st));
+    if (use_generic(h)) {
+        // dense int32 states, step by step; then to the view
+        const size_t nh = (size_t)(T + 1) * B * h->H;
+        const qgru_op &xo = h->p.op[QGRU_OP_X], &ho = h->p.op[QGRU_OP_H];
+        const bool dense = with_slot0 && out.hq && !out.hf && !out.h8;
+        int32_t *hq = out.hq;
+        if (!dense) {
+            if ((rc = ensure(h, h->hq32, nh * 4))) return rc;
+            hq = (int32_t *)h->hq32.p;
+        }
+        const int32_t *x32 = (const int32_t *)in.x;
+        const bool x_dense = in.bs == h->I && in.ts == (long long)B * h->I;
+        if (in.mode != 2 || !x_dense) {
+            int32_t *q = (int32_t *)in.xq;
+            if (!q) {
+                if ((rc = ensure(h, h->x32, (size_t)N * h->I * 4))) return rc;
+                q = (int32_t *)h->x32.p;
+            }
+            k_gather_quantize<<<grid_for(N * h->I, 256, h->sm_count), 256, 0, st>>>(
+                in.x, in.mode == 2 ? 1 : 0, q, N, B, h->I, in.ts, in.bs, h->x_scale, xo.zero_point, op_qmin(xo), op_qmax(xo));
+            h->launches++;
+            x32 = q;
+        }
+        OutView slot;
+        slot.hq = hq + init_slot * B * h->H;
+        slot.bs = h->H;
+        if ((rc = launch_prologue(h, T, B, FwdInput{in.mode, nullptr, 0, 0, in.h0}, nullptr, nullptr, slot, st))) return rc;
+        if (after_prologue) CK(cudaEventRecord(after_prologue, st));
+        if ((rc = run_generic(h, T, B, x32, hq, nullptr, flags, st))) return rc;
+        if (!dense) {
+            const long long slots = with_slot0 ? T + 1 : T, first = with_slot0 ? 0 : (rev ? 0 : 1);
+            const OutView to = with_slot0 || rev ? out : out.shifted(1);
+            k_scatter_states<<<grid_for(slots * B * h->H, 256, h->sm_count), 256, 0, st>>>(
+                hq + (size_t)first * B * h->H, to, slots, rev ? 0 : slots - 1, B, h->H, ho.zero_point, h->h_scale);
+            h->launches++;
+            CK(cudaGetLastError());
+        }
+        return QGRU_OK;
+    }
+    const uint8_t *x8 = x8_shared;
+    if (!x8) {
+        if ((rc = ensure(h, h->x8, (size_t)((N + 127) / 128 * 128) * h->Ipad))) return rc;
+        x8 = (const uint8_t *)h->x8.p;
+    }
+    if ((rc = ensure(h, h->h8, (size_t)(2 * B + 256) * h->Hpad))) return rc;
+    if ((rc = launch_prologue(h, T, B, in, x8_shared ? nullptr : (uint8_t *)h->x8.p, (uint8_t *)h->h8.p,
+                              with_slot0 ? out.shifted(init_slot) : OutView(), st)))
+        return rc;
+    if (after_prologue) CK(cudaEventRecord(after_prologue, st));
+    return run_fast(h, T, B, x8, out, flags, st);
+}
+
 }  // namespace
 
 extern "C" {
@@ -983,32 +1109,9 @@ int qgru_forward_i32(qgru_handle *h, int T, int B, const int32_t *x_q, const int
     int rc = check_forward_args(h, T, B);
     if (rc) return rc;
     CK(cudaSetDevice(h->device));
-    cudaStream_t st = (cudaStream_t)stream;
-    const long long N = (long long)T * B;
-    const qgru_op &xo = h->p.op[QGRU_OP_X], &ho = h->p.op[QGRU_OP_H];
-    const long long init_slot = (flags & QGRU_FLAG_REVERSE) ? T : 0;
-    h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->calls++;
-    CK(cudaEventRecord(h->ev[0], st));
-    CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
-    if (use_generic(h)) {
-        k_init_state<<<grid_for((long long)B * h->Hpad, 256, h->sm_count), 256, 0, st>>>(
-            h0_q, nullptr, nullptr, h_q, nullptr, nullptr, B, h->H, h->Hpad, init_slot, h->h_scale, ho.zero_point,
-            op_qmin(ho), op_qmax(ho), h->d_flags);
-        h->launches++;
-        return run_generic(h, T, B, x_q, h_q, nullptr, flags, st);
-    }
-    if ((rc = ensure(h, h->x8, (size_t)((N + 127) / 128 * 128) * h->Ipad))) return rc;
-    if ((rc = ensure(h, h->h8, (size_t)(2 * B + 256) * h->Hpad))) return rc;
-    k_narrow_rows_i32<<<grid_for(N * (h->Ipad / 4), 256, h->sm_count), 256, 0, st>>>(
-        x_q, (uint8_t *)h->x8.p, N, h->I, h->Ipad, op_qmin(xo), op_qmax(xo), h->d_flags);
-    CK(cudaMemsetAsync(h->h8.p, 0, (size_t)(2 * B + 256) * h->Hpad, st));
-    k_init_state<<<grid_for((long long)B * h->Hpad, 256, h->sm_count), 256, 0, st>>>(
-        h0_q, nullptr, (uint8_t *)h->h8.p, h_q, nullptr, nullptr, B, h->H, h->Hpad, init_slot, h->h_scale,
-        ho.zero_point, op_qmin(ho), op_qmax(ho), h->d_flags);
-    h->launches += 2;
-    CK(cudaGetLastError());
-    return run_fast(h, T, B, h_q, nullptr, flags, st);
+    OutView out = dense_view(h, B);
+    out.hq = h_q;
+    return forward_dir(h, T, B, FwdInput{2, x_q, (long long)B * h->I, h->I, h0_q}, out, true, flags, (cudaStream_t)stream);
 }
 
 int qgru_forward_i32_train(qgru_handle *h, int T, int B, const int32_t *x_q, const int32_t *h0_q,
@@ -1019,17 +1122,15 @@ int qgru_forward_i32_train(qgru_handle *h, int T, int B, const int32_t *x_q, con
     if (rc) return rc;
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
-    const qgru_op &ho = h->p.op[QGRU_OP_H];
     const long long init_slot = (flags & QGRU_FLAG_REVERSE) ? T : 0;
     h->ev = h->ring[h->calls % qgru_handle::kRing];
     h->calls++;
     CK(cudaEventRecord(h->ev[0], st));
-    CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
     // the step-by-step kernels keep every intermediate the training buffer wants
-    k_init_state<<<grid_for((long long)B * h->Hpad, 256, h->sm_count), 256, 0, st>>>(
-        h0_q, nullptr, nullptr, h_q, nullptr, nullptr, B, h->H, h->Hpad, init_slot, h->h_scale, ho.zero_point,
-        op_qmin(ho), op_qmax(ho), h->d_flags);
-    h->launches++;
+    OutView slot;
+    slot.hq = h_q + (size_t)init_slot * B * h->H;
+    slot.bs = h->H;
+    if ((rc = launch_prologue(h, T, B, FwdInput{2, nullptr, 0, 0, h0_q}, nullptr, nullptr, slot, st))) return rc;
     return run_generic(h, T, B, x_q, h_q, v_q, flags, st, masks);
 }
 
@@ -1039,46 +1140,9 @@ int qgru_forward_f32(qgru_handle *h, int T, int B, const float *x, const float *
     int rc = check_forward_args(h, T, B);
     if (rc) return rc;
     CK(cudaSetDevice(h->device));
-    cudaStream_t st = (cudaStream_t)stream;
-    const long long N = (long long)T * B;
-    const qgru_op &xo = h->p.op[QGRU_OP_X], &ho = h->p.op[QGRU_OP_H];
-    const long long init_slot = (flags & QGRU_FLAG_REVERSE) ? T : 0;
-    h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->calls++;
-    CK(cudaEventRecord(h->ev[0], st));
-    CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
-    if (use_generic(h)) {
-        const size_t nh = (size_t)(T + 1) * B * h->H;
-        int32_t *x32 = x_q_out;
-        if (!x32) {
-            if ((rc = ensure(h, h->x32, (size_t)N * h->I * 4))) return rc;
-            x32 = (int32_t *)h->x32.p;
-        }
-        if ((rc = ensure(h, h->hq32, nh * 4))) return rc;
-        k_quantize_f32_i32<<<grid_for(N * h->I, 256, h->sm_count), 256, 0, st>>>(
-            x, x32, N * h->I, h->x_scale, xo.zero_point, op_qmin(xo), op_qmax(xo));
-        k_init_state<<<grid_for((long long)B * h->Hpad, 256, h->sm_count), 256, 0, st>>>(
-            nullptr, h0, nullptr, (int32_t *)h->hq32.p, nullptr, nullptr, B, h->H, h->Hpad, init_slot, h->h_scale,
-            ho.zero_point, op_qmin(ho), op_qmax(ho), h->d_flags);
-        h->launches += 2;
-        if ((rc = run_generic(h, T, B, x32, (int32_t *)h->hq32.p, nullptr, flags, st))) return rc;
-        k_dequantize<<<grid_for((long long)nh, 256, h->sm_count), 256, 0, st>>>(
-            (const int32_t *)h->hq32.p, h_out, (long long)nh, h->h_scale, ho.zero_point);
-        h->launches++;
-        CK(cudaGetLastError());
-        return QGRU_OK;
-    }
-    if ((rc = ensure(h, h->x8, (size_t)((N + 127) / 128 * 128) * h->Ipad))) return rc;
-    if ((rc = ensure(h, h->h8, (size_t)(2 * B + 256) * h->Hpad))) return rc;
-    k_quantize_rows_f32<<<grid_for(N * (h->Ipad / 4), 256, h->sm_count), 256, 0, st>>>(
-        x, (uint8_t *)h->x8.p, x_q_out, N, h->I, h->Ipad, h->x_scale, xo.zero_point, op_qmin(xo), op_qmax(xo));
-    CK(cudaMemsetAsync(h->h8.p, 0, (size_t)(2 * B + 256) * h->Hpad, st));
-    k_init_state<<<grid_for((long long)B * h->Hpad, 256, h->sm_count), 256, 0, st>>>(
-        nullptr, h0, (uint8_t *)h->h8.p, nullptr, h_out, nullptr, B, h->H, h->Hpad, init_slot, h->h_scale,
-        ho.zero_point, op_qmin(ho), op_qmax(ho), h->d_flags);
-    h->launches += 2;
-    CK(cudaGetLastError());
-    return run_fast(h, T, B, nullptr, h_out, flags, st);
+    OutView out = dense_view(h, B);
+    out.hf = h_out;
+    return forward_dir(h, T, B, FwdInput{0, x, (long long)B * h->I, h->I, h0, x_q_out}, out, true, flags, (cudaStream_t)stream);
 }
 
 int qgru_forward_f32_q8(qgru_handle *h, int T, int B, const float *x, const float *h0, uint8_t *h_q8,
@@ -1089,25 +1153,9 @@ int qgru_forward_f32_q8(qgru_handle *h, int T, int B, const float *x, const floa
     if (use_generic(h))
         return fail(h, QGRU_ERR_UNSUPPORTED, "the 8-bit output needs the 8-bit storage plan (x, h, W, R at most 8 bits)");
     CK(cudaSetDevice(h->device));
-    cudaStream_t st = (cudaStream_t)stream;
-    const long long N = (long long)T * B;
-    const qgru_op &xo = h->p.op[QGRU_OP_X], &ho = h->p.op[QGRU_OP_H];
-    const long long init_slot = (flags & QGRU_FLAG_REVERSE) ? T : 0;
-    h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->calls++;
-    CK(cudaEventRecord(h->ev[0], st));
-    CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
-    if ((rc = ensure(h, h->x8, (size_t)((N + 127) / 128 * 128) * h->Ipad))) return rc;
-    if ((rc = ensure(h, h->h8, (size_t)(2 * B + 256) * h->Hpad))) return rc;
-    k_quantize_rows_f32<<<grid_for(N * (h->Ipad / 4), 256, h->sm_count), 256, 0, st>>>(
-        x, (uint8_t *)h->x8.p, nullptr, N, h->I, h->Ipad, h->x_scale, xo.zero_point, op_qmin(xo), op_qmax(xo));
-    CK(cudaMemsetAsync(h->h8.p, 0, (size_t)(2 * B + 256) * h->Hpad, st));
-    k_init_state<<<grid_for((long long)B * h->Hpad, 256, h->sm_count), 256, 0, st>>>(
-        nullptr, h0, (uint8_t *)h->h8.p, nullptr, nullptr, h_q8, B, h->H, h->Hpad, init_slot, h->h_scale,
-        ho.zero_point, op_qmin(ho), op_qmax(ho), h->d_flags);
-    h->launches += 2;
-    CK(cudaGetLastError());
-    return run_fast(h, T, B, nullptr, nullptr, flags, st, h_q8);
+    OutView out = dense_view(h, B);
+    out.h8 = h_q8;
+    return forward_dir(h, T, B, FwdInput{0, x, (long long)B * h->I, h->I, h0}, out, true, flags, (cudaStream_t)stream);
 }
 
 int qgru_synchronize(qgru_handle *h, void *stream) {
@@ -1286,21 +1334,18 @@ extern "C" int qgru_forward_i32_static(qgru_handle *h, int T, int B, const int32
     uint8_t *h8 = ws + off_h8;
     unsigned *bar = reinterpret_cast<unsigned *>(ws + off_bar);
 
-    const qgru_op &xo = h->p.op[QGRU_OP_X], &ho = h->p.op[QGRU_OP_H];
     const long long init_slot = (flags & QGRU_FLAG_REVERSE) ? T : 0;
+    OutView out = dense_view(h, B);
+    out.hq = h_q;
     h->ev = h->ring[h->calls % qgru_handle::kRing];
     h->calls++;
     CK(cudaEventRecord(h->ev[0], st));
-    CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
     // the array keeps what the previous call left: the state buffers' padding columns and the
     // step counters must start at zero
     CK(cudaMemsetAsync(h8, 0, (size_t)2 * B * h->Hpad, st));
     CK(cudaMemsetAsync(bar, 0, (size_t)pl.G * 32 * sizeof(unsigned), st));
-    k_narrow_rows_i32<<<grid_for(N * (h->Ipad / 4), 256, h->sm_count), 256, 0, st>>>(
-        x_q, x8, N, h->I, h->Ipad, op_qmin(xo), op_qmax(xo), h->d_flags);
-    k_init_state<<<grid_for((long long)B * h->Hpad, 256, h->sm_count), 256, 0, st>>>(
-        h0_q, nullptr, h8, h_q, nullptr, nullptr, B, h->H, h->Hpad, init_slot, h->h_scale, ho.zero_point, op_qmin(ho),
-        op_qmax(ho), h->d_flags);
+    if ((rc = launch_prologue(h, T, B, FwdInput{2, x_q, (long long)B * h->I, h->I, h0_q}, x8, h8, out.shifted((size_t)init_slot), st)))
+        return rc;
     CK(cudaEventRecord(h->ev[1], st));
     const LinearConsts lcx = linear_consts(h, 0);
     {
@@ -1322,8 +1367,7 @@ extern "C" int qgru_forward_i32_static(qgru_handle *h, int T, int B, const int32
     a.r8 = h->d_w8[1];
     a.ih = ih;
     a.h8 = h8;
-    a.hq_out = h_q;
-    a.hf_out = nullptr;
+    a.out = out;
     a.lc = linear_consts(h, 1);
     a.gc = h->d_gc;
     a.tables = h->d_tables;
@@ -1334,7 +1378,7 @@ extern "C" int qgru_forward_i32_static(qgru_handle *h, int T, int B, const int32
     if (h->ih_bytes == 1) rc = h->h_uns ? launch_rec<true, int8_t>(h, a, pl, st) : launch_rec<false, int8_t>(h, a, pl, st);
     else rc = h->h_uns ? launch_rec<true, int16_t>(h, a, pl, st) : launch_rec<false, int16_t>(h, a, pl, st);
     if (rc) return rc;
-    h->launches += 3;
+    h->launches += 1;
     CK(cudaEventRecord(h->ev[3], st));
     h->timing_valid = true;
     h->plan_text = "path=int8 gemm=simt_dp4a rec=dp4a workspace=static";
@@ -1342,4 +1386,5 @@ extern "C" int qgru_forward_i32_static(qgru_handle *h, int T, int B, const int32
 }
 
 #include "qgru_fstorage.cuh"
+#include "qgru_layer.cuh"
 #include "qgru_train.cuh"

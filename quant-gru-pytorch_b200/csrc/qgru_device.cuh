@@ -300,6 +300,20 @@ __device__ __forceinline__ float fs_cell(const FsConsts &fc, const float ih[3], 
     return fs_finish(fc, u, r, ih[2], hh[2], h_old);
 }
 
+// One new state to the outputs of OutView.
+__device__ __forceinline__ void put_state(const OutView &o, long long slot, int b, int j, int H, bool last, int32_t hn,
+                                          int32_t zp_h, float h_scale) {
+    const size_t at = (size_t)slot * o.ts + (size_t)b * o.bs + j;
+    const float hf = (float)(hn - zp_h) * h_scale;
+    if (o.hf) o.hf[at] = hf;
+    if (o.hq) o.hq[at] = hn;
+    if (o.h8) o.h8[at] = (uint8_t)hn;
+    if (last) {
+        if (o.hn_f) o.hn_f[(size_t)b * H + j] = hf;
+        if (o.hn_q) o.hn_q[(size_t)b * H + j] = hn;
+    }
+}
+
 // linear_epilogue32 for a scale with the shift-free form.
 template <bool Tie = true>
 __device__ __forceinline__ int32_t linear_epilogue_fast(int32_t acc, const FastLin &f, int32_t zp_out,

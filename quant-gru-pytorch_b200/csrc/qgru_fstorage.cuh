@@ -29,60 +29,6 @@ struct FsChannels {
     const float *inv_gemm_x, *inv_bw, *inv_gemm_h, *inv_br;
 };
 
-// quantize_f (include/quantize_ops_helper.h:514-519): the zero point is added before rounding.
-__device__ __forceinline__ float fs_quantize(float x, float scale, float zp, float lo, float hi) {
-    return fs_clamp(rintf(x / scale + zp), lo, hi);
-}
-
-// fp32 activations -> 8-bit rows padded to Kpad; optionally the quantized values as floats.
-__global__ void k_fs_quantize_rows(const float *__restrict__ x, uint8_t *__restrict__ out8,
-                                   float *__restrict__ xq_out, long long rows, int K, int Kpad,
-                                   float scale, float zp, float lo, float hi,
-                                   uint8_t *__restrict__ keep = nullptr) {
-    const int kw = Kpad >> 2;
-    const long long total = rows * kw;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long row = i / kw;
-        const int k0 = (int)(i - row * kw) * 4;
-        unsigned packed = 0;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int k = k0 + u;
-            int q = 0;
-            if (k < K) {
-                const float raw = rintf(x[row * K + k] / scale + zp);
-                const float qf = fs_clamp(raw, lo, hi);
-                if (xq_out) xq_out[row * K + k] = qf;
-                if (keep) keep[row * K + k] = (raw < lo || raw > hi) ? 0 : 1;
-                q = (int)qf;
-            }
-            packed |= ((unsigned)q & 0xffu) << (8 * u);
-        }
-        reinterpret_cast<unsigned *>(out8)[i] = packed;
-    }
-}
-
-// Initial state: quantize_f(h0) or the zero point (src/gru_interface.cc:949-961), into the
-// 8-bit state rows and, dequantized, into slot `slot` of the output.
-__global__ void k_fs_init_state(const float *__restrict__ h0, uint8_t *__restrict__ h8,
-                                float *__restrict__ h_out, int B, int H, int Hpad, long long slot,
-                                FsConsts fc, uint8_t *__restrict__ keep = nullptr) {
-    const long long total = (long long)B * Hpad;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int b = (int)(i / Hpad), j = (int)(i % Hpad);
-        float q = 0.f;
-        if (j < H) {
-            const float raw = h0 ? rintf(h0[(size_t)b * H + j] / fc.h_scale + fc.zp_h) : fc.zp_h;
-            q = fs_clamp(raw, fc.h_lo, fc.h_hi);
-            h_out[slot * B * H + (long long)b * H + j] = (q - fc.zp_h) * fc.h_scale;
-            if (keep) keep[(size_t)b * H + j] = (raw < fc.h_lo || raw > fc.h_hi) ? 0 : 1;
-        }
-        h8[i] = (uint8_t)(int)q;
-    }
-}
-
 // Per-channel constants of the two linear layers, prepared once per parameter set:
 // chan[0..2] = offset, bias term, GEMM ratio of W*x; chan[3..5] the same for R*h; each [3H].
 __global__ void k_fs_channel_consts(const int32_t *__restrict__ wsum_x, const int32_t *__restrict__ wsum_h,
@@ -112,7 +58,7 @@ __global__ void k_fs_tables(FsConsts fc, float *__restrict__ tab) {
 template <typename IhT>
 __global__ void k_fs_cell(const IhT *__restrict__ ih_q, const int32_t *__restrict__ hh_acc,
                           const float *__restrict__ chan, const uint8_t *__restrict__ h8_in,
-                          uint8_t *__restrict__ h8_out, float *__restrict__ h_out, int B, int H, int Hpad,
+                          uint8_t *__restrict__ h8_out, OutView out, long long slot, int last, int B, int H, int Hpad,
                           FsConsts fc) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int b = blockIdx.y;
@@ -130,7 +76,7 @@ __global__ void k_fs_cell(const IhT *__restrict__ ih_q, const int32_t *__restric
     const float h_old = (float)state_byte(h8_in[(size_t)b * Hpad + j], fc.h_bits);
     const float h_new = fs_cell(fc, ih, hh, h_old);
     h8_out[(size_t)b * Hpad + j] = (uint8_t)(int)h_new;
-    h_out[(size_t)b * H + j] = (h_new - fc.zp_h) * fc.h_scale;
+    put_state(out, slot, b, j, H, last != 0, (int)h_new, (int)fc.zp_h, fc.h_scale);
 }
 
 // ---- training mode (quantGRUForwardFP with is_training): the per-step kernel also keeps the gate
@@ -278,7 +224,6 @@ __global__ void __launch_bounds__(256, 1) k_fs_recurrence(RecArgs a, FsRecArgs f
     const int jl = wj * 32 + lane, j = j0 + jl;
     const bool j_ok = j < a.H;
     constexpr int NB = 4;
-    const size_t BH = (size_t)a.B * a.H;
     unsigned *bar = a.bar + grp * 32;
     const IhT *ihp = reinterpret_cast<const IhT *>(f.ih_q);
     bool dead = false;
@@ -361,7 +306,7 @@ __global__ void __launch_bounds__(256, 1) k_fs_recurrence(RecArgs a, FsRecArgs f
                 const float h_old = HUnsigned ? (float)hb : (float)(int8_t)hb;
                 const float hn = fs_cell(fc, ih, hh, h_old);
                 h_nxt[(size_t)(b0 + b) * a.Hpad + j] = (uint8_t)(int)hn;
-                a.hf_out[(size_t)out_slot * BH + (size_t)(b0 + b) * a.H + j] = (hn - fc.zp_h) * fc.h_scale;
+                put_state(a.out, out_slot, b0 + b, j, a.H, s + 1 == a.T, (int)hn, (int)fc.zp_h, fc.h_scale);
             }
         }
         __syncthreads();
@@ -388,8 +333,7 @@ struct FsTrainArgs {
     qgru_train_masks m;
 };
 
-int fstorage_train_tail(qgru_handle *h, int T, int B, const float *x, const float *h0, float *h_out,
-                        float *xq_out, unsigned flags, cudaStream_t st, const FsConsts &fc, const float *chan,
+int fstorage_train_tail(qgru_handle *h, int T, int B, FwdInput in, float *h_out, unsigned flags, cudaStream_t st, const FsConsts &fc, const float *chan,
                         const FsTrainArgs &tr) {
     const qgru_params &p = h->p;
     const int H = h->H, C = h->C, I = h->I;
@@ -408,20 +352,17 @@ int fstorage_train_tail(qgru_handle *h, int T, int B, const float *x, const floa
     if ((rc = ensure(h, h->h8, (size_t)(2 * B + 256) * h->Hpad))) return rc;
     if ((rc = ensure(h, h->ih32, (size_t)N * C * 4))) return rc;
     if ((rc = ensure(h, h->hh32, (size_t)B * C * 4))) return rc;
-    const qgru_op &ox = p.op[QGRU_OP_X];
     const bool rev = flags & QGRU_FLAG_REVERSE;
-    const long long init_slot = rev ? T : 0;
     uint8_t *h8 = (uint8_t *)h->h8.p;
     const size_t h8_half = (size_t)B * h->Hpad;
     h->ev = h->ring[h->calls % qgru_handle::kRing];
     h->calls++;
     CK(cudaEventRecord(h->ev[0], st));
-    CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
-    k_fs_quantize_rows<<<grid_for(N * (h->Ipad / 4), 256, h->sm_count), 256, 0, st>>>(
-        x, (uint8_t *)h->x8.p, xq_out, N, I, h->Ipad, h->x_scale, fc.zp_x, op_lo(ox), op_hi(ox), tr.m.x);
-    CK(cudaMemsetAsync(h8, 0, (size_t)(2 * B + 256) * h->Hpad, st));
-    k_fs_init_state<<<grid_for((long long)B * h->Hpad, 256, h->sm_count), 256, 0, st>>>(
-        h0, h8, h_out, B, H, h->Hpad, init_slot, fc, tr.m.h0);
+    in.x_keep = tr.m.x;
+    in.h0_keep = tr.m.h0;
+    OutView out = dense_view(h, B);
+    out.hf = h_out;
+    if ((rc = launch_prologue(h, T, B, in, (uint8_t *)h->x8.p, h8, out.shifted(rev ? (size_t)T : 0), st))) return rc;
     // weight masks: W [I][3H], R [H][3H], bw, br [3H] against their per-channel scales
     const float *wsrc[4] = {tr.W, tr.R, tr.bw, tr.br};
     uint8_t *wmask[4] = {tr.m.W, tr.m.R, tr.m.bw, tr.m.br};
@@ -465,7 +406,7 @@ int fstorage_train_tail(qgru_handle *h, int T, int B, const float *x, const floa
             tr.m.gate_output ? tr.m.gate_output + (size_t)t * BC : nullptr, tr.m.h ? tr.m.h + (size_t)t * BH : nullptr,
             B, H, h->Hpad, fc, tc);
     }
-    h->launches += 4 + 2ull * T;
+    h->launches += 3 + 2ull * T;
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->ev[3], st));
     h->timing_valid = true;
@@ -473,9 +414,11 @@ int fstorage_train_tail(qgru_handle *h, int T, int B, const float *x, const floa
     return QGRU_OK;
 }
 
-// Host side of quantGRUForwardFP, inference mode.  x, h0, h_out, xq_out are device pointers.
-int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *h0, float *h_out,
-                     float *xq_out, unsigned flags, cudaStream_t st, const FsTrainArgs *train = nullptr) {
+// Host side of quantGRUForwardFP; `in`, `out`, with_slot0, x8_shared, after_prologue as in forward_dir.  Training
+// mode (`train`) writes the dense slots at out.hf.
+int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const OutView &out, bool with_slot0, unsigned flags,
+                     cudaStream_t st, const uint8_t *x8_shared = nullptr, cudaEvent_t after_prologue = nullptr,
+                     const FsTrainArgs *train = nullptr) {
     if (!h->fast)
         return fail(h, QGRU_ERR_UNSUPPORTED,
                     "float-storage forward needs 8-bit W, R, x and h (the operands of the two products)");
@@ -557,9 +500,10 @@ int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *
         h->launches += 2;
         h->fs_ready = true;
     }
-    if (train) return fstorage_train_tail(h, T, B, x, h0, h_out, xq_out, flags, st, fc, chan, *train);
+    if (train) return fstorage_train_tail(h, T, B, in, out.hf, flags, st, fc, chan, *train);
 
-    if ((rc = ensure(h, h->x8, (size_t)((N + 127) / 128 * 128) * h->Ipad))) return rc;
+    if (!x8_shared && (rc = ensure(h, h->x8, (size_t)((N + 127) / 128 * 128) * h->Ipad))) return rc;
+    const uint8_t *x8 = x8_shared ? x8_shared : (const uint8_t *)h->x8.p;
     if ((rc = ensure(h, h->h8, (size_t)(2 * B + 256) * h->Hpad))) return rc;
     // W*x + bw requantized and clamped to the width of weight_ih_linear: one or two bytes
     const int ih_bytes = (oih.bits <= 8 && !oih.is_unsigned) ? 1 : 2;
@@ -567,7 +511,6 @@ int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *
         return fail(h, QGRU_ERR_UNSUPPORTED, "float-storage forward stores W*x + bw in at most 16 signed bits");
     if ((rc = ensure(h, h->ih, (size_t)N * C * ih_bytes))) return rc;
     const bool rev = flags & QGRU_FLAG_REVERSE;
-    const long long init_slot = rev ? T : 0;
     uint8_t *h8 = (uint8_t *)h->h8.p;
     const size_t h8_half = (size_t)B * h->Hpad;
     const int sms = h->opt_sm_limit > 0 ? std::min(h->opt_sm_limit, h->sm_count) : h->sm_count;
@@ -575,12 +518,10 @@ int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *
     h->ev = h->ring[h->calls % qgru_handle::kRing];
     h->calls++;
     CK(cudaEventRecord(h->ev[0], st));
-    CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
-    k_fs_quantize_rows<<<grid_for(N * (h->Ipad / 4), 256, h->sm_count), 256, 0, st>>>(
-        x, (uint8_t *)h->x8.p, xq_out, N, h->I, h->Ipad, h->x_scale, fc.zp_x, op_lo(ox), op_hi(ox));
-    CK(cudaMemsetAsync(h8, 0, (size_t)(2 * B + 256) * h->Hpad, st));
-    k_fs_init_state<<<grid_for((long long)B * h->Hpad, 256, h->sm_count), 256, 0, st>>>(
-        h0, h8, h_out, B, H, h->Hpad, init_slot, fc);
+    if ((rc = launch_prologue(h, T, B, in, x8_shared ? nullptr : (uint8_t *)h->x8.p, h8,
+                              with_slot0 ? out.shifted(rev ? (size_t)T : 0) : OutView(), st)))
+        return rc;
+    if (after_prologue) CK(cudaEventRecord(after_prologue, st));
     CK(cudaEventRecord(h->ev[1], st));
     // the input projection: exact int32 sums on the tensor cores (dp4a form as fallback), float
     // requantization in the epilogue
@@ -590,7 +531,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *
     bool used_tc = false;
     if (h->opt_gemm != 1) {
         PreScale ps{};
-        rc = tc_gemm_launch(h->tc, (const uint8_t *)h->x8.p, (N + 127) / 128 * 128, h->d_w8[0], h->w8_rows[0],
+        rc = tc_gemm_launch(h->tc, x8, (N + 127) / 128 * 128, h->d_w8[0], h->w8_rows[0],
                             h->ih.p, N, C, h->Ipad, h->x_uns, ih_bytes, lcx, ps, false, false, h->d_flags + 1, sms, st,
                             &h->err);
         if (rc == QGRU_OK) used_tc = true;
@@ -598,7 +539,6 @@ int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *
     }
     if (!used_tc) {
         dim3 grid((unsigned)((N + 63) / 64), (unsigned)((C + 63) / 64));
-        const uint8_t *x8 = (const uint8_t *)h->x8.p;
         if (ih_bytes == 1) {
             if (h->x_uns) k_gemm_wx_simt<true, int8_t><<<grid, 256, 0, st>>>(x8, h->d_w8[0], (int8_t *)h->ih.p, N, C, h->Ipad, lcx);
             else k_gemm_wx_simt<false, int8_t><<<grid, 256, 0, st>>>(x8, h->d_w8[0], (int8_t *)h->ih.p, N, C, h->Ipad, lcx);
@@ -609,7 +549,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *
         CK(cudaGetLastError());
     }
     CK(cudaEventRecord(h->ev[2], st));
-    h->launches += 3;
+    h->launches += 1;
     char buf[256];
     RecPlan pl;
     RecMmaPlan cp;
@@ -621,11 +561,6 @@ int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *
     const bool cluster_ok = !small && h->opt_rec != 1 && h->opt_rec != 3 && h->opt_exchange != 1 &&
                             rec_cluster_plan(H, h->Hpad, B, sms, h->smem_optin, n_tab, h->opt_r_where, h->opt_mt, h->opt_ng, h->opt_kp, &cp);
     if (cluster_ok) {
-        if (cp.G > h->bar_groups) {
-            if ((rc = alloc_dev(h, &h->d_bar, (size_t)cp.G * 32))) return rc;
-            h->bar_groups = cp.G;
-        }
-        CK(cudaMemsetAsync(h->d_bar, 0, (size_t)cp.G * 32 * sizeof(unsigned), st));
         RecMmaArgs a;
         a.T = T; a.B = B; a.H = H; a.Hpad = h->Hpad; a.C = C;
         a.P = cp.P; a.NB = cp.NB; a.b_off = 0; a.b_cnt = B;
@@ -633,8 +568,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *
         a.tmem_cols = (uint32_t)cp.tmem_cols;
         a.ih = h->ih.p;
         a.h8 = h8;
-        a.hq_out = nullptr;
-        a.hf_out = h_out;
+        a.out = out;
         a.lc = linear_consts(h, 1);
         a.tables = (const int32_t *)gate_tab;   // float bit patterns
         a.n_table = n_tab;
@@ -661,7 +595,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *
         a.r8 = h->d_w8[1];
         a.ih = h->ih.p;
         a.h8 = h8;
-        a.hf_out = h_out;
+        a.out = out;
         a.lc = linear_consts(h, 1);
         a.gc = h->d_gc;
         a.tables = (const int32_t *)gate_tab;   // float bit patterns
@@ -709,7 +643,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *
         a.reverse = rev ? 1 : 0;
         a.r8 = h->d_w8[1];
         a.h8 = h8;
-        a.hf_out = h_out;
+        a.out = out;
         a.bar = h->d_bar;
         a.abort_flag = h->d_flags + 1;
         a.spin_limit = h->spin_limit;
@@ -736,7 +670,6 @@ int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *
     } else {
         // two launches per step, as the reference
         if ((rc = ensure(h, h->hh32, (size_t)B * C * 4))) return rc;
-        const size_t BH = (size_t)B * H;
         for (int s = 0; s < T; ++s) {
             const int t = rev ? T - 1 - s : s;
             const size_t out_slot = rev ? (size_t)(T - 1 - s) : (size_t)(s + 1);
@@ -752,10 +685,10 @@ int fstorage_forward(qgru_handle *h, int T, int B, const float *x, const float *
             dim3 g2((H + 127) / 128, B);
             if (ih_bytes == 1)
                 k_fs_cell<int8_t><<<g2, 128, 0, st>>>((const int8_t *)h->ih.p + (size_t)t * B * C, (const int32_t *)h->hh32.p,
-                                                      chan, hin, hout, h_out + out_slot * BH, B, H, h->Hpad, fc);
+                                                      chan, hin, hout, out, (long long)out_slot, s + 1 == T ? 1 : 0, B, H, h->Hpad, fc);
             else
                 k_fs_cell<int16_t><<<g2, 128, 0, st>>>((const int16_t *)h->ih.p + (size_t)t * B * C, (const int32_t *)h->hh32.p,
-                                                       chan, hin, hout, h_out + out_slot * BH, B, H, h->Hpad, fc);
+                                                       chan, hin, hout, out, (long long)out_slot, s + 1 == T ? 1 : 0, B, H, h->Hpad, fc);
             h->launches += 2;
         }
         snprintf(buf, sizeof(buf), "path=float_storage gemm=%s rec=per_step_float_cell ih_bytes=%d",
@@ -779,7 +712,9 @@ int qgru_forward_fstorage(qgru_handle *h, int T, int B, const float *x, const fl
     if (!h->params_set || !h->weights_set)
         return fail(h, QGRU_ERR_NOT_READY, "set_params and set_weights first");
     CK(cudaSetDevice(h->device));
-    return qgru::fstorage_forward(h, T, B, x, h0, h_out, x_q_out, flags, (cudaStream_t)stream);
+    OutView out = dense_view(h, B);
+    out.hf = h_out;
+    return qgru::fstorage_forward(h, T, B, FwdInput{1, x, (long long)B * h->I, h->I, h0, x_q_out}, out, true, flags, (cudaStream_t)stream);
 }
 
 // out[i] = q[i] * scale[i % C]  (dequantizeGRUWeights: weights have zero point 0)
@@ -835,7 +770,10 @@ int qgru_forward_fstorage_train(qgru_handle *h, int T, int B, const float *W, co
         return fail(h, QGRU_ERR_NOT_READY, "set_params and set_weights first");
     CK(cudaSetDevice(h->device));
     qgru::FsTrainArgs tr{W, R, bw, br, v_out, masks ? *masks : qgru_train_masks{}};
-    return qgru::fstorage_forward(h, T, B, x, h0, h_out, x_q_out, flags, (cudaStream_t)stream, &tr);
+    OutView out = dense_view(h, B);
+    out.hf = h_out;
+    return qgru::fstorage_forward(h, T, B, FwdInput{1, x, (long long)B * h->I, h->I, h0, x_q_out}, out, true, flags, (cudaStream_t)stream,
+                                  nullptr, nullptr, &tr);
 }
 
 }  // extern "C"

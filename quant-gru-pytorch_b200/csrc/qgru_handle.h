@@ -77,7 +77,9 @@ struct qgru_handle {
     bool lin_notie[2] = {false, false};       // no channel of that layer's requantization can meet an exact tie
     bool rs_fast[2] = {false, false};   // every per-channel GEMM rescale has the shift-free form
     int *d_flags = nullptr;                   // [0] data errors, [1] barrier abort
-    int *h_flags = nullptr;                   // pinned mirror
+    int *h_flags = nullptr;                   // pinned mirror; [2]: status of an earlier asynchronous forward (written by the GPU)
+    cudaStream_t side = nullptr;              // layer forward: the reverse direction's stream
+    cudaEvent_t ev_split = nullptr, ev_join = nullptr;
     unsigned *d_bar = nullptr;
     int bar_groups = 0;
     // workspace

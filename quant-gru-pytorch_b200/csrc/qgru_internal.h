@@ -111,4 +111,23 @@ struct LinearConsts {
     int32_t fs_C = 0;
 };
 
+// Where a recurrence writes its states: element (slot, row b, unit j) at slot * ts + b * bs + j of whichever
+// outputs are set (slot s + 1 of step s, T - 1 - s in reverse), and the state after the last step, rows
+// dense, at hn_*.
+struct OutView {
+    float *hf = nullptr;       // dequantized
+    int32_t *hq = nullptr;     // int32 containers
+    uint8_t *h8 = nullptr;     // 8-bit containers
+    size_t ts = 0, bs = 0;
+    float *hn_f = nullptr;     // [B][H]
+    int32_t *hn_q = nullptr;   // [B][H]
+    OutView shifted(size_t slots) const {
+        OutView o = *this;
+        if (hf) o.hf += slots * ts;
+        if (hq) o.hq += slots * ts;
+        if (h8) o.h8 += slots * ts;
+        return o;
+    }
+};
+
 }  // namespace qgru

@@ -22,55 +22,114 @@ __device__ __forceinline__ int32_t quantize_one(float x, float scale, int32_t zp
     return clampi((int32_t)q, lo, hi);
 }
 
-// fp32 activations -> 8-bit rows padded to Kpad (zeros), optionally also int32 containers.
-// One thread per group of 4 padded columns.
-__global__ void k_quantize_rows_f32(const float *__restrict__ x, uint8_t *__restrict__ out8,
-                                    int32_t *__restrict__ out32, long long rows, int K, int Kpad,
-                                    float scale, int32_t zp, int32_t lo, int32_t hi) {
-    const int kw = Kpad >> 2;
-    const long long total = rows * kw;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long row = i / kw;
-        const int k0 = (int)(i - row * kw) * 4;
-        unsigned packed = 0;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int k = k0 + u;
-            int32_t q = 0;
-            if (k < K) {
-                q = quantize_one(x[row * K + k], scale, zp, lo, hi);
-                if (out32) out32[row * K + k] = q;
-            }
-            packed |= ((unsigned)q & 0xffu) << (8 * u);
-        }
-        if (out8) reinterpret_cast<unsigned *>(out8)[i] = packed;
+// quantize_f of the float-storage path (include/quantize_ops_helper.h:514-519): the zero point is added before
+// rounding, and the value stays a float.
+__device__ __forceinline__ float fs_quantize_raw(float x, float scale, int32_t zp) { return rintf(x / scale + (float)zp); }
+
+// What every forward does before its first product, in ONE launch: activations to 8-bit rows padded to
+// Kpad (zeros), the initial state to its 8-bit rows and, for the slot layouts, to the outputs' first slot.
+// The status words of the call before are folded into `sticky` (host memory) and cleared.
+// Mode 0: fp32 in, integer quantize; 1: fp32 in, float-storage quantize; 2: int32 containers (values
+// outside the operator's range, which the reference's quantize step would have clamped, raise bit 0
+// of flags[0]; the caller clears the flags).
+struct PrologueArgs {
+    const void *x;               // row n = t * B + b at x + t * x_ts + b * x_bs; null: only the state
+    long long x_ts, x_bs, N;
+    int B, K, Kpad;
+    uint8_t *x8;
+    void *xq;                    // optional dense copy of the quantized values: int32 (mode 0) or float (mode 1)
+    uint8_t *keep;               // optional mask, 1 = the value was not clamped (mode 1)
+    float x_scale;
+    int32_t x_zp, x_lo, x_hi;
+    const void *h0;              // [B][H] fp32 (modes 0, 1) or int32 (mode 2); null: the zero point
+    uint8_t *h8;                 // [B][Hpad]
+    int H, Hpad;
+    OutView slot;                // outputs of the initial slot (slot 0), each may be null
+    float h_scale;
+    int32_t h_zp, h_lo, h_hi;
+    uint8_t *h0_keep;            // optional mask of the initial state (mode 1)
+    int *flags;                  // [2]
+    volatile int *sticky;        // mapped host word or null: do not clear the flags
+    int q_blocks;                // blocks that quantize x; the rest write the state
+};
+
+template <int Mode>
+__device__ __forceinline__ int32_t prologue_quantize(const void *src, long long i, float scale, int32_t zp, int32_t lo, int32_t hi,
+                                                     uint8_t &keep, int *flags) {
+    keep = 1;
+    if constexpr (Mode == 0) {
+        return quantize_one(static_cast<const float *>(src)[i], scale, zp, lo, hi);
+    } else if constexpr (Mode == 1) {
+        const float raw = fs_quantize_raw(static_cast<const float *>(src)[i], scale, zp);
+        keep = (raw < (float)lo || raw > (float)hi) ? 0 : 1;
+        return (int32_t)fmaxf((float)lo, fminf(raw, (float)hi));
+    } else {
+        const int32_t q = static_cast<const int32_t *>(src)[i];
+        if (q < lo || q > hi) atomicOr(flags, 1);
+        return q;
     }
 }
 
-// int32 containers -> 8-bit rows padded to Kpad.  Values outside [lo, hi] (they would have
-// been clamped by the reference's quantize step) raise bit 0 of *err.
-__global__ void k_narrow_rows_i32(const int32_t *__restrict__ x, uint8_t *__restrict__ out8,
-                                  long long rows, int K, int Kpad, int32_t lo, int32_t hi,
-                                  int *err) {
-    const int kw = Kpad >> 2;
-    const long long total = rows * kw;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long row = i / kw;
-        const int k0 = (int)(i - row * kw) * 4;
-        unsigned packed = 0;
+// A thread takes 16 consecutive columns of a row: four 128-bit loads where Vec (rows and base aligned, K a
+// multiple of 4), one 128-bit store.  Memory-bound: 51200 x 256 fp32 (cfg2) 18 us, 37 us with scalar loads.
+template <int Mode, bool Vec>
+__global__ void __launch_bounds__(256) k_prologue(const PrologueArgs a) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && a.sticky) {
+        if (a.flags[1]) *a.sticky = a.flags[1];
+        a.flags[0] = 0;
+        a.flags[1] = 0;
+    }
+    if ((int)blockIdx.x < a.q_blocks) {
+        const int kw = a.Kpad >> 4;
+        const long long total = a.N * kw;
+        for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += a.q_blocks * 256ll) {
+            const long long row = i / kw;
+            const int k0 = (int)(i - row * kw) * 16;
+            const long long t = row / a.B, src = t * a.x_ts + (row - t * a.B) * a.x_bs;
+            unsigned w[4] = {0u, 0u, 0u, 0u};
+            float4 in[4];
+            if constexpr (Vec) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int k = k0 + u;
-            int32_t q = 0;
-            if (k < K) {
-                q = x[row * K + k];
-                if (q < lo || q > hi) atomicOr(err, 1);
+                for (int g = 0; g < 4; ++g)
+                    if (k0 + 4 * g < a.K) in[g] = *reinterpret_cast<const float4 *>(static_cast<const float *>(a.x) + src + k0 + 4 * g);
             }
-            packed |= ((unsigned)q & 0xffu) << (8 * u);
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                if (k0 + 4 * g >= a.K) continue;
+                const float f[4] = {in[g].x, in[g].y, in[g].z, in[g].w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int k = k0 + 4 * g + u;
+                    if (k >= a.K) continue;
+                    uint8_t keep;
+                    const int32_t q = Vec ? prologue_quantize<Mode>(f, u, a.x_scale, a.x_zp, a.x_lo, a.x_hi, keep, a.flags)
+                                          : prologue_quantize<Mode>(a.x, src + k, a.x_scale, a.x_zp, a.x_lo, a.x_hi, keep, a.flags);
+                    w[g] |= ((unsigned)q & 0xffu) << (8 * u);
+                    if (a.xq) {
+                        if constexpr (Mode == 1) static_cast<float *>(a.xq)[row * a.K + k] = (float)q;
+                        else static_cast<int32_t *>(a.xq)[row * a.K + k] = q;
+                    }
+                    if (Mode == 1 && a.keep) a.keep[row * a.K + k] = keep;
+                }
+            }
+            reinterpret_cast<uint4 *>(a.x8)[i] = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        reinterpret_cast<unsigned *>(out8)[i] = packed;
+        return;
+    }
+    // initial state: quantGRUForwardInt32's h_q[0] fill (src/gru_interface.cc:568-574; the float entry point
+    // dequantizes that slot like every other, :704); float storage: src/gru_interface.cc:949-961
+    const long long total = (long long)a.B * a.Hpad;
+    for (long long i = (blockIdx.x - a.q_blocks) * 256ll + threadIdx.x; i < total; i += (long long)(gridDim.x - a.q_blocks) * 256) {
+        const int b = (int)(i / a.Hpad), j = (int)(i % a.Hpad);
+        int32_t q = 0;
+        if (j < a.H) {
+            uint8_t keep = 1;
+            q = a.h0 ? prologue_quantize<Mode>(a.h0, (long long)b * a.H + j, a.h_scale, a.h_zp, a.h_lo, a.h_hi, keep, a.flags)
+                     : (Mode == 1 ? (int32_t)fmaxf((float)a.h_lo, fminf((float)a.h_zp, (float)a.h_hi)) : a.h_zp);
+            put_state(a.slot, 0, b, j, a.H, false, q, a.h_zp, a.h_scale);
+            if (a.h0_keep) a.h0_keep[(size_t)b * a.H + j] = keep;
+        }
+        if (a.h8) a.h8[i] = (uint8_t)q;
     }
 }
 
@@ -80,6 +139,15 @@ __global__ void k_quantize_f32_i32(const float *__restrict__ x, int32_t *__restr
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x)
         out[i] = quantize_one(x[i], scale, zp, lo, hi);
+}
+
+// The same for rows at x + t * ts + b * bs, fp32 or (is_int) already int32.
+__global__ void k_gather_quantize(const void *__restrict__ x, int is_int, int32_t *__restrict__ out, long long N, int B, int K,
+                                  long long ts, long long bs, float scale, int32_t zp, int32_t lo, int32_t hi) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N * K; i += (long long)gridDim.x * blockDim.x) {
+        const long long row = i / K, t = row / B, at = t * ts + (row - t * B) * bs + (i - row * K);
+        out[i] = is_int ? static_cast<const int32_t *>(x)[at] : quantize_one(static_cast<const float *>(x)[at], scale, zp, lo, hi);
+    }
 }
 
 // Per-channel weight quantize, zp = 0 (quantificationPerChannelBitwidth,
@@ -205,36 +273,15 @@ k_gemm_wx_simt(const uint8_t *__restrict__ x8, const int8_t *__restrict__ w8, Ih
     }
 }
 
-// ------------------------------------------------------------ h slot 0 / state init
-
-// Writes the initial state: the 8-bit state buffer (padded rows), and slot `slot` of the
-// int32 / float outputs (quantGRUForwardInt32's h_q[0] fill, src/gru_interface.cc:568-574;
-// the float entry point dequantizes that slot like every other, :704).
-__global__ void k_init_state(const int32_t *__restrict__ h0_q, const float *__restrict__ h0_f,
-                             uint8_t *__restrict__ h8, int32_t *__restrict__ hq_out,
-                             float *__restrict__ hf_out, uint8_t *__restrict__ h8_out, int B, int H, int Hpad,
-                             long long slot,
-                             float scale, int32_t zp, int32_t lo, int32_t hi, int *err) {
-    const long long total = (long long)B * Hpad;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int b = (int)(i / Hpad), j = (int)(i % Hpad);
-        int32_t q = 0;
-        if (j < H) {
-            if (h0_q) {
-                q = h0_q[(size_t)b * H + j];
-                if (q < lo || q > hi) atomicOr(err, 1);
-            } else if (h0_f) {
-                q = quantize_one(h0_f[(size_t)b * H + j], scale, zp, lo, hi);
-            } else {
-                q = zp;
-            }
-            const long long o = slot * B * H + (long long)b * H + j;
-            if (hq_out) hq_out[o] = q;
-            if (hf_out) hf_out[o] = (float)(q - zp) * scale;
-            if (h8_out) h8_out[o] = (uint8_t)q;
-        }
-        if (h8) h8[i] = (uint8_t)q;
+// Dense states of the step-by-step paths [(T+1)][B][H] to the view a caller asked for (slots 0 .. slots - 1 of
+// `src` to slots 0 .. of the view), and the last state.
+__global__ void k_scatter_states(const int32_t *__restrict__ src, OutView o, long long slots, long long hn_slot, int B, int H,
+                                 int32_t zp_h, float h_scale) {
+    const long long BH = (long long)B * H, total = slots * BH;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const long long slot = i / BH;
+        const int r = (int)(i - slot * BH), b = r / H, j = r - b * H;
+        put_state(o, slot, b, j, H, slot == hn_slot, src[i], zp_h, h_scale);
     }
 }
 
@@ -249,9 +296,7 @@ struct RecArgs {
     const int8_t *r8;      // [3H][Hpad]
     const void *ih;        // [T*B][3H] int8 or int16
     uint8_t *h8;           // [2][B][Hpad] ping-pong state
-    int32_t *hq_out;       // [(T+1)][B][H] or null
-    float *hf_out;         // [(T+1)][B][H] or null
-    uint8_t *h8_out = nullptr;   // [(T+1)][B][H] or null: the quantized state in its 8-bit container
+    OutView out;
     LinearConsts lc;       // R*h + br epilogue
     const GateConsts *gc;  // device copy
     const int32_t *tables; // activation tables, gc->table_off indexes into it
@@ -318,7 +363,6 @@ __global__ void __launch_bounds__(256, 1) k_recurrence_dp4a(RecArgs a) {
     const int jl = wj * 32 + lane, j = j0 + jl;
     const bool j_ok = j < a.H;
     constexpr int NB = 4;
-    const size_t BH = (size_t)a.B * a.H;
     const IhT *ihp = reinterpret_cast<const IhT *>(a.ih);
     unsigned *bar = a.bar + grp * 32;
     bool dead = false;
@@ -404,10 +448,7 @@ __global__ void __launch_bounds__(256, 1) k_recurrence_dp4a(RecArgs a) {
                 const int32_t hn = gru_cell<Narrow>(*gc, tables, ihv[u][0], ihv[u][1], ihv[u][2],
                                                     hh[0], hh[1], hh[2], h_old);
                 h_nxt[(size_t)(b0 + b) * a.Hpad + j] = (uint8_t)hn;
-                const size_t o = (size_t)out_slot * BH + (size_t)(b0 + b) * a.H + j;
-                if (a.hq_out) a.hq_out[o] = hn;
-                if (a.hf_out) a.hf_out[o] = (float)(hn - gc->zp_h) * gc->h_scale;
-                if (a.h8_out) a.h8_out[o] = (uint8_t)hn;
+                put_state(a.out, out_slot, b0 + b, j, a.H, s + 1 == a.T, hn, gc->zp_h, gc->h_scale);
             }
         }
         __syncthreads();
@@ -488,7 +529,6 @@ __global__ void __launch_bounds__(1024, 1) k_recurrence_gemv(const __grid_consta
     }
     __syncthreads();
 
-    const size_t BH = (size_t)a.B * a.H;
     const IhT *ihp = reinterpret_cast<const IhT *>(a.ih);
     const uint32_t tab = (uint32_t)__cvta_generic_to_shared(tables);
     const bool worker = qd == 0 && j_ok;
@@ -556,10 +596,7 @@ __global__ void __launch_bounds__(1024, 1) k_recurrence_gemv(const __grid_consta
                 hn = gru_cell<Cell == 1>(gc, tables, ihv[0], ihv[1], ihv[2], hh[0], hh[1], hh[2], h_old);
             }
             h_nxt[j_at] = (unsigned char)hn;
-            const size_t o = (size_t)out_slot * BH + (size_t)b * a.H + j;
-            if (a.hq_out) a.hq_out[o] = hn;
-            if (a.hf_out) a.hf_out[o] = (float)(hn - gc.zp_h) * gc.h_scale;
-            if (a.h8_out) a.h8_out[o] = (uint8_t)hn;
+            put_state(a.out, out_slot, b, j, a.H, s + 1 == a.T, hn, gc.zp_h, gc.h_scale);
         }
         ihv[0] = ihn[0];
         ihv[1] = ihn[1];
@@ -631,7 +668,6 @@ __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_con
         }
     __syncthreads();
 
-    const size_t BH = (size_t)a.B * a.H;
     const IhT *ihp = reinterpret_cast<const IhT *>(a.ih);
     const uint32_t tab = (uint32_t)__cvta_generic_to_shared(tables);
     const bool worker = half == 0 && j_ok;
@@ -694,10 +730,7 @@ __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_con
                 hn = (int32_t)fs_finish_tab(a.fs, tab, u_g, r_g, fih[2], fhh[2], (float)h_old);
             }
             h_nxt[j_at] = (unsigned char)hn;
-            const size_t o = (size_t)out_slot * BH + (size_t)b * a.H + j;
-            if (a.hq_out) a.hq_out[o] = hn;
-            if (a.hf_out) a.hf_out[o] = (float)(hn - gc.zp_h) * gc.h_scale;
-            if (a.h8_out) a.h8_out[o] = (uint8_t)hn;
+            put_state(a.out, out_slot, b, j, a.H, s + 1 == a.T, hn, gc.zp_h, gc.h_scale);
         }
         ihv[0] = ihn[0];
         ihv[1] = ihn[1];

@@ -202,7 +202,6 @@ k_recurrence_c64(const __grid_constant__ CUtensorMap map_r, const __grid_constan
         const int ul = 16 * q + (lane & 15);         // unit within the CTA's 64, shared with lane ^ 16
         const int j = j0 + ul;
         const bool j_ok = j < a.H;
-        const size_t BH = (size_t)a.B * a.H;
         const IhT *ihp = reinterpret_cast<const IhT *>(a.ih);
         const int nchunks = a.NB / 4;
         const uint32_t tab = tc::smem_u32(tables);
@@ -370,10 +369,7 @@ k_recurrence_c64(const __grid_constant__ CUtensorMap map_r, const __grid_constan
 #pragma unroll
                         for (int k = 0; k < 2; ++k)
                             if (f0 + k < nb && j_ok) {
-                                const size_t o = (size_t)out_slot * BH + (size_t)(bg0 + f0 + k) * a.H + j;
-                                if (a.hq_out) a.hq_out[o] = hn[k];
-                                if (a.hf_out) a.hf_out[o] = (float)(hn[k] - gc.zp_h) * gc.h_scale;
-                                if (a.h8_out) a.h8_out[o] = (uint8_t)hn[k];
+                                put_state(a.out, out_slot, bg0 + f0 + k, j, a.H, s + 1 == a.T, hn[k], gc.zp_h, gc.h_scale);
                             }
                     } else {
                         hn_last[0] = hn[0];
@@ -399,10 +395,7 @@ k_recurrence_c64(const __grid_constant__ CUtensorMap map_r, const __grid_constan
 #pragma unroll
                     for (int k = 0; k < 2; ++k)
                         if (f_last + k < nb && j_ok) {
-                            const size_t o = (size_t)out_slot * BH + (size_t)(bg0 + f_last + k) * a.H + j;
-                            if (a.hq_out) a.hq_out[o] = hn_last[k];
-                            if (a.hf_out) a.hf_out[o] = (float)(hn_last[k] - gc.zp_h) * gc.h_scale;
-                            if (a.h8_out) a.h8_out[o] = (uint8_t)hn_last[k];
+                            put_state(a.out, out_slot, bg0 + f_last + k, j, a.H, s + 1 == a.T, hn_last[k], gc.zp_h, gc.h_scale);
                         }
                 }
                 STAMP((warp % 15) == 1 && lane == 0, 12 + 8 * (warp / 15));

@@ -312,7 +312,6 @@ k_recurrence_cluster(const __grid_constant__ CUtensorMap map_r, const __grid_con
         const int q = warp & 3;                      // TMEM lane quadrant this warp may read
         const int rank = (warp - 1) >> 2;            // 0..EPW-1 among the warps of that quadrant
         const int u = q * 32 + lane;                 // unit within a 128-unit tile = TMEM lane
-        const size_t BH = (size_t)a.B * a.H;
         const IhT *ihp = reinterpret_cast<const IhT *>(a.ih);
         const int nchunks = a.NB / CH;
         const uint32_t tab = tc::smem_u32(tables);          // fused-cell tables, shared-window address
@@ -399,30 +398,39 @@ k_recurrence_cluster(const __grid_constant__ CUtensorMap map_r, const __grid_con
 #pragma unroll
             for (int i = 0; i < CH; ++i) h_keep[mt][i] = 0;
         // the CH cells of a chunk to whichever outputs the caller asked for: the choice is made once
-        // per chunk, not per cell; `base` is the element offset of (time slot, first row of the sub-group)
-        auto store_outputs = [&](const int32_t(&v)[MT][CH], int c0, int nb, size_t base) {
+        // per chunk, not per cell; `base` is the element offset of (time slot, first row of the sub-group);
+        // `last`: the sequence's last step, `hn_base` its first row in the dense last state
+        const uint32_t obs = (uint32_t)a.out.bs;
+        auto store_outputs = [&](const int32_t(&v)[MT][CH], int c0, int nb, size_t base, bool last, size_t hn_base) {
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) {
                 if (!j_ok[mt]) continue;
-                const uint32_t oj = (uint32_t)(c0 * a.H + j0 + mt * 128 + u);
-                if (a.hf_out) {
-                    float *o = a.hf_out + base;
+                const uint32_t oj = (uint32_t)c0 * obs + (uint32_t)(j0 + mt * 128 + u);
+                if (a.out.hf) {
+                    float *o = a.out.hf + base;
 #pragma unroll
                     for (int i = 0; i < CH; ++i)
-                        if (c0 + i < nb) o[oj + (uint32_t)(i * a.H)] = (float)(v[mt][i] - gc.zp_h) * gc.h_scale;
+                        if (c0 + i < nb) o[oj + (uint32_t)i * obs] = (float)(v[mt][i] - gc.zp_h) * gc.h_scale;
                 }
-                if (a.hq_out) {
-                    int32_t *o = a.hq_out + base;
+                if (a.out.hq) {
+                    int32_t *o = a.out.hq + base;
 #pragma unroll
                     for (int i = 0; i < CH; ++i)
-                        if (c0 + i < nb) o[oj + (uint32_t)(i * a.H)] = v[mt][i];
+                        if (c0 + i < nb) o[oj + (uint32_t)i * obs] = v[mt][i];
                 }
-                if (a.h8_out) {
-                    uint8_t *o = a.h8_out + base;
+                if (a.out.h8) {
+                    uint8_t *o = a.out.h8 + base;
 #pragma unroll
                     for (int i = 0; i < CH; ++i)
-                        if (c0 + i < nb) o[oj + (uint32_t)(i * a.H)] = (uint8_t)v[mt][i];
+                        if (c0 + i < nb) o[oj + (uint32_t)i * obs] = (uint8_t)v[mt][i];
                 }
+                if (last && (a.out.hn_f || a.out.hn_q))
+                    for (int i = 0; i < CH; ++i)
+                        if (c0 + i < nb) {
+                            const size_t at = hn_base + (size_t)(c0 + i) * a.H + j0 + mt * 128 + u;
+                            if (a.out.hn_f) a.out.hn_f[at] = (float)(v[mt][i] - gc.zp_h) * gc.h_scale;
+                            if (a.out.hn_q) a.out.hn_q[at] = v[mt][i];
+                        }
             }
         };
         for (int s = 0; s < a.T; ++s) {
@@ -436,7 +444,7 @@ k_recurrence_cluster(const __grid_constant__ CUtensorMap map_r, const __grid_con
             // this step's rows of W*x+bw and of the outputs: one warp-uniform base each, 32-bit offsets
             // per cell (a sub-group's rows of one step span far less than 2^32 elements)
             const IhT *ih_s = ihp + ((size_t)t * a.B + bg0) * a.C;
-            const size_t out_base = (size_t)out_slot * BH + (size_t)bg0 * a.H;
+            const size_t out_base = (size_t)out_slot * a.out.ts + (size_t)bg0 * a.out.bs, hn_base = (size_t)bg0 * a.H;
             const bool from_regs = keep_h && s > 0;
             const bool from_priv = priv_h && s > 0;
             int kc = 0;   // ordinal of the chunk among this warp's chunks
@@ -672,7 +680,7 @@ k_recurrence_cluster(const __grid_constant__ CUtensorMap map_r, const __grid_con
                     for (int r = 0; r < a.P; ++r)
                         if (r != p) st_async_u32(map_to_rank(at, (uint32_t)r), word, map_to_rank(bar_nx, (uint32_t)r));
                 }
-                if (!last) store_outputs(hn, c0, nb, out_base);
+                if (!last) store_outputs(hn, c0, nb, out_base, s + 1 == a.T, hn_base);
                 if (a.write_final && s + 1 == a.T) {
 #pragma unroll
                     for (int mt = 0; mt < MT; ++mt)
@@ -706,7 +714,7 @@ k_recurrence_cluster(const __grid_constant__ CUtensorMap map_r, const __grid_con
             if (lane == 0 && s + 1 < a.T) tc::mbar_arrive(&h_ready[2 * g + ((s + 1) & 1)]);
             // Outputs of the last chunk leave for global memory after the arrive: nothing in the next
             // step waits for them, so they overlap the exchange and the next MMAs.
-            if (c_last >= 0) store_outputs(hn_last, c_last * CH, nb, out_base);
+            if (c_last >= 0) store_outputs(hn_last, c_last * CH, nb, out_base, s + 1 == a.T, hn_base);
             }   // sub-groups
         }
         if (!ok && lane == 0) atomicOr(a.abort_flag, 1);

@@ -168,7 +168,6 @@ k_recurrence_mma(const __grid_constant__ CUtensorMap map_r, const __grid_constan
         const int q = warp & 3;                      // TMEM lane quadrant this warp may read
         const int rank = (warp - 1) >> 2;            // 0..EPW-1 among the warps of that quadrant
         const int u = q * 32 + lane;                 // unit within a 128-unit tile = TMEM lane
-        const size_t BH = (size_t)a.B * a.H;
         const IhT *ihp = reinterpret_cast<const IhT *>(a.ih);
         const int nchunks = a.NB / CH;
         int64_t corr[MT][3];
@@ -248,10 +247,7 @@ k_recurrence_mma(const __grid_constant__ CUtensorMap map_r, const __grid_constan
                             hn = gru_cell<Narrow>(gc, tables, ihv[mt][i][0], ihv[mt][i][1], ihv[mt][i][2], hh_z,
                                                   hh_r, hh_n, hold[mt][i]);
                         h_nxt[(size_t)(b0 + b) * a.Hpad + j] = (uint8_t)hn;
-                        const size_t o = (size_t)out_slot * BH + (size_t)(b0 + b) * a.H + j;
-                        if (a.hq_out) a.hq_out[o] = hn;
-                        if (a.hf_out) a.hf_out[o] = (float)(hn - gc.zp_h) * gc.h_scale;
-                        if (a.h8_out) a.h8_out[o] = (uint8_t)hn;
+                        put_state(a.out, out_slot, b0 + b, j, a.H, s + 1 == a.T, hn, gc.zp_h, gc.h_scale);
                     }
                 }
             }

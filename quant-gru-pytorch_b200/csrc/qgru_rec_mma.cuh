@@ -27,9 +27,7 @@ struct RecMmaArgs {
     int r_slots;      // cluster kernel: 16 KB shared-memory tile slots for R
     const void *ih;         // [T*B][3H]: raw W*x+bw (int8/int16) or pre-rescaled for the fused cell (int16/int32)
     uint8_t *h8;            // [2][B][Hpad] ping-pong state (+ slack rows)
-    int32_t *hq_out;        // [(T+1)][B][H] or null
-    float *hf_out;          // [(T+1)][B][H] or null
-    uint8_t *h8_out = nullptr;   // [(T+1)][B][H] or null: the quantized state in its 8-bit container
+    OutView out;
     int write_final = 0;    // cluster kernel: the last step also writes its state to h8 (rows [B][Hpad]), where the
                             // launch over the next chunk of timesteps picks it up as its initial state
     LinearConsts lc;        // R*h + br epilogue

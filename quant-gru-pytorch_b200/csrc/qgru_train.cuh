@@ -68,15 +68,15 @@ int qgru_forward_f32_train(qgru_handle *h, int T, int B, const float *W, const f
     h->ev = h->ring[h->calls % qgru_handle::kRing];
     h->calls++;
     CK(cudaEventRecord(h->ev[0], st));
-    CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
     k_quantize_f32_i32<<<grid_for(N * I, 256, h->sm_count), 256, 0, st>>>(x, x32, N * I, h->x_scale, xo.zero_point,
                                                                          op_qmin(xo), op_qmax(xo));
     if (m.x)
         qgru::k_quantize_keep<<<grid_for(N * I, 256, h->sm_count), 256, 0, st>>>(x, N * I, h->x_scale, xo.zero_point,
                                                                              op_qmin(xo), op_qmax(xo), m.x);
-    k_init_state<<<grid_for((long long)B * h->Hpad, 256, h->sm_count), 256, 0, st>>>(
-        nullptr, h0, nullptr, (int32_t *)h->hq32.p, nullptr, nullptr, B, H, h->Hpad, init_slot, h->h_scale, ho.zero_point,
-        op_qmin(ho), op_qmax(ho), h->d_flags);
+    OutView slot;
+    slot.hq = (int32_t *)h->hq32.p + (size_t)init_slot * B * H;
+    slot.bs = H;
+    if ((rc = launch_prologue(h, T, B, FwdInput{0, nullptr, 0, 0, h0}, nullptr, nullptr, slot, st))) return rc;
     if (m.h0 && h0)
         qgru::k_quantize_keep<<<grid_for((long long)B * H, 256, h->sm_count), 256, 0, st>>>(
             h0, (long long)B * H, h->h_scale, ho.zero_point, op_qmin(ho), op_qmax(ho), m.h0);
@@ -88,7 +88,7 @@ int qgru_forward_f32_train(qgru_handle *h, int T, int B, const float *W, const f
         if (wsrc[k] && wmask[k])
             qgru::k_fs_weight_mask<<<grid_for(wn[k], 256, h->sm_count), 256, 0, st>>>(
                 wsrc[k], wn[k], C, h->d_wscale[k], (float)op_qmin(p.op[wop[k]]), (float)op_qmax(p.op[wop[k]]), wmask[k]);
-    h->launches += 8;
+    h->launches += 7;
     const qgru_masks cm{m.ih_linear, m.hh_linear, m.gate_input, m.gate_output, m.h};
     if ((rc = run_generic(h, T, B, x32, (int32_t *)h->hq32.p, (int32_t *)h->vq32.p, flags, st, &cm))) return rc;
     k_dequantize<<<grid_for((long long)nh, 256, h->sm_count), 256, 0, st>>>((const int32_t *)h->hq32.p, h_out,

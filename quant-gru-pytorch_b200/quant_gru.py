@@ -12,8 +12,11 @@ float-storage path with real sigmoid / tanh, both in eval mode), ``forward_quant
 What differs by design: each direction owns a ``gru_ops.Handle`` whose packed weights are
 re-quantized only when a parameter tensor or the quant params change (the reference
 re-quantizes weights and regenerates LUTs on every call); the reverse direction runs on the
-same input with reversed time indexing instead of two ``flip`` copies; the two directions
-are queued on two CUDA streams.  Training: in train() mode with gradients enabled, forward
+same input with reversed time indexing instead of two ``flip`` copies; a quantized forward is one library
+call for both directions (they run beside each other on two CUDA streams) that reads and writes
+the module's own tensors, batch-first ones too, and does not wait for the GPU: like any torch
+operation its results are ordered on the current stream.  A device-side error of a forward is
+raised by the next forward (``forward_quantized``, which checks its input's range, waits).  Training: in train() mode with gradients enabled, forward
 runs through an autograd function whose backward is qgru_backward - the fp32 GRU in float mode,
 and with use_quantization the quantized forward in training mode (float-storage path, or the
 integer path with quant_storage_dtype="int32") with its clamp masks as straight-through
@@ -108,7 +111,6 @@ class _Direction:
         self.weights = None
         self.weights_key = None
         self.loaded_key = None
-        self.stream = None
 
 
 class QuantGRU(nn.Module):
@@ -266,7 +268,6 @@ class QuantGRU(nn.Module):
         st = self._dirs[d]
         if st.handle is None or st.handle.device != (device.index or 0):
             st.handle = gru_ops.Handle(self.input_size, self.hidden_size, device=device.index or 0)
-            st.stream = torch.cuda.Stream(device=device)
             if self.bidirectional:
                 # the two directions run side by side: each persistent kernel takes half the SMs
                 sms = torch.cuda.get_device_properties(device).multi_processor_count
@@ -328,20 +329,36 @@ class QuantGRU(nn.Module):
         orv = outs[1][:T]
         return torch.cat([of, orv], dim=-1), torch.cat([hn, outs[1][0:1]], dim=0)
 
-    def _run_directions(self, fn, device):
-        """Queue fn(d, state) for each direction on its own stream, then join."""
-        cur = torch.cuda.current_stream(device)
-        outs = []
-        for d in range(self.num_directions):
-            st = self._dirs[d]
-            st.stream.wait_stream(cur)
-            with torch.cuda.stream(st.stream):
-                outs.append(fn(d, st))
-        for d in range(self.num_directions):
-            cur.wait_stream(self._dirs[d].stream)
-        for d in range(self.num_directions):
-            self._dirs[d].handle.synchronize()
-        return outs
+    def _layer_forward(self, input, hx, device, dtype):
+        """One quantized forward of every direction in one library call: (output, h_n)."""
+        x = input
+        if x.dtype != dtype or x.device != device or x.stride(-1) != 1:
+            x = x.to(device=device, dtype=dtype).contiguous()
+        B, T = x.shape[:2] if self.batch_first else (x.shape[1], x.shape[0])
+        if x.dim() != 3 or x.shape[2] != self.input_size:
+            raise ValueError(f"input must have {self.input_size} features in three dimensions, got {list(x.shape)}")
+        t_dim, b_dim = (1, 0) if self.batch_first else (0, 1)
+        H, D = self.hidden_size, self.num_directions
+        if hx is not None:
+            if tuple(hx.shape) != (D, B, H):
+                raise ValueError(f"hx must have shape {[D, B, H]}, got {list(hx.shape)}")
+            hx = hx.to(device=device, dtype=dtype).contiguous()
+        states = [self._ready_quant(d, device) for d in range(D)]
+        # (the library keeps offsets inside a timestep in 32 bits: very long batch-first outputs are transposed)
+        direct = not self.batch_first or T * D * H <= 1 << 25
+        out = torch.empty((B, T, D * H) if self.batch_first and direct else (T, B, D * H), dtype=dtype, device=device)
+        ot, ob = (t_dim, b_dim) if direct else (0, 1)
+        h_n = torch.empty((D, B, H), dtype=dtype, device=device)
+        h = states[0].handle
+        args = (T, B, x.data_ptr(), x.stride(t_dim), x.stride(b_dim), hx.data_ptr() if hx is not None else None,
+                out.data_ptr(), out.stride(ot), out.stride(ob), h_n.data_ptr(),
+                torch._C._cuda_getCurrentRawStream(device.index or 0))
+        rev = states[1].handle._h if D == 2 else None
+        if dtype == torch.int32:
+            h._ck(h._lib.qgru_layer_forward_i32(h._h, rev, *args), "qgru_layer_forward_i32")
+        else:
+            h._ck(h._lib.qgru_layer_forward(h._h, rev, self.quant_storage_dtype != "int32", *args), "qgru_layer_forward")
+        return out if direct else out.transpose(0, 1).contiguous(), h_n
 
     def _forward_float_train(self, input, hx):
         """Float mode and QAT with autograd: every tensor operation outside the two library calls is a
@@ -396,9 +413,12 @@ class QuantGRU(nn.Module):
             return self._forward_impl(input, hx)
 
     def _forward_impl(self, input, hx=None):
+        device = input.device if input.is_cuda else torch.device("cuda", torch.cuda.current_device())
+        if self.use_quantization and not self.calibrating:
+            self._ensure_quant_ready()
+            return self._layer_forward(input, hx, device, torch.float32)
         if self.batch_first:
             input = input.transpose(0, 1)
-        device = input.device if input.is_cuda else torch.device("cuda", torch.cuda.current_device())
         x = input.to(device=device, dtype=torch.float32).contiguous()
         T, B, _ = x.shape
         h0 = self._split_h0(hx, B, device, torch.float32)
@@ -423,15 +443,6 @@ class QuantGRU(nn.Module):
                     h = st.handle.forward_float(*st.weights, xd, h0[d])
                 outs.append(torch.cat([h[1:].flip(0), h[0:1]], 0) if d == 1 else h)
             self._quant_params_dirty = True
-        elif self.use_quantization:
-            self._ensure_quant_ready()
-            for d in range(self.num_directions):
-                self._ready_quant(d, device)
-            if self.quant_storage_dtype == "int32":
-                run = lambda d, st: st.handle.forward_f32(x, h0[d], reverse=(d == 1), sync=False)  # noqa: E731
-            else:
-                run = lambda d, st: st.handle.forward_fstorage(x, h0[d], reverse=(d == 1), sync=False)  # noqa: E731
-            outs = self._run_directions(run, device)
         else:
             outs = []
             for d in range(self.num_directions):
@@ -452,20 +463,11 @@ class QuantGRU(nn.Module):
         if input.is_floating_point():
             raise TypeError("forward_quantized only accepts already quantized integer input "
                             f"(int in / int out); got dtype={input.dtype}")
-        if self.batch_first:
-            input = input.transpose(0, 1)
         device = input.device if input.is_cuda else torch.device("cuda", torch.cuda.current_device())
-        x_q = input.to(device=device, dtype=torch.int32).contiguous()
-        T, B, _ = x_q.shape
-        h0 = self._split_h0(hx, B, device, torch.int32)
-        for d in range(self.num_directions):
-            self._ready_quant(d, device)
-        outs = self._run_directions(
-            lambda d, st: st.handle.forward_i32(x_q, h0[d], reverse=(d == 1), sync=False), device)
-        output, h_n = self._combine(outs, T)
-        if self.batch_first:
-            output = output.transpose(0, 1).contiguous()
-        return output, h_n
+        out = self._layer_forward(input, hx, device, torch.int32)
+        for st in self._dirs:
+            st.handle.synchronize()     # values outside the operators' ranges are an error of this call
+        return out
 
     def last_plans(self):
         return [st.handle.describe_plan() if st.handle else "" for st in self._dirs]
