@@ -503,6 +503,11 @@ typedef struct qgru_hist qgru_hist;
 #define QGRU_HIST_CHANNEL0 29
 
 QGRU_API int qgru_hist_create(qgru_hist **out, int device, int hidden_size, int num_bins);
+/* The same in device memory of the caller's (qgru_hist_bytes of it, 16-byte aligned, contents immaterial),
+ * which has to outlive the object and every call queued on it. */
+QGRU_API size_t qgru_hist_bytes(int hidden_size, int num_bins);
+QGRU_API int qgru_hist_create_in(qgru_hist **out, int device, int hidden_size, int num_bins, void *storage,
+                                 size_t bytes);
 QGRU_API void qgru_hist_destroy(qgru_hist *hs);
 QGRU_API int qgru_hist_reset(qgru_hist *hs);
 QGRU_API int qgru_hist_count(const qgru_hist *hs);
@@ -528,6 +533,11 @@ QGRU_API int qgru_calibrate_hist(qgru_handle *h, qgru_hist *hs, int T, int B, co
                                  const float *R, const float *bw, const float *br,
                                  const float *x, const float *h0, const int32_t *granularity,
                                  void *stream);
+/* The same, returning the float forward's states too (h_out [(T+1),B,H] or NULL). */
+QGRU_API int qgru_calibrate_hist_h(qgru_handle *h, qgru_hist *hs, int T, int B, const float *W,
+                                   const float *R, const float *bw, const float *br,
+                                   const float *x, const float *h0, const int32_t *granularity,
+                                   float *h_out, void *stream);
 
 /* calculateGRUQuantitativeParametersFromHistograms (src/gru_interface.cc:1079-1153):
  * histograms + bit-width config (fields of `p` as for qgru_calc_params_from_ranges) ->

@@ -115,6 +115,8 @@ SYMBOLS = {
                                         C.POINTER(Ranges), _P, _P]),
     "qgru_ranges_reset": (None, [C.POINTER(Ranges), C.c_int]),
     "qgru_hist_create": (C.c_int, [C.POINTER(_P), C.c_int, C.c_int, C.c_int]),
+    "qgru_hist_bytes": (C.c_size_t, [C.c_int, C.c_int]),
+    "qgru_hist_create_in": (C.c_int, [C.POINTER(_P), C.c_int, C.c_int, C.c_int, _P, C.c_size_t]),
     "qgru_hist_destroy": (None, [_P]),
     "qgru_hist_reset": (C.c_int, [_P]),
     "qgru_hist_count": (C.c_int, [_P]),
@@ -124,6 +126,8 @@ SYMBOLS = {
     "qgru_hist_import": (C.c_int, [_P, C.c_int, _F, C.c_float, C.c_float, C.c_int64]),
     "qgru_calibrate_hist": (C.c_int, [_P, _P, C.c_int, C.c_int, _P, _P, _P, _P, _P, _P,
                                       C.POINTER(C.c_int32), _P]),
+    "qgru_calibrate_hist_h": (C.c_int, [_P, _P, C.c_int, C.c_int, _P, _P, _P, _P, _P, _P,
+                                        C.POINTER(C.c_int32), _P, _P]),
     "qgru_calc_params_from_hist": (C.c_int, [_P, C.c_int, C.c_float, C.POINTER(Params), _F, _F, _F, _F]),
     "qgru_calibrate_from_histogram": (C.c_int, [_F, C.c_int, C.c_float, C.c_float, C.c_int64, C.c_int,
                                                 C.c_int, C.c_float, C.POINTER(Op)]),

@@ -8,9 +8,13 @@
 // finite values, the host range rules (first batch fixes the range limit, later batches grow
 // the range inside it), a proportional redistribution of the old counts when the range
 // changes, and the binning pass.  Differences in how the work is done, not in what is counted:
-// the gate tensors are not materialised (a generator computes each value from the float
-// forward's buffers inside both passes), one privatised binning kernel serves every tensor, and
-// the per-channel weight histograms are built by one block per channel.
+// the gate tensors are not materialised - one pass over the float forward's buffers takes the ranges of
+// all twelve operators of the cell, a second one bins them (each value is computed in registers and
+// counted in the block's own twelve histograms) - and a batch is two such passes with ONE host
+// synchronisation between them, where all ranges come back at once; the per-channel weight
+// histograms are built by one block per channel.  The SQNR search over the candidates of every
+// histogram and the percentile scan run on the GPU; what decides a result is re-evaluated by the host
+// functions that define it (see k_sqnr_search).
 //
 // Float expressions that decide a bin keep the reference kernels' operand order, with explicit
 // round-to-nearest multiplies and adds so that no fused multiply-add changes a boundary case.
@@ -32,8 +36,6 @@ namespace qgru {
 int float_forward(qgru_handle *h, int T, int B, const float *W, const float *R, const float *bw,
                   const float *br, const float *x, const float *h0, float *h_out, float *v_out,
                   int v_stride, cudaStream_t st);
-int calibrate_histogram_op(const float *counts, int bins, float min_val, float max_val, long long total,
-                           bool pot2, bool use_percentile, float percentile, qgru_op *op);
 }  // namespace qgru
 
 // One collector: counts live on the device, range and bookkeeping on the host.
@@ -41,15 +43,20 @@ struct HistMeta {
     float min_val = FLT_MAX, max_val = -FLT_MAX;
     long long total = 0;
     bool valid = false;
+    bool stored = false;           // the counts hold something (else they read as zeros)
     bool limit_set = false;
     float limit_min = 0.f, limit_max = 0.f;
 };
 
 struct qgru_hist {
     int device = 0, H = 0, bins = 0, n = 0;
-    float *d_counts = nullptr;     // [n][bins]
+    void *own = nullptr;           // storage, where it was allocated here
+    float *d_counts = nullptr;     // [n][bins]; a histogram that holds nothing yet is not cleared
     float *d_tmp = nullptr;        // [bins] redistribution target
-    float *d_mm = nullptr;         // [2] min / max of one pass, then per-channel [2 * 3H]
+    unsigned *d_keys = nullptr;    // [MAX_JOBS][2] min / max keys of one batch's collections
+    float *d_mm = nullptr;         // [4][2][3H] per-channel minima and maxima of W, R, bw, br
+    char *d_scratch = nullptr;     // parameter derivation: per histogram an index, a search job and its result
+    float *d_gather = nullptr;     // [GATHER][bins] histograms on their way to the host
     std::vector<HistMeta> meta;
     bool channels_done[4] = {false, false, false, false};
     std::string err;
@@ -57,75 +64,57 @@ struct qgru_hist {
 
 namespace {
 
-// ---- value generators: element i of a logical tensor, computed from the float forward's buffers
-enum GenKind : int {
-    GEN_PLAIN = 0,     // p0[i]
-    GEN_WX_BIAS,       // p0[i] + p1[i % C]                         (W*x + bw, C = 3H)
-    GEN_V3,            // v slots 3..5 as one [N][3H] tensor        (R*h + br)
-    GEN_V_SLOT,        // v slot `slot` as an [N][H] tensor          (z, r, n)
-    GEN_PRE_ZR,        // (wx[g] + bw[g]) + v[3 + g]                (update / reset gate input, g = slot)
-    GEN_PRE_N,         // (wx[2] + bw[2]) + v[1] * v[5]             (new gate input)
-    GEN_RH,            // v[1] * v[5]                               (r * (R*h + br)_n)
-    GEN_NEW,           // (1 - v[0]) * v[2]
-    GEN_OLD,           // v[0] * h[t]                               (h = p1: [(T+1)][B][H], row n of slot t)
-    GEN_COLS,          // p0[k * ld + c0 + j], j < width             (a column block of a [K][ld] matrix)
-};
+constexpr int GATHER = 128;
+constexpr size_t DERIVE_BYTES = 144;   // of scratch per histogram
+constexpr int MAX_JOBS = 32;     // collections of one batch: x, twelve operators of the cell, at most twelve weight tensors
 
+// ---- a tensor, or a column block of a [K][ld] matrix
 struct Gen {
-    int kind, slot;
-    const float *p0, *p1, *v, *wx;
-    int H, ld, c0, width;
-    long long n;   // number of elements
+    const float *p0;
+    int ld, c0, width;   // width 0: p0[i]; else p0[k * ld + c0 + j], i = k * width + j
+    long long n;         // number of elements
 };
 
 __device__ __forceinline__ float gen_value(const Gen &g, long long i) {
-    const int H = g.H;
-    switch (g.kind) {
-        case GEN_PLAIN: return g.p0[i];
-        case GEN_WX_BIAS: return g.p0[i] + g.p1[i % (3 * H)];
-        case GEN_V3: {
-            const long long row = i / (3 * H);
-            const int c = (int)(i % (3 * H));
-            return g.v[row * 6 * H + 3 * H + c];
-        }
-        case GEN_V_SLOT: {
-            const long long row = i / H;
-            const int j = (int)(i % H);
-            return g.v[row * 6 * H + (long long)g.slot * H + j];
-        }
-        case GEN_PRE_ZR: {
-            const long long row = i / H;
-            const int j = (int)(i % H);
-            const float w = g.wx[row * 3 * H + (long long)g.slot * H + j] + g.p1[g.slot * H + j];
-            return w + g.v[row * 6 * H + (long long)(3 + g.slot) * H + j];
-        }
-        case GEN_PRE_N: {
-            const long long row = i / H;
-            const int j = (int)(i % H);
-            const float w = g.wx[row * 3 * H + 2LL * H + j] + g.p1[2 * H + j];
-            return w + __fmul_rn(g.v[row * 6 * H + H + j], g.v[row * 6 * H + 5LL * H + j]);
-        }
-        case GEN_RH: {
-            const long long row = i / H;
-            const int j = (int)(i % H);
-            return __fmul_rn(g.v[row * 6 * H + H + j], g.v[row * 6 * H + 5LL * H + j]);
-        }
-        case GEN_NEW: {
-            const long long row = i / H;
-            const int j = (int)(i % H);
-            return __fmul_rn(1.0f - g.v[row * 6 * H + j], g.v[row * 6 * H + 2LL * H + j]);
-        }
-        case GEN_OLD: {
-            const long long row = i / H;
-            const int j = (int)(i % H);
-            return __fmul_rn(g.v[row * 6 * H + j], g.p1[row * H + j]);
-        }
-        default: {   // GEN_COLS
-            const long long k = i / g.width;
-            const int j = (int)(i % g.width);
-            return g.p0[k * g.ld + g.c0 + j];
-        }
-    }
+    if (g.width == 0) return g.p0[i];
+    const long long k = i / g.width;
+    return g.p0[k * g.ld + g.c0 + (int)(i - k * g.width)];
+}
+
+// ---- the cell's twelve operators from the float forward's buffers: wx (W*x), v (z, r, n, R*h + br) with six slots
+// per row, h with the initial state in front.  CELL_SLOT: the operator each value counts for.
+constexpr int CELL_VALUES = 16;   // h; three of W*x + bw; three of R*h + br; gate inputs; gate outputs; three products
+constexpr int CELL_COUNT = 12;
+__device__ constexpr int CELL_SLOT[CELL_VALUES] = {0, 1, 1, 1, 2, 2, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11};
+constexpr int CELL_OPS[CELL_COUNT] = {QGRU_OP_H, QGRU_OP_IH_LINEAR, QGRU_OP_HH_LINEAR, QGRU_OP_UPDATE_IN, QGRU_OP_RESET_IN,
+                                      QGRU_OP_NEW_IN, QGRU_OP_UPDATE_OUT, QGRU_OP_RESET_OUT, QGRU_OP_NEW_OUT,
+                                      QGRU_OP_MUL_RESET_HIDDEN, QGRU_OP_MUL_NEW_CONTRIB, QGRU_OP_MUL_OLD_CONTRIB};
+struct CellSrc {
+    const float *wx, *v, *h, *bw;
+    long long N;
+    int B, H;
+};
+__device__ __forceinline__ void cell_values(const CellSrc &c, long long n, int j, float bz, float br, float bn, float (&x)[CELL_VALUES]) {
+    const int H = c.H;
+    const float *w = c.wx + n * 3 * H + j, *q = c.v + n * 6 * H + j;
+    const float z = q[0], r = q[H], g = q[2 * H], rz = q[3 * H], rr = q[4 * H], rg = q[5 * H];
+    const float h_old = c.h[n * H + j];
+    x[0] = c.h[(n + c.B) * H + j];
+    x[1] = w[0] + bz;
+    x[2] = w[H] + br;
+    x[3] = w[2 * H] + bn;
+    x[4] = rz;
+    x[5] = rr;
+    x[6] = rg;
+    x[7] = x[1] + rz;
+    x[8] = x[2] + rr;
+    x[13] = __fmul_rn(r, rg);
+    x[9] = x[3] + x[13];
+    x[10] = z;
+    x[11] = r;
+    x[12] = g;
+    x[14] = __fmul_rn(1.0f - z, g);
+    x[15] = __fmul_rn(z, h_old);
 }
 
 // ordered-integer keys so that float min/max can use integer atomics
@@ -162,26 +151,117 @@ __global__ void __launch_bounds__(256) k_hist_minmax(Gen g, unsigned *mm) {
     }
 }
 
+// keys of a batch's collections before the range pass
+__global__ void k_hist_clear_keys(unsigned *keys) {
+    if (threadIdx.x < MAX_JOBS * 2) keys[threadIdx.x] = threadIdx.x & 1 ? KEY_MAX_EMPTY : KEY_MIN_EMPTY;
+}
+
+// ranges of the cell's operators: a thread walks rows of one unit
+__global__ void __launch_bounds__(128) k_hist_cell_minmax(CellSrc c, unsigned *keys) {
+    const int j = blockIdx.x * 128 + threadIdx.x;
+    float mn[CELL_COUNT], mx[CELL_COUNT];
+#pragma unroll
+    for (int k = 0; k < CELL_COUNT; ++k) {
+        mn[k] = FLT_MAX;
+        mx[k] = -FLT_MAX;
+    }
+    if (j < c.H) {
+        const float bz = c.bw[j], br = c.bw[c.H + j], bn = c.bw[2 * c.H + j];
+        // two rows at a time (the second may be the first again): twenty loads in flight per thread
+        for (long long n = blockIdx.y; n < c.N; n += 2ll * gridDim.y) {
+            float x[CELL_VALUES], x2[CELL_VALUES];
+            cell_values(c, n, j, bz, br, bn, x);
+            cell_values(c, n + gridDim.y < c.N ? n + gridDim.y : n, j, bz, br, bn, x2);
+#pragma unroll
+            for (int k = 0; k < CELL_VALUES; ++k)
+                if (isfinite(x2[k])) {
+                    mn[CELL_SLOT[k]] = fminf(mn[CELL_SLOT[k]], x2[k]);
+                    mx[CELL_SLOT[k]] = fmaxf(mx[CELL_SLOT[k]], x2[k]);
+                }
+#pragma unroll
+            for (int k = 0; k < CELL_VALUES; ++k)
+                if (isfinite(x[k])) {
+                    mn[CELL_SLOT[k]] = fminf(mn[CELL_SLOT[k]], x[k]);
+                    mx[CELL_SLOT[k]] = fmaxf(mx[CELL_SLOT[k]], x[k]);
+                }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < CELL_COUNT; ++k) {
+        for (int o = 16; o > 0; o >>= 1) {
+            mn[k] = fminf(mn[k], __shfl_xor_sync(0xffffffffu, mn[k], o));
+            mx[k] = fmaxf(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+        }
+    }
+    // one pair of atomics per operator and block: they all go to 24 words
+    __shared__ float red[2][CELL_COUNT][4];
+    if ((threadIdx.x & 31) == 0)
+#pragma unroll
+        for (int k = 0; k < CELL_COUNT; ++k) {
+            red[0][k][threadIdx.x >> 5] = mn[k];
+            red[1][k][threadIdx.x >> 5] = mx[k];
+        }
+    __syncthreads();
+    if (threadIdx.x < CELL_COUNT) {
+        const int k = threadIdx.x;
+        const float lo = fminf(fminf(red[0][k][0], red[0][k][1]), fminf(red[0][k][2], red[0][k][3]));
+        const float hi = fmaxf(fmaxf(red[1][k][0], red[1][k][1]), fmaxf(red[1][k][2], red[1][k][3]));
+        if (lo <= hi) {
+            atomicMin(keys + 2 * k, fkey(lo));
+            atomicMax(keys + 2 * k + 1, fkey(hi));
+        }
+    }
+}
+
 // histogram_kernel_shared (src/calibration_gpu.cu:66-104): values below / above the range go to
-// the first / last bin, non-finite values are skipped; counts are whole numbers held as float.
-__global__ void __launch_bounds__(256) k_hist_add(Gen g, float *counts, float min_val, float max_val,
-                                                  float inv_bw, int bins) {
-    extern __shared__ float sh[];
-    for (int i = threadIdx.x; i < bins; i += blockDim.x) sh[i] = 0.0f;
+// the first / last bin, non-finite values are skipped; counts are whole numbers held as float.  The block
+// counts in integers (native shared-memory atomics; a float add there is a compare-and-swap loop).
+struct BinRange {
+    float min_val, max_val, inv_bw;
+    float *counts;
+};
+__device__ __forceinline__ void bin_value(float v, const BinRange &r, int bins, unsigned *sh) {
+    if (!isfinite(v)) return;
+    int b;
+    if (v < r.min_val) b = 0;
+    else if (v > r.max_val) b = bins - 1;
+    else b = min((int)__fmul_rn(v - r.min_val, r.inv_bw), bins - 1);
+    atomicAdd(&sh[b], 1u);
+}
+
+__global__ void __launch_bounds__(256) k_hist_add(Gen g, BinRange r, int bins) {
+    extern __shared__ unsigned sh[];
+    for (int i = threadIdx.x; i < bins; i += blockDim.x) sh[i] = 0u;
     __syncthreads();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < g.n;
-         i += (long long)gridDim.x * blockDim.x) {
-        const float v = gen_value(g, i);
-        if (!isfinite(v)) continue;
-        int b;
-        if (v < min_val) b = 0;
-        else if (v > max_val) b = bins - 1;
-        else b = min((int)__fmul_rn(v - min_val, inv_bw), bins - 1);
-        atomicAdd(&sh[b], 1.0f);
-    }
+         i += (long long)gridDim.x * blockDim.x)
+        bin_value(gen_value(g, i), r, bins, sh);
     __syncthreads();
     for (int i = threadIdx.x; i < bins; i += blockDim.x)
-        if (sh[i] > 0) atomicAdd(&counts[i], sh[i]);
+        if (sh[i]) atomicAdd(&r.counts[i], (float)sh[i]);
+}
+
+struct CellRanges {
+    BinRange r[CELL_COUNT];
+};
+// The twelve operators of the cell in one pass: twelve histograms per block (98 KB at 2048 bins, two
+// blocks per SM).  Bound by the shared-memory atomics, 16 per cell.
+__global__ void __launch_bounds__(512) k_hist_cell_add(CellSrc c, const __grid_constant__ CellRanges rg, int bins) {
+    extern __shared__ unsigned sh[];
+    for (int i = threadIdx.x; i < CELL_COUNT * bins; i += blockDim.x) sh[i] = 0u;
+    __syncthreads();
+    const long long total = c.N * c.H;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const long long n = i / c.H;
+        const int j = (int)(i - n * c.H);
+        float x[CELL_VALUES];
+        cell_values(c, n, j, c.bw[j], c.bw[c.H + j], c.bw[2 * c.H + j], x);
+#pragma unroll
+        for (int k = 0; k < CELL_VALUES; ++k) bin_value(x[k], rg.r[CELL_SLOT[k]], bins, sh + CELL_SLOT[k] * bins);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < CELL_COUNT * bins; i += blockDim.x)
+        if (sh[i]) atomicAdd(&rg.r[i / bins].counts[i % bins], (float)sh[i]);
 }
 
 // redistribute_histogram_kernel (src/calibration_gpu.cu:116-158): each source bin goes to the
@@ -209,17 +289,37 @@ __global__ void k_hist_redistribute(const float *__restrict__ src, float src_min
     }
 }
 
-// per-channel min / max of a [K][C] matrix (compute_per_channel_minmax_kernel, :232-275)
-__global__ void k_channel_minmax(const float *__restrict__ w, int K, int C, float *mins, float *maxs) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
+// per-channel ranges of a [K][C] matrix (compute_per_channel_minmax_kernel, :232-275; degenerate ranges widened
+// as collect_per_channel_histograms_batch does on the host, :600-620).  32 channels x 8 row lanes a block.
+__global__ void __launch_bounds__(256) k_channel_range(const float *__restrict__ w, int K, int C, float tiny_range, float *mins, float *maxs) {
+    __shared__ float smn[8][32], smx[8][32];
+    const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5, c = blockIdx.x * 32 + cx;
     float mn = FLT_MAX, mx = -FLT_MAX;
-    for (int k = 0; k < K; ++k) {
-        const float v = w[(size_t)k * C + c];
-        if (isfinite(v)) {
-            mn = fminf(mn, v);
-            mx = fmaxf(mx, v);
+    if (c < C)
+        for (int k = ry; k < K; k += 8) {
+            const float v = w[(size_t)k * C + c];
+            if (isfinite(v)) {
+                mn = fminf(mn, v);
+                mx = fmaxf(mx, v);
+            }
         }
+    smn[ry][cx] = mn;
+    smx[ry][cx] = mx;
+    __syncthreads();
+    if (ry || c >= C) return;
+    for (int k = 1; k < 8; ++k) {
+        mn = fminf(mn, smn[k][cx]);
+        mx = fmaxf(mx, smx[k][cx]);
+    }
+    if (mn > mx) mn = mx = 0.0f;
+    if (mn == mx) {
+        mn -= 0.5f;
+        mx += 0.5f;
+    }
+    const float range = mx - mn;
+    if (range < tiny_range || isnan(range) || isinf(range)) {
+        mn = fminf(mn, 0.0f);
+        mx = mn + tiny_range;
     }
     mins[c] = mn;
     maxs[c] = mx;
@@ -229,26 +329,144 @@ __global__ void k_channel_minmax(const float *__restrict__ w, int K, int C, floa
 __global__ void __launch_bounds__(128) k_channel_hist(const float *__restrict__ w, int K, int C,
                                                       const float *__restrict__ mins,
                                                       const float *__restrict__ maxs, float *counts, int bins) {
-    extern __shared__ float sh[];
+    extern __shared__ unsigned sh[];
     const int c = blockIdx.x;
-    for (int i = threadIdx.x; i < bins; i += blockDim.x) sh[i] = 0.0f;
+    for (int i = threadIdx.x; i < bins; i += blockDim.x) sh[i] = 0u;
     __syncthreads();
     const float mn = mins[c], mx = maxs[c];
     float bw = (mx - mn) / bins;
     if (bw < 1e-9f) bw = 1e-9f;
-    const float inv = 1.0f / bw;
-    for (int k = threadIdx.x; k < K; k += blockDim.x) {
-        const float v = w[(size_t)k * C + c];
-        if (!isfinite(v)) continue;
-        int b;
-        if (v < mn) b = 0;
-        else if (v > mx) b = bins - 1;
-        else b = min((int)__fmul_rn(v - mn, inv), bins - 1);
-        atomicAdd(&sh[b], 1.0f);
-    }
+    const BinRange r{mn, mx, 1.0f / bw, nullptr};
+    for (int k = threadIdx.x; k < K; k += blockDim.x) bin_value(w[(size_t)k * C + c], r, bins, sh);
     __syncthreads();
     float *out = counts + (size_t)c * bins;
-    for (int i = threadIdx.x; i < bins; i += blockDim.x) out[i] = sh[i];
+    for (int i = threadIdx.x; i < bins; i += blockDim.x) out[i] = (float)sh[i];
+}
+
+// ---- parameter derivation
+// Which candidates of a histogram's SQNR search can be the best: noise of every candidate, one thread each, over
+// the histogram's occupied bins; then the candidates within `margin` of the smallest, as a bit mask.  The
+// result is defined by the host's sums, whose terms come from the C library's powf and may differ from
+// a product in the last bit.  Two fp32 sums of n such terms in the same order differ by less than
+// (2 n + 16) * 2^-24 of themselves, so with a margin of twice that the host's winner is always in the
+// mask, and where the mask holds one candidate (nearly always: the candidates' noises differ by far
+// more) nothing is left to compute.
+// One block per histogram.  3101 histograms (H = 256, per-channel weights), 101 or 357 candidates: 0.37 ms;
+// the whole derivation took 61 ms on 16 host threads.
+constexpr int SQNR_WORDS = 12;   // at most 17 * 21 = 357 candidates
+__global__ void __launch_bounds__(128) k_sqnr_search(const float *__restrict__ counts, const int *__restrict__ index,
+                                                     const SqnrSearch *__restrict__ jobs, int bins,
+                                                     unsigned *__restrict__ mask) {
+    __shared__ float val[2048], cnt[2048];
+    __shared__ float noise_s[SQNR_WORDS * 32];
+    __shared__ unsigned err_s[SQNR_WORDS * 32];   // one occupied bin: the candidate's error and clip flag
+    __shared__ int warp_n[4], base;
+    __shared__ unsigned best_key;
+    const SqnrSearch q = jobs[blockIdx.x];
+    const float *src = counts + (size_t)index[blockIdx.x] * bins;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        base = 0;
+        best_key = 0xffffffffu;
+    }
+    __syncthreads();
+    for (int i0 = 0; i0 < bins; i0 += 128) {   // occupied bins, in order
+        const int i = i0 + tid;
+        const float c = i < bins ? src[i] : 0.f;
+        const bool on = i < bins && !(c < 1e-6f);
+        const unsigned b = __ballot_sync(0xffffffffu, on);
+        if (lane == 0) warp_n[warp] = __popc(b);
+        __syncthreads();
+        int at = base + __popc(b & ((1u << lane) - 1u));
+        for (int w = 0; w < warp; ++w) at += warp_n[w];
+        if (on) {
+            val[at] = __fadd_rn(q.hmin, __fmul_rn((float)i + 0.5f, q.bw));
+            cnt[at] = c;
+        }
+        __syncthreads();
+        if (tid == 0) base += warp_n[0] + warp_n[1] + warp_n[2] + warp_n[3];
+        __syncthreads();
+    }
+    const int n = base;
+    for (int c = tid; c < q.n; c += 128) {
+        float delta, offset;
+        sqnr_candidate(q, c, &delta, &offset);
+        float noise = delta > 0 ? 0.f : FLT_MAX;
+        unsigned err_bits = 0;
+        if (delta > 0) {
+#pragma unroll 4
+            for (int i = 0; i < n; ++i) {
+                const float x = val[i];
+                float t = rintf(__fsub_rn(__fdiv_rn(x, delta), offset));
+                const bool clipped = t < 0 || t > q.steps;
+                t = fmaxf(0.0f, fminf(q.steps, t));
+                const float e = __fsub_rn(__fmul_rn(__fadd_rn(t, offset), delta), x);
+                err_bits = (__float_as_uint(e) & 0x7fffffffu) | (clipped ? 0x80000000u : 0u);
+                float err = __fmul_rn(e, e);
+                if (clipped) err = __fmul_rn(err, 3.0f);
+                noise = __fadd_rn(noise, __fmul_rn(err, cnt[i]));
+            }
+        }
+        noise_s[c] = noise;
+        err_s[c] = err_bits;
+        if (noise < FLT_MAX) atomicMin(&best_key, __float_as_uint(noise));   // non-negative: ordered as integers
+    }
+    __syncthreads();
+    if (best_key == 0xffffffffu) {
+        if (tid < SQNR_WORDS) mask[blockIdx.x * SQNR_WORDS + tid] = 0u;
+        return;
+    }
+    const float limit = __uint_as_float(best_key) * (1.0f + (float)(4 * n + 32) * 0x1p-24f);
+    for (int c0 = warp * 32; c0 < SQNR_WORDS * 32; c0 += 128) {
+        const int c = c0 + lane;
+        bool in = c < q.n && noise_s[c] <= limit;
+        // a bias: one value, and the same error from candidates that are multiples of each other; the first wins
+        if (in && n == 1)
+            for (int k = 0; k < c && in; ++k) in = err_s[k] != err_s[c] || noise_s[k] > limit;
+        const unsigned b = __ballot_sync(0xffffffffu, in);
+        if (lane == 0) mask[blockIdx.x * SQNR_WORDS + c0 / 32] = b;
+    }
+}
+
+// Histogram::getPercentileRange's two bins (include/histogram_collector.h:105-165): the cumulative counts are
+// summed one after another in fp32, as the reference does (above 2^24 the order matters).  One warp per
+// histogram.  out: first bin at or above each threshold, or -1, -1 where the whole range is taken.
+__global__ void __launch_bounds__(32) k_percentile_bins(const float *__restrict__ counts, const int *__restrict__ index, int bins,
+                                                        float clip, int2 *__restrict__ out) {
+    __shared__ float cum[2048];
+    const float *src = counts + (size_t)index[blockIdx.x] * bins;
+    for (int i = threadIdx.x; i < bins; i += 32) cum[i] = src[i];
+    __syncwarp();
+    if (threadIdx.x != 0) return;
+    float s = cum[0];
+#pragma unroll 8
+    for (int i = 1; i < bins; ++i) {
+        s = __fadd_rn(s, cum[i]);
+        cum[i] = s;
+    }
+    int lo = 0, hi = bins - 1;
+    if (s < 1e-6f) {
+        lo = hi = -1;
+    } else {
+        // (the sums do not decrease: binary search)
+        const auto first = [&](float thr, int none) {
+            int a = 0, b = bins;
+            while (a < b) {
+                const int m = (a + b) / 2;
+                if (cum[m] >= thr) b = m;
+                else a = m + 1;
+            }
+            return a < bins ? a : none;
+        };
+        lo = first(__fmul_rn(s, clip), 0);
+        hi = first(__fmul_rn(s, 1.0f - clip), bins - 1);
+    }
+    out[blockIdx.x] = make_int2(lo, hi);
+}
+
+__global__ void k_gather_hist(const float *__restrict__ counts, const int *__restrict__ index, int bins, float *__restrict__ out) {
+    const float *src = counts + (size_t)index[blockIdx.x] * bins;
+    for (int i = threadIdx.x; i < bins; i += blockDim.x) out[(size_t)blockIdx.x * bins + i] = src[i];
 }
 
 int hfail(qgru_hist *hs, int code, const std::string &msg) {
@@ -268,23 +486,17 @@ float min_scale_bins(int bins) { return std::min(1.19209290e-07f, 0.01f / static
 
 int blocks_for(long long n) { return (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, 1184)); }
 
-void add_data(qgru_hist *hs, const Gen &g, float *counts, float min_val, float max_val, cudaStream_t st) {
+BinRange bin_range(const qgru_hist *hs, float *counts, float min_val, float max_val) {
     float bw = (max_val - min_val) / hs->bins;                  // build_histogram, :503-505
     if (bw < 1e-9f) bw = 1e-9f;
-    const float inv = 1.0f / bw;
-    k_hist_add<<<blocks_for(g.n), 256, (size_t)hs->bins * 4, st>>>(g, counts, min_val, max_val, inv, hs->bins);
+    return BinRange{min_val, max_val, 1.0f / bw, counts};
 }
 
-// GPUHistogramCollector::collect for collector `idx` with the values `g` generates.
-int collect(qgru_hist *hs, int idx, const Gen &g, cudaStream_t st) {
-    if (g.n <= 0) return QGRU_OK;
+// The host rules of GPUHistogramCollector::collect for collector `idx` and a batch of n values whose range keys
+// are `keys`: new range, old counts moved into it, and where the new values are to be counted.
+int begin_collect(qgru_hist *hs, int idx, const unsigned *keys, long long n, BinRange *out, cudaStream_t st) {
     HistMeta &m = hs->meta[idx];
     float *counts = hs->d_counts + (size_t)idx * hs->bins;
-    unsigned keys[2] = {KEY_MIN_EMPTY, KEY_MAX_EMPTY};
-    HCK(cudaMemcpyAsync(hs->d_mm, keys, 8, cudaMemcpyHostToDevice, st));
-    k_hist_minmax<<<blocks_for(g.n), 256, 0, st>>>(g, reinterpret_cast<unsigned *>(hs->d_mm));
-    HCK(cudaMemcpyAsync(keys, hs->d_mm, 8, cudaMemcpyDeviceToHost, st));
-    HCK(cudaStreamSynchronize(st));
     float dmin, dmax;
     if (keys[0] == KEY_MIN_EMPTY && keys[1] == KEY_MAX_EMPTY) {
         dmin = dmax = 0.0f;                                     // nothing finite
@@ -308,9 +520,8 @@ int collect(qgru_hist *hs, int idx, const Gen &g, cudaStream_t st) {
         HCK(cudaMemsetAsync(counts, 0, (size_t)hs->bins * 4, st));
         m.min_val = dmin;
         m.max_val = dmax;
-        add_data(hs, g, counts, dmin, dmax, st);
-        m.total = g.n;
-        m.valid = true;
+        m.total = n;
+        m.valid = m.stored = true;
         // growth limit is infinite (HistogramCollector::Config), as in the reference's default
         m.limit_min = dmin - range * INFINITY / 2.0f;
         m.limit_max = dmax + range * INFINITY / 2.0f;
@@ -324,9 +535,7 @@ int collect(qgru_hist *hs, int idx, const Gen &g, cudaStream_t st) {
             new_min = std::min(dmin, m.min_val);
             new_max = std::max(dmax, m.max_val);
         }
-        if (new_min == m.min_val && new_max == m.max_val) {
-            add_data(hs, g, counts, m.min_val, m.max_val, st);
-        } else {
+        if (new_min != m.min_val || new_max != m.max_val) {
             // _merge_with_extended_range_gpu, :924-955
             HCK(cudaMemsetAsync(hs->d_tmp, 0, (size_t)hs->bins * 4, st));
             const float src_bw = (hs->bins <= 0 || m.max_val <= m.min_val) ? 1.0f : (m.max_val - m.min_val) / hs->bins;
@@ -337,67 +546,125 @@ int collect(qgru_hist *hs, int idx, const Gen &g, cudaStream_t st) {
                 k_hist_redistribute<<<(hs->bins + 255) / 256, 256, 0, st>>>(counts, m.min_val, s_bw, hs->d_tmp,
                                                                             new_min, d_bw, hs->bins);
             }
-            add_data(hs, g, hs->d_tmp, new_min, new_max, st);
             HCK(cudaMemcpyAsync(counts, hs->d_tmp, (size_t)hs->bins * 4, cudaMemcpyDeviceToDevice, st));
             m.min_val = new_min;
             m.max_val = new_max;
         }
-        m.total += g.n;
+        m.total += n;
     }
-    HCK(cudaGetLastError());
+    *out = bin_range(hs, counts, m.min_val, m.max_val);
     return QGRU_OK;
 }
 
 Gen plain(const float *p, long long n) {
     Gen g{};
-    g.kind = GEN_PLAIN;
     g.p0 = p;
     g.n = n;
     return g;
 }
 
-// collect_per_channel_histograms_batch (src/calibration_gpu.cu:581-676): built once.
-int collect_channels(qgru_hist *hs, int k, const float *w, int K, cudaStream_t st) {
-    const int C = 3 * hs->H, bins = hs->bins;
-    float *d_min = hs->d_mm + 2, *d_max = d_min + C;
-    k_channel_minmax<<<(C + 127) / 128, 128, 0, st>>>(w, K, C, d_min, d_max);
-    std::vector<float> mn(C), mx(C);
-    HCK(cudaMemcpyAsync(mn.data(), d_min, (size_t)C * 4, cudaMemcpyDeviceToHost, st));
-    HCK(cudaMemcpyAsync(mx.data(), d_max, (size_t)C * 4, cudaMemcpyDeviceToHost, st));
-    HCK(cudaStreamSynchronize(st));
+struct Job {
+    int idx;
+    Gen g;
+};
+
+// One batch: the ranges of every tensor (and of the cell's operators), one synchronisation, then the counts.
+// chan: per-channel histograms to build (matrix, rows), null where not asked for.
+int collect_batch(qgru_hist *hs, const std::vector<Job> &jobs, const CellSrc *cell, const float *const chan[4], const int chan_rows[4],
+                  cudaStream_t st) {
+    const int C = 3 * hs->H, bins = hs->bins, base_job = cell ? CELL_COUNT : 0;
+    if (base_job + (int)jobs.size() > MAX_JOBS) return hfail(hs, QGRU_ERR_BAD_ARG, "too many collections in one batch");
+    k_hist_clear_keys<<<1, 2 * MAX_JOBS, 0, st>>>(hs->d_keys);
     const float tiny_range = min_scale_bins(bins) * bins;
-    for (int c = 0; c < C; ++c) {
-        if (mn[c] > mx[c]) mn[c] = mx[c] = 0.0f;
-        if (mn[c] == mx[c]) {
-            mn[c] -= 0.5f;
-            mx[c] += 0.5f;
+    std::vector<float> mm;
+    for (int k = 0; k < 4 && chan; ++k)
+        if (chan[k]) {
+            k_channel_range<<<(C + 31) / 32, 256, 0, st>>>(chan[k], chan_rows[k], C, tiny_range, hs->d_mm + (size_t)2 * k * C,
+                                                          hs->d_mm + (size_t)(2 * k + 1) * C);
+            k_channel_hist<<<C, 128, (size_t)bins * 4, st>>>(chan[k], chan_rows[k], C, hs->d_mm + (size_t)2 * k * C,
+                                                            hs->d_mm + (size_t)(2 * k + 1) * C,
+                                                            hs->d_counts + (size_t)(QGRU_HIST_CHANNEL0 + k * C) * bins, bins);
+            mm.resize((size_t)8 * C);
         }
-        const float range = mx[c] - mn[c];
-        if (range < tiny_range || std::isnan(range) || std::isinf(range)) {
-            mn[c] = std::min(mn[c], 0.0f);
-            mx[c] = std::max(mx[c], 0.0f);
-            mx[c] = mn[c] + tiny_range;
-        }
+    if (cell) {
+        const int bx = (cell->H + 127) / 128;
+        const dim3 grid(bx, (unsigned)std::min<long long>(cell->N, std::max(1, 1184 / bx)));
+        k_hist_cell_minmax<<<grid, 128, 0, st>>>(*cell, hs->d_keys);
     }
-    HCK(cudaMemcpyAsync(d_min, mn.data(), (size_t)C * 4, cudaMemcpyHostToDevice, st));
-    HCK(cudaMemcpyAsync(d_max, mx.data(), (size_t)C * 4, cudaMemcpyHostToDevice, st));
-    const int base = QGRU_HIST_CHANNEL0 + k * C;
-    k_channel_hist<<<C, 128, (size_t)bins * 4, st>>>(w, K, C, d_min, d_max, hs->d_counts + (size_t)base * bins, bins);
+    for (size_t i = 0; i < jobs.size(); ++i)
+        if (jobs[i].g.n > 0)
+            k_hist_minmax<<<blocks_for(jobs[i].g.n), 256, 0, st>>>(jobs[i].g, hs->d_keys + 2 * (base_job + i));
+    unsigned keys[2 * MAX_JOBS];
+    HCK(cudaMemcpyAsync(keys, hs->d_keys, sizeof(keys), cudaMemcpyDeviceToHost, st));
+    if (!mm.empty()) HCK(cudaMemcpyAsync(mm.data(), hs->d_mm, mm.size() * 4, cudaMemcpyDeviceToHost, st));
     HCK(cudaStreamSynchronize(st));
-    for (int c = 0; c < C; ++c) {
-        HistMeta &m = hs->meta[base + c];
-        m.min_val = mn[c];
-        m.max_val = mx[c];
-        m.total = K;
-        m.valid = true;
+    int rc;
+    if (cell) {
+        CellRanges rg;
+        for (int k = 0; k < CELL_COUNT; ++k) {
+            const int op = CELL_OPS[k];
+            const long long n = cell->N * cell->H * (op == QGRU_OP_IH_LINEAR || op == QGRU_OP_HH_LINEAR ? 3 : 1);
+            if ((rc = begin_collect(hs, op, keys + 2 * k, n, &rg.r[k], st))) return rc;
+        }
+        const size_t smem = (size_t)CELL_COUNT * bins * 4;
+        HCK(cudaFuncSetAttribute(k_hist_cell_add, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const long long blocks = std::max<long long>(1, std::min<long long>((cell->N * cell->H + 8191) / 8192, 296));
+        k_hist_cell_add<<<(unsigned)blocks, 512, smem, st>>>(*cell, rg, bins);
     }
-    hs->channels_done[k] = true;
+    for (size_t i = 0; i < jobs.size(); ++i) {
+        if (jobs[i].g.n <= 0) continue;
+        BinRange r;
+        if ((rc = begin_collect(hs, jobs[i].idx, keys + 2 * (base_job + i), jobs[i].g.n, &r, st))) return rc;
+        k_hist_add<<<blocks_for(jobs[i].g.n), 256, (size_t)bins * 4, st>>>(jobs[i].g, r, bins);
+    }
+    HCK(cudaGetLastError());
+    for (int k = 0; k < 4 && chan; ++k)
+        if (chan[k]) {
+            for (int c = 0; c < C; ++c) {
+                HistMeta &m = hs->meta[QGRU_HIST_CHANNEL0 + k * C + c];
+                m.min_val = mm[(size_t)2 * k * C + c];
+                m.max_val = mm[(size_t)(2 * k + 1) * C + c];
+                m.total = chan_rows[k];
+                m.valid = m.stored = true;
+            }
+            hs->channels_done[k] = true;
+        }
     return QGRU_OK;
+}
+
+size_t hist_storage(int H, int bins) {
+    const size_t n = QGRU_HIST_CHANNEL0 + (size_t)4 * 3 * H;
+    return ((n + 1 + GATHER) * bins + (size_t)8 * 3 * H + 2 * MAX_JOBS) * 4 + 64 + n * DERIVE_BYTES;
 }
 
 }  // namespace
 
 extern "C" {
+
+size_t qgru_hist_bytes(int hidden_size, int num_bins) {
+    return hidden_size > 0 && num_bins > 0 && num_bins <= 2048 ? hist_storage(hidden_size, num_bins) : 0;
+}
+
+int qgru_hist_create_in(qgru_hist **out, int device, int hidden_size, int num_bins, void *storage, size_t bytes) {
+    if (!out || hidden_size <= 0 || num_bins <= 0 || num_bins > 2048 || !storage || bytes < hist_storage(hidden_size, num_bins))
+        return QGRU_ERR_BAD_ARG;
+    *out = nullptr;
+    qgru_hist *hs = new qgru_hist();
+    hs->device = device;
+    hs->H = hidden_size;
+    hs->bins = num_bins;
+    hs->n = QGRU_HIST_CHANNEL0 + 4 * 3 * hidden_size;
+    hs->meta.resize(hs->n);
+    float *p = (float *)storage;
+    hs->d_counts = p;
+    hs->d_tmp = p += (size_t)hs->n * num_bins;
+    hs->d_mm = p += num_bins;
+    hs->d_gather = p += (size_t)8 * 3 * hidden_size;
+    hs->d_keys = (unsigned *)(p += (size_t)GATHER * num_bins);
+    hs->d_scratch = (char *)(((uintptr_t)(p + 2 * MAX_JOBS) + 63) & ~(uintptr_t)63);
+    *out = hs;
+    return QGRU_OK;
+}
 
 int qgru_hist_create(qgru_hist **out, int device, int hidden_size, int num_bins) {
     if (!out || hidden_size <= 0 || num_bins <= 0 || num_bins > 2048) return QGRU_ERR_BAD_ARG;
@@ -407,33 +674,25 @@ int qgru_hist_create(qgru_hist **out, int device, int hidden_size, int num_bins)
         cudaGetLastError();
         return QGRU_ERR_CUDA;
     }
-    qgru_hist *hs = new qgru_hist();
-    hs->device = device;
-    hs->H = hidden_size;
-    hs->bins = num_bins;
-    hs->n = QGRU_HIST_CHANNEL0 + 4 * 3 * hidden_size;
-    hs->meta.resize(hs->n);
-    bool ok = cudaSetDevice(device) == cudaSuccess;
-    ok = ok && cudaMalloc(&hs->d_counts, (size_t)hs->n * num_bins * 4) == cudaSuccess;
-    ok = ok && cudaMalloc(&hs->d_tmp, (size_t)num_bins * 4) == cudaSuccess;
-    ok = ok && cudaMalloc(&hs->d_mm, (size_t)(2 + 2 * 3 * hidden_size) * 4) == cudaSuccess;
-    ok = ok && cudaMemset(hs->d_counts, 0, (size_t)hs->n * num_bins * 4) == cudaSuccess;
-    if (!ok) {
+    void *p = nullptr;
+    const size_t bytes = hist_storage(hidden_size, num_bins);
+    if (cudaSetDevice(device) != cudaSuccess || cudaMalloc(&p, bytes) != cudaSuccess) {
         cudaGetLastError();
-        qgru_hist_destroy(hs);
         return QGRU_ERR_NOMEM;
     }
-    *out = hs;
-    return QGRU_OK;
+    const int rc = qgru_hist_create_in(out, device, hidden_size, num_bins, p, bytes);
+    if (rc == QGRU_OK) (*out)->own = p;
+    else cudaFree(p);
+    return rc;
 }
 
 void qgru_hist_destroy(qgru_hist *hs) {
     if (!hs) return;
-    cudaSetDevice(hs->device);
-    cudaFree(hs->d_counts);
-    cudaFree(hs->d_tmp);
-    cudaFree(hs->d_mm);
-    cudaGetLastError();
+    if (hs->own) {
+        cudaSetDevice(hs->device);
+        cudaFree(hs->own);
+        cudaGetLastError();
+    }
     delete hs;
 }
 
@@ -443,8 +702,6 @@ int qgru_hist_count(const qgru_hist *hs) { return hs ? hs->n : 0; }
 
 int qgru_hist_reset(qgru_hist *hs) {
     if (!hs) return QGRU_ERR_BAD_ARG;
-    HCK(cudaSetDevice(hs->device));
-    HCK(cudaMemset(hs->d_counts, 0, (size_t)hs->n * hs->bins * 4));
     for (HistMeta &m : hs->meta) m = HistMeta();
     for (bool &b : hs->channels_done) b = false;
     return QGRU_OK;
@@ -453,7 +710,8 @@ int qgru_hist_reset(qgru_hist *hs) {
 int qgru_hist_collect(qgru_hist *hs, int index, const float *data, long long n, void *stream) {
     if (!hs || !data || index < 0 || index >= hs->n || n < 0) return QGRU_ERR_BAD_ARG;
     HCK(cudaSetDevice(hs->device));
-    return collect(hs, index, plain(data, n), (cudaStream_t)stream);
+    if (n == 0) return QGRU_OK;
+    return collect_batch(hs, {Job{index, plain(data, n)}}, nullptr, nullptr, nullptr, (cudaStream_t)stream);
 }
 
 int qgru_hist_export(const qgru_hist *hs_c, int index, float *counts, float *min_val, float *max_val,
@@ -464,8 +722,11 @@ int qgru_hist_export(const qgru_hist *hs_c, int index, float *counts, float *min
     if (min_val) *min_val = m.min_val;
     if (max_val) *max_val = m.max_val;
     if (total_count) *total_count = m.valid ? m.total : 0;
-    if (counts) {
+    if (counts && !m.stored) {
+        std::fill(counts, counts + hs->bins, 0.0f);
+    } else if (counts) {
         HCK(cudaSetDevice(hs->device));
+        HCK(cudaDeviceSynchronize());   // the last batch's counts may still be on their way, on any stream
         HCK(cudaMemcpy(counts, hs->d_counts + (size_t)index * hs->bins, (size_t)hs->bins * 4, cudaMemcpyDeviceToHost));
     }
     return QGRU_OK;
@@ -482,6 +743,7 @@ int qgru_hist_import(qgru_hist *hs, int index, const float *counts, float min_va
     m.max_val = max_val;
     m.total = total_count;
     m.valid = total_count > 0;
+    m.stored = true;
     // GPUHistogramCollector::merge into an empty collector, src/calibration_gpu.cu:961-979
     const float tiny_range = min_scale_bins(hs->bins) * hs->bins;
     float range = max_val - min_val;
@@ -496,6 +758,12 @@ int qgru_hist_import(qgru_hist *hs, int index, const float *counts, float min_va
 int qgru_calibrate_hist(qgru_handle *h, qgru_hist *hs, int T, int B, const float *W, const float *R,
                         const float *bw, const float *br, const float *x, const float *h0,
                         const int32_t *granularity, void *stream) {
+    return qgru_calibrate_hist_h(h, hs, T, B, W, R, bw, br, x, h0, granularity, nullptr, stream);
+}
+
+int qgru_calibrate_hist_h(qgru_handle *h, qgru_hist *hs, int T, int B, const float *W, const float *R,
+                          const float *bw, const float *br, const float *x, const float *h0,
+                          const int32_t *granularity, float *h_out, void *stream) {
     if (!h || !hs || !W || !R || !bw || !br || !x || !granularity) return QGRU_ERR_BAD_ARG;
     if (T <= 0 || B <= 0) return fail(h, QGRU_ERR_BAD_ARG, "T and B must be positive");
     if (hs->H != h->H || hs->device != h->device)
@@ -503,70 +771,38 @@ int qgru_calibrate_hist(qgru_handle *h, qgru_hist *hs, int T, int B, const float
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
     const int H = h->H, C = h->C, I = h->I;
-    const long long N = (long long)T * B, NH = N * H;
+    const long long N = (long long)T * B;
     int rc;
-    if ((rc = ensure(h, h->f_h, (size_t)(T + 1) * B * H * 4))) return rc;
+    float *hbuf = h_out;
+    if (!hbuf) {
+        if ((rc = ensure(h, h->f_h, (size_t)(T + 1) * B * H * 4))) return rc;
+        hbuf = (float *)h->f_h.p;
+    }
     if ((rc = ensure(h, h->f_v, (size_t)N * 6 * H * 4))) return rc;
-    float *hbuf = (float *)h->f_h.p, *v = (float *)h->f_v.p;
+    float *v = (float *)h->f_v.p;
     if ((rc = float_forward(h, T, B, W, R, bw, br, x, h0, hbuf, v, 6, st))) return rc;
-    const float *wx = (const float *)h->f_wx.p;
-
-    auto run = [&](int idx, Gen g) -> int {
-        g.H = H;
-        g.v = v;
-        g.wx = wx;
-        const int r = collect(hs, idx, g, st);
-        if (r) h->err = "histogram collection: " + hs->err;
-        return r;
-    };
-    auto make = [&](int kind, int slot, const float *p0, const float *p1, long long n) {
-        Gen g{};
-        g.kind = kind;
-        g.slot = slot;
-        g.p0 = p0;
-        g.p1 = p1;
-        g.n = n;
-        return g;
-    };
-    // x, h (without the initial state), W*x + bw, R*h + br  (collectAllHistogramsGPU, :27-48)
-    if ((rc = run(QGRU_OP_X, make(GEN_PLAIN, 0, x, nullptr, N * I)))) return rc;
-    if ((rc = run(QGRU_OP_H, make(GEN_PLAIN, 0, hbuf + (size_t)B * H, nullptr, NH)))) return rc;
-    if ((rc = run(QGRU_OP_IH_LINEAR, make(GEN_WX_BIAS, 0, wx, bw, N * C)))) return rc;
-    if ((rc = run(QGRU_OP_HH_LINEAR, make(GEN_V3, 0, nullptr, nullptr, N * C)))) return rc;
+    // the cell's operators: h (without the initial state), W*x + bw, R*h + br, gate inputs and outputs, products
+    // (collectAllHistogramsGPU, :27-48, :109-117; collect_gate_histograms, src/calibration_gpu.cu:542-574)
+    const CellSrc cell{(const float *)h->f_wx.p, v, hbuf, bw, N, B, H};
+    std::vector<Job> jobs{Job{QGRU_OP_X, plain(x, N * I)}};
     // weights and biases by granularity (:50-97): per tensor and per gate every batch, per channel once
-    const float *mats[4] = {W, R, bw, br};
+    const float *mats[4] = {W, R, bw, br}, *chan[4] = {};
     const int rows[4] = {I, H, 1, 1};
     static const int tensor_idx[4] = {QGRU_OP_W, QGRU_OP_R, QGRU_OP_BW, QGRU_OP_BR};
     for (int k = 0; k < 4; ++k) {
         if (granularity[k] == QGRU_PER_TENSOR) {
-            if ((rc = run(tensor_idx[k], make(GEN_PLAIN, 0, mats[k], nullptr, (long long)rows[k] * C)))) return rc;
+            jobs.push_back(Job{tensor_idx[k], plain(mats[k], (long long)rows[k] * C)});
         } else if (granularity[k] == QGRU_PER_GATE) {
-            for (int g3 = 0; g3 < 3; ++g3) {
-                Gen g = make(GEN_COLS, 0, mats[k], nullptr, (long long)rows[k] * H);
-                g.ld = C;
-                g.c0 = g3 * H;
-                g.width = H;
-                if ((rc = run(QGRU_HIST_GATE0 + 3 * k + g3, g))) return rc;
-            }
+            for (int g3 = 0; g3 < 3; ++g3) jobs.push_back(Job{QGRU_HIST_GATE0 + 3 * k + g3, Gen{mats[k], C, g3 * H, H, (long long)rows[k] * H}});
         } else if (!hs->channels_done[k]) {
-            if ((rc = collect_channels(hs, k, mats[k], rows[k], st))) {
-                h->err = "histogram collection: " + hs->err;
-                return rc;
-            }
+            chan[k] = mats[k];
         }
     }
-    // gate outputs and products (collect_gate_histograms, src/calibration_gpu.cu:542-574)
-    if ((rc = run(QGRU_OP_UPDATE_OUT, make(GEN_V_SLOT, 0, nullptr, nullptr, NH)))) return rc;
-    if ((rc = run(QGRU_OP_RESET_OUT, make(GEN_V_SLOT, 1, nullptr, nullptr, NH)))) return rc;
-    if ((rc = run(QGRU_OP_NEW_OUT, make(GEN_V_SLOT, 2, nullptr, nullptr, NH)))) return rc;
-    if ((rc = run(QGRU_OP_MUL_RESET_HIDDEN, make(GEN_RH, 0, nullptr, nullptr, NH)))) return rc;
-    if ((rc = run(QGRU_OP_MUL_NEW_CONTRIB, make(GEN_NEW, 0, nullptr, nullptr, NH)))) return rc;
-    if ((rc = run(QGRU_OP_MUL_OLD_CONTRIB, make(GEN_OLD, 0, nullptr, hbuf, NH)))) return rc;
-    // gate inputs (:109-117)
-    if ((rc = run(QGRU_OP_UPDATE_IN, make(GEN_PRE_ZR, 0, nullptr, bw, NH)))) return rc;
-    if ((rc = run(QGRU_OP_RESET_IN, make(GEN_PRE_ZR, 1, nullptr, bw, NH)))) return rc;
-    if ((rc = run(QGRU_OP_NEW_IN, make(GEN_PRE_N, 0, nullptr, bw, NH)))) return rc;
-    h->launches += 2 * 13 + 8;
+    if ((rc = collect_batch(hs, jobs, &cell, chan, rows, st))) {
+        h->err = "histogram collection: " + hs->err;
+        return rc;
+    }
+    h->launches += 4 + 2 * jobs.size();
     return QGRU_OK;
 }
 
@@ -579,64 +815,122 @@ int qgru_calc_params_from_hist(const qgru_hist *hs_c, int use_percentile, float 
         !p->op[QGRU_OP_BR].symmetric)
         return QGRU_ERR_UNSUPPORTED;
     HCK(cudaSetDevice(hs->device));
+    HCK(cudaDeviceSynchronize());   // the last batch's counts may still be on their way, on any stream
     const int H = hs->H, C = 3 * H, bins = hs->bins;
     const bool pot2 = p->use_pot2 != 0;
     p->hidden = H;
-    std::vector<float> counts((size_t)hs->n * bins);
-    HCK(cudaMemcpy(counts.data(), hs->d_counts, counts.size() * 4, cudaMemcpyDeviceToHost));
-    auto one = [&](int idx, qgru_op *op) -> int {
-        const HistMeta &m = hs->meta[idx];
-        if (!m.valid) return hfail(hs, QGRU_ERR_NOT_READY, "histogram " + std::to_string(idx) + " is empty");
-        return calibrate_histogram_op(counts.data() + (size_t)idx * bins, bins, m.min_val, m.max_val, m.total, pot2,
-                                      use_percentile != 0, percentile, op);
-    };
-    // calculateGRUQuantitativeParametersFromHistograms, src/gru_interface.cc:1079-1153
+    // every histogram that is needed, and the operator it derives a scale for
+    // (calculateGRUQuantitativeParametersFromHistograms, src/gru_interface.cc:1079-1153)
     static const int scalar_ops[] = {QGRU_OP_X, QGRU_OP_H, QGRU_OP_IH_LINEAR, QGRU_OP_HH_LINEAR,
                                      QGRU_OP_UPDATE_IN, QGRU_OP_RESET_IN, QGRU_OP_NEW_IN,
                                      QGRU_OP_UPDATE_OUT, QGRU_OP_RESET_OUT, QGRU_OP_NEW_OUT,
                                      QGRU_OP_MUL_RESET_HIDDEN, QGRU_OP_MUL_NEW_CONTRIB, QGRU_OP_MUL_OLD_CONTRIB};
-    int rc;
-    for (int k : scalar_ops)
-        if ((rc = one(k, &p->op[k]))) return rc;
     static const int tensor_idx[4] = {QGRU_OP_W, QGRU_OP_R, QGRU_OP_BW, QGRU_OP_BR};
+    std::vector<int> index;
+    std::vector<qgru_op> ops;
+    for (int k : scalar_ops) {
+        index.push_back(k);
+        ops.push_back(p->op[k]);
+    }
+    for (int k = 0; k < 4; ++k) {
+        const int n = p->granularity[k] == QGRU_PER_TENSOR ? 1 : p->granularity[k] == QGRU_PER_GATE ? 3 : C;
+        const int first = p->granularity[k] == QGRU_PER_TENSOR ? tensor_idx[k]
+                          : p->granularity[k] == QGRU_PER_GATE ? QGRU_HIST_GATE0 + 3 * k : QGRU_HIST_CHANNEL0 + k * C;
+        for (int i = 0; i < n; ++i) {
+            index.push_back(first + i);
+            ops.push_back(p->op[tensor_idx[k]]);
+        }
+    }
+    const int n = (int)index.size();
+    for (int i = 0; i < n; ++i) {
+        const HistMeta &m = hs->meta[index[i]];
+        if (!m.valid || m.total <= 0) return hfail(hs, QGRU_ERR_NOT_READY, "histogram " + std::to_string(index[i]) + " is empty");
+        if ((int64_t)op_qmax(ops[i]) - op_qmin(ops[i]) <= 0) return hfail(hs, QGRU_ERR_BAD_ARG, "operator without a range");
+    }
+    std::vector<SqnrSearch> search(use_percentile ? 0 : n);
+    for (size_t i = 0; i < search.size(); ++i) {
+        const HistMeta &m = hs->meta[index[i]];
+        search[i] = hist_sqnr_search(bins, m.min_val, m.max_val, ops[i]);
+    }
+    // device scratch: indices, then search jobs and masks, or percentile bins
+    const size_t idx_b = ((size_t)n * 4 + 15) & ~size_t(15), job_b = (search.size() * sizeof(SqnrSearch) + 15) & ~size_t(15);
+    static_assert(sizeof(SqnrSearch) + SQNR_WORDS * 4 + 4 + 32 <= DERIVE_BYTES, "scratch per histogram (each part rounded up)");
+    HCK(cudaMemcpyAsync(hs->d_scratch, index.data(), (size_t)n * 4, cudaMemcpyHostToDevice, 0));
+    const int *d_index = (const int *)hs->d_scratch;
+    int rc = QGRU_OK;
+    if (use_percentile) {
+        const float clip = (100.0f - percentile) / 100.0f;
+        std::vector<int2> found(n, make_int2(-1, -1));
+        if (clip > 0.0f) {
+            int2 *d_out = (int2 *)(hs->d_scratch + idx_b);
+            k_percentile_bins<<<n, 32, 0, 0>>>(hs->d_counts, d_index, bins, clip, d_out);
+            HCK(cudaGetLastError());
+            HCK(cudaMemcpyAsync(found.data(), d_out, (size_t)n * sizeof(int2), cudaMemcpyDeviceToHost, 0));
+        }
+        HCK(cudaStreamSynchronize(0));
+        for (int i = 0; i < n && rc == QGRU_OK; ++i) {
+            const HistMeta &m = hs->meta[index[i]];
+            rc = hist_percentile_finish(bins, m.min_val, m.max_val, found[i].x < 0, found[i].x, found[i].y, pot2, &ops[i]);
+        }
+    } else {
+        SqnrSearch *d_jobs = (SqnrSearch *)(hs->d_scratch + idx_b);
+        unsigned *d_mask = (unsigned *)(hs->d_scratch + idx_b + job_b);
+        HCK(cudaMemcpyAsync(d_jobs, search.data(), search.size() * sizeof(SqnrSearch), cudaMemcpyHostToDevice, 0));
+        k_sqnr_search<<<n, 128, 0, 0>>>(hs->d_counts, d_index, d_jobs, bins, d_mask);
+        HCK(cudaGetLastError());
+        std::vector<unsigned> mask((size_t)n * SQNR_WORDS);
+        HCK(cudaMemcpyAsync(mask.data(), d_mask, mask.size() * 4, cudaMemcpyDeviceToHost, 0));
+        HCK(cudaStreamSynchronize(0));
+        // histograms with more than one candidate left: their counts come to the host, GATHER at a time
+        std::vector<int> open, best(n, -1);
+        for (int i = 0; i < n; ++i) {
+            int left = 0;
+            for (int w = 0; w < SQNR_WORDS; ++w) {
+                const unsigned b = mask[(size_t)i * SQNR_WORDS + w];
+                left += __builtin_popcount(b);
+                if (b && best[i] < 0) best[i] = w * 32 + __builtin_ctz(b);
+            }
+            if (left > 1) open.push_back(i);
+        }
+        std::vector<float> counts(std::min<size_t>(open.size(), GATHER) * bins);
+        for (size_t o = 0; o < open.size(); o += GATHER) {
+            const int no = (int)std::min<size_t>(GATHER, open.size() - o);
+            std::vector<int> which(no);
+            for (int i = 0; i < no; ++i) which[i] = index[open[o + i]];
+            HCK(cudaMemcpyAsync(hs->d_scratch, which.data(), (size_t)no * 4, cudaMemcpyHostToDevice, 0));
+            k_gather_hist<<<no, 256, 0, 0>>>(hs->d_counts, d_index, bins, hs->d_gather);
+            HCK(cudaMemcpyAsync(counts.data(), hs->d_gather, (size_t)no * bins * 4, cudaMemcpyDeviceToHost, 0));
+            HCK(cudaStreamSynchronize(0));
+            const auto settle = [&](int k) {
+                const int i = open[o + k];
+                std::vector<int> list;
+                for (int c = 0; c < SQNR_WORDS * 32; ++c)
+                    if (mask[(size_t)i * SQNR_WORDS + c / 32] >> (c & 31) & 1) list.push_back(c);
+                best[i] = hist_sqnr_best(counts.data() + (size_t)k * bins, bins, search[i], ops[i], list.data(), (int)list.size());
+            };
+            const unsigned nt = no < 32 ? 1u : std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
+            std::vector<std::thread> pool;
+            for (unsigned w = 1; w < nt; ++w)
+                pool.emplace_back([&, w]() { for (int k = (int)w; k < no; k += (int)nt) settle(k); });
+            for (int k = 0; k < no; k += (int)nt) settle(k);
+            for (std::thread &t : pool) t.join();
+        }
+        for (int i = 0; i < n && rc == QGRU_OK; ++i) rc = hist_sqnr_finish(search[i], best[i], pot2, &ops[i]);
+    }
+    if (rc) return hfail(hs, rc, "histogram calibration failed");
+    int at = 0;
+    for (int k : scalar_ops) p->op[k] = ops[at++];
     float *scales[4] = {scale_W, scale_R, scale_bw, scale_br};
     for (int k = 0; k < 4; ++k) {
-        qgru_op *op = &p->op[tensor_idx[k]];
         if (p->granularity[k] == QGRU_PER_TENSOR) {
-            qgru_op t = *op;
-            if ((rc = one(tensor_idx[k], &t))) return rc;
-            std::fill(scales[k], scales[k] + C, t.scale);
+            std::fill(scales[k], scales[k] + C, ops[at++].scale);
         } else if (p->granularity[k] == QGRU_PER_GATE) {
-            for (int g = 0; g < 3; ++g) {
-                qgru_op t = *op;
-                if ((rc = one(QGRU_HIST_GATE0 + 3 * k + g, &t))) return rc;
-                std::fill(scales[k] + g * H, scales[k] + (g + 1) * H, t.scale);
-            }
+            for (int g = 0; g < 3; ++g) std::fill(scales[k] + g * H, scales[k] + (g + 1) * H, ops[at++].scale);
         } else {
-            // 3H independent searches: spread over the host threads
-            const int base = QGRU_HIST_CHANNEL0 + k * C;
-            const unsigned nt = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-            std::vector<int> status(nt, QGRU_OK);
-            std::vector<std::thread> pool;
-            for (unsigned w = 0; w < nt; ++w)
-                pool.emplace_back([&, w]() {
-                    for (int c = (int)w; c < C; c += (int)nt) {
-                        const HistMeta &m = hs->meta[base + c];
-                        qgru_op t = *op;
-                        const int r = m.valid ? calibrate_histogram_op(counts.data() + (size_t)(base + c) * bins, bins,
-                                                                       m.min_val, m.max_val, m.total, pot2,
-                                                                       use_percentile != 0, percentile, &t)
-                                              : QGRU_ERR_NOT_READY;
-                        if (r) status[w] = r;
-                        scales[k][c] = t.scale;
-                    }
-                });
-            for (std::thread &t : pool) t.join();
-            for (int r : status)
-                if (r) return hfail(hs, r, "per-channel histogram calibration failed");
+            for (int c = 0; c < C; ++c) scales[k][c] = ops[at++].scale;
         }
-        op->scale = scales[k][0];
-        op->zero_point = 0;
+        p->op[tensor_idx[k]].scale = scales[k][0];
+        p->op[tensor_idx[k]].zero_point = 0;
     }
     return qgru_generate_luts(p);
 }

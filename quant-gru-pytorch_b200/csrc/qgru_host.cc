@@ -316,6 +316,15 @@ float hist_bin_width(const float min_val, const float max_val, int bins) {
     return (max_val - min_val) / bins;
 }
 
+// The tail of Histogram::getPercentileRange once the two bins are known (include/histogram_collector.h:150-165).
+void percentile_from_bins(int bins, float min_val, float max_val, int lo_i, int hi_i, float *pmin, float *pmax) {
+    const float bw = hist_bin_width(min_val, max_val, bins);
+    float a = min_val + lo_i * bw, b = min_val + hi_i * bw;
+    if (b <= a) b = max_val;
+    *pmin = a;
+    *pmax = b;
+}
+
 // Histogram::getPercentileRange, include/histogram_collector.h:105-165.
 void percentile_range(const float *counts, int bins, float min_val, float max_val, long long total,
                       float clip, float *pmin, float *pmax) {
@@ -327,7 +336,6 @@ void percentile_range(const float *counts, int bins, float min_val, float max_va
     for (int i = 1; i < bins; ++i) cum[i] = cum[i - 1] + counts[i];
     const float sum = cum[bins - 1];
     if (sum < 1e-6f) return;
-    const float bw = hist_bin_width(min_val, max_val, bins);
     const float keep = 1.0f - clip;
     const float lo_thr = sum * clip, hi_thr = sum * keep;
     int lo_i = 0, hi_i = bins - 1;
@@ -335,19 +343,12 @@ void percentile_range(const float *counts, int bins, float min_val, float max_va
         if (cum[i] >= lo_thr) { lo_i = i; break; }
     for (int i = 0; i < bins; ++i)
         if (cum[i] >= hi_thr) { hi_i = i; break; }
-    float a = min_val + lo_i * bw, b = min_val + hi_i * bw;
-    if (b <= a) b = max_val;
-    *pmin = a;
-    *pmax = b;
+    percentile_from_bins(bins, min_val, max_val, lo_i, hi_i, pmin, pmax);
 }
 
-// calibratePercentile, include/pot_sqnr_calibrator.h:99-186.
-ContScale calibrate_percentile(const float *counts, int bins, float min_val, float max_val, long long total,
-                               int64_t steps, bool sym, bool uns, float percentile) {
+// calibratePercentile, include/pot_sqnr_calibrator.h:99-186, from the two ends of the percentile range on.
+ContScale percentile_scale(float pmin, float pmax, int64_t steps, bool sym, bool uns) {
     const float tiny = minimum_scale(steps);
-    const float clip = (100.0f - percentile) / 100.0f;
-    float pmin, pmax;
-    percentile_range(counts, bins, min_val, max_val, total, clip, &pmin, &pmax);
     pmin = std::min(pmin, 0.0f);
     pmax = std::max(pmax, 0.0f);
     pmin = std::max(-FLT_MAX, std::min(pmin, 0.0f));
@@ -403,75 +404,66 @@ float sqnr_noise(const float *counts, int bins, float min_val, float bw, float d
     return noise;
 }
 
-// calibrateSqnr with searchSymmetric / searchAsymmetric, include/pot_sqnr_calibrator.h:246-381
-// (101 symmetric deltas; 17 deltas x min(steps + 2, 21) offsets otherwise).
-bool calibrate_sqnr(const float *counts, int bins, float hmin, float hmax, int64_t steps, bool sym,
-                    bool uns, ContScale *out) {
-    const float tiny = minimum_scale(steps);
-    const float bw = hist_bin_width(hmin, hmax, bins);
+// The candidates of calibrateSqnr, searchSymmetric / searchAsymmetric (include/pot_sqnr_calibrator.h:246-381;
+// 101 symmetric deltas; 17 deltas x min(steps + 2, 21) offsets otherwise), in the reference's order.
+SqnrSearch sqnr_search(int bins, float hmin, float hmax, int64_t steps, bool sym, bool uns) {
+    SqnrSearch q{};
+    q.tiny = minimum_scale(steps);
+    q.steps = static_cast<float>(steps);
+    q.hmin = hmin;
+    q.bw = hist_bin_width(hmin, hmax, bins);
     const float min_val = std::min(hmin, 0.0f);
     float max_val = std::max(hmax, 0.0f);
-    const float floor_max = min_val + tiny * static_cast<float>(steps);
+    const float floor_max = min_val + q.tiny * q.steps;
     max_val = (max_val > floor_max) ? max_val : floor_max;
-    float best_noise = FLT_MAX;
-    ContScale best{0, 0, 0};
+    q.sym = sym ? 1 : 0;
     if (sym) {
-        float max_delta, offset;
         if (uns) {
-            max_delta = max_val / static_cast<float>(steps);
-            offset = 0.0f;
+            q.max_delta = max_val / q.steps;
+            q.offset = 0.0f;
         } else {
-            max_delta = 2.0f * std::max(max_val, -min_val) / static_cast<float>(steps);
-            offset = -static_cast<float>((steps + 1) / 2);
+            q.max_delta = 2.0f * std::max(max_val, -min_val) / q.steps;
+            q.offset = -static_cast<float>((steps + 1) / 2);
         }
-        max_delta = std::max(max_delta, tiny);
-        const int cand = 101, div = cand - 1;
-        for (int d = 1; d <= cand; ++d) {
-            float delta = max_delta * d / div;
-            delta = std::max(delta, tiny);
-            const float noise = sqnr_noise(counts, bins, hmin, bw, delta, offset, steps);
-            if (noise < best_noise) {
-                best_noise = noise;
-                best.scale = delta;
-                best.min = offset * delta;
-                best.max = best.min + steps * delta;
-            }
-        }
+        q.max_delta = std::max(q.max_delta, q.tiny);
+        q.n = 101;
     } else {
-        const float max_delta = (max_val - min_val) / static_cast<float>(steps);
-        const float obs_off = rintf(min_val / max_delta);
-        const float obs_min = max_delta * obs_off;
-        const float obs_max = obs_min + max_delta * static_cast<float>(steps);
-        const int n_off = std::min(static_cast<int>(steps + 2), 21);
-        std::vector<float> offs(n_off);
-        const float step = static_cast<float>(steps) / (n_off - 2);
-        for (int o = 0; o < n_off - 1; ++o) offs[o] = rintf(-static_cast<float>(steps) + o * step);
-        offs[n_off - 1] = obs_off;
-        const int cand = 17;
-        for (int d = 1; d <= cand; ++d) {
-            float delta = max_delta * d / (cand - 1);
-            delta = std::max(delta, tiny);
-            for (int o = 0; o < n_off; ++o) {
-                float t_min = delta * offs[o];
-                float t_max = t_min + delta * static_cast<float>(steps);
-                t_min = std::max(obs_min, t_min);
-                t_max = std::min(obs_max, t_max);
-                float cd = (t_max - t_min) / static_cast<float>(steps);
-                cd = std::max(cd, tiny);
-                const float co = rintf(t_min / cd);
-                const float noise = sqnr_noise(counts, bins, hmin, bw, cd, co, steps);
-                if (noise < best_noise) {
-                    best_noise = noise;
-                    best.scale = cd;
-                    best.min = co * cd;
-                    best.max = best.min + steps * cd;
-                }
-            }
+        q.max_delta = (max_val - min_val) / q.steps;
+        q.obs_off = rintf(min_val / q.max_delta);
+        q.obs_min = q.max_delta * q.obs_off;
+        q.obs_max = q.obs_min + q.max_delta * q.steps;
+        q.n_off = static_cast<int>(std::min<int64_t>(steps + 2, 21));
+        q.off_step = q.steps / (q.n_off - 2);
+        q.n = 17 * q.n_off;
+    }
+    return q;
+}
+
+ContScale sqnr_result(const SqnrSearch &q, int c) {
+    float delta, offset;
+    sqnr_candidate(q, c, &delta, &offset);
+    ContScale r;
+    r.scale = delta;
+    r.min = offset * delta;
+    r.max = r.min + q.steps * delta;
+    return r;
+}
+
+// calibrateSqnr over the candidates of `list` (null: all), in order; -1: none has a finite noise.
+int sqnr_best(const float *counts, int bins, const SqnrSearch &q, int64_t steps, const int *list, int n_list) {
+    float best_noise = FLT_MAX;
+    int best = -1;
+    for (int i = 0; i < (list ? n_list : q.n); ++i) {
+        const int c = list ? list[i] : i;
+        float delta, offset;
+        sqnr_candidate(q, c, &delta, &offset);
+        const float noise = sqnr_noise(counts, bins, q.hmin, q.bw, delta, offset, steps);
+        if (noise < best_noise) {
+            best_noise = noise;
+            best = c;
         }
     }
-    if (best_noise == FLT_MAX) return false;
-    *out = best;
-    return true;
+    return best;
 }
 
 // encodeScaleResult(coverage_round = false) + storedScaleForMode, include/pot_sqnr_calibrator.h:
@@ -509,9 +501,14 @@ int calibrate_histogram(const float *counts, int bins, float min_val, float max_
     if (steps <= 0) return QGRU_ERR_BAD_ARG;
     ContScale c;
     if (use_percentile) {
-        c = calibrate_percentile(counts, bins, min_val, max_val, total, steps, sym, uns, percentile);
-    } else if (!calibrate_sqnr(counts, bins, min_val, max_val, steps, sym, uns, &c)) {
-        return QGRU_ERR_RANGE;
+        float pmin, pmax;
+        percentile_range(counts, bins, min_val, max_val, total, (100.0f - percentile) / 100.0f, &pmin, &pmax);
+        c = percentile_scale(pmin, pmax, steps, sym, uns);
+    } else {
+        const SqnrSearch q = sqnr_search(bins, min_val, max_val, steps, sym, uns);
+        const int best = sqnr_best(counts, bins, q, steps, nullptr, 0);
+        if (best < 0) return QGRU_ERR_RANGE;
+        c = sqnr_result(q, best);
     }
     return encode_histogram_scale(c, pot2, op) ? QGRU_OK : QGRU_ERR_RANGE;
 }
@@ -520,9 +517,23 @@ int calibrate_histogram(const float *counts, int bins, float min_val, float max_
 }  // namespace qgru
 
 namespace qgru {
-int calibrate_histogram_op(const float *counts, int bins, float min_val, float max_val, long long total,
-                           bool pot2, bool use_percentile, float percentile, qgru_op *op) {
-    return calibrate_histogram(counts, bins, min_val, max_val, total, pot2, use_percentile, percentile, op);
+// The derivation of one histogram in pieces, for a caller that has counted or searched on the GPU
+// (qgru_calc_params_from_hist): everything that decides a result is computed by the functions above.
+SqnrSearch hist_sqnr_search(int bins, float min_val, float max_val, const qgru_op &op) {
+    return sqnr_search(bins, min_val, max_val, (int64_t)op_qmax(op) - op_qmin(op), op.symmetric != 0, op.bits < 32 && op.is_unsigned);
+}
+int hist_sqnr_best(const float *counts, int bins, const SqnrSearch &q, const qgru_op &op, const int *list, int n_list) {
+    return sqnr_best(counts, bins, q, (int64_t)op_qmax(op) - op_qmin(op), list, n_list);
+}
+int hist_sqnr_finish(const SqnrSearch &q, int best, bool pot2, qgru_op *op) {
+    return best >= 0 && encode_histogram_scale(sqnr_result(q, best), pot2, op) ? QGRU_OK : QGRU_ERR_RANGE;
+}
+int hist_percentile_finish(int bins, float min_val, float max_val, bool whole_range, int lo_i, int hi_i, bool pot2, qgru_op *op) {
+    float pmin = min_val, pmax = max_val;
+    if (!whole_range) percentile_from_bins(bins, min_val, max_val, lo_i, hi_i, &pmin, &pmax);
+    const ContScale c = percentile_scale(pmin, pmax, (int64_t)op_qmax(*op) - op_qmin(*op), op->symmetric != 0,
+                                         op->bits < 32 && op->is_unsigned);
+    return encode_histogram_scale(c, pot2, op) ? QGRU_OK : QGRU_ERR_RANGE;
 }
 }  // namespace qgru
 

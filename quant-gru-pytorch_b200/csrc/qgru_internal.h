@@ -1,6 +1,7 @@
 // qgru_internal.h - declarations shared by the host set-up code and the CUDA translation
 // units of libqgru_b200.  Nothing here is part of the public ABI (include/qgru.h).
 #pragma once
+#include <math.h>
 #include <stdint.h>
 
 #include <string>
@@ -18,9 +19,47 @@ float decode_scale(Rescale r);
 bool make_rescale(float src, float dst, bool pot2, Rescale *out);
 bool make_rescale_product(float a, float b, float dst, bool pot2, Rescale *out);
 bool make_rescale_to_product(float src, float a, float b, bool pot2, Rescale *out);
-// one histogram -> op->scale / op->zero_point by Percentile or SQNR (qgru_host.cc)
-int calibrate_histogram_op(const float *counts, int bins, float min_val, float max_val, long long total,
-                           bool pot2, bool use_percentile, float percentile, qgru_op *op);
+// One histogram -> op->scale / op->zero_point by Percentile or SQNR (qgru_host.cc), in pieces.
+// The SQNR search's candidates: delta and offset of number c come from these scalars.
+struct SqnrSearch {
+    float hmin, bw;                       // histogram: value of bin i = hmin + (i + 0.5) * bw
+    float tiny, steps, max_delta, offset; // symmetric: delta = max(max_delta * (c + 1) / 100, tiny)
+    float obs_off, obs_min, obs_max, off_step;
+    int sym, n, n_off;
+};
+// Both sides round every product (no fused multiply-add): a candidate that differs in its last bit would move the
+// small errors of a histogram with few values by more than any margin.
+QG_HD float sqnr_mul(float a, float b) {
+#if defined(__CUDA_ARCH__)
+    return __fmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+QG_HD void sqnr_candidate(const SqnrSearch &q, int c, float *delta, float *offset) {
+    if (q.sym) {
+        const float d = sqnr_mul(q.max_delta, (float)(c + 1)) / 100.0f;
+        *delta = d > q.tiny ? d : q.tiny;
+        *offset = q.offset;
+        return;
+    }
+    const int d = c / q.n_off + 1, o = c % q.n_off;
+    float dl = sqnr_mul(q.max_delta, (float)d) / 16.0f;
+    dl = dl > q.tiny ? dl : q.tiny;
+    const float off = o == q.n_off - 1 ? q.obs_off : rintf(-q.steps + sqnr_mul((float)o, q.off_step));
+    float t_min = sqnr_mul(dl, off);
+    float t_max = t_min + sqnr_mul(dl, q.steps);
+    t_min = q.obs_min > t_min ? q.obs_min : t_min;
+    t_max = q.obs_max < t_max ? q.obs_max : t_max;
+    float cd = (t_max - t_min) / q.steps;
+    cd = cd > q.tiny ? cd : q.tiny;
+    *delta = cd;
+    *offset = rintf(t_min / cd);
+}
+SqnrSearch hist_sqnr_search(int bins, float min_val, float max_val, const qgru_op &op);
+int hist_sqnr_best(const float *counts, int bins, const SqnrSearch &q, const qgru_op &op, const int *list, int n_list);
+int hist_sqnr_finish(const SqnrSearch &q, int best, bool pot2, qgru_op *op);
+int hist_percentile_finish(int bins, float min_val, float max_val, bool whole_range, int lo_i, int hi_i, bool pot2, qgru_op *op);
 int32_t op_qmin(const qgru_op &o);
 int32_t op_qmax(const qgru_op &o);
 int32_t lut_eval(const qgru_lut &lut, int32_t q_x, const qgru_op &in_bw, const qgru_op &out_bw);

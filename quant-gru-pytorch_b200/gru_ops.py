@@ -374,9 +374,10 @@ class Handle:
         ranges.load(rs)
         return h
 
-    def calibrate_hist(self, W, R, bw, br, x, hist, granularity, h0=None):
+    def calibrate_hist(self, W, R, bw, br, x, hist, granularity, h0=None, want_h=False):
         """Float forward + fold of every operator's values of this batch into ``hist``
-        (a params.Histograms); granularity = QGRU_PER_* of W, R, bw, br."""
+        (a params.Histograms); granularity = QGRU_PER_* of W, R, bw, br.  want_h: returns the float
+        forward's h [(T+1),B,H]."""
         T, B = int(x.shape[0]), int(x.shape[1])
         H = self.hidden_size
         args = [_check_tensor(t, n, torch.float32) for t, n in
@@ -384,8 +385,10 @@ class Handle:
         if h0 is not None:
             h0 = _check_tensor(h0, "h0", torch.float32, (B, H))
         gran = (C.c_int32 * 4)(*[int(g) for g in granularity])
-        self._ck(self._lib.qgru_calibrate_hist(self._h, hist._h, T, B, *[_ptr(t) for t in args], _ptr(h0),
-                                               gran, _stream(self._tdev)), "qgru_calibrate_hist")
+        h = torch.empty((T + 1, B, H), dtype=torch.float32, device=self._tdev) if want_h else None
+        self._ck(self._lib.qgru_calibrate_hist_h(self._h, hist._h, T, B, *[_ptr(t) for t in args], _ptr(h0), gran, _ptr(h),
+                                                 hist._on(torch.cuda.current_stream(self._tdev))), "qgru_calibrate_hist")
+        return h
 
     # -- introspection
     def synchronize(self):
@@ -573,8 +576,7 @@ def forward_calibrate(is_training, time_steps, batch_size, input_size, hidden_si
         x = _check_tensor(x, "x", torch.float32, (time_steps, batch_size, input_size))
         hd = _handle_for(x.device.index or 0, input_size, hidden_size, "fp")
         h0 = h0 if (h0 is not None and h0.numel() > 0) else None
-        hd.calibrate_hist(W, R, bw, br, x, hist_collectors, bitwidth_config.granularity_list(), h0)
-        h = hd.forward_float(W, R, bw, br, x, h0)
+        h = hd.calibrate_hist(W, R, bw, br, x, hist_collectors, bitwidth_config.granularity_list(), h0, want_h=True)
         return h, torch.empty(0, dtype=torch.float32, device=x.device)
     if method != "minmax":
         raise ValueError(f"unknown calibration method {calib_method_str!r}")

@@ -173,18 +173,35 @@ class Histograms:
     """One direction's histogram collectors (GRUGPUHistogramCollectors,
     include/histogram_gpu.cuh): 2048-bin histograms with range growth for the 13 activation
     operators and, by granularity, per-tensor / per-gate / per-channel ones for W, R, bw, br.
-    Counts live on the GPU inside the library."""
+    Counts live on the GPU, in a block of torch's caching allocator: collectors come and go with
+    every calibration, and allocating their 12 MB to 50 MB from the driver took longer than filling
+    them."""
 
     def __init__(self, hidden, device=0, num_bins=2048):
+        import torch
         self.hidden, self.device, self.num_bins = hidden, device, num_bins
         self._lib = _cabi.lib()
         self._h = C.c_void_p()
-        _cabi.check(self._lib.qgru_hist_create(C.byref(self._h), device, hidden, num_bins), "qgru_hist_create")
+        n = self._lib.qgru_hist_bytes(hidden, num_bins)
+        if n == 0:
+            raise ValueError("hidden must be positive and num_bins between 1 and 2048")
+        self._storage = torch.empty(n, dtype=torch.uint8, device=torch.device("cuda", device))
+        self._streams = {torch.cuda.current_stream(device).cuda_stream}
+        _cabi.check(self._lib.qgru_hist_create_in(C.byref(self._h), device, hidden, num_bins,
+                                                  C.c_void_p(self._storage.data_ptr()), n), "qgru_hist_create_in")
+
+    def _on(self, stream):
+        """Work on the counts is queued on this stream: the allocator must not reuse them before it is done."""
+        if stream.cuda_stream not in self._streams:
+            self._streams.add(stream.cuda_stream)
+            self._storage.record_stream(stream)
+        return C.c_void_p(stream.cuda_stream)
 
     def close(self):
         if getattr(self, "_h", None) is not None and self._h.value:
             self._lib.qgru_hist_destroy(self._h)
             self._h = C.c_void_p()
+            self._storage = None
 
     def __del__(self):
         try:
@@ -208,7 +225,7 @@ class Histograms:
         import torch
         if not (data.is_cuda and data.dtype == torch.float32 and data.is_contiguous()):
             raise ValueError("data must be a contiguous float32 CUDA tensor")
-        stream = C.c_void_p(torch.cuda.current_stream(data.device).cuda_stream)
+        stream = self._on(torch.cuda.current_stream(data.device))
         self._ck(self._lib.qgru_hist_collect(self._h, int(index), C.c_void_p(data.data_ptr()),
                                              int(data.numel()), stream), "qgru_hist_collect")
 

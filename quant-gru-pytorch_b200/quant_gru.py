@@ -438,9 +438,8 @@ class QuantGRU(nn.Module):
                     name = "hist_collectors_reverse" if d == 1 else "hist_collectors"
                     if getattr(self, name) is None:
                         setattr(self, name, Histograms(self.hidden_size, device.index or 0))
-                    st.handle.calibrate_hist(*st.weights, xd, getattr(self, name),
-                                             self._bitwidth_config.granularity_list(), h0[d])
-                    h = st.handle.forward_float(*st.weights, xd, h0[d])
+                    h = st.handle.calibrate_hist(*st.weights, xd, getattr(self, name),
+                                                 self._bitwidth_config.granularity_list(), h0[d], want_h=True)
                 outs.append(torch.cat([h[1:].flip(0), h[0:1]], 0) if d == 1 else h)
             self._quant_params_dirty = True
         else:
