@@ -446,7 +446,10 @@ QGRU_API double qgru_probe_last_bulk_rate(void);
  *                                           stream beside this chunk's recurrence).  0: one chunk;
  *                                           auto: eight chunks where the recurrence leaves half of
  *                                           the SMs free and T >= 256
- *   "rec"      auto | dp4a | mma | generic  recurrence kernel (generic = int32 storage path)
+ *   "rec"      auto | dp4a | mma | gemv | reg | fast | generic
+ *                                           recurrence kernel (generic = int32 storage path; reg: R in
+ *                                           registers, warp-level tensor instructions, H <= 1024; fast:
+ *                                           auto, and reg at the sizes where it is the faster one)
  *   "exchange" auto | global | cluster      how the CTAs of a batch group exchange h_t
  *   "cell"     auto | fused | generic       gate datapath: tabulated (auto also allows its
  *                                           shift-free form), or the reference's step by step

@@ -166,7 +166,9 @@ int qgru_set_option(qgru_handle *h, const char *name, const char *value) {
         else if (v == "mma") h->opt_rec = 2;
         else if (v == "generic") h->opt_rec = 3;
         else if (v == "gemv") h->opt_rec = 4;
-        else return fail(h, QGRU_ERR_BAD_ARG, "rec: auto|dp4a|mma|gemv|generic");
+        else if (v == "reg") h->opt_rec = 5;
+        else if (v == "fast") h->opt_rec = 6;
+        else return fail(h, QGRU_ERR_BAD_ARG, "rec: auto|dp4a|mma|gemv|reg|fast|generic");
     } else if (n == "exchange") {
         if (v == "auto") h->opt_exchange = 0;
         else if (v == "global") h->opt_exchange = 1;
@@ -466,6 +468,7 @@ int qgru_set_params(qgru_handle *h, const qgru_params *p, const float *scale_W,
         CK(cudaMemcpy(h->d_wscale[k], wscale[k].data(), C * sizeof(float), cudaMemcpyHostToDevice));
     h->params_set = true;
     h->fs_ready = false;
+    h->plan_reg = RecRegPlan{};   // its tables have other sizes now
     return QGRU_OK;
 }
 
@@ -718,6 +721,81 @@ int launch_prologue(qgru_handle *h, int T, int B, const FwdInput &in, uint8_t *x
     return QGRU_OK;
 }
 
+// What the W*x product stores for the tabulated cell: the value already at its gate's input scale.
+PreScale pre_scale(const qgru_handle *h, bool fused) {
+    PreScale ps{};
+    ps.H = h->H;
+    if (!fused) return ps;
+    ps.enabled = 1;
+    ps.zp_ih = h->gc_host.zp_ih;
+    for (int a = 0; a < 3; ++a) {
+        ps.to[a] = h->gc_host.ih_to[a];
+        ps.zp_in[a] = h->gc_host.zp_in[a];
+    }
+    if (h->gc_host.ft_ih_n > 0) {
+        ps.table = h->d_ftables + h->gc_host.ft_ih_off;
+        ps.table_n = h->gc_host.ft_ih_n;
+        ps.lo = h->gc_host.ih_lo;
+    }
+    return ps;
+}
+
+// Where rec=fast takes the register-resident recurrence (us per step against the other forms, integer cell):
+// - not where one CTA per row with R in registers and no tile of eight rows fits (one row at H = 256: 1.66 / 1.07);
+// - one CTA per row group, H <= 256: always (256 rows 2.29 / 2.70, 4096 rows of H = 64 1.8 / 5.5);
+// - clusters, H <= 512: up to four rows each, where the exchange costs less than tcgen05's fixed latencies (H = 512:
+//   one and two rows 2.4 / 2.88, four 2.87 / 2.89, eight 2.95 / 2.94, 31 rows 10.2 / 5.7); the longer cells of the
+//   generic and the float form keep it ahead up to a full tile of eight (3.2 / 3.8);
+// - larger clusters: one tile of eight rows (H = 1024: six rows 2.56 / 4.29, ten 4.51 / 4.29).
+bool reg_is_faster(const RecRegPlan &pl, bool gemv) {
+    if (gemv) return false;
+    if (pl.P == 1) return true;
+    return pl.Bt <= (pl.KS == 2 && pl.cell <= CELL_INT_FAST_NOTIE ? 4 : 8);
+}
+
+// The 8-bit path with the register-resident recurrence.
+int run_reg(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out, unsigned flags, RecCell cell, const RecRegPlan &pl,
+            int ih_bytes, int n_table, cudaStream_t st) {
+    const long long N = (long long)T * B;
+    const int sms = h->opt_sm_limit > 0 ? std::min(h->opt_sm_limit, h->sm_count) : h->sm_count;
+    const bool fused = cell <= CELL_INT_FAST_NOTIE;
+    int rc;
+    if ((rc = ensure(h, h->ih, pl.ih_elements(N) * ih_bytes))) return rc;
+    PreScale ps = pre_scale(h, fused);
+    ps.slice = pl.U;
+    CK(cudaEventRecord(h->ev[1], st));
+    const LinearConsts lcx = linear_consts(h, 0);
+    if ((rc = tc_gemm_launch(h->tc, x8, (N + 127) / 128 * 128, h->d_w8[0], h->w8_rows[0], h->ih.p, N, h->C, h->Ipad, h->x_uns, ih_bytes, lcx,
+                             ps, lcx.fits32 && h->rs_fast[0] && h->opt_cell != 2, h->lin_notie[0] && h->opt_tie != 1, h->d_flags + 1, sms, st,
+                             &h->err)))
+        return rc;
+    h->launches++;
+    CK(cudaEventRecord(h->ev[2], st));
+    RecRegArgs a{};
+    a.T = T;
+    a.B = B;
+    a.H = h->H;
+    a.Hpad = h->Hpad;
+    a.reverse = (flags & QGRU_FLAG_REVERSE) ? 1 : 0;
+    a.r8 = h->d_w8[1];
+    a.ih = h->ih.p;
+    a.h8 = (const uint8_t *)h->h8.p;
+    a.out = out;
+    a.lc = linear_consts(h, 1);
+    a.gc = h->d_gc;
+    a.tables = fused ? h->d_ftables : h->d_tables;
+    a.n_table = n_table;
+    a.abort_flag = h->d_flags + 1;
+    if ((rc = rec_reg_launch(h, pl, a, cell, ih_bytes, st))) return rc;
+    CK(cudaEventRecord(h->ev[3], st));
+    h->timing_valid = true;
+    char buf[300];
+    snprintf(buf, sizeof(buf), "path=int8 gemm=tcgen05_i8 rec=mma_sync_i8 r_in=registers cell=%s U=%d KS=%d KST=%d P=%d G=%d Bt=%d D=%d smem=%zu ih_bytes=%d",
+             fused ? "fused_shiftfree" : "generic", pl.U, pl.KS, pl.KST, pl.P, pl.G, pl.Bt, pl.D, pl.smem, ih_bytes);
+    h->plan_text = buf;
+    return QGRU_OK;
+}
+
 // Shared tail of the device entry points, 8-bit path: x8 and the initial state are ready.
 int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out, unsigned flags, cudaStream_t st) {
     const long long N = (long long)T * B;
@@ -746,13 +824,26 @@ int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out
     // while the rows fit one wave of SMs (beyond that the tensor-core tiles win on throughput).
     const bool gemv_ok = gemv_fits(h) && h->opt_rec != 1 && h->opt_rec != 2;
     if (h->opt_rec == 4 && !gemv_ok) return fail(h, QGRU_ERR_UNSUPPORTED, "rec=gemv needs H <= 256");
-    const bool use_gemv = gemv_ok && (h->opt_rec == 4 || (h->opt_rec == 0 && B <= sms));
+    const bool use_gemv = gemv_ok && (h->opt_rec == 4 || ((h->opt_rec == 0 || h->opt_rec == 6) && B <= sms));
     if (use_gemv) use_mma = false;
     const bool use_cluster = use_mma && cluster_ok;
     if (h->opt_exchange == 2 && use_mma && !use_cluster)
         return fail(h, QGRU_ERR_UNSUPPORTED, "cluster exchange does not fit shared memory");
     if (use_cluster) mp = cp;
     if (!use_mma && !use_gemv && !dp4a_ok) return fail(h, QGRU_ERR_UNSUPPORTED, "no recurrence plan fits shared memory");
+    // R in registers with warp-level tensor instructions (qgru_rec_reg.cu)
+    if ((h->opt_rec == 5 || (h->opt_rec == 6 && h->opt_exchange == 0)) && h->opt_gemm != 1 && !h->opt_floor) {
+        const bool lin_fast = h->lin_fits32[1] && h->rs_fast[1];
+        const bool cell_fast = h->opt_cell == 0 && h->gc_host.fused_ok && lin_fast && h->gc_host.rh_to_n.mq != 0 && h->gc_host.uh_to_h.mq != 0;
+        const bool notie = h->lin_notie[1] && h->gc_host.cell_notie != 0 && h->opt_tie != 1;
+        const RecCell cell = !cell_fast ? CELL_INT_GENERIC : notie ? CELL_INT_FAST_NOTIE : CELL_INT_FAST;
+        const int bytes = cell_fast ? h->gc_host.ih_pre_bytes : h->ih_bytes;
+        const int n_tab = cell_fast ? h->gc_host.ft_ih_off : h->n_table;
+        RecRegPlan &rp = h->plan_reg;
+        const bool fits = rec_reg_plan(h, B, sms, bytes, cell, n_tab, &rp);
+        if (!fits && h->opt_rec == 5) return fail(h, QGRU_ERR_UNSUPPORTED, "rec=reg needs H <= 1024 and room for its tables");
+        if (fits && (h->opt_rec == 5 || reg_is_faster(rp, use_gemv))) return run_reg(h, T, B, x8, out, flags, cell, rp, bytes, n_tab, st);
+    }
     // the fused cell needs the GEMM epilogue to pre-rescale W*x+bw: tensor-core GEMM only
     // (the one-CTA-per-row form takes it only in its branch-free shape: every scale shift-free)
     const bool gemv_fused = use_gemv && h->opt_cell == 0 && h->lin_fits32[1] && h->rs_fast[1] &&
@@ -769,21 +860,7 @@ int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out
     if (h->opt_ut == 64 && use_mma && !use_c64)
         return fail(h, QGRU_ERR_UNSUPPORTED, "unit_tile=64 needs the fused shift-free cell, H <= 512 and at most 96 rows per cluster");
     if (use_c64) mp = c64;
-    PreScale ps{};
-    if (fused) {
-        ps.enabled = 1;
-        ps.H = h->H;
-        ps.zp_ih = h->gc_host.zp_ih;
-        for (int a = 0; a < 3; ++a) {
-            ps.to[a] = h->gc_host.ih_to[a];
-            ps.zp_in[a] = h->gc_host.zp_in[a];
-        }
-        if (h->gc_host.ft_ih_n > 0) {
-            ps.table = h->d_ftables + h->gc_host.ft_ih_off;
-            ps.table_n = h->gc_host.ft_ih_n;
-            ps.lo = h->gc_host.ih_lo;
-        }
-    }
+    const PreScale ps = pre_scale(h, fused);
     // ---- chunks of timesteps (cluster recurrence with the tensor-core GEMM): W*x+bw exists for two
     // chunks at a time instead of the whole sequence, and the GEMM of chunk k+1 runs on a second,
     // low-priority stream beside the recurrence of chunk k, which picks up its initial state where

@@ -509,11 +509,21 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
     const int ih_bytes = (oih.bits <= 8 && !oih.is_unsigned) ? 1 : 2;
     if (oih.bits > 16 || (oih.bits == 16 && oih.is_unsigned))
         return fail(h, QGRU_ERR_UNSUPPORTED, "float-storage forward stores W*x + bw in at most 16 signed bits");
-    if ((rc = ensure(h, h->ih, (size_t)N * C * ih_bytes))) return rc;
     const bool rev = flags & QGRU_FLAG_REVERSE;
     uint8_t *h8 = (uint8_t *)h->h8.p;
     const size_t h8_half = (size_t)B * h->Hpad;
     const int sms = h->opt_sm_limit > 0 ? std::min(h->opt_sm_limit, h->sm_count) : h->sm_count;
+    // (small batches of a narrow layer run faster on the SIMT forms below than on the clusters: measured 0.17 ms
+    // against 0.28 ms at H = 128, B = 32 and 4.1 against 4.6 us per step at H = 256, B = 1)
+    const bool small = (h->opt_rec == 0 || h->opt_rec == 4 || h->opt_rec == 6) && h->Hpad <= 256 && B <= sms;
+    RecRegPlan &rp = h->plan_reg;
+    bool use_reg = false;
+    if ((h->opt_rec == 5 || (h->opt_rec == 6 && h->opt_exchange == 0)) && h->opt_gemm != 1) {
+        use_reg = rec_reg_plan(h, B, sms, ih_bytes, CELL_FS, n_tab, &rp);
+        if (!use_reg && h->opt_rec == 5) return fail(h, QGRU_ERR_UNSUPPORTED, "rec=reg needs H <= 1024 and room for its tables");
+        use_reg = use_reg && (h->opt_rec == 5 || reg_is_faster(rp, small));
+    }
+    if ((rc = ensure(h, h->ih, (use_reg ? rp.ih_elements(N) : (size_t)N * C) * ih_bytes))) return rc;
 
     h->ev = h->ring[h->calls % qgru_handle::kRing];
     h->calls++;
@@ -531,11 +541,12 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
     bool used_tc = false;
     if (h->opt_gemm != 1) {
         PreScale ps{};
+        ps.slice = use_reg ? rp.U : H;
         rc = tc_gemm_launch(h->tc, x8, (N + 127) / 128 * 128, h->d_w8[0], h->w8_rows[0],
                             h->ih.p, N, C, h->Ipad, h->x_uns, ih_bytes, lcx, ps, false, false, h->d_flags + 1, sms, st,
                             &h->err);
         if (rc == QGRU_OK) used_tc = true;
-        else if (rc != QGRU_ERR_UNSUPPORTED || h->opt_gemm == 2) return rc;
+        else if (rc != QGRU_ERR_UNSUPPORTED || h->opt_gemm == 2 || use_reg) return rc;
     }
     if (!used_tc) {
         dim3 grid((unsigned)((N + 63) / 64), (unsigned)((C + 63) / 64));
@@ -555,12 +566,25 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
     RecMmaPlan cp;
     // the tensor-core recurrence of the integer path (one cluster per group of batch rows, h_t
     // exchanged through distributed shared memory) with the float cell as its epilogue
-    // (small batches of a narrow layer run faster on the SIMT forms below: measured 0.17 ms against
-    // 0.28 ms at H = 128, B = 32 and 4.1 against 4.6 us per step at H = 256, B = 1)
-    const bool small = (h->opt_rec == 0 || h->opt_rec == 4) && h->Hpad <= 256 && B <= sms;
-    const bool cluster_ok = !small && h->opt_rec != 1 && h->opt_rec != 3 && h->opt_exchange != 1 &&
+    const bool cluster_ok = !small && !use_reg && h->opt_rec != 1 && h->opt_rec != 3 && h->opt_exchange != 1 &&
                             rec_cluster_plan(H, h->Hpad, B, sms, h->smem_optin, n_tab, h->opt_r_where, h->opt_mt, h->opt_ng, h->opt_kp, &cp);
-    if (cluster_ok) {
+    if (use_reg) {
+        RecRegArgs a{};
+        a.T = T; a.B = B; a.H = H; a.Hpad = h->Hpad;
+        a.reverse = rev ? 1 : 0;
+        a.r8 = h->d_w8[1];
+        a.ih = h->ih.p;
+        a.h8 = h8;
+        a.out = out;
+        a.tables = (const int32_t *)gate_tab;   // float bit patterns
+        a.n_table = n_tab;
+        a.abort_flag = h->d_flags + 1;
+        a.fs_chan = chan + (size_t)3 * C;
+        a.fs = fc;
+        if ((rc = rec_reg_launch(h, rp, a, CELL_FS, ih_bytes, st))) return rc;
+        snprintf(buf, sizeof(buf), "path=float_storage gemm=tcgen05_i8 rec=mma_sync_i8_float_cell r_in=registers U=%d KS=%d P=%d G=%d Bt=%d smem=%zu ih_bytes=%d gates=%s",
+                 rp.U, rp.KS, rp.P, rp.G, rp.Bt, rp.smem, ih_bytes, fc.tab_on ? "tabulated" : "evaluated");
+    } else if (cluster_ok) {
         RecMmaArgs a;
         a.T = T; a.B = B; a.H = H; a.Hpad = h->Hpad; a.C = C;
         a.P = cp.P; a.NB = cp.NB; a.b_off = 0; a.b_cnt = B;
@@ -586,7 +610,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
         snprintf(buf, sizeof(buf), "path=float_storage gemm=%s rec=tcgen05_i8_float_cell exchange=cluster_dsmem NB=%d NG=%d P=%d G=%d smem=%zu tmem_cols=%d ih_bytes=%d gates=%s",
                  used_tc ? "tcgen05_i8" : "simt_dp4a", cp.NB, cp.NG, cp.P, cp.G, cp.smem, cp.tmem_cols, ih_bytes,
                  fc.tab_on ? "tabulated" : "evaluated");
-    } else if ((h->opt_rec == 0 || h->opt_rec == 4) && h->Hpad <= 256 && B <= sms &&
+    } else if (small &&
                gemv_smem(h, n_tab) <= (size_t)h->smem_optin) {
         // one CTA per batch row, the whole R in shared memory, no synchronisation between CTAs
         RecArgs a{};

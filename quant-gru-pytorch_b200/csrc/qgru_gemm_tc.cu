@@ -349,6 +349,7 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
                 done += cnt;
             }
         }
+        const int slice = ps.slice, ld = 3 * slice;
         ChanConsts cur = load_consts(0);
         int m0;
         long long n0;
@@ -361,14 +362,15 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
             const Rescale rs = cur.rs;
             const FastLin fl = cur.fl;
             // fused-cell mode: the channel's gate decides the second rescale (to its input scale)
-            const int gate = (ps.enabled && m_ok) ? m / ps.H : 0;
+            const int gate = m_ok ? m / ps.H : 0;
             const Rescale pre_rs = ps.to[gate];
             const int32_t pre_zp = ps.zp_in[gate];
             const int32_t c32 = (int32_t)corr;
             ok = WAITED(4, tc::mbar_wait(&acc_full[buf], (uint32_t)((local / nacc) & 1), WAIT_BUDGET));
             if (!ok) break;
             tc::tc_fence_after_sync();
-            IhT *out = ih + m;
+            const int unit = m - gate * ps.H, sl = unit / slice;
+            IhT *out = ih + ((size_t)sl * N * ld + gate * slice + (unit - sl * slice));
             // this warp's COLS accumulator columns: both halves are fetched before anything is
             // computed, and the buffer goes back to the MMA warp as soon as they have arrived
             static_assert(COLS == 32, "two 16-column loads per warp and tile");
@@ -423,14 +425,14 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
                         y[i] = t;
                     }
                 }
-                // token n of channel m lives at ih[n * C + m]: one pointer walked by C elements
-                IhT *po = out + (n0 + c0) * C;
+                // token n of channel m: one pointer walked by rows of 3 * slice values
+                IhT *po = out + (n0 + c0) * ld;
                 if (m_ok && n0 + c0 + 16 <= N) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i, po += C) *po = (IhT)y[i];
+                    for (int i = 0; i < 16; ++i, po += ld) *po = (IhT)y[i];
                 } else if (m_ok) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i, po += C)
+                    for (int i = 0; i < 16; ++i, po += ld)
                         if (n0 + c0 + i < N) *po = (IhT)y[i];
                 }
             }
@@ -523,6 +525,8 @@ int tc_gemm_launch(TcGemmState &s, const uint8_t *x8, long long x_rows_alloc, co
     const CUtensorMap &mx = *reinterpret_cast<const CUtensorMap *>(s.map_x);
     // the branch-free epilogue applies the second rescale from the table, or needs its shift-free form
     const bool tab = ps.enabled && ps.table != nullptr && 3 * ps.table_n <= PRE_TAB_MAX;
+    if (ps.H == 0) ps.H = C / 3;
+    if (ps.slice == 0) ps.slice = ps.H;
     fast = fast && (!ps.enabled || tab || (ps.to[0].mq != 0 && ps.to[1].mq != 0 && ps.to[2].mq != 0));
     cudaError_t e;
     if (ih_bytes == 1)

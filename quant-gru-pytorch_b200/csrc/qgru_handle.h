@@ -10,6 +10,7 @@
 #include "qgru_gemm_tc.cuh"
 #include "qgru_rec_f32.cuh"
 #include "qgru_rec_mma.cuh"
+#include "qgru_rec_reg.cuh"
 #include "qgru_internal.h"
 
 using qgru::GateConsts;
@@ -37,7 +38,7 @@ struct qgru_handle {
     GateConsts gc_host{};
     // options
     int opt_gemm = 0;      // 0 auto, 1 simt, 2 tcgen05
-    int opt_rec = 0;       // 0 auto, 1 dp4a, 3 generic
+    int opt_rec = 0;       // 0 auto, 1 dp4a, 2 mma, 3 generic, 4 gemv, 5 reg (forced), 6 fast (auto, and reg where it is faster)
     int opt_sm_limit = 0;  // 0: all SMs
     int opt_exchange = 0;  // 0 auto (cluster where it fits), 1 global counter, 2 cluster only
     int opt_cell = 0;      // 0 auto (fused cell where valid), 1 generic cell
@@ -99,6 +100,7 @@ struct qgru_handle {
     bool timing_valid = false;
     uint64_t launches = 0;
     TcGemmState tc;
+    qgru::RecRegPlan plan_reg;   // register-resident recurrence: the plan of the last call
     qgru::RecMmaState rec;       // tensor maps of the global-exchange recurrence
     qgru::RecMmaState rec_cl;    // tensor maps of the cluster-exchange recurrence
     qgru::RecMmaState rec_c64;   // tensor maps of its 64-units-per-CTA form

@@ -104,7 +104,9 @@ struct GateConsts {
 // What the input-projection GEMM applies after the requantization when the recurrence runs the
 // fused cell: out = rescale(ih - zp_ih -> gate input scale of the channel's gate) + zp_in[gate].
 struct PreScale {
-    int32_t enabled, H, zp_ih;
+    int32_t enabled, zp_ih;
+    int32_t H;              // hidden size: channel m belongs to gate m / H
+    int32_t slice;          // hidden units per slice of the stored tensor [H / slice][N][3][slice]; 0: H, i.e. [N][3H]
     Rescale to[3];
     int32_t zp_in[3];
     // optional table of that function over the clamped W*x+bw range (gate-major, n entries per

@@ -268,6 +268,7 @@ class QuantGRU(nn.Module):
         st = self._dirs[d]
         if st.handle is None or st.handle.device != (device.index or 0):
             st.handle = gru_ops.Handle(self.input_size, self.hidden_size, device=device.index or 0)
+            st.handle.set_option("rec", "fast")
             if self.bidirectional:
                 # the two directions run side by side: each persistent kernel takes half the SMs
                 sms = torch.cuda.get_device_properties(device).multi_processor_count

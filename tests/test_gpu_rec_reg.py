@@ -1,0 +1,42 @@
+"""GPU tests of the recurrence with R in registers (option rec=reg, qgru_rec_reg.cu) against the oracle: every split of
+K over warps and of the units over CTAs, ragged rows and units, both directions, all cells."""
+import importlib
+
+import numpy as np
+import pytest
+
+from __graft_entry__ import PKG_NAME
+from tests.cases import config_named, make_case
+
+gru_ops = importlib.import_module(PKG_NAME + ".gru_ops")
+pytestmark = pytest.mark.gpu
+
+# (T, B, H): one CTA with 64 .. 256 inputs a warp (one row, full and ragged tiles of eight, several tiles), K over two
+# warps in clusters of 3 and 4, over four warps in clusters of 9 and 16
+SHAPES = [(1, 1, 1), (4, 3, 64), (5, 300, 60), (3, 1500, 33), (6, 9, 130), (4, 19, 192), (5, 1, 255), (3, 1400, 256),
+          (5, 2, 257), (6, 37, 321), (4, 70, 384), (5, 41, 512), (3, 300, 500), (4, 2, 513), (5, 5, 600), (3, 90, 1001), (4, 1, 1024)]
+
+
+@pytest.mark.parametrize("T,B,H", SHAPES)
+@pytest.mark.parametrize("cfg", ["default", "cfg2", "cfg3", "ih16", "unsigned_x"])
+def test_reg_recurrence_equals_oracle(oracle, cuda_device, cfg, T, B, H):
+    import torch
+    I = 7
+    case = make_case(T * 131 + H, T, B, I, H, oracle, config_named(cfg))
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda_device)
+    want = oracle.forward_i32(T, B, I, H, case.wq, case.x_q, case.h0_q, case.params.c, case.params.scale_list())
+    with gru_ops.Handle(I, H, device=cuda_device.index or 0) as hd:
+        hd.set_params(case.params)
+        hd.set_weights_i32(*[dev(a) for a in case.wq])
+        x, xf = dev(case.x_q), dev(case.x)
+        h0 = None if case.h0_q is None else dev(case.h0_q)
+        f0 = None if case.h0 is None else dev(case.h0)
+        base = [hd.forward_f32(xf, f0, reverse=True), hd.forward_fstorage(xf, f0), hd.forward_i32(x, h0, reverse=True)]
+        hd.set_option("rec", "reg")
+        assert np.array_equal(hd.forward_i32(x, h0).cpu().numpy(), want)
+        assert "r_in=registers" in hd.describe_plan()
+        for cell in ("auto", "generic"):
+            hd.set_option("cell", cell)
+            got = [hd.forward_f32(xf, f0, reverse=True), hd.forward_fstorage(xf, f0), hd.forward_i32(x, h0, reverse=True)]
+            for a, b in zip(base, got):
+                assert torch.equal(a, b), hd.describe_plan()
