@@ -306,6 +306,27 @@ QGRU_API int qgru_backward(qgru_handle *h, int T, int B, const float *W_t, const
                            float *dx, float *dW, float *dR, float *dbw, float *dbr, float *dh,
                            const qgru_bwd_masks *masks, void *stream);
 
+/* Training of a whole layer (GRUFunction, pytorch/quant_gru.py:760-1058, for one or both directions): weights and
+ * gradients in the module's layout, W [3H,I], R [3H,H], gates r, z, n; x and out strided as in qgru_layer_forward
+ * (mode 0: x dense [T,B,I]); h0, h_n, dh_n, dh0 [directions][B,H].  mode 0: fp32 GRU; 1: float-storage quantized
+ * forward; 2: integer forward (1, 2: after qgru_set_params; weights are quantized by the call and not left
+ * loaded).  `saved`: qgru_train_saved_bytes bytes per direction, written by the forward, read by the
+ * backward; 0 bytes: this layer has no such form, use the entry points above.  Gradient pointers
+ * (dx, dh0, dW ... dbr), biases, h0 and dh_n may be NULL.  Nothing waits for the GPU. */
+typedef struct qgru_train_dir {
+    const float *W, *R, *bw, *br;
+    void *saved;
+    float *dW, *dR, *dbw, *dbr;
+    int shares_x;               /* written by the forward, read by the backward of the same pass */
+} qgru_train_dir;
+QGRU_API int qgru_train_saved_bytes(qgru_handle *h, int mode, int T, int B, size_t *bytes);
+QGRU_API int qgru_train_forward(qgru_handle *h, qgru_handle *reverse, int mode, int T, int B, const float *x, long long x_ts, long long x_bs,
+                                const float *h0, qgru_train_dir *dirs, float *out, long long out_ts, long long out_bs, float *h_n,
+                                void *stream);
+QGRU_API int qgru_train_backward(qgru_handle *h, qgru_handle *reverse, int mode, int T, int B, const float *x, const float *dout,
+                                 long long do_ts, long long do_bs, const float *dh_n, float *dx, float *dh0, const qgru_train_dir *dirs,
+                                 void *stream);
+
 /* quantGRUForwardInt (src/gru_interface.cc:610-725), inference mode: float in, float out.
  *   x [T,B,I] f32 device, h0 [B,H] f32 device or NULL, h [(T+1),B,H] f32 device out,
  *   x_q_out [T,B,I] int32 device or NULL. */

@@ -46,6 +46,11 @@ class Masks(C.Structure):
                 ("gate_output", C.c_void_p), ("h", C.c_void_p)]
 
 
+class TrainDir(C.Structure):
+    """qgru_train_dir: weights, saved block and gradients of one direction (device pointers, 0 = absent)."""
+    _fields_ = [(n, C.c_void_p) for n in ("W", "R", "bw", "br", "saved", "dW", "dR", "dbw", "dbr")] + [("shares_x", C.c_int)]
+
+
 class BwdMasks(C.Structure):
     """qgru_bwd_masks: straight-through masks of the quantized backward (device pointers, 0 = absent)."""
     _fields_ = [(n, C.c_void_p) for n in ("x", "h0", "W", "R", "bw", "br", "ih_linear", "hh_linear",
@@ -105,6 +110,9 @@ SYMBOLS = {
     "qgru_timing_window": (C.c_int, [_P, C.POINTER(C.c_int), _F, _F, _F]),
     "qgru_launch_count": (C.c_uint64, [_P]),
     "qgru_describe_plan": (C.c_char_p, [_P, C.c_int, C.c_int]),
+    "qgru_train_saved_bytes": (C.c_int, [_P, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_size_t)]),
+    "qgru_train_forward": (C.c_int, [_P, _P, C.c_int, C.c_int, C.c_int, _P, C.c_longlong, C.c_longlong, _P, _P, _P, C.c_longlong, C.c_longlong, _P, _P]),
+    "qgru_train_backward": (C.c_int, [_P, _P, C.c_int, C.c_int, C.c_int, _P, _P, C.c_longlong, C.c_longlong, _P, _P, _P, _P, _P]),
     "qgru_set_option": (C.c_int, [_P, C.c_char_p, C.c_char_p]),
     "qgru_probe_mma_i8": (C.c_int, [C.c_int] * 7 + [C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "qgru_probe_mma_i8_commits": (C.c_int, [C.c_int] * 11 + [C.POINTER(C.c_double), C.POINTER(C.c_double)]),

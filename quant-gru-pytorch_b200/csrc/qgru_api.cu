@@ -112,6 +112,7 @@ void qgru_destroy(qgru_handle *h) {
     cudaDeviceSynchronize();
     cudaFree(h->d_gc);
     cudaFree(h->d_tables);
+    cudaFree(h->d_ttables);
     cudaFree(h->d_ftables);
     for (int i = 0; i < 2; ++i) {
         cudaFree(h->d_rs[i]);
@@ -341,7 +342,8 @@ int qgru_set_params(qgru_handle *h, const qgru_params *p, const float *scale_W,
                narrow_ok(g.n_to_h, max_abs_diff(op[QGRU_OP_NEW_OUT]));
 
     // Tabulate each activation over its whole clamped input range when that range is small.
-    std::vector<int32_t> tables;
+    std::vector<int32_t> tables, ttables;
+    bool flags_fit = true;
     for (int a = 0; a < 3; ++a) {
         g.table_size[a] = 0;
         g.table_off[a] = 0;
@@ -351,9 +353,15 @@ int qgru_set_params(qgru_handle *h, const qgru_params *p, const float *scale_W,
             g.table_size[a] = n;
             for (int q = g.in_lo[a]; q <= g.in_hi[a]; ++q)
                 tables.push_back(lut_eval(p->lut[a], q, op[in_op[a]], op[out_op[a]]));
+            for (int q = g.in_lo[a]; q <= g.in_hi[a]; ++q) {
+                const int32_t y = tables[ttables.size()];
+                ttables.push_back(2 * y + (y == lut_raw(p->lut[a], q) ? 1 : 0));
+            }
+            flags_fit = flags_fit && op[out_op[a]].bits <= 30;
         }
     }
     h->n_table = (int)tables.size();
+    h->n_ttable = flags_fit ? h->n_table : 0;
 
     // Tables of the fused cell (gru_cell_fused): every entry is computed with the same host
     // functions the kernels' generic path uses, so both forms give identical results.
@@ -444,19 +452,21 @@ int qgru_set_params(qgru_handle *h, const qgru_params *p, const float *scale_W,
               (ih8 || ih16) && (int64_t)std::max(h->I, h->H) * 128 * 255 < (int64_t)0x7fffffff;
 
     int rc;
-    if ((rc = alloc_dev(h, &h->d_gc, 1))) return rc;
+    if ((rc = alloc_once(h, &h->d_gc, 1))) return rc;
     if ((rc = alloc_dev(h, &h->d_tables, tables.size()))) return rc;
+    if ((rc = alloc_dev(h, &h->d_ttables, ttables.size()))) return rc;
+    if (!ttables.empty()) CK(cudaMemcpy(h->d_ttables, ttables.data(), ttables.size() * 4, cudaMemcpyHostToDevice));
     if ((rc = alloc_dev(h, &h->d_ftables, ft.size()))) return rc;
     if (!ft.empty()) CK(cudaMemcpy(h->d_ftables, ft.data(), ft.size() * 4, cudaMemcpyHostToDevice));
     for (int s = 0; s < 2; ++s) {
-        if ((rc = alloc_dev(h, &h->d_rs[s], C))) return rc;
-        if ((rc = alloc_dev(h, &h->d_brs[s], C))) return rc;
-        if ((rc = alloc_dev(h, &h->d_fl[s], C))) return rc;
-        if ((rc = alloc_dev(h, &h->d_corr[s], C))) return rc;
-        if ((rc = alloc_dev(h, &h->d_wsum[s], C))) return rc;
+        if ((rc = alloc_once(h, &h->d_rs[s], C))) return rc;
+        if ((rc = alloc_once(h, &h->d_brs[s], C))) return rc;
+        if ((rc = alloc_once(h, &h->d_fl[s], C))) return rc;
+        if ((rc = alloc_once(h, &h->d_corr[s], C))) return rc;
+        if ((rc = alloc_once(h, &h->d_wsum[s], C))) return rc;
     }
     for (int k = 0; k < 4; ++k)
-        if ((rc = alloc_dev(h, &h->d_wscale[k], C))) return rc;
+        if ((rc = alloc_once(h, &h->d_wscale[k], C))) return rc;
     CK(cudaMemcpy(h->d_gc, &g, sizeof(g), cudaMemcpyHostToDevice));
     if (!tables.empty())
         CK(cudaMemcpy(h->d_tables, tables.data(), tables.size() * 4, cudaMemcpyHostToDevice));
@@ -467,8 +477,8 @@ int qgru_set_params(qgru_handle *h, const qgru_params *p, const float *scale_W,
     for (int k = 0; k < 4; ++k)
         CK(cudaMemcpy(h->d_wscale[k], wscale[k].data(), C * sizeof(float), cudaMemcpyHostToDevice));
     h->params_set = true;
-    h->fs_ready = false;
-    h->plan_reg = RecRegPlan{};   // its tables have other sizes now
+    h->fs_uploaded = h->fs_ready = false;
+    h->plan_reg = h->plan_train = RecRegPlan{};   // their tables have other sizes now
     return QGRU_OK;
 }
 
@@ -476,19 +486,26 @@ int qgru_set_params(qgru_handle *h, const qgru_params *p, const float *scale_W,
 
 namespace {
 
+// The packed weights: rows are allocated (and zeroed) past 3H so that every 128-row tile load stays inside.  Whoever
+// packs writes whole rows, so the zeros are written once.
+int alloc_packed(qgru_handle *h, cudaStream_t st) {
+    int rc;
+    h->w8_rows[0] = (h->C + 127) / 128 * 128;
+    h->w8_rows[1] = h->C + 256;
+    for (int s = 0; s < 2; ++s) {
+        if (h->d_w8[s]) continue;
+        const size_t n = (size_t)h->w8_rows[s] * (s ? h->Hpad : h->Ipad);
+        if ((rc = alloc_once(h, &h->d_w8[s], n))) return rc;
+        CK(cudaMemsetAsync(h->d_w8[s], 0, n, st));
+    }
+    return QGRU_OK;
+}
+
 // Pack int32 weights already resident in h->d_wq[] and derive the per-channel corrections.
 int finish_weights(qgru_handle *h, cudaStream_t st) {
     const int C = h->C;
     int rc;
-    if (h->fast) {
-        // rows are allocated (and zeroed) past 3H so that every 128-row tile load stays inside
-        h->w8_rows[0] = (C + 127) / 128 * 128;
-        h->w8_rows[1] = C + 256;
-        if ((rc = alloc_dev(h, &h->d_w8[0], (size_t)h->w8_rows[0] * h->Ipad))) return rc;
-        if ((rc = alloc_dev(h, &h->d_w8[1], (size_t)h->w8_rows[1] * h->Hpad))) return rc;
-        CK(cudaMemsetAsync(h->d_w8[0], 0, (size_t)h->w8_rows[0] * h->Ipad, st));
-        CK(cudaMemsetAsync(h->d_w8[1], 0, (size_t)h->w8_rows[1] * h->Hpad, st));
-    }
+    if (h->fast && (rc = alloc_packed(h, st))) return rc;
     CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
     k_pack_weights<<<C, 128, 0, st>>>(h->d_wq[0], h->fast ? h->d_w8[0] : nullptr, h->d_wsum[0], h->I,
                                       h->Ipad, C, h->d_flags);
@@ -511,10 +528,6 @@ int finish_weights(qgru_handle *h, cudaStream_t st) {
     h->lin_fits32[1] = !(h->h_flags[0] & 16);
     h->lin_notie[0] = !(h->h_flags[0] & 32);
     h->lin_notie[1] = !(h->h_flags[0] & 64);
-    h->tc.valid = false;
-    h->rec.valid = false;
-    h->rec_cl.valid = false;
-    h->rec_c64.valid = false;
     h->weights_set = true;
     h->fs_ready = false;
     return QGRU_OK;
@@ -536,7 +549,7 @@ int qgru_set_weights_f32(qgru_handle *h, const float *W, const float *R, const f
     const int opi[4] = {QGRU_OP_W, QGRU_OP_R, QGRU_OP_BW, QGRU_OP_BR};
     int rc;
     for (int k = 0; k < 4; ++k) {
-        if ((rc = alloc_dev(h, &h->d_wq[k], n[k]))) return rc;
+        if ((rc = alloc_once(h, &h->d_wq[k], n[k]))) return rc;
         k_quantize_weights<<<grid_for((long long)n[k], 256, h->sm_count), 256, 0, st>>>(
             src[k], h->d_wq[k], (long long)n[k], C, h->d_wscale[k], op_qmin(h->p.op[opi[k]]),
             op_qmax(h->p.op[opi[k]]));
@@ -557,7 +570,7 @@ int qgru_set_weights_i32(qgru_handle *h, const int32_t *W_q, const int32_t *R_q,
     const int32_t *src[4] = {W_q, R_q, bw_q, br_q};
     int rc;
     for (int k = 0; k < 4; ++k) {
-        if ((rc = alloc_dev(h, &h->d_wq[k], n[k]))) return rc;
+        if ((rc = alloc_once(h, &h->d_wq[k], n[k]))) return rc;
         CK(cudaMemcpyAsync(h->d_wq[k], src[k], n[k] * 4, cudaMemcpyDeviceToDevice, st));
     }
     return finish_weights(h, st);
@@ -671,6 +684,7 @@ struct FwdInput {
     const void *h0;
     void *xq = nullptr;              // optional dense copy of the quantized x
     uint8_t *x_keep = nullptr, *h0_keep = nullptr;
+    float *xd = nullptr;             // optional dense copy of the dequantized x
 };
 
 // The first launch of a forward (k_prologue); x8: null where another handle has quantized the same x.
@@ -687,6 +701,7 @@ int launch_prologue(qgru_handle *h, int T, int B, const FwdInput &in, uint8_t *x
     a.x8 = x8;
     a.xq = in.xq;
     a.keep = in.x_keep;
+    a.xd = in.xd;
     a.x_scale = h->x_scale;
     a.x_zp = xo.zero_point;
     a.x_lo = op_qmin(xo);
@@ -1465,3 +1480,4 @@ extern "C" int qgru_forward_i32_static(qgru_handle *h, int T, int B, const int32
 #include "qgru_fstorage.cuh"
 #include "qgru_layer.cuh"
 #include "qgru_train.cuh"
+#include "qgru_train_layer.cuh"

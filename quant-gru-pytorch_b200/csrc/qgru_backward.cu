@@ -112,16 +112,31 @@ __global__ void k_bwd_apply_mask(float *__restrict__ data, const uint8_t *__rest
 // The bias gradients from the sums the recurrence leaves per group of batch rows: part [G][6][H] (z, r, n of
 // dp, then of dq), added in group order.
 __global__ void k_bwd_bias(const float *__restrict__ part, int G, int H, const uint8_t *__restrict__ m_bw,
-                           const uint8_t *__restrict__ m_br, float *__restrict__ dbw, float *__restrict__ dbr) {
+                           const uint8_t *__restrict__ m_br, float *__restrict__ dbw, float *__restrict__ dbr, int accumulate) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x, C = 3 * H;
     if (c >= 2 * C) return;
     float s = 0.f;
     for (int g = 0; g < G; ++g) s += part[(size_t)g * 2 * C + c];
-    if (c < C) dbw[c] += m_bw ? s * (float)m_bw[c] : s;
-    else dbr[c - C] += m_br ? s * (float)m_br[c - C] : s;
+    const bool x_side = c < C;
+    const int k = x_side ? c : c - C;
+    const uint8_t *mask = x_side ? m_bw : m_br;
+    float *out = x_side ? dbw : dbr;
+    if (!out) return;
+    if (mask) s *= (float)mask[k];
+    out[k] = accumulate ? out[k] + s : s;
 }
 
 }  // namespace
+
+namespace qgru {
+
+void bwd_bias_launch(qgru_handle *h, const float *part, int G, const uint8_t *m_bw, const uint8_t *m_br, float *dbw, float *dbr, int accumulate,
+                     cudaStream_t st) {
+    k_bwd_bias<<<(2 * h->C + 127) / 128, 128, 0, st>>>(part, G, h->H, m_bw, m_br, dbw, dbr, accumulate);
+    h->launches++;
+}
+
+}  // namespace qgru
 
 extern "C" {
 
@@ -155,10 +170,9 @@ int qgru_backward(qgru_handle *h, int T, int B, const float *W_t, const float *R
     if (bwd_chain_fits(h, B, &G)) {
         if ((rc = ensure(h, h->bwd_bias, (size_t)G * 2 * C * sizeof(float)))) return rc;
         float *part = (float *)h->bwd_bias.p;
-        if ((rc = bwd_chain_launch(h, BwdChainArgs{T, B, H, R_t, 1, h_all, v, dh_new, dh, pm, dp, dq, part}, st)))
+        if ((rc = bwd_chain_launch(h, BwdChainArgs{T, B, H, R_t, 1, 0, 0, h_all, v, dh_new + NH, (long long)NH, H, dh, dh, m.h0, pm, dp, dq, part}, st)))
             return rc;
-        k_bwd_bias<<<(2 * C + 127) / 128, 128, 0, st>>>(part, G, H, m.bw, m.br, dbw, dbr);
-        h->launches++;
+        bwd_bias_launch(h, part, G, m.bw, m.br, dbw, dbr, 1, st);
     } else {
         // wide layers, step by step: the pointwise part, then dh[b][k] += sum_m dq[b][m] * R_t[m][k]
         const dim3 pw_grid((H + 255) / 256, B);
@@ -173,7 +187,8 @@ int qgru_backward(qgru_handle *h, int T, int B, const float *W_t, const float *R
         k_bwd_colsum<<<(C + 31) / 32, 256, 0, st>>>(dq, N, C, m.br, dbr);
         if (m.ih_linear)
             k_bwd_apply_mask<<<grid_for(N * C, 256, h->sm_count), 256, 0, st>>>(dp, m.ih_linear, N * C);
-        h->launches += T + 2 + (m.ih_linear ? 1 : 0);
+        if (m.h0) k_bwd_apply_mask<<<grid_for((long long)NH, 256, h->sm_count), 256, 0, st>>>(dh, m.h0, (long long)NH);
+        h->launches += T + 2 + (m.ih_linear ? 1 : 0) + (m.h0 ? 1 : 0);
     }
     // dx[n][i] = sum_m dp[n][m] * W_t[m][i]
     if ((rc = gemm_f32(h, GemmF32{dp, false, W_t, false, dx, N, C, I, false, m.x}, st))) return rc;
@@ -181,10 +196,6 @@ int qgru_backward(qgru_handle *h, int T, int B, const float *W_t, const float *R
     if ((rc = gemm_f32(h, GemmF32{h_all, true, dq, false, dR, H, N, C, true, m.R}, st))) return rc;
     // dW[i][m] += sum_n x_t[i][n] * dp[n][m]
     if ((rc = gemm_f32(h, GemmF32{x_t, false, dp, false, dW, I, N, C, true, m.W}, st))) return rc;
-    if (m.h0) {
-        k_bwd_apply_mask<<<grid_for((long long)NH, 256, h->sm_count), 256, 0, st>>>(dh, m.h0, (long long)NH);
-        h->launches++;
-    }
     CK(cudaGetLastError());
     return QGRU_OK;
 }

@@ -106,34 +106,39 @@ __device__ __forceinline__ int32_t gru_cell(const GateConsts &gc, const int32_t 
     return clampi(h_new, gc.h_lo, gc.h_hi);
 }
 
-// piecewise_linear in the training branch (include/quantize_ops_helper.h:760-783): always the
-// segment evaluation, and the two clamp flags (1 = inside the range) are kept.
-__device__ __forceinline__ int32_t activation_keep(const GateConsts &gc, int which, int32_t pre,
-                                                   uint8_t &keep_in, uint8_t &keep_out) {
+// piecewise_linear in the training branch (include/quantize_ops_helper.h:760-783): the two clamp flags
+// (1 = inside the range) are kept.  ttab: null, or a table over the whole clamped input range
+// (offsets as `tables` of gru_cell) of 2 * output + keep_out.
+__device__ __forceinline__ int32_t activation_keep(const GateConsts &gc, const int32_t *ttab, int which, int32_t pre,
+                                                   uint32_t &keep) {
     const int32_t q = clampi(pre, gc.in_lo[which], gc.in_hi[which]);
-    keep_in = q == pre;
+    keep |= (uint32_t)(q == pre) << (PM_IN + which);
+    if (ttab && gc.table_size[which] > 0) {
+        const int32_t e = ttab[gc.table_off[which] + (q - gc.in_lo[which])];
+        keep |= (uint32_t)(e & 1) << (PM_OUT + which);
+        return e >> 1;
+    }
     const int32_t raw = lut_raw(gc.lut[which], q);
     const int32_t out = clampi(raw, gc.out_lo[which], gc.out_hi[which]);
-    keep_out = out == raw;
+    keep |= (uint32_t)(out == raw) << (PM_OUT + which);
     return out;
 }
 
-// gru_cell in training mode: the gate outputs and the seven clamp flags of one cell
-// (src/gru_forward_gpu_quant.cu:296-348).  keep[0..2] gate inputs z, r, n; keep[3..5] gate
-// outputs; keep[6] the new state.
-__device__ __forceinline__ int32_t gru_cell_train(const GateConsts &gc, int32_t ih_z, int32_t ih_r,
+// gru_cell in training mode: the gate outputs and the clamp flags of one cell
+// (src/gru_forward_gpu_quant.cu:296-348), PM_IN, PM_OUT and PM_H bits added to `keep`.
+__device__ __forceinline__ int32_t gru_cell_train(const GateConsts &gc, const int32_t *ttab, int32_t ih_z, int32_t ih_r,
                                                   int32_t ih_n, int32_t hh_z, int32_t hh_r, int32_t hh_n,
-                                                  int32_t h_old, int32_t *gates, uint8_t *keep) {
+                                                  int32_t h_old, int32_t *gates, uint32_t &keep) {
     const int32_t z_pre = rescale_diff<false>(ih_z, gc.zp_ih, gc.ih_to[ACT_Z]) +
                           rescale_diff<false>(hh_z, gc.zp_hh, gc.hh_to[ACT_Z]) + gc.zp_in[ACT_Z];
-    const int32_t z = activation_keep(gc, ACT_Z, z_pre, keep[0], keep[3]);
+    const int32_t z = activation_keep(gc, ttab, ACT_Z, z_pre, keep);
     const int32_t r_pre = rescale_diff<false>(ih_r, gc.zp_ih, gc.ih_to[ACT_R]) +
                           rescale_diff<false>(hh_r, gc.zp_hh, gc.hh_to[ACT_R]) + gc.zp_in[ACT_R];
-    const int32_t r = activation_keep(gc, ACT_R, r_pre, keep[1], keep[4]);
+    const int32_t r = activation_keep(gc, ttab, ACT_R, r_pre, keep);
     const int64_t r_hh = ((int64_t)r - gc.zp_out[ACT_R]) * ((int64_t)hh_n - gc.zp_hh);
     const int32_t n_pre = rescale_diff<false>(ih_n, gc.zp_ih, gc.ih_to[ACT_N]) +
                           (int32_t)rescale64(r_hh, gc.rh_to_n) + gc.zp_in[ACT_N];
-    const int32_t n = activation_keep(gc, ACT_N, n_pre, keep[2], keep[5]);
+    const int32_t n = activation_keep(gc, ttab, ACT_N, n_pre, keep);
     const int32_t n_h = rescale_diff<false>(n, gc.zp_out[ACT_N], gc.n_to_h) + gc.zp_h;
     const int64_t z_d = (int64_t)z - gc.zp_out[ACT_Z];
     const int64_t old_c = z_d * ((int64_t)h_old - gc.zp_h);
@@ -144,7 +149,7 @@ __device__ __forceinline__ int32_t gru_cell_train(const GateConsts &gc, int32_t 
     gates[1] = r;
     gates[2] = n;
     const int32_t h_c = clampi(h_new, gc.h_lo, gc.h_hi);
-    keep[6] = h_c == h_new;
+    keep |= (uint32_t)(h_c == h_new) << PM_H;
     return h_c;
 }
 
@@ -232,11 +237,14 @@ __device__ __forceinline__ float fs_clamp(float v, float lo, float hi) { return 
 // sum_k W*x; off = float(sum_k W) * zp_in as computeWeightSumKernel leaves it (:442-458, one
 // rounded product); bias_term = round(bias * inv_bias).  Sub, add and multiply are kept as
 // separate roundings, as in the reference's compiled kernel (none of them is an a*b+c there).
-__device__ __forceinline__ float fs_linear(int acc, float off, float bias_term, float inv_gemm,
-                                           float zp_out, float lo, float hi) {
+__device__ __forceinline__ float fs_linear_raw(int acc, float off, float bias_term, float inv_gemm, float zp_out) {
     const float val = __fsub_rn((float)acc, off);
     const float combined = __fadd_rn(val, bias_term);
-    return fs_clamp(rintf(__fmul_rn(combined, inv_gemm)) + zp_out, lo, hi);
+    return rintf(__fmul_rn(combined, inv_gemm)) + zp_out;
+}
+__device__ __forceinline__ float fs_linear(int acc, float off, float bias_term, float inv_gemm,
+                                           float zp_out, float lo, float hi) {
+    return fs_clamp(fs_linear_raw(acc, off, bias_term, inv_gemm, zp_out), lo, hi);
 }
 __device__ __forceinline__ float fs_offset(int wsum, float zp_in) { return __fmul_rn((float)wsum, zp_in); }
 __device__ __forceinline__ float fs_bias_term(int bias_q, float inv_bias) {
@@ -250,10 +258,13 @@ __device__ __forceinline__ float fs_sigmoid(float x) { return 1.0f / (1.0f + exp
 // ih / hh are the requantized, clamped linear outputs, h_old the quantized previous state.
 // The activation half of a gate: real_sigmoid_f / real_tanh_f (include/quantize_ops_helper.h:
 // 687-720) on a clamped gate input; g = 0 update, 1 reset (sigmoid), 2 new (tanh).
-__device__ __forceinline__ float fs_activation(const FsConsts &fc, int g, float in) {
+__device__ __forceinline__ float fs_activation_raw(const FsConsts &fc, int g, float in) {
     const float x = (in - fc.zp_in[g]) * fc.s_in[g];
     const float y = g == 2 ? tanhf(x) : fs_sigmoid(x);
-    return fs_clamp(rintf(y / fc.s_out[g] + fc.zp_out[g]), fc.out_lo[g], fc.out_hi[g]);
+    return rintf(y / fc.s_out[g] + fc.zp_out[g]);
+}
+__device__ __forceinline__ float fs_activation(const FsConsts &fc, int g, float in) {
+    return fs_clamp(fs_activation_raw(fc, g, in), fc.out_lo[g], fc.out_hi[g]);
 }
 // The same through the table (tab: shared-window address of the float table), or directly.
 __device__ __forceinline__ float fs_activation_tab(const FsConsts &fc, uint32_t tab, int g, float in) {
@@ -298,6 +309,47 @@ __device__ __forceinline__ float fs_cell(const FsConsts &fc, const float ih[3], 
     const float u = fs_sigmoid_gate(fc, 0, ih[0], hh[0]);
     const float r = fs_sigmoid_gate(fc, 1, ih[1], hh[1]);
     return fs_finish(fc, u, r, ih[2], hh[2], h_old);
+}
+
+// The cell in training mode (PointwiseOperationsFP<true, false>, src/gru_forward_gpu_quant_fp.cu:572-770):
+// ih, hh requantized but not clamped yet; q: the four values of v (update, reset, new gate outputs, R*h + br of the
+// new gate); keep: PM_* bits, 1 = inside the range before the clamp (clamp_f<true>,
+// include/quantize_ops_helper.h:416-431).  tab: shared-window address of a table whose entries carry "clamped" in
+// the lowest mantissa bit (whole numbers of at most 17 bits: free), or tab_on = 0.
+__device__ __forceinline__ float fs_clamp_keep(float v, float lo, float hi, uint32_t &keep, int bit) {
+    keep |= (uint32_t)(!(v < lo || v > hi)) << bit;
+    return fs_clamp(v, lo, hi);
+}
+__device__ __forceinline__ float fs_activation_keep(const FsConsts &fc, int tab_on, uint32_t tab, int g, float in, uint32_t &keep) {
+    if (tab_on) {
+        const uint32_t e = (uint32_t)lds_i32(tab + 4u * (uint32_t)(fc.tab_off[g] + (int)(in - fc.in_lo[g])));
+        keep |= (~e & 1u) << (PM_OUT + g);
+        return __uint_as_float(e & ~1u);
+    }
+    return fs_clamp_keep(fs_activation_raw(fc, g, in), fc.out_lo[g], fc.out_hi[g], keep, PM_OUT + g);
+}
+__device__ __forceinline__ float fs_cell_train(const FsConsts &fc, int tab_on, uint32_t tab, const float (&ih_raw)[3], const float (&hh_raw)[3],
+                                               float h_old, float (&q)[4], uint32_t &keep) {
+    float ih[3], hh[3];
+#pragma unroll
+    for (int g = 0; g < 3; ++g) {
+        ih[g] = fs_clamp_keep(ih_raw[g], fc.ih_lo, fc.ih_hi, keep, PM_IH + g);
+        hh[g] = fs_clamp_keep(hh_raw[g], fc.hh_lo, fc.hh_hi, keep, PM_HH + g);
+    }
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+        const float a = rintf((ih[g] - fc.zp_ih) * fc.ih_to[g]);
+        const float c = rintf((hh[g] - fc.zp_hh) * fc.hh_to[g]);
+        q[g] = fs_activation_keep(fc, tab_on, tab, g, fs_clamp_keep(a + c + fc.zp_in[g], fc.in_lo[g], fc.in_hi[g], keep, PM_IN + g), keep);
+    }
+    const float rh = rintf(((q[1] - fc.zp_out[1]) * (hh[2] - fc.zp_hh)) * fc.rh_to_n);
+    const float a_n = rintf((ih[2] - fc.zp_ih) * fc.ih_to[2]);
+    q[2] = fs_activation_keep(fc, tab_on, tab, 2, fs_clamp_keep(a_n + rh + fc.zp_in[2], fc.in_lo[2], fc.in_hi[2], keep, PM_IN + 2), keep);
+    q[3] = hh[2];
+    const float n_h = rintf((q[2] - fc.zp_out[2]) * fc.n_to_h) + fc.zp_h;
+    const float old_c = (q[0] - fc.zp_out[0]) * (h_old - fc.zp_h);
+    const float new_c = ((fc.one_q - q[0]) - fc.zp_out[0]) * (n_h - fc.zp_h);
+    return fs_clamp_keep(rintf((old_c + new_c) * fc.uh_to_h) + fc.zp_h, fc.h_lo, fc.h_hi, keep, PM_H);
 }
 
 // One new state to the outputs of OutView.

@@ -172,7 +172,7 @@ int float_forward(qgru_handle *h, int T, int B, const float *W, const float *R, 
     h->launches++;
     if ((rc = gemm_f32(h, GemmF32{x, false, W, false, wx, N, I, Cn}, st))) return rc;
     if (float_chain_fits(h, B))
-        return float_chain_launch(h, FloatFwdArgs{T, B, H, R, wx, bw, br, h_out, v_out, v_stride}, st);
+        return float_chain_launch(h, FloatFwdArgs{T, B, H, R, wx, bw, br, h_out, v_out, v_stride, 0, 0, OutView()}, st);
     // wide layers, step by step: R*h as a tiled product, then the pointwise gates
     if ((rc = ensure(h, h->f_acc2, (size_t)B * Cn * 4))) return rc;
     float *rh = (float *)h->f_acc2.p;

@@ -53,6 +53,17 @@ __global__ void k_fs_tables(FsConsts fc, float *__restrict__ tab) {
         tab[fc.tab_off[g] + i] = fs_activation(fc, g, fc.in_lo[g] + (float)i);
 }
 
+// The same for fs_cell_train: the lowest bit says that the clamp changed the value.
+__global__ void k_fs_train_tables(FsConsts fc, uint32_t *__restrict__ tab) {
+    const int g = blockIdx.x;
+    const int n = (int)(fc.in_hi[g] - fc.in_lo[g]) + 1;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        uint32_t keep = 0;
+        const float y = fs_clamp_keep(fs_activation_raw(fc, g, fc.in_lo[g] + (float)i), fc.out_lo[g], fc.out_hi[g], keep, 0);
+        tab[fc.tab_off[g] + i] = __float_as_uint(y) | (keep ^ 1u);
+    }
+}
+
 // PointwiseOperationsFP<false, false> (src/gru_forward_gpu_quant_fp.cu:572-770) as its own launch:
 // one thread per (hidden unit, batch row).  Used where the persistent kernel below has no plan.
 template <typename IhT>
@@ -80,32 +91,7 @@ __global__ void k_fs_cell(const IhT *__restrict__ ih_q, const int32_t *__restric
 }
 
 // ---- training mode (quantGRUForwardFP with is_training): the per-step kernel also keeps the gate
-// buffer v and the clamp masks, 1 = the value was inside its range before the clamp
-// (clamp_f<true>, include/quantize_ops_helper.h:416-431).
-
-// Dequantization constants of the four slots of v (dequantificationVFPInplace,
-// src/quantize_ops.cu:368-397): update, reset, new gate outputs, R*h + br row of the new gate.
-struct FsTrainConsts {
-    float scale[4], zp[4];
-};
-
-__device__ __forceinline__ float fs_clamp_keep(float v, float lo, float hi, uint8_t &keep) {
-    keep = (v < lo || v > hi) ? 0 : 1;
-    return fs_clamp(v, lo, hi);
-}
-// biasRescaleInline<true>
-__device__ __forceinline__ float fs_linear_keep(int acc, float off, float bias_term, float inv_gemm,
-                                                float zp_out, float lo, float hi, uint8_t &keep) {
-    const float val = __fsub_rn((float)acc, off);
-    const float combined = __fadd_rn(val, bias_term);
-    return fs_clamp_keep(rintf(__fmul_rn(combined, inv_gemm)) + zp_out, lo, hi, keep);
-}
-// real_sigmoid_f<true> / real_tanh_f<true> on an already clamped gate input
-__device__ __forceinline__ float fs_activation_keep(const FsConsts &fc, int g, float in, uint8_t &keep) {
-    const float x = (in - fc.zp_in[g]) * fc.s_in[g];
-    const float y = g == 2 ? tanhf(x) : fs_sigmoid(x);
-    return fs_clamp_keep(rintf(y / fc.s_out[g] + fc.zp_out[g]), fc.out_lo[g], fc.out_hi[g], keep);
-}
+// buffer v and the clamp masks.
 
 // PointwiseOperationsFP<true, false> (src/gru_forward_gpu_quant_fp.cu:572-770) for one timestep.
 // ih_acc / hh_acc: exact sums of W*x and R*h; masks point at this step's rows, any may be null.
@@ -120,49 +106,28 @@ __global__ void k_fs_cell_train(const int32_t *__restrict__ ih_acc, const int32_
     if (j >= H || b >= B) return;
     const int C = 3 * H;
     const size_t w = (size_t)b * C + j;
-    float ih[3], hh[3];
-    uint8_t k_ih[3], k_hh[3], k_in[3], k_out[3], k_h;
+    float ih[3], hh[3], q[4];
+    uint32_t keep = 0;
 #pragma unroll
     for (int g = 0; g < 3; ++g) {
         const int m = j + g * H;
-        ih[g] = fs_linear_keep(ih_acc[w + g * H], chan[m], chan[C + m], chan[2 * C + m], fc.zp_ih, fc.ih_lo,
-                               fc.ih_hi, k_ih[g]);
-        hh[g] = fs_linear_keep(hh_acc[w + g * H], chan[3 * C + m], chan[4 * C + m], chan[5 * C + m], fc.zp_hh,
-                               fc.hh_lo, fc.hh_hi, k_hh[g]);
+        ih[g] = fs_linear_raw(ih_acc[w + g * H], chan[m], chan[C + m], chan[2 * C + m], fc.zp_ih);
+        hh[g] = fs_linear_raw(hh_acc[w + g * H], chan[3 * C + m], chan[4 * C + m], chan[5 * C + m], fc.zp_hh);
     }
-    float gate[2];
-#pragma unroll
-    for (int g = 0; g < 2; ++g) {
-        const float a = rintf((ih[g] - fc.zp_ih) * fc.ih_to[g]);
-        const float c = rintf((hh[g] - fc.zp_hh) * fc.hh_to[g]);
-        const float in = fs_clamp_keep(a + c + fc.zp_in[g], fc.in_lo[g], fc.in_hi[g], k_in[g]);
-        gate[g] = fs_activation_keep(fc, g, in, k_out[g]);
-    }
-    const float u = gate[0], r = gate[1];
-    const float rh = rintf(((r - fc.zp_out[1]) * (hh[2] - fc.zp_hh)) * fc.rh_to_n);
-    const float a_n = rintf((ih[2] - fc.zp_ih) * fc.ih_to[2]);
-    const float in_n = fs_clamp_keep(a_n + rh + fc.zp_in[2], fc.in_lo[2], fc.in_hi[2], k_in[2]);
-    const float n = fs_activation_keep(fc, 2, in_n, k_out[2]);
-    const float h_old = (float)state_byte(h8_in[(size_t)b * Hpad + j], fc.h_bits);
-    const float n_h = rintf((n - fc.zp_out[2]) * fc.n_to_h) + fc.zp_h;
-    const float old_c = (u - fc.zp_out[0]) * (h_old - fc.zp_h);
-    const float new_c = ((fc.one_q - u) - fc.zp_out[0]) * (n_h - fc.zp_h);
-    const float h_new = fs_clamp_keep(rintf((old_c + new_c) * fc.uh_to_h) + fc.zp_h, fc.h_lo, fc.h_hi, k_h);
+    const float h_new = fs_cell_train(fc, 0, 0, ih, hh, (float)state_byte(h8_in[(size_t)b * Hpad + j], fc.h_bits), q, keep);
     h8_out[(size_t)b * Hpad + j] = (uint8_t)(int)h_new;
     h_out[(size_t)b * H + j] = (h_new - fc.zp_h) * fc.h_scale;
     float *vb = v + (size_t)b * 4 * H + j;
-    vb[0] = (u - tc.zp[0]) * tc.scale[0];
-    vb[H] = (r - tc.zp[1]) * tc.scale[1];
-    vb[2 * H] = (n - tc.zp[2]) * tc.scale[2];
-    vb[3 * H] = (hh[2] - tc.zp[3]) * tc.scale[3];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) vb[k * H] = (q[k] - tc.zp[k]) * tc.scale[k];
 #pragma unroll
     for (int g = 0; g < 3; ++g) {
-        if (m_ih) m_ih[w + g * H] = k_ih[g];
-        if (m_hh) m_hh[w + g * H] = k_hh[g];
-        if (m_gin) m_gin[w + g * H] = k_in[g];
-        if (m_gout) m_gout[w + g * H] = k_out[g];
+        if (m_ih) m_ih[w + g * H] = keep >> (PM_IH + g) & 1;
+        if (m_hh) m_hh[w + g * H] = keep >> (PM_HH + g) & 1;
+        if (m_gin) m_gin[w + g * H] = keep >> (PM_IN + g) & 1;
+        if (m_gout) m_gout[w + g * H] = keep >> (PM_OUT + g) & 1;
     }
-    if (m_h) m_h[(size_t)b * H + j] = k_h;
+    if (m_h) m_h[(size_t)b * H + j] = keep >> PM_H & 1;
 }
 
 // Clamp masks of the weight quantization (quantificationPerChannelFP<true>, src/quantize_ops.cu:
@@ -414,20 +379,25 @@ int fstorage_train_tail(qgru_handle *h, int T, int B, FwdInput in, float *h_out,
     return QGRU_OK;
 }
 
-// Host side of quantGRUForwardFP; `in`, `out`, with_slot0, x8_shared, after_prologue as in forward_dir.  Training
-// mode (`train`) writes the dense slots at out.hf.
-int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const OutView &out, bool with_slot0, unsigned flags,
-                     cudaStream_t st, const uint8_t *x8_shared = nullptr, cudaEvent_t after_prologue = nullptr,
-                     const FsTrainArgs *train = nullptr) {
-    if (!h->fast)
-        return fail(h, QGRU_ERR_UNSUPPORTED,
-                    "float-storage forward needs 8-bit W, R, x and h (the operands of the two products)");
+// Constants of the float-storage cell, and on the device (once per parameter set) what the channels and the gate
+// tables need: fs_ch holds 4 x C scale ratios from the host, 6 x C per-channel constants that also depend on the
+// weights (chan: k_fs_channel_consts, k_train_weights), the gate tables, their training form.
+struct FsSetup {
+    FsConsts fc;
+    int n_tab = 0;              // entries of the gate tables, 0: gates are evaluated
+    int n_train_tab = 0;        // the same for the training form (its outputs need the lowest mantissa bit free)
+    FsChannels ch;
+    float *chan, *gate_tab;
+    uint32_t *train_tab;
+};
+
+int fs_setup(qgru_handle *h, FsSetup &s, cudaStream_t st) {
     const qgru_params &p = h->p;
-    const int H = h->H, C = h->C;
-    const long long N = (long long)T * B;
+    const int C = h->C;
+    FsConsts &fc = s.fc;
     // ---- constants (setRescaleParam, src/gru_forward_gpu_quant_fp.cu:821-1003): float ratios
     // of the stored scales, computed in the same float operations
-    FsConsts fc{};
+    fc = FsConsts{};
     const qgru_op &ox = p.op[QGRU_OP_X], &oh = p.op[QGRU_OP_H], &oih = p.op[QGRU_OP_IH_LINEAR],
                   &ohh = p.op[QGRU_OP_HH_LINEAR];
     const int op_in[3] = {QGRU_OP_UPDATE_IN, QGRU_OP_RESET_IN, QGRU_OP_NEW_IN};
@@ -471,16 +441,18 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
         tab_total += n;
     }
     fc.tab_on = (tab_possible && h->opt_cell != 1) ? 1 : 0;
-    const int n_tab = fc.tab_on ? tab_total : 0;
-
+    s.n_tab = fc.tab_on ? tab_total : 0;
+    s.n_train_tab = s.n_tab;
+    for (int g = 0; g < 3; ++g)
+        if (p.op[op_out[g]].bits > 16) s.n_train_tab = 0;
     int rc;
-    // per-channel constants: 4 x C scale ratios from the host, then 6 x C derived on the device
-    // from the packed weights (column sums, quantized biases); then the gate tables
-    if ((rc = ensure(h, h->fs_ch, ((size_t)10 * C + 3 * 1024) * sizeof(float)))) return rc;
+    if ((rc = ensure(h, h->fs_ch, ((size_t)10 * C + 6 * 1024) * sizeof(float)))) return rc;
     float *chp = (float *)h->fs_ch.p;
-    float *chan = chp + (size_t)4 * C;
-    float *gate_tab = chp + (size_t)10 * C;
-    if (!h->fs_ready) {
+    s.ch = FsChannels{chp, chp + C, chp + 2 * C, chp + 3 * C};
+    s.chan = chp + (size_t)4 * C;
+    s.gate_tab = chp + (size_t)10 * C;
+    s.train_tab = reinterpret_cast<uint32_t *>(s.gate_tab + 3 * 1024);
+    if (!h->fs_uploaded) {
         std::vector<float> hostc((size_t)4 * C);
         for (int m = 0; m < C; ++m) {
             const float s_wx = h->sc[0][m] * ox.scale;
@@ -492,12 +464,39 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
         }
         CK(cudaMemcpyAsync(chp, hostc.data(), hostc.size() * sizeof(float), cudaMemcpyHostToDevice, st));
         CK(cudaStreamSynchronize(st));   // hostc leaves scope
-        const FsChannels ch{chp, chp + C, chp + 2 * C, chp + 3 * C};
-        k_fs_channel_consts<<<(C + 127) / 128, 128, 0, st>>>(h->d_wsum[0], h->d_wsum[1], h->d_wq[2], h->d_wq[3], ch,
-                                                            fc.zp_x, fc.zp_h, chan, C);
-        if (tab_possible) k_fs_tables<<<3, 256, 0, st>>>(fc, gate_tab);
+        if (tab_possible) {
+            k_fs_tables<<<3, 256, 0, st>>>(fc, s.gate_tab);
+            k_fs_train_tables<<<3, 256, 0, st>>>(fc, s.train_tab);
+        }
         CK(cudaGetLastError());
         h->launches += 2;
+        h->fs_uploaded = true;
+    }
+    return QGRU_OK;
+}
+
+// Host side of quantGRUForwardFP; `in`, `out`, with_slot0, x8_shared, after_prologue as in forward_dir.  Training
+// mode (`train`) writes the dense slots at out.hf.
+int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const OutView &out, bool with_slot0, unsigned flags,
+                     cudaStream_t st, const uint8_t *x8_shared = nullptr, cudaEvent_t after_prologue = nullptr,
+                     const FsTrainArgs *train = nullptr) {
+    if (!h->fast)
+        return fail(h, QGRU_ERR_UNSUPPORTED,
+                    "float-storage forward needs 8-bit W, R, x and h (the operands of the two products)");
+    const qgru_params &p = h->p;
+    const int H = h->H, C = h->C;
+    const long long N = (long long)T * B;
+    int rc;
+    FsSetup su;
+    if ((rc = fs_setup(h, su, st))) return rc;
+    const FsConsts &fc = su.fc;
+    const int n_tab = su.n_tab;
+    float *chan = su.chan, *gate_tab = su.gate_tab;
+    if (!h->fs_ready) {
+        k_fs_channel_consts<<<(C + 127) / 128, 128, 0, st>>>(h->d_wsum[0], h->d_wsum[1], h->d_wq[2], h->d_wq[3], su.ch,
+                                                            fc.zp_x, fc.zp_h, chan, C);
+        CK(cudaGetLastError());
+        h->launches++;
         h->fs_ready = true;
     }
     if (train) return fstorage_train_tail(h, T, B, in, out.hf, flags, st, fc, chan, *train);
@@ -506,6 +505,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
     const uint8_t *x8 = x8_shared ? x8_shared : (const uint8_t *)h->x8.p;
     if ((rc = ensure(h, h->h8, (size_t)(2 * B + 256) * h->Hpad))) return rc;
     // W*x + bw requantized and clamped to the width of weight_ih_linear: one or two bytes
+    const qgru_op &oih = p.op[QGRU_OP_IH_LINEAR];
     const int ih_bytes = (oih.bits <= 8 && !oih.is_unsigned) ? 1 : 2;
     if (oih.bits > 16 || (oih.bits == 16 && oih.is_unsigned))
         return fail(h, QGRU_ERR_UNSUPPORTED, "float-storage forward stores W*x + bw in at most 16 signed bits");

@@ -143,8 +143,9 @@ k_gemm_f32(const float *__restrict__ A, const float *__restrict__ Bm, float *__r
                 if (c >= M) continue;
                 float y = v[e];
                 if (!split) {
-                    if (accumulate) y += out[n * M + c];
+                    if (accumulate == 1) y += out[n * M + c];
                     if (mask) y *= (float)mask[n * M + c];
+                    if (accumulate == 2) y += out[n * M + c];
                 }
                 out[n * M + c] = y;
             }
@@ -156,9 +157,10 @@ k_gemm_f32(const float *__restrict__ A, const float *__restrict__ Bm, float *__r
 __global__ void k_gemm_f32_join(const float *__restrict__ part, float *__restrict__ C, long long n, int parts, int accumulate,
                                 const uint8_t *__restrict__ mask) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        float y = accumulate ? C[i] : 0.f;
+        float y = accumulate == 1 ? C[i] : 0.f;
         for (int p = 0; p < parts; ++p) y += part[(size_t)p * n + i];
         if (mask) y *= (float)mask[i];
+        if (accumulate == 2) y += C[i];
         C[i] = y;
     }
 }
@@ -169,7 +171,7 @@ void launch(const GemmF32 &g, int parts, long long k_part, float *ws, bool va, b
     const int threads = (BT / 8) * (BT / 8);
     auto kern = va ? (vb ? k_gemm_f32<BT, AT, BTr, true, true> : k_gemm_f32<BT, AT, BTr, true, false>)
                    : (vb ? k_gemm_f32<BT, AT, BTr, false, true> : k_gemm_f32<BT, AT, BTr, false, false>);
-    kern<<<grid, threads, 0, st>>>(g.A, g.B, g.C, g.N, g.K, g.M, k_part, g.accumulate ? 1 : 0, g.mask, ws);
+    kern<<<grid, threads, 0, st>>>(g.A, g.B, g.C, g.N, g.K, g.M, k_part, g.accumulate, g.mask, ws);
 }
 
 template <int BT>
@@ -210,7 +212,7 @@ int gemm_f32(qgru_handle *h, const GemmF32 &g, cudaStream_t st) {
     h->launches++;
     if (parts > 1) {
         const long long n = g.N * g.M;
-        k_gemm_f32_join<<<grid_for(n, 256, h->sm_count), 256, 0, st>>>(ws, g.C, n, (int)parts, g.accumulate ? 1 : 0, g.mask);
+        k_gemm_f32_join<<<grid_for(n, 256, h->sm_count), 256, 0, st>>>(ws, g.C, n, (int)parts, g.accumulate, g.mask);
         h->launches++;
     }
     CK(cudaGetLastError());

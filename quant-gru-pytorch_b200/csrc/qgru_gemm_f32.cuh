@@ -18,7 +18,7 @@ struct GemmF32 {
     float *C;
     long long N, K;
     int M;
-    bool accumulate = false;
+    int accumulate = 0;              // 1: mask * (C + product), 2: C + mask * product
     const uint8_t *mask = nullptr;
 };
 int gemm_f32(qgru_handle *h, const GemmF32 &g, cudaStream_t st);

@@ -63,6 +63,8 @@ struct qgru_handle {
     GateConsts *d_gc = nullptr;
     int32_t *d_tables = nullptr;
     int n_table = 0;
+    int32_t *d_ttables = nullptr;  // tables with clamp flags (training cell), or n_ttable = 0
+    int n_ttable = 0;
     int32_t *d_ftables = nullptr;  // tables of the fused cell
     int n_ftable = 0;
     Rescale *d_rs[2] = {nullptr, nullptr};    // gemm rescale: x side, h side
@@ -92,7 +94,7 @@ struct qgru_handle {
     DevBuf f_split;                        // fp32 matrix product: partial tiles where K is split
     qgru::F32RecPlan plan_fwd, plan_bwd;   // fp32 recurrences: the plan of the last batch size
     DevBuf fs_ch;                          // float-storage forward: 4 x 3H per-channel scale ratios
-    bool fs_ready = false;                 // fs_ch matches the current parameters
+    bool fs_uploaded = false, fs_ready = false;   // fs_ch matches the current parameters; and the current weights
     static constexpr int kRing = 64;
     cudaEvent_t ring[kRing][4] = {};   // per forward: start, gemm start, gemm end, recurrence end
     cudaEvent_t *ev = ring[0];          // the slot the current forward records into
@@ -100,7 +102,7 @@ struct qgru_handle {
     bool timing_valid = false;
     uint64_t launches = 0;
     TcGemmState tc;
-    qgru::RecRegPlan plan_reg;   // register-resident recurrence: the plan of the last call
+    qgru::RecRegPlan plan_reg, plan_train;   // register-resident recurrence: the plan of the last call, of the last training forward
     qgru::RecMmaState rec;       // tensor maps of the global-exchange recurrence
     qgru::RecMmaState rec_cl;    // tensor maps of the cluster-exchange recurrence
     qgru::RecMmaState rec_c64;   // tensor maps of its 64-units-per-CTA form
@@ -149,6 +151,12 @@ inline int alloc_dev(qgru_handle *h, T **p, size_t n) {
         return QGRU_ERR_NOMEM;
     }
     return QGRU_OK;
+}
+
+// A buffer whose size depends on the layer's sizes alone.
+template <class T>
+inline int alloc_once(qgru_handle *h, T **p, size_t n) {
+    return *p ? QGRU_OK : alloc_dev(h, p, n);
 }
 
 inline int grid_for(long long n, int block, int sm_count) {

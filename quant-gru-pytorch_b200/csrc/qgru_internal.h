@@ -136,6 +136,16 @@ struct FsConsts {
     int tab_off[3];
 };
 
+// Clamp masks of a quantized training forward, one word per (timestep, row, unit): bit g (z, r, n)
+// W*x + bw, 3 + g R*h + br, 6 + g gate input, 9 + g gate output, 12 the new state; 1 = not clamped.
+constexpr int PM_IH = 0, PM_HH = 3, PM_IN = 6, PM_OUT = 9, PM_H = 12;
+
+// Dequantization constants of the four slots of v (dequantificationVFPInplace,
+// src/quantize_ops.cu:368-397): update, reset, new gate outputs, R*h + br row of the new gate.
+struct FsTrainConsts {
+    float scale[4], zp[4];
+};
+
 // Per output channel constants of one fused linear layer:
 //   out = clamp( int32( rescale( acc + corr[m], rs[m] ) ) + zp_out )
 // with corr[m] = rescale(bias_q[m], bias_rs[m]) - zp_in * sum_k W_q[k][m]

@@ -38,7 +38,8 @@ struct PrologueArgs {
     int B, K, Kpad;
     uint8_t *x8;
     void *xq;                    // optional dense copy of the quantized values: int32 (mode 0) or float (mode 1)
-    uint8_t *keep;               // optional mask, 1 = the value was not clamped (mode 1)
+    float *xd;                   // optional dense copy of what the quantized values stand for: (q - zp) * scale (modes 0, 1)
+    uint8_t *keep;               // optional mask, 1 = the value was not clamped (modes 0, 1)
     float x_scale;
     int32_t x_zp, x_lo, x_hi;
     const void *h0;              // [B][H] fp32 (modes 0, 1) or int32 (mode 2); null: the zero point
@@ -47,7 +48,7 @@ struct PrologueArgs {
     OutView slot;                // outputs of the initial slot (slot 0), each may be null
     float h_scale;
     int32_t h_zp, h_lo, h_hi;
-    uint8_t *h0_keep;            // optional mask of the initial state (mode 1)
+    uint8_t *h0_keep;            // optional mask of the initial state (modes 0, 1)
     int *flags;                  // [2]
     volatile int *sticky;        // mapped host word or null: do not clear the flags
     int q_blocks;                // blocks that quantize x; the rest write the state
@@ -58,7 +59,10 @@ __device__ __forceinline__ int32_t prologue_quantize(const void *src, long long 
                                                      uint8_t &keep, int *flags) {
     keep = 1;
     if constexpr (Mode == 0) {
-        return quantize_one(static_cast<const float *>(src)[i], scale, zp, lo, hi);
+        // (quantize_one with its flag: quantize<true>, include/quantize_ops_helper.h:528-533)
+        const int32_t q = (int32_t)(rintf(__fdiv_rn(static_cast<const float *>(src)[i], scale)) + (float)zp);
+        keep = (q < lo || q > hi) ? 0 : 1;
+        return clampi(q, lo, hi);
     } else if constexpr (Mode == 1) {
         const float raw = fs_quantize_raw(static_cast<const float *>(src)[i], scale, zp);
         keep = (raw < (float)lo || raw > (float)hi) ? 0 : 1;
@@ -109,7 +113,8 @@ __global__ void __launch_bounds__(256) k_prologue(const PrologueArgs a) {
                         if constexpr (Mode == 1) static_cast<float *>(a.xq)[row * a.K + k] = (float)q;
                         else static_cast<int32_t *>(a.xq)[row * a.K + k] = q;
                     }
-                    if (Mode == 1 && a.keep) a.keep[row * a.K + k] = keep;
+                    if (Mode != 2 && a.xd) a.xd[row * a.K + k] = (float)(q - a.x_zp) * a.x_scale;
+                    if (Mode != 2 && a.keep) a.keep[row * a.K + k] = keep;
                 }
             }
             reinterpret_cast<uint4 *>(a.x8)[i] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -789,17 +794,20 @@ __global__ void k_gates_train(const int32_t *__restrict__ ih, const int32_t *__r
     if (j >= H || b >= B) return;
     const size_t w = (size_t)b * 3 * H + j;
     int32_t gates[3];
-    uint8_t keep[7];
-    h_out[(size_t)b * H + j] = gru_cell_train(*gcp, ih[w], ih[w + H], ih[w + 2 * H], hh[w], hh[w + H],
+    uint32_t keep = 0;
+    h_out[(size_t)b * H + j] = gru_cell_train(*gcp, nullptr, ih[w], ih[w + H], ih[w + 2 * H], hh[w], hh[w + H],
                                               hh[w + 2 * H], h_in[(size_t)b * H + j], gates, keep);
     int32_t *vb = v + (size_t)b * 4 * H + j;
     vb[0] = gates[0];
     vb[H] = gates[1];
     vb[2 * H] = gates[2];
     vb[3 * H] = hh[w + 2 * H];
-    if (m_in) { m_in[w] = keep[0]; m_in[w + H] = keep[1]; m_in[w + 2 * H] = keep[2]; }
-    if (m_out) { m_out[w] = keep[3]; m_out[w + H] = keep[4]; m_out[w + 2 * H] = keep[5]; }
-    if (m_h) m_h[(size_t)b * H + j] = keep[6];
+#pragma unroll
+    for (int g = 0; g < 3; ++g) {
+        if (m_in) m_in[w + g * H] = keep >> (PM_IN + g) & 1;
+        if (m_out) m_out[w + g * H] = keep >> (PM_OUT + g) & 1;
+    }
+    if (m_h) m_h[(size_t)b * H + j] = keep >> PM_H & 1;
 }
 
 }  // namespace qgru

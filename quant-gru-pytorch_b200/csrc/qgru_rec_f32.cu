@@ -32,6 +32,9 @@ namespace {
 constexpr int MAX_ROWS = 40;                 // batch rows per cluster
 constexpr int RB = 8;                        // forward: rows between two block barriers
 
+// block of gate g (z, r, n) in weights, W*x and gradients
+__device__ __forceinline__ int gate_block(int torch, int g) { return torch && g < 2 ? 1 - g : g; }
+
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ float4 ld_remote4(uint32_t addr) {
     float4 v;
@@ -91,8 +94,9 @@ __global__ void __launch_bounds__(512, 1) k_float_chain(const FloatFwdArgs a) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int k = kg * 32 + 2 * i;
-                const float lo = (j < H && k < H) ? a.R[(size_t)k * C + g * H + j] : 0.f;
-                const float hi = (j < H && k + 1 < H) ? a.R[(size_t)(k + 1) * C + g * H + j] : 0.f;
+                const size_t at = a.torch ? ((size_t)gate_block(1, g) * H + j) * H + k : (size_t)k * C + g * H + j;
+                const float lo = (j < H && k < H) ? a.R[at] : 0.f;
+                const float hi = (j < H && k + 1 < H) ? a.R[at + (a.torch ? 1 : C)] : 0.f;
                 R2[g][i] = pack2(lo, hi);
             }
     }
@@ -101,26 +105,34 @@ __global__ void __launch_bounds__(512, 1) k_float_chain(const FloatFwdArgs a) {
     const bool j_ok = cj < H;
     for (int i = tid; i < 6 * U; i += NT) {
         const int g = i / U, j = p * U + i % U;
-        bias[i] = j < H ? (g < 3 ? a.bw[g * H + j] : a.br[(g - 3) * H + j]) : 0.f;
+        const float *src = g < 3 ? a.bw : a.br;
+        bias[i] = j < H && src ? src[gate_block(a.torch, g % 3) * H + j] : 0.f;
     }
     // the initial state
+    const float *h_init = a.h + (a.reverse ? (size_t)a.T * a.B * H : 0);
     if (P == 1) {
         for (int i = tid; i < 2 * Bt * PU; i += NT) {
             const int b = i / PU, j = i % PU;
-            hs[i] = (b < nb && j < H) ? a.h[(size_t)(b0 + b) * H + j] : 0.f;
+            hs[i] = (b < nb && j < H) ? h_init[(size_t)(b0 + b) * H + j] : 0.f;
         }
     } else {
         for (int i = tid; i < 2 * BtU; i += NT) {
             const int b = i / U, j = p * U + i % U;
-            own[i] = (b < nb && j < H) ? a.h[(size_t)(b0 + b) * H + j] : 0.f;
+            own[i] = (b < nb && j < H) ? h_init[(size_t)(b0 + b) * H + j] : 0.f;
         }
     }
     // running pointers of this thread's unit: one add per step instead of 64-bit products per access
-    const float *wx_next = a.wx + (size_t)b0 * C + cj;
-    float *h_out = a.h + (size_t)(a.B + b0) * H + cj;
     const int vs = a.v_stride * H;
-    float *v_out = a.v ? a.v + (size_t)b0 * vs + cj : nullptr;
-    const size_t wx_step = (size_t)a.B * C, h_step = (size_t)a.B * H, v_step = (size_t)a.B * vs;
+    const long long dir = a.reverse ? -1 : 1;
+    const size_t row0 = (size_t)(a.reverse ? a.T - 1 : 0) * a.B + b0;      // first row of the first step
+    const float *wx_next = a.wx + row0 * C + cj;
+    float *h_out = a.h + (row0 + (a.reverse ? 0 : a.B)) * H + cj;
+    float *v_out = a.v ? a.v + row0 * vs + cj : nullptr;
+    float *u_out = a.out.hf ? a.out.hf + (size_t)(a.reverse ? a.T - 1 : 1) * a.out.ts + (size_t)b0 * a.out.bs + cj : nullptr;
+    const long long wx_step = dir * a.B * C, h_step = dir * a.B * H, v_step = dir * a.B * vs, u_step = dir * (long long)a.out.ts;
+    int g_off[3];
+#pragma unroll
+    for (int g = 0; g < 3; ++g) g_off[g] = gate_block(a.torch, g) * H;
     int slot_in = 0, fetched = 0;
     auto fetch_wx = [&]() {   // each thread fetches what its own cells will read
         if (fetched < a.T && j_ok) {
@@ -129,7 +141,7 @@ __global__ void __launch_bounds__(512, 1) k_float_chain(const FloatFwdArgs a) {
                 for (int b = r0 + cb; b < min(nb, r0 + RB); b += KG) {
                     const float *src = wx_next + b * C;
 #pragma unroll
-                    for (int g = 0; g < 3; ++g) cp_async4(dst + (b * 3 + g) * U, src + g * H);
+                    for (int g = 0; g < 3; ++g) cp_async4(dst + (b * 3 + g) * U, src + g_off[g]);
                 }
         }
         wx_next += wx_step;
@@ -260,7 +272,10 @@ __global__ void __launch_bounds__(512, 1) k_float_chain(const FloatFwdArgs a) {
         if (j_ok)
             for (int r0 = 0; r0 < nb; r0 += RB)
                 for (int c = r0 + cb; c < min(nb, r0 + RB); c += KG) {
-                    h_out[c * H] = next[c * U];
+                    const float hn = next[c * U];
+                    h_out[c * H] = hn;
+                    if (u_out) u_out[(size_t)c * a.out.bs] = hn;
+                    if (s + 1 == a.T && a.out.hn_f) a.out.hn_f[(size_t)(b0 + c) * H + cj] = hn;
                     if (v_out) {
                         const float *t = vst + c * U + cu;
                         float *vb = v_out + c * vs;
@@ -274,6 +289,7 @@ __global__ void __launch_bounds__(512, 1) k_float_chain(const FloatFwdArgs a) {
                 }
         h_out += h_step;
         if (v_out) v_out += v_step;
+        if (u_out) u_out += u_step;
         slot = slot + 1 == D ? 0 : slot + 1;
         fetch_wx();
         if (P > 1) cluster_wait();
@@ -316,7 +332,7 @@ __global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
                 const int m = in0 + 2 * i + e, g = m / U, j = p * U + m % U;
-                w[e] = (k < H && j < H) ? (a.r_trans ? a.R[((size_t)g * H + j) * H + k] : a.R[(size_t)k * C + (size_t)g * H + j]) : 0.f;
+                w[e] = (k < H && j < H) ? (a.r_trans ? a.R[((size_t)gate_block(a.torch, g) * H + j) * H + k] : a.R[(size_t)k * C + (size_t)g * H + j]) : 0.f;
             }
             R2[o][i] = pack2(w[0], w[1]);
         }
@@ -329,11 +345,15 @@ __global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
     for (int k = 0; k < 6; ++k) bsum[k * NT + tid] = 0.f;
     // Running pointers, last step first.  The cell's operands of a step, each thread its own: v (4), dh_new,
     // h_{t-1}, the 32-bit word that holds the cell's 16 mask bits.
-    const size_t BH = (size_t)a.B * H;
-    const size_t last = (size_t)(a.T - 1) * a.B + b0;      // first row of the last step
-    const float *v_in = a.v + last * 4 * H + cj, *dn_in = a.dh_new + (last + a.B) * H + cj, *h_in = a.h + last * H + cj;
+    const long long dir = a.reverse ? 1 : -1, BH = dir * a.B * H;
+    const size_t t_last = a.reverse ? 0 : a.T - 1, last = t_last * a.B + b0;      // first row of the last step
+    const float *v_in = a.v + last * 4 * H + cj, *dn_in = a.dh_new + (long long)t_last * a.dn_ts + b0 * a.dn_bs + cj,
+                *h_in = a.h + (last + (a.reverse ? a.B : 0)) * H + cj;
     size_t m_at = last * H + cj;
     float *dp_out = a.dp + last * C + cj, *dq_out = a.dq + last * C + cj;
+    int g_off[3];
+#pragma unroll
+    for (int g = 0; g < 3; ++g) g_off[g] = gate_block(a.torch, g) * H;
     int slot_in = 0, left = a.T;
     auto fetch = [&]() {
         if (left > 0 && j_ok) {
@@ -343,15 +363,15 @@ __global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
                 const float *vb = v_in + b * 4 * H;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) cp_async4(d + k * BtU, vb + k * H);
-                cp_async4(d + 4 * BtU, dn_in + b * H);
+                cp_async4(d + 4 * BtU, dn_in + b * a.dn_bs);
                 cp_async4(d + 5 * BtU, h_in + b * H);
                 if (a.pm) cp_async4(d + 6 * BtU, reinterpret_cast<const float *>(a.pm + ((m_at + b * H) & ~(size_t)1)));
             }
         }
-        v_in -= 4 * BH;
-        dn_in -= BH;
-        h_in -= BH;
-        m_at -= BH;
+        v_in += 4 * BH;
+        dn_in += dir * a.dn_ts;
+        h_in += BH;
+        m_at += BH;
         --left;
         slot_in = slot_in + 1 == D ? 0 : slot_in + 1;
         cp_async_commit();
@@ -381,7 +401,7 @@ __global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
         return s;
     };
     int slot = 0;
-    if (P == 1) __syncthreads();
+    __syncthreads();                                        // the zeros of dqs and dps are complete
 
     for (int i = a.T - 1; i >= 0; --i) {
         const int buf = i & 1;
@@ -391,7 +411,7 @@ __global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
                 const int at = b * U + cu;
                 const float *d = stage + slot * 7 * BtU + at;
                 const float z = d[0], r = d[BtU], g = d[2 * BtU], q_g = d[3 * BtU], h_old = d[5 * BtU];
-                const float in = i == a.T - 1 ? a.dh[(size_t)(b0 + b) * H + cj] : carry(buf ^ 1, b);
+                const float in = i == a.T - 1 ? (a.dh_in ? a.dh_in[(size_t)(b0 + b) * H + cj] : 0.f) : carry(buf ^ 1, b);
                 uint32_t m = 0xffffffffu;
                 if (a.pm) m = __float_as_uint(d[6 * BtU]) >> (((m_par + b * H) & 1) * 16);
                 float dh = d[4 * BtU] + in;
@@ -458,26 +478,30 @@ __global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
                 const float *dpb = dps + b * 3 * U + cu, *dqb = dqs + b * 3 * U + cu;
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
-                    dp_out[b * C + k * H] = dpb[k * U];
-                    dq_out[b * C + k * H] = dqb[k * U];
+                    dp_out[b * C + g_off[k]] = dpb[k * U];
+                    dq_out[b * C + g_off[k]] = dqb[k * U];
                 }
             }
-        dp_out -= 3 * BH;
-        dq_out -= 3 * BH;
-        m_par -= BH;
+        dp_out += 3 * BH;
+        dq_out += 3 * BH;
+        m_par += BH;
         slot = slot + 1 == D ? 0 : slot + 1;
         fetch();
         if (P > 1) cluster_wait();
     }
     if (j_ok)
-        for (int b = cb; b < nb; b += KG) a.dh[(size_t)(b0 + b) * H + cj] = carry(0, b);
+        for (int b = cb; b < nb; b += KG) {
+            const size_t at = (size_t)(b0 + b) * H + cj;
+            const float dh = carry(0, b);
+            a.dh_out[at] = a.h0_mask ? dh * (float)a.h0_mask[at] : dh;
+        }
     __syncthreads();
     for (int c = tid; c < 6 * U; c += NT) {
         const int k = c / U, uu = c % U;
         if (p * U + uu >= H) continue;
         float s = 0.f;
         for (int t = 0; t < KG; ++t) s += bsum[k * NT + t * U + uu];
-        a.bias_part[((size_t)grp * 6 + k) * H + p * U + uu] = s;
+        a.bias_part[((size_t)grp * 6 + (k < 3 ? 0 : 3) + gate_block(a.torch, k % 3)) * H + p * U + uu] = s;
     }
     if (P > 1) {   // nobody leaves while a peer may still read its partial sums
         cluster_arrive();

@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "qgru_internal.h"
+
 struct qgru_handle;
 
 namespace qgru {
@@ -17,16 +19,17 @@ struct F32RecPlan {
     size_t smem = 0;
 };
 
-// Clamp masks of a quantized training forward, one word per (timestep, row, unit): bit g (z, r, n)
-// W*x + bw, 3 + g R*h + br, 6 + g gate input, 9 + g gate output, 12 the new state; 1 = not clamped.
-constexpr int PM_IH = 0, PM_HH = 3, PM_IN = 6, PM_OUT = 9, PM_H = 12;
-
+// Weights come in one of two layouts: R [H][3H] with the gates in the order of v (z, r, n), or the module's own
+// (torch): R [3H][H], gates in the order r, z, n.  In the second, W*x and the gradients dp, dq have
+// that gate order as well, so that no weight and no gradient is transposed or reordered anywhere.
 struct FloatFwdArgs {
     int T, B, H;
-    const float *R, *wx, *bw, *br;    // R [H][3H]; wx = W*x of all steps [T*B][3H]
-    float *h;                         // [(T+1)][B][H], slot 0 holds the initial state
+    const float *R, *wx, *bw, *br;    // wx = W*x of all steps [T*B][3H]; biases may be null
+    float *h;                         // [(T+1)][B][H], slot 0 (in reverse slot T) holds the initial state
     float *v;                         // [T*B][v_stride * H] or null
     int v_stride;
+    int torch, reverse;               // weight layout; reverse: step s consumes time T - 1 - s
+    OutView out;                      // further copies of the states: hf, hn_f
     int U, P, KG, Bt, D;              // set by the launcher
 };
 // False: no plan for this shape (H > 512), the caller runs step by step.
@@ -35,16 +38,24 @@ int float_chain_launch(qgru_handle *h, FloatFwdArgs a, cudaStream_t st);
 
 struct BwdChainArgs {
     int T, B, H;
-    const float *R;                   // [H][3H], or its transpose [3H][H] with r_trans
-    int r_trans;
-    const float *h, *v, *dh_new;      // [(T+1)][B][H], [T*B][4H], [(T+1)][B][H]
-    float *dh;                        // [B][H] in / out
+    const float *R;                   // [H][3H]; its transpose [3H][H] with r_trans; [3H][H] in the module's gate order with torch
+    int r_trans, torch, reverse;
+    const float *h, *v;               // [(T+1)][B][H], [T*B][4H]
+    const float *dh_new;              // gradient of the state after the step at time t, row b: dh_new + t * dn_ts + b * dn_bs
+    long long dn_ts, dn_bs;
+    const float *dh_in;               // [B][H] gradient of the last state, or null
+    float *dh_out;                    // [B][H] gradient of the initial state, times h0_mask where there is one
+    const uint8_t *h0_mask;
     const uint16_t *pm;               // packed clamp masks [T*B][H] or null
     float *dp, *dq;                   // [T*B][3H]: gradients of W*x + bw (masked) and of R*h + br
-    float *bias_part;                 // [G][6][H]: column sums of dp (before the W*x + bw mask) and of dq
+    float *bias_part;                 // [G][6][H]: sums of dp (before its mask) and of dq over the group's rows
     int U, P, KG, Bt, D;              // set by the launcher
 };
 bool bwd_chain_fits(qgru_handle *h, int B, int *groups);
 int bwd_chain_launch(qgru_handle *h, BwdChainArgs a, cudaStream_t st);
+
+// Bias gradients from bias_part; masks and either output may be null.
+void bwd_bias_launch(qgru_handle *h, const float *part, int G, const uint8_t *m_bw, const uint8_t *m_br, float *dbw, float *dbr, int accumulate,
+                     cudaStream_t st);
 
 }  // namespace qgru

@@ -57,7 +57,7 @@ struct GenLin {
 };
 
 __host__ __device__ constexpr size_t cell_const_bytes(int cell) {
-    return cell <= CELL_INT_FAST_NOTIE ? sizeof(FastLin) : cell == CELL_INT_GENERIC ? sizeof(GenLin) : 3 * sizeof(float);
+    return cell <= CELL_INT_FAST_NOTIE ? sizeof(FastLin) : cell == CELL_INT_GENERIC || cell == CELL_INT_TRAIN ? sizeof(GenLin) : 3 * sizeof(float);
 }
 
 // State rows are 64 bytes modulo 128 apart: the four 16-byte pieces of two neighbouring rows that a quarter warp
@@ -73,7 +73,7 @@ __host__ __device__ inline RegSmem reg_smem(int K, int U, int KS, int NT, int D,
     RegSmem s;
     s.tables = 128;                                                        // barriers in front
     s.consts = s.tables + up((size_t)n_table * 4);
-    s.hs = s.consts + up((size_t)3 * U * cell_const_bytes(cell)) + (cell == CELL_INT_GENERIC ? up(sizeof(GateConsts)) : 0);
+    s.hs = s.consts + up((size_t)3 * U * cell_const_bytes(cell));
     s.ihs = s.hs + up((size_t)2 * NT * 8 * state_stride(K));
     s.red = s.ihs + up((size_t)D * NT * 8 * 3 * U * ih_bytes);
     s.total = s.red + (KS > 1 ? up((size_t)(U / 16) * KS * 12 * RED_STRIDE * 4) : 0);
@@ -83,7 +83,7 @@ __host__ __device__ inline RegSmem reg_smem(int K, int U, int KS, int NT, int D,
 template <typename IhT, int KST, int Cell, bool HU, bool Split>
 __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ GateConsts gc, const __grid_constant__ RecRegArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr bool Tie = Cell != CELL_INT_FAST_NOTIE;
+    constexpr bool Tie = Cell != CELL_INT_FAST_NOTIE, Train = Cell >= CELL_INT_TRAIN;
     const int U = a.U, KS = Split ? a.KS : 1, P = Split ? a.P : 1, NT = a.NT, D = a.D, H = a.H;
     const int K = KS * KST * 32, HS = state_stride(K);
     const RegSmem L = reg_smem(K, U, KS, NT, D, (int)sizeof(IhT), Cell, a.n_table);
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
         const bool ok = j < H;
         if constexpr (Cell <= CELL_INT_FAST_NOTIE) {
             reinterpret_cast<FastLin *>(consts)[i] = ok ? a.lc.fl[g * H + j] : FastLin{0, 0, 0, 0, 0, 0};
-        } else if constexpr (Cell == CELL_INT_GENERIC) {
+        } else if constexpr (Cell == CELL_INT_GENERIC || Cell == CELL_INT_TRAIN) {
             reinterpret_cast<GenLin *>(consts)[i] = ok ? GenLin{a.lc.corr[g * H + j], a.lc.rs[g * H + j]} : GenLin{0, Rescale{1, 1, 0, 0, 0, 0, 0, 0}};
         } else {
             for (int k = 0; k < 3; ++k) reinterpret_cast<float *>(consts)[k * 3 * U + i] = ok ? a.fs_chan[(size_t)k * 3 * H + g * H + j] : 0.f;
@@ -181,7 +181,8 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
     }
     // N cells side by side: sums, W*x + bw, previous states; ui[i]: which of the thread's units.  Gate by gate over all
     // of them, so that their table lookups overlap.
-    auto cells = [&](auto n_c, const int (*acc)[2], const int (*ihv)[2], const int32_t *h_old, const int *ui, int32_t *hn) {
+    // Training: also the four values of v (zero point taken off) and the mask bits of each.
+    auto cells = [&](auto n_c, const int (*acc)[2], const int (*ihv)[2], const int32_t *h_old, const int *ui, int32_t *hn, float (*vq)[4], uint32_t *keep) {
         constexpr int N = decltype(n_c)::value;
         if constexpr (Cell <= CELL_INT_FAST_NOTIE) {
             const auto lin = [&](int v, int g, int i) {
@@ -204,6 +205,40 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
                 const int32_t hg = linear_epilogue(acc[2][i], f[2 * U].corr, f[2 * U].rs, a.lc.zp_out, a.lc.lo, a.lc.hi);
                 hn[i] = gru_cell<false>(gc, tables, ihv[0][i], ihv[1][i], ihv[2][i], hz, hr, hg, h_old[i]);
             }
+        } else if constexpr (Cell == CELL_INT_TRAIN) {
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const GenLin *f = reinterpret_cast<const GenLin *>(consts) + u0 + ui[i];
+                int32_t ih[3], hh[3], gates[3];
+                uint32_t m = 0;
+#pragma unroll
+                for (int g = 0; g < 3; ++g) {
+                    const int32_t w = (int32_t)rescale64(acc[g][i] + f[g * U].corr, f[g * U].rs) + a.lc.zp_out;
+                    hh[g] = clampi(w, a.lc.lo, a.lc.hi);
+                    ih[g] = clampi(ihv[g][i], gc.ih_lo, gc.ih_hi);
+                    m |= (uint32_t)(hh[g] == w) << (PM_HH + g) | (uint32_t)(ih[g] == ihv[g][i]) << (PM_IH + g);
+                }
+                hn[i] = gru_cell_train(gc, a.n_table ? tables : nullptr, ih[0], ih[1], ih[2], hh[0], hh[1], hh[2], h_old[i], gates, m);
+#pragma unroll
+                for (int g = 0; g < 3; ++g) vq[i][g] = (float)(gates[g] - (int32_t)a.tc.zp[g]);
+                vq[i][3] = (float)(hh[2] - (int32_t)a.tc.zp[3]);
+                keep[i] = m;
+            }
+        } else if constexpr (Cell == CELL_FS_TRAIN) {
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const float *f = reinterpret_cast<const float *>(consts) + u0 + ui[i];
+                float ih[3], hh[3];
+#pragma unroll
+                for (int g = 0; g < 3; ++g) {
+                    ih[g] = (float)ihv[g][i];
+                    hh[g] = fs_linear_raw(acc[g][i], f[g * U], f[(3 + g) * U], f[(6 + g) * U], a.fs.zp_hh);
+                }
+                keep[i] = 0;
+                hn[i] = (int32_t)fs_cell_train(a.fs, a.n_table, tab, ih, hh, (float)h_old[i], vq[i], keep[i]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) vq[i][k] -= a.tc.zp[k];
+            }
         } else {
             const auto lin = [&](int v, int g, int i) {
                 const float *f = reinterpret_cast<const float *>(consts) + g * U + u0 + ui[i];
@@ -224,6 +259,23 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
     const ptrdiff_t out_step = a.reverse ? -(ptrdiff_t)a.out.ts : (ptrdiff_t)a.out.ts;
     float *hf = a.out.hf ? a.out.hf + (size_t)(a.reverse ? a.T - 1 : 1) * a.out.ts + (size_t)b0 * a.out.bs + out_j : nullptr;
     const int obs = (int)a.out.bs;
+    // training: units j .. j + N - 1 of row n of the gate buffer, the masks and the states (two units: both exist and H is even)
+    const auto keep_cells = [&](auto n_c, size_t n, size_t slot_row, int j, const float (*vq)[4], const uint32_t *keep, const float *f) {
+        constexpr int N = decltype(n_c)::value;
+        float *v = a.v + n * 4 * H + j;
+        if constexpr (N == 2) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                *reinterpret_cast<float2 *>(v + (size_t)k * H) = make_float2(vq[0][k] * a.tc.scale[k], vq[1][k] * a.tc.scale[k]);
+            *reinterpret_cast<uint32_t *>(a.pm + n * H + j) = keep[0] | keep[1] << 16;
+            if (a.h_all) *reinterpret_cast<float2 *>(a.h_all + slot_row * H + j) = make_float2(f[0], f[1]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[(size_t)k * H] = vq[0][k] * a.tc.scale[k];
+            a.pm[n * H + j] = (uint16_t)keep[0];
+            if (a.h_all) a.h_all[slot_row * H + j] = f[0];
+        }
+    };
     int slot = 0;
     uint32_t ih_phase = 0;
     // (a wait that has run out is not repeated: the steps go on with whatever is there, so that every barrier is met)
@@ -266,7 +318,9 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
                     const int32_t h_old[2] = {state_byte(hb2, h_bits), state_byte(hb2 >> 8, h_bits)};
                     const int ui[2] = {0, 1};
                     int32_t hn[2];
-                    cells(std::integral_constant<int, 2>(), sums, ihv, h_old, ui, hn);
+                    float vq[2][4];
+                    uint32_t keep[2];
+                    cells(std::integral_constant<int, 2>(), sums, ihv, h_old, ui, hn, vq, keep);
                     if (row < rows) {
                         *reinterpret_cast<uint16_t *>(h_nxt + b * HS + out_j) = (uint16_t)(((uint32_t)hn[0] & 0xffu) | ((uint32_t)hn[1] << 8));
                         if (a.vec2) {
@@ -278,6 +332,16 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
                         } else {
                             if (out_j < H) put_state(a.out, out_slot, b0 + b, out_j, H, last, hn[0], gc.zp_h, gc.h_scale);
                             if (out_j + 1 < H) put_state(a.out, out_slot, b0 + b, out_j + 1, H, last, hn[1], gc.zp_h, gc.h_scale);
+                        }
+                        if constexpr (Train) {
+                            const size_t n = (size_t)(a.reverse ? a.T - 1 - s : s) * a.B + b0 + b, at = (size_t)out_slot * a.B + b0 + b;
+                            const float f[2] = {(float)(hn[0] - gc.zp_h) * gc.h_scale, (float)(hn[1] - gc.zp_h) * gc.h_scale};
+                            if ((H & 1) == 0) {
+                                if (out_j < H) keep_cells(std::integral_constant<int, 2>(), n, at, out_j, vq, keep, f);
+                            } else {
+                                if (out_j < H) keep_cells(std::integral_constant<int, 1>(), n, at, out_j, vq, keep, f);
+                                if (out_j + 1 < H) keep_cells(std::integral_constant<int, 1>(), n, at, out_j + 1, vq + 1, keep + 1, f + 1);
+                            }
                         }
                     }
                 }
@@ -292,6 +356,8 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
                 asm volatile("bar.sync %0, %1;" ::"r"(1 + ug), "r"(KS * 32) : "memory");
                 const int ul = lane & 15, j = out_j, per = 8 / KS;
                 int32_t hn[2] = {0, 0};
+                float vq[2][4];
+                uint32_t keep[2];
                 const int row0 = ks * per + (lane >> 4);         // this lane's rows: row0 and, with two slices, row0 + 2
                 if (ks * per < rows) {                           // (warp-uniform)
                     int sums[3][2] = {}, ihv[3][2];
@@ -311,8 +377,8 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
                         ihv[2][i] = iv[2 * U];
                         h_old[i] = state_byte(h_cur[b * HS + j], h_bits);
                     }
-                    if (per == 2 || ks * per + 2 >= rows) cells(std::integral_constant<int, 1>(), sums, ihv, h_old, ui, hn);
-                    else cells(std::integral_constant<int, 2>(), sums, ihv, h_old, ui, hn);
+                    if (per == 2 || ks * per + 2 >= rows) cells(std::integral_constant<int, 1>(), sums, ihv, h_old, ui, hn, vq, keep);
+                    else cells(std::integral_constant<int, 2>(), sums, ihv, h_old, ui, hn, vq, keep);
 #pragma unroll
                     for (int i = 0; i < 2; ++i) {
                         if (2 * i >= per || ks * per + 2 * i >= rows) continue;
@@ -343,6 +409,12 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
                             if (last && a.out.hn_f) a.out.hn_f[(size_t)(b0 + nt * 8 + row) * H + j] = f;
                         } else {
                             put_state(a.out, out_slot, b0 + nt * 8 + row, j, H, last, hn[i], gc.zp_h, gc.h_scale);
+                        }
+                        if constexpr (Train) {
+                            const int b = b0 + nt * 8 + row;
+                            const float f = (float)(hn[i] - gc.zp_h) * gc.h_scale;
+                            keep_cells(std::integral_constant<int, 1>(), (size_t)(a.reverse ? a.T - 1 - s : s) * a.B + b, (size_t)out_slot * a.B + b, j,
+                                       vq + i, keep + i, &f);
                         }
                     }
                 }
@@ -396,6 +468,8 @@ RegKernel pick(RecCell cell, int ih_bytes, int kst, bool hu, bool split) {
             return ih_bytes == 2 ? pick_kst<int16_t, CELL_INT_FAST_NOTIE>(kst, hu, split) : pick_kst<int32_t, CELL_INT_FAST_NOTIE>(kst, hu, split);
         case CELL_INT_GENERIC:
             return ih_bytes == 1 ? pick_kst<int8_t, CELL_INT_GENERIC>(kst, hu, split) : pick_kst<int16_t, CELL_INT_GENERIC>(kst, hu, split);
+        case CELL_INT_TRAIN: return ih_bytes == 2 ? pick_kst<int16_t, CELL_INT_TRAIN>(kst, hu, split) : pick_kst<int32_t, CELL_INT_TRAIN>(kst, hu, split);
+        case CELL_FS_TRAIN: return ih_bytes == 2 ? pick_kst<int16_t, CELL_FS_TRAIN>(kst, hu, split) : pick_kst<int32_t, CELL_FS_TRAIN>(kst, hu, split);
         default: return ih_bytes == 1 ? pick_kst<int8_t, CELL_FS>(kst, hu, split) : pick_kst<int16_t, CELL_FS>(kst, hu, split);
     }
 }

@@ -20,7 +20,9 @@ struct RecRegPlan {
     size_t ih_elements(long long N) const { return (size_t)N * 3 * P * U; }
 };
 
-enum RecCell { CELL_INT_FAST = 0, CELL_INT_FAST_NOTIE = 1, CELL_INT_GENERIC = 2, CELL_FS = 3 };
+// The training cells keep the gate buffer and the packed clamp masks; their W*x + bw comes clamped to one step
+// beyond the operator's range on either side, so that it still tells what the clamp changed.
+enum RecCell { CELL_INT_FAST = 0, CELL_INT_FAST_NOTIE = 1, CELL_INT_GENERIC = 2, CELL_FS = 3, CELL_INT_TRAIN = 4, CELL_FS_TRAIN = 5 };
 
 struct RecRegArgs {
     int T, B, H, Hpad, reverse, h_unsigned;
@@ -34,6 +36,10 @@ struct RecRegArgs {
     int n_table;
     const float *fs_chan;         // float-storage cell: [3][C] offset, bias term, scale ratio of R*h + br
     FsConsts fs;
+    // training cells: all states [(T+1)][B][H] or null, gate buffer [T*B][4H], clamp masks [T*B][H] (PM_* bits)
+    float *h_all, *v;
+    uint16_t *pm;
+    FsTrainConsts tc;
     int KS, U, P, Bt, NT, D, vec2;   // set by the launcher
     int *abort_flag;
 };

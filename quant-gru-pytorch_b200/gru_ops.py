@@ -324,6 +324,12 @@ class Handle:
         self.synchronize()
         return dx, dW, dR, dbw, dbr, dh
 
+    def train_saved_bytes(self, mode, T, B):
+        """Bytes per direction that qgru_train_forward keeps for the backward; 0: no such form."""
+        n = C.c_size_t(0)
+        self._ck(self._lib.qgru_train_saved_bytes(self._h, mode, T, B, C.byref(n)), "qgru_train_saved_bytes")
+        return n.value
+
     # -- forward (host tensors; copies are part of the call)
     def forward_i32_host(self, x_q, h0_q=None, reverse=False, out=None):
         x_q = _check_tensor(x_q, "x_q", torch.int32, cuda=False)

@@ -29,7 +29,7 @@ import math
 import torch
 from torch import nn
 
-from . import gru_ops
+from . import _cabi, gru_ops
 from .params import GRUQuantParams, Histograms, OperatorQuantConfig, Ranges
 
 
@@ -103,6 +103,74 @@ class _QuantGRUFunction(torch.autograd.Function):
         return None, None, None, dx, dW, dR, dbw, dbr, dh0 + dh_all[0]
 
 
+class _LayerFunction(torch.autograd.Function):
+    """Training of the whole layer, both directions, weights in the module's layout: one library call forward,
+    one backward (qgru_train_forward / qgru_train_backward; modes as there).  Inputs: x and hx as the
+    module takes them (fp32), then w_ih, w_hh, b_ih, b_hh per direction (biases may be None)."""
+
+    @staticmethod
+    def forward(ctx, module, mode, saved_bytes, x, hx, *params):
+        H, D = module.hidden_size, module.num_directions
+        t_dim, b_dim = (1, 0) if module.batch_first else (0, 1)
+        T, B = x.shape[t_dim], x.shape[b_dim]
+        handles = [module._dirs[d].handle for d in range(D)]
+        if mode == 0:
+            x = x.transpose(0, 1).contiguous() if module.batch_first else x.contiguous()
+            x_ts, x_bs = B * x.shape[2], x.shape[2]
+        else:
+            if x.stride(-1) != 1:
+                x = x.contiguous()
+            x_ts, x_bs = x.stride(t_dim), x.stride(b_dim)
+        saved = torch.empty((D, (saved_bytes + 255) // 256 * 64), dtype=torch.float32, device=x.device)
+        dirs = (_cabi.TrainDir * D)()
+        params = [p if p is None else p.contiguous() for p in params]
+        for d in range(D):
+            for name, p in zip(("W", "R", "bw", "br"), params[4 * d:4 * d + 4]):
+                setattr(dirs[d], name, p.data_ptr() if p is not None else None)
+            dirs[d].saved = saved[d].data_ptr()
+        out = torch.empty((B, T, D * H) if module.batch_first else (T, B, D * H), device=x.device)
+        h_n = torch.empty((D, B, H), device=x.device)
+        h = handles[0]
+        h._ck(h._lib.qgru_train_forward(h._h, handles[1]._h if D == 2 else None, mode, T, B, x.data_ptr(), x_ts, x_bs,
+                                        hx.data_ptr() if hx is not None else None, dirs, out.data_ptr(), out.stride(t_dim),
+                                        out.stride(b_dim), h_n.data_ptr(), gru_ops._stream(x.device)), "qgru_train_forward")
+        ctx.handles, ctx.mode, ctx.saved, ctx.dirs, ctx.batch_first = handles, mode, saved, dirs, module.batch_first
+        ctx.shape, ctx.param_shapes = (T, B, x.shape[2], H), [None if p is None else p.shape for p in params]
+        ctx.set_materialize_grads(False)
+        if mode == 0:
+            ctx.save_for_backward(x)
+        return out, h_n
+
+    @staticmethod
+    def backward(ctx, dout, dh_n):
+        T, B, I, H = ctx.shape
+        D, dev = len(ctx.handles), ctx.saved.device
+        t_dim, b_dim = (1, 0) if ctx.batch_first else (0, 1)
+        if dout is None:
+            dout = torch.zeros((B, T, D * H) if ctx.batch_first else (T, B, D * H), device=dev)
+        elif dout.stride(-1) != 1:
+            dout = dout.contiguous()
+        if dh_n is not None:
+            dh_n = dh_n.contiguous()
+        need = ctx.needs_input_grad
+        dx = torch.empty((T, B, I), device=dev) if need[3] else None
+        dh0 = torch.empty((D, B, H), device=dev) if need[4] else None
+        grads = [torch.empty(s, device=dev) if s is not None and n else None for s, n in zip(ctx.param_shapes, need[5:])]
+        for d in range(D):
+            for name, g in zip(("dW", "dR", "dbw", "dbr"), grads[4 * d:4 * d + 4]):
+                setattr(ctx.dirs[d], name, g.data_ptr() if g is not None else None)
+        x = ctx.saved_tensors[0] if ctx.mode == 0 else None
+        h = ctx.handles[0]
+        h._ck(h._lib.qgru_train_backward(h._h, ctx.handles[1]._h if D == 2 else None, ctx.mode, T, B,
+                                         x.data_ptr() if x is not None else None, dout.data_ptr(), dout.stride(t_dim),
+                                         dout.stride(b_dim), dh_n.data_ptr() if dh_n is not None else None,
+                                         dx.data_ptr() if dx is not None else None, dh0.data_ptr() if dh0 is not None else None,
+                                         ctx.dirs, gru_ops._stream(dev)), "qgru_train_backward")
+        if dx is not None and ctx.batch_first:
+            dx = dx.transpose(0, 1)
+        return (None, None, None, dx, dh0, *grads)
+
+
 class _Direction:
     """Per-direction run-time state: handle, haste-layout weights, what the handle holds."""
 
@@ -110,6 +178,7 @@ class _Direction:
         self.handle = None
         self.weights = None
         self.weights_key = None
+        self.params_key = None
         self.loaded_key = None
 
 
@@ -264,7 +333,7 @@ class QuantGRU(nn.Module):
         suffix = "_reverse" if d == 1 else ""
         return [getattr(self, n + suffix) for n in ("weight_ih_l0", "weight_hh_l0", "bias_ih_l0", "bias_hh_l0")]
 
-    def _direction(self, d, device):
+    def _handle(self, d, device):
         st = self._dirs[d]
         if st.handle is None or st.handle.device != (device.index or 0):
             st.handle = gru_ops.Handle(self.input_size, self.hidden_size, device=device.index or 0)
@@ -273,7 +342,11 @@ class QuantGRU(nn.Module):
                 # the two directions run side by side: each persistent kernel takes half the SMs
                 sms = torch.cuda.get_device_properties(device).multi_processor_count
                 st.handle.set_option("sm_limit", max(1, sms // 2))
-            st.weights_key = st.loaded_key = None
+            st.weights_key = st.params_key = st.loaded_key = None
+        return st
+
+    def _direction(self, d, device):
+        st = self._handle(d, device)
         ps = self._params_of(d)
         key = tuple((p.data_ptr(), p._version) if p is not None else None for p in ps)
         if key != st.weights_key:
@@ -282,12 +355,20 @@ class QuantGRU(nn.Module):
             st.loaded_key = None
         return st
 
+    def _load_params(self, st, d):
+        """The direction's quant params on its handle; returns what identifies them."""
+        qp = self.quant_params_reverse if d == 1 else self.quant_params
+        key = (id(qp), qp.to_bytes())
+        if key != st.params_key:
+            st.params_key = st.loaded_key = None
+            st.handle.set_params(qp)
+            st.params_key = key
+        return key
+
     def _ready_quant(self, d, device):
         st = self._direction(d, device)
-        qp = self.quant_params_reverse if d == 1 else self.quant_params
-        key = (st.weights_key, id(qp), qp.to_bytes())
+        key = (st.weights_key, self._load_params(st, d))
         if key != st.loaded_key:
-            st.handle.set_params(qp)
             st.handle.set_weights_f32(*st.weights)
             st.loaded_key = key
         return st
@@ -361,8 +442,35 @@ class QuantGRU(nn.Module):
             h._ck(h._lib.qgru_layer_forward(h._h, rev, self.quant_storage_dtype != "int32", *args), "qgru_layer_forward")
         return out if direct else out.transpose(0, 1).contiguous(), h_n
 
-    def _forward_float_train(self, input, hx):
-        """Float mode and QAT with autograd: every tensor operation outside the two library calls is a
+    def _forward_train(self, input, hx):
+        """Float mode and QAT with autograd."""
+        device = input.device
+        if input.dim() != 3 or input.shape[2] != self.input_size:
+            raise ValueError(f"input must have {self.input_size} features in three dimensions, got {list(input.shape)}")
+        params = [p for d in range(self.num_directions) for p in self._params_of(d)]
+        for p in params:
+            if p is not None and p.device != device:
+                raise ValueError(f"input is on {device}, the parameters on {p.device}")
+        states = [self._handle(d, device) for d in range(self.num_directions)]
+        mode = 0 if not self.use_quantization else 2 if self.quant_storage_dtype == "int32" else 1
+        if mode:
+            for d, st in enumerate(states):
+                self._load_params(st, d)
+        B, T = input.shape[:2] if self.batch_first else (input.shape[1], input.shape[0])
+        sizes = [st.handle.train_saved_bytes(mode, T, B) for st in states]
+        if not all(sizes):
+            return self._forward_train_stepwise(input, hx)
+        for st in states:
+            st.loaded_key = None        # the quantized weights of this step replace the loaded ones
+        # (conversions outside the autograd function: torch carries the gradients back through them)
+        params = [p if p is None or p.dtype == torch.float32 else p.to(torch.float32) for p in params]
+        if hx is not None:
+            hx = hx.to(device=device, dtype=torch.float32).contiguous()
+        return _LayerFunction.apply(self, mode, max(sizes), input.to(torch.float32), hx, *params)
+
+    def _forward_train_stepwise(self, input, hx):
+        """Layers without the one-call form (H > 512, operands wider than 8 bit).
+        Every tensor operation outside the two library calls is a
         torch operation, so gradients reach the module's parameters in their PyTorch layout."""
         x = input.transpose(0, 1) if self.batch_first else input
         device = x.device
@@ -386,7 +494,7 @@ class QuantGRU(nn.Module):
             if self.use_quantization:
                 qp = self.quant_params_reverse if d == 1 else self.quant_params
                 h = _QuantGRUFunction.apply(st.handle, qp, self.quant_storage_dtype == "int32", xd, W, R, bw, br, h0)
-                st.loaded_key = None        # the handle was reloaded outside the module's cache
+                st.params_key = st.loaded_key = None   # the handle was reloaded outside the module's cache
             else:
                 h = _FloatGRUFunction.apply(st.handle, xd, W, R, bw, br, h0)
             outs.append(h[1:].flip(0) if d == 1 else h[1:])
@@ -409,7 +517,7 @@ class QuantGRU(nn.Module):
             want = (self.num_directions, input.shape[0 if self.batch_first else 1], self.hidden_size)
             if hx is not None and tuple(hx.shape) != want:
                 raise ValueError(f"hx must have shape {list(want)}, got {list(hx.shape)}")
-            return self._forward_float_train(input, hx)
+            return self._forward_train(input, hx)
         with torch.no_grad():
             return self._forward_impl(input, hx)
 
