@@ -758,14 +758,11 @@ PreScale pre_scale(const qgru_handle *h, bool fused) {
 // Where rec=fast takes the register-resident recurrence (us per step against the other forms, integer cell):
 // - not where one CTA per row with R in registers and no tile of eight rows fits (one row at H = 256: 1.66 / 1.07);
 // - one CTA per row group, H <= 256: always (256 rows 2.29 / 2.70, 4096 rows of H = 64 1.8 / 5.5);
-// - clusters, H <= 512: up to four rows each, where the exchange costs less than tcgen05's fixed latencies (H = 512:
-//   one and two rows 2.4 / 2.88, four 2.87 / 2.89, eight 2.95 / 2.94, 31 rows 10.2 / 5.7); the longer cells of the
-//   generic and the float form keep it ahead up to a full tile of eight (3.2 / 3.8);
-// - larger clusters: one tile of eight rows (H = 1024: six rows 2.56 / 4.29, ten 4.51 / 4.29).
+// - clusters, H <= 512: one tile of eight rows (H = 512: two rows 2.15 / 2.86, eight 2.57 / 2.96, sixteen 4.37 / 2.96);
+// - larger clusters: two tiles (H = 1024: six rows 1.98 / 4.29, ten 3.16 / 4.29, 22 rows 4.74 / 4.30).
 bool reg_is_faster(const RecRegPlan &pl, bool gemv) {
     if (gemv) return false;
-    if (pl.P == 1) return true;
-    return pl.Bt <= (pl.KS == 2 && pl.cell <= CELL_INT_FAST_NOTIE ? 4 : 8);
+    return pl.P == 1 || pl.Bt <= (pl.KS == 2 ? 8 : 16);
 }
 
 // The 8-bit path with the register-resident recurrence.

@@ -31,6 +31,15 @@ __device__ __forceinline__ void st_async_u32(uint32_t peer_addr, uint32_t v, uin
 __device__ __forceinline__ void sts_u32(uint32_t addr, uint32_t v) {
     asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
+// 16 bytes (both addresses on a 16-byte boundary)
+__device__ __forceinline__ void st_async_v4(uint32_t peer_addr, const uint32_t (&v)[4], uint32_t peer_bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(peer_addr),
+                 "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(peer_bar)
+                 : "memory");
+}
+__device__ __forceinline__ void sts_v4(uint32_t addr, const uint32_t (&v)[4]) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
 __device__ __forceinline__ void fence_proxy_async_cta() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Byte offset of element (row b, byte k) inside a K-major tile of `rows` rows stored as 128-byte

@@ -40,9 +40,12 @@ struct RecRegArgs {
     float *h_all, *v;
     uint16_t *pm;
     FsTrainConsts tc;
-    int KS, U, P, Bt, NT, D, vec2;   // set by the launcher
+    int U, P, Bt, NT, D, vec2;       // set by the launcher
     int *abort_flag;
 };
+
+typedef void (*RegKernel)(const GateConsts, const RecRegArgs);
+RegKernel rec_reg_float_kernel(RecCell cell, int ih_bytes, int kst, int ks, bool hu);   // qgru_rec_reg_float.cu
 
 // False where the form does not exist (H > 1024, no shared memory left).
 bool rec_reg_plan(qgru_handle *h, int B, int sms, int ih_bytes, RecCell cell, int n_table, RecRegPlan *pl);
