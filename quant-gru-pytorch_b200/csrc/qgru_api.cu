@@ -651,7 +651,9 @@ size_t gemv_reg_smem(const qgru_handle *h, int n_table) {
 
 template <bool HU, typename IhT>
 int launch_gemv_reg(qgru_handle *h, RecArgs &a, cudaStream_t st) {
-    auto kern = h->Hpad == 128 ? k_recurrence_gemv_reg<HU, IhT, 64> : k_recurrence_gemv_reg<HU, IhT, 128>;
+    const bool notie = h->lin_notie[1] && h->gc_host.cell_notie != 0 && h->opt_tie != 1;
+    auto kern = h->Hpad == 128 ? (notie ? k_recurrence_gemv_reg<HU, IhT, 64, 2, false> : k_recurrence_gemv_reg<HU, IhT, 64, 2, true>)
+                               : (notie ? k_recurrence_gemv_reg<HU, IhT, 128, 2, false> : k_recurrence_gemv_reg<HU, IhT, 128, 2, true>);
     const size_t smem = gemv_reg_smem(h, a.n_table);
     CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int threads = 2 * ((h->H + 31) / 32 * 32);

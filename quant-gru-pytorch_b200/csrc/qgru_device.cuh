@@ -180,6 +180,14 @@ __device__ __forceinline__ int32_t lds_i32(uint32_t addr) {
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
+// The same from a table that a kernel fills before its first lookup and never changes: independent lookups may
+// overlap and change places (in volatile order the update and the reset gate of a cell take turns).  The
+// index has to be inside the table whatever the data.
+__device__ __forceinline__ int32_t lds_table(uint32_t addr) {
+    int32_t v;
+    asm("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
 // Sign- or zero-extend a state byte held in the low bits of x: bits = 8 for int8 storage, 9 for
 // uint8 (bit 8 is zero, so the value stays non-negative).
 __device__ __forceinline__ int32_t state_byte(uint32_t x, uint32_t bits) {
@@ -198,7 +206,7 @@ __device__ __forceinline__ int32_t state_byte(uint32_t x, uint32_t bits) {
 // point (lin_round).
 __device__ __forceinline__ int32_t ft_lookup(const GateConsts &gc, uint32_t tab, int k, int32_t v) {
     const int32_t idx = min(max(v + gc.fi_c[k], gc.fi_lo[k]), gc.fi_hi[k]);
-    return lds_i32(tab + 4u * (uint32_t)idx);
+    return lds_table(tab + 4u * (uint32_t)idx);
 }
 //   which = ACT_Z / ACT_R: sigmoid LUT output minus its zero point
 __device__ __forceinline__ int32_t fused_gate_fast(const GateConsts &gc, uint32_t tab, int which, int32_t a_pre,

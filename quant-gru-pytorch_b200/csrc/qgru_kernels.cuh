@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(1024, 1) k_recurrence_gemv(const __grid_consta
 // lane busy.  The per-unit constants of the R*h + br requantization live in shared memory (the
 // registers belong to R).
 // Cell: 2 the tabulated integer cell, 3 the float cell of the float-storage forward (as in k_recurrence_gemv).
-template <bool HUnsigned, typename IhT, int KT, int Cell = 2>
+template <bool HUnsigned, typename IhT, int KT, int Cell = 2, bool Tie = true>
 __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_constant__ GateConsts gc, RecArgs a) {
     static_assert(Cell == 2 || Cell == 3, "the branch-free cells only");
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -684,10 +684,13 @@ __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_con
         v[1] = (int32_t)src[a.H];
         v[2] = (int32_t)src[2 * a.H];
     };
+    // fp32 output alone, as a module asks for it: a running pointer instead of the address arithmetic of every view
+    const bool plain = a.out.hf && !a.out.hq && !a.out.h8;
+    float *hf = plain ? a.out.hf + (size_t)(a.reverse ? a.T - 1 : 1) * a.out.ts + (size_t)b * a.out.bs + j : nullptr;
+    const long long hf_step = a.reverse ? -(long long)a.out.ts : (long long)a.out.ts;
     int32_t ihv[3] = {0, 0, 0};
     if (worker) load_ih(0, ihv);
     for (int s = 0; s < a.T; ++s) {
-        const long long out_slot = a.reverse ? (a.T - 1 - s) : (s + 1);
         const unsigned char *h_cur = hs + (size_t)(s & 1) * HS;
         unsigned char *h_nxt = hs + (size_t)((s + 1) & 1) * HS;
         int32_t ihn[3] = {0, 0, 0};
@@ -720,9 +723,9 @@ __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_con
             const int32_t h_old = HUnsigned ? (int32_t)hb : (int32_t)(int8_t)hb;
             int32_t hn;
             if constexpr (Cell == 2) {
-                const int32_t z_d = fused_gate_fast(gc, tab, ACT_Z, ihv[0], lin_round(acc[0], fls[j]));
-                const int32_t r_d = fused_gate_fast(gc, tab, ACT_R, ihv[1], lin_round(acc[1], fls[units + j]));
-                hn = fused_finish_fast(gc, tab, ihv[2], lin_round(acc[2], fls[2 * units + j]), z_d, r_d, h_old);
+                const int32_t z_d = fused_gate_fast(gc, tab, ACT_Z, ihv[0], lin_round<Tie>(acc[0], fls[j]));
+                const int32_t r_d = fused_gate_fast(gc, tab, ACT_R, ihv[1], lin_round<Tie>(acc[1], fls[units + j]));
+                hn = fused_finish_fast<Tie>(gc, tab, ihv[2], lin_round<Tie>(acc[2], fls[2 * units + j]), z_d, r_d, h_old);
             } else {
                 const float fih[3] = {(float)ihv[0], (float)ihv[1], (float)ihv[2]};
                 float fhh[3];
@@ -735,8 +738,15 @@ __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_con
                 hn = (int32_t)fs_finish_tab(a.fs, tab, u_g, r_g, fih[2], fhh[2], (float)h_old);
             }
             h_nxt[j_at] = (unsigned char)hn;
-            put_state(a.out, out_slot, b, j, a.H, s + 1 == a.T, hn, gc.zp_h, gc.h_scale);
+            if (plain) {
+                const float f = (float)(hn - gc.zp_h) * gc.h_scale;
+                *hf = f;
+                if (s + 1 == a.T && a.out.hn_f) a.out.hn_f[(size_t)b * a.H + j] = f;
+            } else {
+                put_state(a.out, a.reverse ? (a.T - 1 - s) : (s + 1), b, j, a.H, s + 1 == a.T, hn, gc.zp_h, gc.h_scale);
+            }
         }
+        hf += hf_step;
         ihv[0] = ihn[0];
         ihv[1] = ihn[1];
         ihv[2] = ihn[2];
