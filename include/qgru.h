@@ -470,7 +470,8 @@ QGRU_API double qgru_probe_last_bulk_rate(void);
  *   "rec"      auto | dp4a | mma | gemv | reg | fast | generic
  *                                           recurrence kernel (generic = int32 storage path; reg: R in
  *                                           registers, warp-level tensor instructions, H <= 1024; fast:
- *                                           auto, and reg at the sizes where it is the faster one)
+ *                                           auto, and reg at the sizes where it is the faster one; layers
+ *                                           with 16-bit states and H <= 256 in one launch)
  *   "exchange" auto | global | cluster      how the CTAs of a batch group exchange h_t
  *   "cell"     auto | fused | generic       gate datapath: tabulated (auto also allows its
  *                                           shift-free form), or the reference's step by step

@@ -450,6 +450,8 @@ int qgru_set_params(qgru_handle *h, const qgru_params *p, const float *scale_W,
     h->fast = fits8(op[QGRU_OP_X]) && fits8(op[QGRU_OP_H]) && fits8(op[QGRU_OP_W]) &&
               !op[QGRU_OP_W].is_unsigned && fits8(op[QGRU_OP_R]) && !op[QGRU_OP_R].is_unsigned &&
               (ih8 || ih16) && (int64_t)std::max(h->I, h->H) * 128 * 255 < (int64_t)0x7fffffff;
+    h->wide = !h->fast && fits8(op[QGRU_OP_R]) && !op[QGRU_OP_R].is_unsigned && op[QGRU_OP_H].bits <= 16 && h->Hpad <= 256 &&
+              wide_smem(h->H, h->Hpad, h->n_table) <= (size_t)h->smem_optin;
 
     int rc;
     if ((rc = alloc_once(h, &h->d_gc, 1))) return rc;
@@ -505,11 +507,11 @@ int alloc_packed(qgru_handle *h, cudaStream_t st) {
 int finish_weights(qgru_handle *h, cudaStream_t st) {
     const int C = h->C;
     int rc;
-    if (h->fast && (rc = alloc_packed(h, st))) return rc;
+    if ((h->fast || h->wide) && (rc = alloc_packed(h, st))) return rc;
     CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
     k_pack_weights<<<C, 128, 0, st>>>(h->d_wq[0], h->fast ? h->d_w8[0] : nullptr, h->d_wsum[0], h->I,
                                       h->Ipad, C, h->d_flags);
-    k_pack_weights<<<C, 128, 0, st>>>(h->d_wq[1], h->fast ? h->d_w8[1] : nullptr, h->d_wsum[1], h->H,
+    k_pack_weights<<<C, 128, 0, st>>>(h->d_wq[1], h->fast || h->wide ? h->d_w8[1] : nullptr, h->d_wsum[1], h->H,
                                       h->Hpad, C, h->d_flags);
     const int gb = (C + 127) / 128;
     k_channel_consts<<<gb, 128, 0, st>>>(h->d_wq[2], h->d_brs[0], h->d_wsum[0],
@@ -522,7 +524,7 @@ int finish_weights(qgru_handle *h, cudaStream_t st) {
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(h->h_flags, h->d_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (h->fast && (h->h_flags[0] & 2))
+    if (h->h_flags[0] & 2)
         return fail(h, QGRU_ERR_BAD_ARG, "quantized weight outside the 8-bit range its operator declares");
     h->lin_fits32[0] = !(h->h_flags[0] & 8);
     h->lin_fits32[1] = !(h->h_flags[0] & 16);
@@ -1064,6 +1066,31 @@ int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out
     return QGRU_OK;
 }
 
+dim3 linear_grid(long long N, int C) { return dim3((unsigned)((N + 31) / 32), (unsigned)((C + 63) / 64)); }
+
+// Operands wider than 8 bits, R of 8 and states of up to 16, H <= 256: the recurrence in one launch.
+int run_wide(qgru_handle *h, int T, int B, const int32_t *x32, const int32_t *h0, const OutView &out, unsigned flags, cudaStream_t st) {
+    const long long N = (long long)T * B;
+    const int C = h->C;
+    int rc;
+    if ((rc = ensure(h, h->ih32, (size_t)N * C * 4))) return rc;
+    CK(cudaEventRecord(h->ev[1], st));
+    k_linear_generic<<<linear_grid(N, C), 256, 0, st>>>(h->d_wq[0], x32, (int32_t *)h->ih32.p, N, h->I, C, linear_consts(h, 0), nullptr);
+    CK(cudaEventRecord(h->ev[2], st));
+    WideArgs a{T, B, h->H, h->Hpad, C, (flags & QGRU_FLAG_REVERSE) ? 1 : 0, h->d_w8[1], (const int32_t *)h->ih32.p, h0, out, linear_consts(h, 1),
+               h->d_tables, h->n_table};
+    const size_t smem = wide_smem(h->H, h->Hpad, h->n_table);
+    auto kern = h->h_uns ? k_recurrence_wide<true> : k_recurrence_wide<false>;
+    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<B, 4 * ((h->H + 31) / 32 * 32), smem, st>>>(h->gc_host, a);
+    CK(cudaGetLastError());
+    h->launches += 2;
+    CK(cudaEventRecord(h->ev[3], st));
+    h->timing_valid = true;
+    h->plan_text = "path=wide gemm=simt_i64 rec=dp4a_two_planes rows_per_cta=1";
+    return QGRU_OK;
+}
+
 // Generic path: int32 operands, 64-bit accumulation, one launch pair per step.
 int run_generic(qgru_handle *h, int T, int B, const int32_t *x32, int32_t *hq, int32_t *vq, unsigned flags,
                 cudaStream_t st, const qgru_masks *mk = nullptr) {
@@ -1075,9 +1102,8 @@ int run_generic(qgru_handle *h, int T, int B, const int32_t *x32, int32_t *hq, i
     CK(cudaEventRecord(h->ev[1], st));
     const LinearConsts lcx = linear_consts(h, 0), lch = linear_consts(h, 1);
     {
-        dim3 grid((C + 127) / 128, (unsigned)N);
-        k_linear_generic<<<grid, 128, 0, st>>>(h->d_wq[0], x32, (int32_t *)h->ih32.p, N, h->I, C, lcx,
-                                               mk ? mk->ih_linear : nullptr);
+        k_linear_generic<<<linear_grid(N, C), 256, 0, st>>>(h->d_wq[0], x32, (int32_t *)h->ih32.p, N, h->I, C, lcx,
+                                                           mk ? mk->ih_linear : nullptr);
         h->launches++;
     }
     CK(cudaEventRecord(h->ev[2], st));
@@ -1087,9 +1113,8 @@ int run_generic(qgru_handle *h, int T, int B, const int32_t *x32, int32_t *hq, i
         const int t = rev ? T - 1 - s : s;
         const size_t in_slot = rev ? (size_t)(T - s) : (size_t)s;
         const size_t out_slot = rev ? (size_t)(T - 1 - s) : (size_t)(s + 1);
-        dim3 g1((C + 127) / 128, B);
         const size_t row = (size_t)t * B;
-        k_linear_generic<<<g1, 128, 0, st>>>(h->d_wq[1], hq + in_slot * BH, (int32_t *)h->hh32.p, B, H, C, lch,
+        k_linear_generic<<<linear_grid(B, C), 256, 0, st>>>(h->d_wq[1], hq + in_slot * BH, (int32_t *)h->hh32.p, B, H, C, lch,
                                              mk && mk->hh_linear ? mk->hh_linear + row * C : nullptr);
         dim3 g2((H + 127) / 128, B);
         if (mk)
@@ -1160,6 +1185,17 @@ int forward_dir(qgru_handle *h, int T, int B, const FwdInput &in, const OutView 
                 in.x, in.mode == 2 ? 1 : 0, q, N, B, h->I, in.ts, in.bs, h->x_scale, xo.zero_point, op_qmin(xo), op_qmax(xo));
             h->launches++;
             x32 = q;
+        }
+        if (h->wide && h->opt_rec == 6) {
+            if ((rc = ensure(h, h->hq32, (size_t)B * h->H * 4))) return rc;
+            OutView init;
+            init.hq = (int32_t *)h->hq32.p;
+            init.bs = h->H;
+            const FwdInput state{in.mode, nullptr, 0, 0, in.h0};
+            if ((rc = launch_prologue(h, T, B, state, nullptr, nullptr, init, st))) return rc;
+            if (with_slot0 && (rc = launch_prologue(h, T, B, state, nullptr, nullptr, out.shifted(init_slot), st))) return rc;
+            if (after_prologue) CK(cudaEventRecord(after_prologue, st));
+            return run_wide(h, T, B, x32, (const int32_t *)h->hq32.p, out, flags, st);
         }
         OutView slot;
         slot.hq = hq + init_slot * B * h->H;

@@ -32,6 +32,7 @@ struct qgru_handle {
     std::vector<float> sc[4];  // W, R, bw, br scales
     // storage plan
     bool fast = false;         // 8-bit operands, int32 accumulation
+    bool wide = false;         // not fast, but R of 8 and states of at most 16 bits, H <= 256
     bool x_uns = false, h_uns = false;
     int ih_bytes = 1;
     float x_scale = 1.f, h_scale = 1.f;

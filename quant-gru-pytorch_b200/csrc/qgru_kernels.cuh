@@ -184,7 +184,7 @@ __global__ void k_pack_weights(const int32_t *__restrict__ wq, int8_t *__restric
         if (k < K) {
             v = wq[(size_t)k * C + m];
             local += v;
-            if (v < -128 || v > 127) atomicOr(err, 2);
+            if (w8 && (v < -128 || v > 127)) atomicOr(err, 2);
         }
         if (w8) w8[(size_t)m * Kpad + k] = (int8_t)v;
     }
@@ -757,17 +757,184 @@ __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_con
 // --------------------------------------------- generic fallback (any bit width, int32 data)
 
 // out[n][m] = epilogue( sum_k W_q[k][m] * in[n][k] ) with 64-bit accumulation
-// (quantizedGemmBiasFused's arithmetic, src/gru_forward_gpu_quant.cu:110-180).
-__global__ void k_linear_generic(const int32_t *__restrict__ wq, const int32_t *__restrict__ in,
-                                 int32_t *__restrict__ out, long long N, int K, int C,
-                                 LinearConsts lc, uint8_t *__restrict__ keep = nullptr) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    const long long n = blockIdx.y;
-    if (m >= C || n >= N) return;
-    int64_t acc = 0;
-    for (int k = 0; k < K; ++k) acc += (int64_t)wq[(size_t)k * C + m] * (int64_t)in[n * K + k];
-    out[n * C + m] = linear_epilogue(acc, lc.corr[m], lc.rs[m], lc.zp_out, lc.lo, lc.hi,
-                                     keep ? keep + n * C + m : nullptr);
+// (quantizedGemmBiasFused's arithmetic, src/gru_forward_gpu_quant.cu:110-180).  32 x 64 tiles, 2 x 4 outputs
+// per thread, K in slabs of 32 through shared memory; bound by the widening multiply-adds.
+__global__ void __launch_bounds__(256)
+k_linear_generic(const int32_t *__restrict__ wq, const int32_t *__restrict__ in, int32_t *__restrict__ out, long long N, int K, int C,
+                 LinearConsts lc, uint8_t *__restrict__ keep = nullptr) {
+    __shared__ int32_t xs[32][33];
+    __shared__ __align__(16) int32_t ws[32][64];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const long long n0 = (long long)blockIdx.x * 32;
+    const int m0 = blockIdx.y * 64;
+    int64_t acc[2][4] = {};
+    for (int k0 = 0; k0 < K; k0 += 32) {
+        for (int i = tid; i < 32 * 32; i += 256) {
+            const int r = i >> 5, k = i & 31;
+            xs[r][k] = n0 + r < N && k0 + k < K ? in[(n0 + r) * K + k0 + k] : 0;
+        }
+        for (int i = tid; i < 32 * 64; i += 256) {
+            const int k = i >> 6, m = i & 63;
+            ws[k][m] = m0 + m < C && k0 + k < K ? wq[(size_t)(k0 + k) * C + m0 + m] : 0;
+        }
+        __syncthreads();
+        const int kn = min(32, K - k0);
+        for (int k = 0; k < kn; ++k) {
+            const int4 w = *reinterpret_cast<const int4 *>(&ws[k][tx * 4]);
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const int64_t x = xs[ty * 2 + r][k];
+                acc[r][0] += (int64_t)w.x * x;
+                acc[r][1] += (int64_t)w.y * x;
+                acc[r][2] += (int64_t)w.z * x;
+                acc[r][3] += (int64_t)w.w * x;
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const long long n = n0 + ty * 2 + r;
+            const int m = m0 + tx * 4 + c;
+            if (n < N && m < C) out[n * C + m] = linear_epilogue(acc[r][c], lc.corr[m], lc.rs[m], lc.zp_out, lc.lo, lc.hi, keep ? keep + n * C + m : nullptr);
+        }
+}
+
+// The recurrence with states of up to 16 bits and 8-bit R, H <= 256, in one launch instead of two per step: one CTA per
+// batch row keeps R in shared memory (as k_recurrence_gemv) and the state as two bytes per unit in planes of
+// their own, low bytes unsigned, high bytes with the operator's sign, so that both products are dp4a and
+// sum = 256 * high + low is exact.  A quad of threads owns a unit: after the shuffles lanes 0, 1, 2 requantize
+// the rows of one gate each, lanes 0 and 1 run the update and the reset gate side by side, lane 2 the rest.
+// Bound by that chain of 64-bit rescales and segment searches: 21 rows of H = 100, 61 steps, 16-bit operators 122 us
+// (two launches per step: 800).
+struct WideArgs {
+    int T, B, H, Hpad, C, reverse;
+    const int8_t *r8;          // [3H][Hpad]
+    const int32_t *ih;         // [T*B][3H] W*x + bw
+    const int32_t *h0;         // [B][H]
+    OutView out;
+    LinearConsts lc;           // R*h + br epilogue
+    const int32_t *tables;
+    int n_table;
+};
+// shared memory: tables | thresholds [3][16] | segments [3][16] | state [2 buffers][2 planes] | R
+__host__ __device__ inline size_t wide_smem(int H, int Hpad, int n_table) {
+    const size_t units = (size_t)(H + 31) / 32 * 32;
+    return (((size_t)n_table * 4 + 15) & ~size_t(15)) + 3 * 16 * 4 + 3 * 16 * sizeof(qgru_lut_segment) + (size_t)4 * (Hpad + 64) + 3 * units * Hpad;
+}
+
+template <bool HUnsigned>
+__global__ void __launch_bounds__(1024, 1) k_recurrence_wide(const __grid_constant__ GateConsts gc, const __grid_constant__ WideArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int NT = blockDim.x, Kq = a.Hpad >> 2, nch = Kq >> 4, Qs = Kq + 16, Hs = 4 * Qs;
+    int32_t *tables = reinterpret_cast<int32_t *>(smem_raw);
+    size_t off = ((size_t)a.n_table * 4 + 15) & ~size_t(15);
+    int32_t *thr = reinterpret_cast<int32_t *>(smem_raw + off);
+    off += 3 * 16 * 4;
+    qgru_lut_segment *seg = reinterpret_cast<qgru_lut_segment *>(smem_raw + off);
+    off += 3 * 16 * sizeof(qgru_lut_segment);
+    unsigned char *hs = smem_raw + off;                   // [buffer][plane][Hs]
+    off += (size_t)4 * Hs;
+    uint4 *Rq = reinterpret_cast<uint4 *>(smem_raw + off);
+    const int tid = threadIdx.x, qd = tid & 3, j = tid >> 2, b = blockIdx.x;
+    const bool j_ok = j < a.H;
+    for (int i = tid; i < a.n_table; i += NT) tables[i] = a.tables[i];
+    for (int i = tid; i < 48; i += NT) {
+        thr[i] = gc.lut[i >> 4].seg[i & 15].threshold;
+        seg[i] = gc.lut[i >> 4].seg[i & 15];
+    }
+    for (int i = tid; i < a.Hpad; i += NT) {
+        const int at = (i / Kq) * Qs + (i % Kq);
+        const int32_t q = i < a.H ? a.h0[(size_t)b * a.H + i] : 0;
+        hs[at] = (unsigned char)q;
+        hs[Hs + at] = (unsigned char)(q >> 8);
+        hs[2 * Hs + at] = hs[3 * Hs + at] = 0;
+    }
+    for (int g = 0; g < 3; ++g)
+        for (int c = 0; c < nch; ++c) {
+            uint4 w = make_uint4(0u, 0u, 0u, 0u);
+            if (j_ok) w = *reinterpret_cast<const uint4 *>(a.r8 + (size_t)(g * a.H + j) * a.Hpad + qd * Kq + 16 * c);
+            Rq[(size_t)(c * 3 + g) * NT + tid] = w;
+        }
+    // this lane's gate
+    const int g = min(qd, 2), gs = min(qd, 1);
+    const int64_t corr = j_ok ? a.lc.corr[g * a.H + j] : 0;
+    const Rescale rs = j_ok ? a.lc.rs[g * a.H + j] : Rescale{1, 1, 0, 0, 0, 0, 0, 0};
+    const Rescale ih_to = gc.ih_to[g], hh_to = gc.hh_to[gs];
+    const int32_t zp_in = gc.zp_in[g], in_lo = gc.in_lo[g], in_hi = gc.in_hi[g], out_lo = gc.out_lo[g], out_hi = gc.out_hi[g];
+    const int32_t t_size = gc.table_size[g], t_off = gc.table_off[g], lut_zp = gc.lut[g].zp_x;
+    const auto act = [&](int32_t pre) {                   // activation() for this lane's gate
+        const int32_t q = clampi(pre, in_lo, in_hi);
+        if (t_size > 0) return tables[t_off + (q - in_lo)];
+        int sg = QGRU_LUT_SEGMENTS - 1;
+#pragma unroll
+        for (int i = QGRU_LUT_SEGMENTS - 2; i >= 0; --i)
+            if (q < thr[g * 16 + i]) sg = i;
+        return clampi(lut_segment(seg[g * 16 + sg], lut_zp, q), out_lo, out_hi);
+    };
+    const int j_at = (j / Kq) * Qs + (j % Kq);
+    const long long dir = a.reverse ? -1 : 1;
+    const int32_t *src = a.ih + ((size_t)(a.reverse ? a.T - 1 : 0) * a.B + b) * a.C + g * a.H + j;
+    const long long src_step = dir * a.B * a.C;
+    int32_t ihv = j_ok ? *src : 0;
+    __syncthreads();
+    for (int s = 0; s < a.T; ++s) {
+        const unsigned char *h_cur = hs + (s & 1) * 2 * Hs;
+        unsigned char *h_nxt = hs + ((s + 1) & 1) * 2 * Hs;
+        int32_t ihn = 0;
+        src += src_step;
+        if (j_ok && s + 1 < a.T) ihn = *src;
+        int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
+        const uint4 *l4 = reinterpret_cast<const uint4 *>(h_cur + qd * Qs), *h4 = reinterpret_cast<const uint4 *>(h_cur + Hs + qd * Qs);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (c >= nch) break;
+            const uint4 x = l4[c], y = h4[c];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const uint4 w = Rq[(size_t)(c * 3 + k) * NT + tid];
+                lo[k] = dp4a_w<true>((int)w.x, x.x, lo[k]);
+                hi[k] = dp4a_w<HUnsigned>((int)w.x, y.x, hi[k]);
+                lo[k] = dp4a_w<true>((int)w.y, x.y, lo[k]);
+                hi[k] = dp4a_w<HUnsigned>((int)w.y, y.y, hi[k]);
+                lo[k] = dp4a_w<true>((int)w.z, x.z, lo[k]);
+                hi[k] = dp4a_w<HUnsigned>((int)w.z, y.z, hi[k]);
+                lo[k] = dp4a_w<true>((int)w.w, x.w, lo[k]);
+                hi[k] = dp4a_w<HUnsigned>((int)w.w, y.w, hi[k]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            lo[k] += __shfl_xor_sync(0xffffffffu, lo[k], 1);
+            hi[k] += __shfl_xor_sync(0xffffffffu, hi[k], 1);
+            lo[k] += __shfl_xor_sync(0xffffffffu, lo[k], 2);
+            hi[k] += __shfl_xor_sync(0xffffffffu, hi[k], 2);
+        }
+        const int my_lo = g == 0 ? lo[0] : g == 1 ? lo[1] : lo[2], my_hi = g == 0 ? hi[0] : g == 1 ? hi[1] : hi[2];
+        const int32_t hh = linear_epilogue((int64_t)my_hi * 256 + my_lo, corr, rs, a.lc.zp_out, a.lc.lo, a.lc.hi);
+        const int32_t a_ih = rescale_diff<false>(ihv, gc.zp_ih, ih_to);
+        // gru_cell<false>, the update and the reset gate in lanes 0 and 1
+        const int32_t gate = act(a_ih + rescale_diff<false>(hh, gc.zp_hh, hh_to) + zp_in);
+        const int32_t z = __shfl_sync(0xffffffffu, gate, 0, 4), r = __shfl_sync(0xffffffffu, gate, 1, 4);
+        if (qd == 2 && j_ok) {
+            const int64_t r_hh = ((int64_t)r - gc.zp_out[ACT_R]) * ((int64_t)hh - gc.zp_hh);
+            const int32_t n = act(a_ih + (int32_t)rescale64(r_hh, gc.rh_to_n) + zp_in);
+            const int32_t n_h = rescale_diff<false>(n, gc.zp_out[ACT_N], gc.n_to_h) + gc.zp_h;
+            const int32_t h_old = (HUnsigned ? (int32_t)h_cur[Hs + j_at] : (int32_t)(int8_t)h_cur[Hs + j_at]) * 256 + (int32_t)h_cur[j_at];
+            const int64_t z_d = (int64_t)z - gc.zp_out[ACT_Z];
+            const int64_t old_c = z_d * ((int64_t)h_old - gc.zp_h);
+            const int64_t one_minus = ((int64_t)gc.one_q - z) - gc.zp_out[ACT_Z];
+            const int64_t new_c = one_minus * ((int64_t)n_h - gc.zp_h);
+            const int32_t hn = clampi((int32_t)rescale64(old_c + new_c, gc.uh_to_h) + gc.zp_h, gc.h_lo, gc.h_hi);
+            h_nxt[j_at] = (unsigned char)hn;
+            h_nxt[Hs + j_at] = (unsigned char)(hn >> 8);
+            put_state(a.out, a.reverse ? (a.T - 1 - s) : (s + 1), b, j, a.H, s + 1 == a.T, hn, gc.zp_h, gc.h_scale);
+        }
+        ihv = ihn;
+        __syncthreads();
+    }
 }
 
 // v: optional [B][4H] out of this step: update, reset, new gate outputs and the R*h + br row of

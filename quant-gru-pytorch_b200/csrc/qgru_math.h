@@ -173,6 +173,14 @@ QG_HD int32_t clampi(int32_t v, int32_t lo, int32_t hi) {
     return t < hi ? t : hi;
 }
 
+// One segment of a piecewise-linear activation at q.
+QG_HD int32_t lut_segment(const qgru_lut_segment &s, int32_t zp_x, int32_t q) {
+    const int64_t bx = (int64_t)s.q_b * (int64_t)(q - zp_x);
+    const int n = (int)(int8_t)s.n_bx;
+    const int32_t term = (n >= 0) ? (int32_t)rshift_round64(bx, n) : (int32_t)((uint64_t)bx << (-n));
+    return (int32_t)((uint32_t)term + (uint32_t)s.term_c);
+}
+
 // piecewise_linear_raw on an already clamped input (include/quantize_ops_helper.h:560-589):
 // first segment whose threshold exceeds q, else the last one.
 QG_HD int32_t lut_raw(const qgru_lut &lut, int32_t q) {
@@ -182,11 +190,7 @@ QG_HD int32_t lut_raw(const qgru_lut &lut, int32_t q) {
 #endif
     for (int i = QGRU_LUT_SEGMENTS - 2; i >= 0; --i)
         if (q < lut.seg[i].threshold) seg = i;
-    const qgru_lut_segment s = lut.seg[seg];
-    const int64_t bx = (int64_t)s.q_b * (int64_t)(q - lut.zp_x);
-    const int n = (int)(int8_t)s.n_bx;
-    const int32_t term = (n >= 0) ? (int32_t)rshift_round64(bx, n) : (int32_t)((uint64_t)bx << (-n));
-    return (int32_t)((uint32_t)term + (uint32_t)s.term_c);
+    return lut_segment(lut.seg[seg], lut.zp_x, q);
 }
 
 }  // namespace qgru

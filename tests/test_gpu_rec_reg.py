@@ -40,3 +40,31 @@ def test_reg_recurrence_equals_oracle(oracle, cuda_device, cfg, T, B, H):
             got = [hd.forward_f32(xf, f0, reverse=True), hd.forward_fstorage(xf, f0), hd.forward_i32(x, h0, reverse=True)]
             for a, b in zip(base, got):
                 assert torch.equal(a, b), hd.describe_plan()
+
+
+# one unit, ragged units, one and several 16-byte chunks per thread, every row count a CTA wave can end with
+@pytest.mark.parametrize("T,B,H", [(1, 1, 1), (5, 3, 33), (4, 21, 100), (3, 300, 130), (4, 2, 256), (3, 2, 257)])
+@pytest.mark.parametrize("cfg", ["wide16", "pot2_wide16", "unsigned_wide16"])
+def test_wide_recurrence_equals_oracle(oracle, cuda_device, cfg, T, B, H):
+    """States of up to 16 bits in one launch (option rec=fast; H > 256: step by step)."""
+    import torch
+    I = 9
+    c = config_named("wide16")
+    if cfg == "pot2_wide16":
+        c.use_pot2 = True
+    if cfg == "unsigned_wide16":
+        c.unsigned["h"] = c.unsigned["x"] = True
+        c.bits["h"] = 12
+    case = make_case(T * 17 + H, T, B, I, H, oracle, c)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda_device)
+    want = oracle.forward_i32(T, B, I, H, case.wq, case.x_q, case.h0_q, case.params.c, case.params.scale_list())
+    with gru_ops.Handle(I, H, device=cuda_device.index or 0) as hd:
+        hd.set_params(case.params)
+        hd.set_weights_i32(*[dev(a) for a in case.wq])
+        x, h0 = dev(case.x_q), None if case.h0_q is None else dev(case.h0_q)
+        xf, f0 = dev(case.x), None if case.h0 is None else dev(case.h0)
+        base = [hd.forward_i32(x, h0, reverse=True), hd.forward_f32(xf, f0)]
+        hd.set_option("rec", "fast")
+        assert np.array_equal(hd.forward_i32(x, h0).cpu().numpy(), want)
+        assert ("path=wide" in hd.describe_plan()) == (H <= 256)
+        assert torch.equal(base[0], hd.forward_i32(x, h0, reverse=True)) and torch.equal(base[1], hd.forward_f32(xf, f0))
