@@ -17,8 +17,8 @@
 // the partial sums instead, again H values per row.  Sums are added in a fixed order.
 //
 // Measured on a B200 against the two launches per step (tiled product, pointwise kernel) that it replaces, in us
-// per step: backward H = 512, B = 256: 221 -> 21; H = 262, B = 65: 112 -> 4.1; H = 128, B = 32: 48 -> 2.8.
-// Forward H = 262, B = 65: 36 -> 3.9; H = 256, B = 64: 31 -> 3.0.
+// per step: backward H = 512, B = 256: 221 -> 21; H = 262, B = 65: 112 -> 3.1; H = 128, B = 32: 48 -> 1.85.
+// Forward with gate buffer H = 262, B = 65: 36 -> 3.0; H = 256, B = 64: 31 -> 3.8; H = 128, B = 32: 2.0.
 #include "qgru_rec_f32.cuh"
 
 #include "qgru_cluster.cuh"
@@ -69,7 +69,11 @@ __host__ __device__ inline size_t fwd_smem_floats(int P, int U, int KG, int Bt, 
            (size_t)(Bt > RB ? 2 : 1) * KG * (Bt > RB ? RB : Bt) * 3 * U + (size_t)D * Bt * 3 * U + (size_t)6 * Bt * U + (size_t)6 * U;
 }
 
-__global__ void __launch_bounds__(512, 1) k_float_chain(const FloatFwdArgs a) {
+// One: a thread has at most one cell a step (Bt <= KG and one block of rows): its results stay in registers between the
+// cell and the stores, and no loop, staging buffer or 64-bit index is left around them.  A step of few rows
+// is a chain of some 900 dependent instructions at about five cycles each, so their number is what counts.
+template <bool One, int MaxThreads>
+__global__ void __launch_bounds__(MaxThreads, 1) k_float_chain(const FloatFwdArgs a) {
     extern __shared__ __align__(16) float sm[];
     const int U = a.U, P = a.P, KG = a.KG, Bt = a.Bt, D = a.D, PU = P * U, H = a.H, C = 3 * H;
     const int rb_max = min(Bt, RB), BtU = Bt * U;
@@ -134,8 +138,17 @@ __global__ void __launch_bounds__(512, 1) k_float_chain(const FloatFwdArgs a) {
 #pragma unroll
     for (int g = 0; g < 3; ++g) g_off[g] = gate_block(a.torch, g) * H;
     int slot_in = 0, fetched = 0;
+    const bool act = One && j_ok && cb < nb;                 // One: this thread's cell is (row cb, unit cu)
+    if constexpr (One) wx_next += (size_t)cb * C;
+    long long row = (long long)row0 + cb;                    // One: this cell's row of the step
     auto fetch_wx = [&]() {   // each thread fetches what its own cells will read
-        if (fetched < a.T && j_ok) {
+        if constexpr (One) {
+            if (act && fetched < a.T) {
+                float *dst = wxs + (slot_in * Bt + cb) * 3 * U + cu;
+#pragma unroll
+                for (int g = 0; g < 3; ++g) cp_async4(dst + g * U, wx_next + g_off[g]);
+            }
+        } else if (fetched < a.T && j_ok) {
             float *dst = wxs + slot_in * 3 * BtU + cu;
             for (int r0 = 0; r0 < nb; r0 += RB)
                 for (int b = r0 + cb; b < min(nb, r0 + RB); b += KG) {
@@ -185,11 +198,13 @@ __global__ void __launch_bounds__(512, 1) k_float_chain(const FloatFwdArgs a) {
         const float *hk = hcur + kg * 32;
         const float *wxc = wxs + slot * 3 * BtU + cu;
         float *next = P > 1 ? own + ((s + 1) & 1) * BtU + cu : hs + ((s + 1) & 1) * BtU + cu;
+        float o_z = 0.f, o_r = 0.f, o_g = 0.f, o_rz = 0.f, o_rr = 0.f, o_rg = 0.f, o_h = 0.f;   // One: this step's cell
         for (int r0 = 0, pb = 0; r0 < nb; r0 += RB, pb ^= 1) {
             const int r1 = min(nb, r0 + RB);
             float *pk = part + pb * part_n + kg * rb_max * 3 * U + u;
             int b = r0;
-            for (; b + 2 <= r1; b += 2, pk += 6 * U) {
+            // (two rows at a time where there are registers for it)
+            if constexpr (!One || MaxThreads < 512) for (; b + 2 <= r1; b += 2, pk += 6 * U) {
                 uint64_t acc[2][3] = {};
                 const float *h0 = hk + b * PU, *h1 = h0 + PU;
 #pragma unroll
@@ -213,7 +228,7 @@ __global__ void __launch_bounds__(512, 1) k_float_chain(const FloatFwdArgs a) {
                         pk[(r * 3 + g) * U] = lo + hi;
                     }
             }
-            if (b < r1) {
+            for (; b < r1; ++b, pk += 3 * U) {
                 uint64_t acc[3] = {};
                 const float *h0 = hk + b * PU;
 #pragma unroll
@@ -234,7 +249,37 @@ __global__ void __launch_bounds__(512, 1) k_float_chain(const FloatFwdArgs a) {
             }
             if (r0 == 0) cp_async_wait_depth(D);
             __syncthreads();
-            if (j_ok) {
+            if constexpr (One) {
+                if (act) {
+                    // (loads of several slices in flight, added in slice order)
+                    const float *q = part + cb * 3 * U + cu, *w = wxc + cb * 3 * U, *bi = bias + cu;
+                    const int step = rb_max * 3 * U;
+                    float sum[3] = {0.f, 0.f, 0.f};
+                    int k = 0;
+                    for (; k + 4 <= KG; k += 4, q += 4 * step) {
+                        float y[4][3];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+#pragma unroll
+                            for (int g = 0; g < 3; ++g) y[e][g] = q[e * step + g * U];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+#pragma unroll
+                            for (int g = 0; g < 3; ++g) sum[g] += y[e][g];
+                    }
+                    for (; k < KG; ++k, q += step)
+#pragma unroll
+                        for (int g = 0; g < 3; ++g) sum[g] += q[g * U];
+                    o_rz = sum[0] + bi[3 * U];
+                    o_rr = sum[1] + bi[4 * U];
+                    o_rg = sum[2] + bi[5 * U];
+                    o_z = 1.0f / (1.0f + expf(-((w[0] + bi[0]) + o_rz)));
+                    o_r = 1.0f / (1.0f + expf(-((w[U] + bi[U]) + o_rr)));
+                    o_g = tanhf((w[2 * U] + bi[2 * U]) + o_r * o_rg);
+                    o_h = o_z * hcur[cb * PU + cj] + (1.0f - o_z) * o_g;
+                    next[cb * U] = o_h;
+                }
+            } else if (j_ok) {
                 for (int c = r0 + cb; c < r1; c += KG) {
                     float sum[3] = {0.f, 0.f, 0.f};
                     const float *q = part + pb * part_n + (c - r0) * 3 * U + cu;
@@ -269,7 +314,26 @@ __global__ void __launch_bounds__(512, 1) k_float_chain(const FloatFwdArgs a) {
         else __syncthreads();
         // Results leave for global memory behind the arrive: a cluster barrier's release waits for
         // every store before it, and nothing in the next step waits for these.
-        if (j_ok)
+        if constexpr (One) {
+            if (act) {
+                // (addresses from the row index: a pointer per output would not fit beside R)
+                a.h[(row + (a.reverse ? 0 : a.B)) * H + cj] = o_h;
+                if (a.out.hf) a.out.hf[(size_t)(a.reverse ? a.T - 1 - s : s + 1) * a.out.ts + (size_t)(b0 + cb) * a.out.bs + cj] = o_h;
+                if (s + 1 == a.T && a.out.hn_f) a.out.hn_f[(size_t)(b0 + cb) * H + cj] = o_h;
+                if (a.v) {
+                    float *vb = a.v + row * vs + cj;
+                    vb[0] = o_z;
+                    vb[H] = o_r;
+                    vb[2 * H] = o_g;
+                    vb[3 * H] = a.v_stride == 6 ? o_rz : o_rg;
+                    if (a.v_stride == 6) {
+                        vb[4 * H] = o_rr;
+                        vb[5 * H] = o_rg;
+                    }
+                }
+            }
+            row += dir * a.B;
+        } else if (j_ok)
             for (int r0 = 0; r0 < nb; r0 += RB)
                 for (int c = r0 + cb; c < min(nb, r0 + RB); c += KG) {
                     const float hn = next[c * U];
@@ -287,9 +351,11 @@ __global__ void __launch_bounds__(512, 1) k_float_chain(const FloatFwdArgs a) {
                         }
                     }
                 }
-        h_out += h_step;
-        if (v_out) v_out += v_step;
-        if (u_out) u_out += u_step;
+        if constexpr (!One) {
+            h_out += h_step;
+            if (v_out) v_out += v_step;
+            if (u_out) u_out += u_step;
+        }
         slot = slot + 1 == D ? 0 : slot + 1;
         fetch_wx();
         if (P > 1) cluster_wait();
@@ -306,7 +372,9 @@ __host__ __device__ inline size_t bwd_smem_floats(int P, int U, int KG, int Bt, 
     return (size_t)2 * Bt * 3 * U + (size_t)2 * KG * Bt * U + (size_t)D * 7 * Bt * U + (size_t)Bt * U + (size_t)6 * U * KG;
 }
 
-__global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
+// One: a thread has at most one cell a step (Bt <= KG), see the forward; its bias sums stay in registers too.
+template <bool One, int MaxThreads>
+__global__ void __launch_bounds__(MaxThreads, 1) k_bwd_chain(const BwdChainArgs a) {
     extern __shared__ __align__(16) float sm[];
     const int U = a.U, P = a.P, KG = a.KG, Bt = a.Bt, D = a.D, H = a.H, C = 3 * H, BtU = Bt * U;
     float *dqs = sm;                                        // [Bt][3U]
@@ -354,9 +422,27 @@ __global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
     int g_off[3];
 #pragma unroll
     for (int g = 0; g < 3; ++g) g_off[g] = gate_block(a.torch, g) * H;
+    const bool act = One && j_ok && cb < nb;                 // One: this thread's cell is (row cb, unit cu)
+    if constexpr (One) {
+        v_in += (size_t)cb * 4 * H;
+        dn_in += cb * a.dn_bs;
+        h_in += (size_t)cb * H;
+        m_at += (size_t)cb * H;
+        dp_out += (size_t)cb * C;
+        dq_out += (size_t)cb * C;
+    }
     int slot_in = 0, left = a.T;
     auto fetch = [&]() {
-        if (left > 0 && j_ok) {
+        if constexpr (One) {
+            if (act && left > 0) {
+                float *d = stage + slot_in * 7 * BtU + cb * U + cu;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) cp_async4(d + k * BtU, v_in + k * H);
+                cp_async4(d + 4 * BtU, dn_in);
+                cp_async4(d + 5 * BtU, h_in);
+                if (a.pm) cp_async4(d + 6 * BtU, reinterpret_cast<const float *>(a.pm + (m_at & ~(size_t)1)));
+            }
+        } else if (left > 0 && j_ok) {
             float *dst = stage + slot_in * 7 * BtU + cu;
             for (int b = cb; b < nb; b += KG) {
                 float *d = dst + b * U;
@@ -377,7 +463,7 @@ __global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
         cp_async_commit();
     };
     for (int d = 0; d < D; ++d) fetch();
-    size_t m_par = last * H + cj;                           // parity of the cell's mask index
+    size_t m_par = last * H + cj + (One ? (size_t)cb * H : 0);   // parity of the cell's mask index
     const uint32_t part_u32 = smem_addr(part);
     // gradient of the state of (row b, own unit): the part through the update gate plus the KG partial sums,
     // added in a fixed order, eight remote loads in flight
@@ -400,20 +486,20 @@ __global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
         }
         return s;
     };
+    float o_sum[6] = {}, o_dp[3] = {}, o_dq[3] = {};
     int slot = 0;
     __syncthreads();                                        // the zeros of dqs and dps are complete
 
     for (int i = a.T - 1; i >= 0; --i) {
         const int buf = i & 1;
         cp_async_wait_depth(D);
-        if (j_ok) {
-            for (int b = cb; b < nb; b += KG) {
+        const auto cell = [&](int b) {
                 const int at = b * U + cu;
                 const float *d = stage + slot * 7 * BtU + at;
                 const float z = d[0], r = d[BtU], g = d[2 * BtU], q_g = d[3 * BtU], h_old = d[5 * BtU];
                 const float in = i == a.T - 1 ? (a.dh_in ? a.dh_in[(size_t)(b0 + b) * H + cj] : 0.f) : carry(buf ^ 1, b);
                 uint32_t m = 0xffffffffu;
-                if (a.pm) m = __float_as_uint(d[6 * BtU]) >> (((m_par + b * H) & 1) * 16);
+                if (a.pm) m = __float_as_uint(d[6 * BtU]) >> ((One ? m_par & 1 : (m_par + b * H) & 1) * 16);
                 float dh = d[4 * BtU] + in;
                 if (!(m >> PM_H & 1)) dh *= 0.f;
                 zdh[at] = z * dh;
@@ -431,12 +517,26 @@ __global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
                     dq[k] *= keep;
                     if (!(m >> (PM_HH + k) & 1)) dq[k] *= 0.f;
                     dqs[b * 3 * U + k * U + cu] = dq[k];
-                    bsum[k * NT + tid] += dp[k];
-                    bsum[(3 + k) * NT + tid] += dq[k];
+                    if constexpr (One) {
+                        o_sum[k] += dp[k];
+                        o_sum[3 + k] += dq[k];
+                    } else {
+                        bsum[k * NT + tid] += dp[k];
+                        bsum[(3 + k) * NT + tid] += dq[k];
+                    }
                     if (!(m >> (PM_IH + k) & 1)) dp[k] *= 0.f;
-                    dps[b * 3 * U + k * U + cu] = dp[k];
+                    if constexpr (One) {
+                        o_dp[k] = dp[k];
+                        o_dq[k] = dq[k];
+                    } else {
+                        dps[b * 3 * U + k * U + cu] = dp[k];
+                    }
                 }
-            }
+        };
+        if constexpr (One) {
+            if (act) cell(cb);
+        } else if (j_ok) {
+            for (int b = cb; b < nb; b += KG) cell(b);
         }
         __syncthreads();
         const float *x = dqs + in0;
@@ -473,7 +573,14 @@ __global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
         if (P > 1) cluster_arrive();
         else __syncthreads();
         // (behind the arrive: see the forward)
-        if (j_ok)
+        if constexpr (One) {
+            if (act)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    dp_out[g_off[k]] = o_dp[k];
+                    dq_out[g_off[k]] = o_dq[k];
+                }
+        } else if (j_ok)
             for (int b = cb; b < nb; b += KG) {
                 const float *dpb = dps + b * 3 * U + cu, *dqb = dqs + b * 3 * U + cu;
 #pragma unroll
@@ -495,6 +602,9 @@ __global__ void __launch_bounds__(512, 1) k_bwd_chain(const BwdChainArgs a) {
             const float dh = carry(0, b);
             a.dh_out[at] = a.h0_mask ? dh * (float)a.h0_mask[at] : dh;
         }
+    if constexpr (One)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) bsum[k * NT + tid] = o_sum[k];
     __syncthreads();
     for (int c = tid; c < 6 * U; c += NT) {
         const int k = c / U, uu = c % U;
@@ -603,24 +713,31 @@ void make_plan(qgru_handle *h, int B, Kern kern, size_t (*floats)(int, int, int,
 }  // namespace
 
 bool float_chain_fits(qgru_handle *h, int B) {
-    make_plan(h, B, k_float_chain, fwd_smem_floats, &h->plan_fwd);
+    make_plan(h, B, k_float_chain<false, 512>, fwd_smem_floats, &h->plan_fwd);
     return h->plan_fwd.ok;
 }
 
+// (forms of at most 384 threads have registers to spare beside R: no spills)
 int float_chain_launch(qgru_handle *h, FloatFwdArgs a, cudaStream_t st) {
-    CK(launch_chain(k_float_chain, h->plan_fwd, a, st));
+    const F32RecPlan &pl = h->plan_fwd;
+    const bool one = pl.Bt <= std::min(pl.KG, RB), small = pl.U * pl.KG <= 384;
+    CK(launch_chain(one ? (small ? k_float_chain<true, 384> : k_float_chain<true, 512>)
+                        : (small ? k_float_chain<false, 384> : k_float_chain<false, 512>), pl, a, st));
     h->launches++;
     return QGRU_OK;
 }
 
 bool bwd_chain_fits(qgru_handle *h, int B, int *groups) {
-    make_plan(h, B, k_bwd_chain, bwd_smem_floats, &h->plan_bwd);
+    make_plan(h, B, k_bwd_chain<false, 512>, bwd_smem_floats, &h->plan_bwd);
     *groups = h->plan_bwd.G;
     return h->plan_bwd.ok;
 }
 
 int bwd_chain_launch(qgru_handle *h, BwdChainArgs a, cudaStream_t st) {
-    CK(launch_chain(k_bwd_chain, h->plan_bwd, a, st));
+    const F32RecPlan &pl = h->plan_bwd;
+    const bool one = pl.Bt <= pl.KG, small = pl.U * pl.KG <= 384;
+    CK(launch_chain(one ? (small ? k_bwd_chain<true, 384> : k_bwd_chain<true, 512>) : (small ? k_bwd_chain<false, 384> : k_bwd_chain<false, 512>),
+                    pl, a, st));
     h->launches++;
     return QGRU_OK;
 }
