@@ -330,8 +330,9 @@ class QuantGRU(nn.Module):
 
     # ----------------------------------------------------------------- run-time plumbing
     def _params_of(self, d):
-        suffix = "_reverse" if d == 1 else ""
-        return [getattr(self, n + suffix) for n in ("weight_ih_l0", "weight_hh_l0", "bias_ih_l0", "bias_hh_l0")]
+        if d == 1:
+            return [self.weight_ih_l0_reverse, self.weight_hh_l0_reverse, self.bias_ih_l0_reverse, self.bias_hh_l0_reverse]
+        return [self.weight_ih_l0, self.weight_hh_l0, self.bias_ih_l0, self.bias_hh_l0]
 
     def _handle(self, d, device):
         st = self._dirs[d]
@@ -346,7 +347,9 @@ class QuantGRU(nn.Module):
         return st
 
     def _direction(self, d, device):
-        st = self._handle(d, device)
+        st = self._dirs[d]
+        if st.handle is None or st.handle.device != (device.index or 0):
+            st = self._handle(d, device)
         ps = self._params_of(d)
         key = tuple((p.data_ptr(), p._version) if p is not None else None for p in ps)
         if key != st.weights_key:
@@ -413,33 +416,46 @@ class QuantGRU(nn.Module):
 
     def _layer_forward(self, input, hx, device, dtype):
         """One quantized forward of every direction in one library call: (output, h_n)."""
+        # (one frame of a stream is host time from end to end: no conversion, attribute or temporary that is not needed)
         x = input
-        if x.dtype != dtype or x.device != device or x.stride(-1) != 1:
+        if x.dtype is not dtype or x.device != device or x.stride(-1) != 1:
             x = x.to(device=device, dtype=dtype).contiguous()
-        B, T = x.shape[:2] if self.batch_first else (x.shape[1], x.shape[0])
-        if x.dim() != 3 or x.shape[2] != self.input_size:
-            raise ValueError(f"input must have {self.input_size} features in three dimensions, got {list(x.shape)}")
-        t_dim, b_dim = (1, 0) if self.batch_first else (0, 1)
-        H, D = self.hidden_size, self.num_directions
+        shape = x.shape
+        if len(shape) != 3 or shape[2] != self.input_size:
+            raise ValueError(f"input must have {self.input_size} features in three dimensions, got {list(shape)}")
+        H, D, batch_first = self.hidden_size, self.num_directions, self.batch_first
+        if batch_first:
+            B, T, _ = shape
+            x_bs, x_ts, _ = x.stride()
+        else:
+            T, B, _ = shape
+            x_ts, x_bs, _ = x.stride()
+        h0 = None
         if hx is not None:
             if tuple(hx.shape) != (D, B, H):
                 raise ValueError(f"hx must have shape {[D, B, H]}, got {list(hx.shape)}")
-            hx = hx.to(device=device, dtype=dtype).contiguous()
-        states = [self._ready_quant(d, device) for d in range(D)]
+            if hx.dtype is not dtype or hx.device != device or not hx.is_contiguous():
+                hx = hx.to(device=device, dtype=dtype).contiguous()
+            h0 = hx.data_ptr()
+        h = self._ready_quant(0, device).handle
+        rev = self._ready_quant(1, device).handle._h if D == 2 else None
         # (the library keeps offsets inside a timestep in 32 bits: very long batch-first outputs are transposed)
-        direct = not self.batch_first or T * D * H <= 1 << 25
-        out = torch.empty((B, T, D * H) if self.batch_first and direct else (T, B, D * H), dtype=dtype, device=device)
-        ot, ob = (t_dim, b_dim) if direct else (0, 1)
-        h_n = torch.empty((D, B, H), dtype=dtype, device=device)
-        h = states[0].handle
-        args = (T, B, x.data_ptr(), x.stride(t_dim), x.stride(b_dim), hx.data_ptr() if hx is not None else None,
-                out.data_ptr(), out.stride(ot), out.stride(ob), h_n.data_ptr(),
-                torch._C._cuda_getCurrentRawStream(device.index or 0))
-        rev = states[1].handle._h if D == 2 else None
-        if dtype == torch.int32:
-            h._ck(h._lib.qgru_layer_forward_i32(h._h, rev, *args), "qgru_layer_forward_i32")
+        direct = not batch_first or T * D * H <= 1 << 25
+        if batch_first and direct:
+            out = x.new_empty((B, T, D * H))
+            o_ts, o_bs = D * H, T * D * H
         else:
-            h._ck(h._lib.qgru_layer_forward(h._h, rev, self.quant_storage_dtype != "int32", *args), "qgru_layer_forward")
+            out = x.new_empty((T, B, D * H))
+            o_ts, o_bs = B * D * H, D * H
+        h_n = x.new_empty((D, B, H))
+        stream = torch._C._cuda_getCurrentRawStream(device.index or 0)
+        if dtype is torch.int32:
+            rc = h._lib.qgru_layer_forward_i32(h._h, rev, T, B, x.data_ptr(), x_ts, x_bs, h0, out.data_ptr(), o_ts, o_bs, h_n.data_ptr(), stream)
+        else:
+            rc = h._lib.qgru_layer_forward(h._h, rev, self.quant_storage_dtype != "int32", T, B, x.data_ptr(), x_ts, x_bs, h0, out.data_ptr(),
+                                           o_ts, o_bs, h_n.data_ptr(), stream)
+        if rc:
+            h._ck(rc, "qgru_layer_forward")
         return out if direct else out.transpose(0, 1).contiguous(), h_n
 
     def _forward_train(self, input, hx):
@@ -507,8 +523,10 @@ class QuantGRU(nn.Module):
 
     # --------------------------------------------------------------------------- forward
     def forward(self, input, hx=None):
-        needs_grad = torch.is_grad_enabled() and (input.requires_grad or (hx is not None and hx.requires_grad) or
-                                                  any(p.requires_grad for p in self.parameters()))
+        if not torch.is_grad_enabled():
+            return self._forward_impl(input, hx)
+        needs_grad = (input.requires_grad or (hx is not None and hx.requires_grad) or
+                      any(p.requires_grad for p in self.parameters()))
         if needs_grad and self.training and not self.calibrating:
             if self.use_quantization:
                 self._ensure_quant_ready()
