@@ -138,6 +138,7 @@ void qgru_destroy(qgru_handle *h) {
     if (h->ev_split) cudaEventDestroy(h->ev_split);
     if (h->ev_join) cudaEventDestroy(h->ev_join);
     if (h->side) cudaStreamDestroy(h->side);
+    cudaFree(h->d_stamps);
     cudaFree(h->d_flags);
     if (h->h_flags) cudaFreeHost(h->h_flags);
     cudaFree(h->d_bar);
@@ -168,7 +169,11 @@ int qgru_set_option(qgru_handle *h, const char *name, const char *value) {
         else if (v == "generic") h->opt_rec = 3;
         else if (v == "gemv") h->opt_rec = 4;
         else if (v == "reg") h->opt_rec = 5;
-        else if (v == "fast") h->opt_rec = 6;
+        else if (v == "fast") {
+            CK(cudaSetDevice(h->device));
+            if (int rc = alloc_once(h, &h->d_stamps, (size_t)qgru_handle::kRing * 3)) return rc;
+            h->opt_rec = 6;
+        }
         else return fail(h, QGRU_ERR_BAD_ARG, "rec: auto|dp4a|mma|gemv|reg|fast|generic");
     } else if (n == "exchange") {
         if (v == "auto") h->opt_exchange = 0;
@@ -658,9 +663,17 @@ int launch_gemv_reg(qgru_handle *h, RecArgs &a, cudaStream_t st) {
                                : (notie ? k_recurrence_gemv_reg<HU, IhT, 128, 2, false> : k_recurrence_gemv_reg<HU, IhT, 128, 2, true>);
     const size_t smem = gemv_reg_smem(h, a.n_table);
     CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int threads = 2 * ((h->H + 31) / 32 * 32);
-    kern<<<a.B, threads, smem, st>>>(h->gc_host, a);
-    CK(cudaGetLastError());
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)a.B);
+    cfg.blockDim = dim3(2u * (unsigned)((h->H + 31) / 32 * 32));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = a.stamp ? 1 : 0;
+    CK(cudaLaunchKernelEx(&cfg, kern, (const GateConsts)h->gc_host, a));
     h->launches++;
     return QGRU_OK;
 }
@@ -689,6 +702,7 @@ struct FwdInput {
     void *xq = nullptr;              // optional dense copy of the quantized x
     uint8_t *x_keep = nullptr, *h0_keep = nullptr;
     float *xd = nullptr;             // optional dense copy of the dequantized x
+    unsigned long long *stamp = nullptr;   // start time of the prologue, or null
 };
 
 // The first launch of a forward (k_prologue); x8: null where another handle has quantized the same x.
@@ -722,6 +736,7 @@ int launch_prologue(qgru_handle *h, int T, int B, const FwdInput &in, uint8_t *x
     a.h0_keep = in.h0_keep;
     a.flags = h->d_flags;
     a.sticky = in.mode == 2 ? nullptr : h->h_flags + 2;
+    a.stamp = in.stamp;
     if (in.mode == 2) CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
     a.q_blocks = x8 ? grid_for(a.N * (h->Ipad / 16), 256, h->sm_count) : 0;
     const int blocks = a.q_blocks + grid_for((long long)B * h->Hpad, 256, h->sm_count);
@@ -769,9 +784,11 @@ bool reg_is_faster(const RecRegPlan &pl, bool gemv) {
     return pl.P == 1 || pl.Bt <= (pl.KS == 2 ? 8 : 16);
 }
 
-// The 8-bit path with the register-resident recurrence.
+// The 8-bit path with the register-resident recurrence.  chained: the three launches of the forward as dependent launches,
+// each prepares itself (tensor maps, R to registers, tables) beside the one before; nothing may be recorded between
+// them, so that start times come from the kernels.
 int run_reg(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out, unsigned flags, RecCell cell, const RecRegPlan &pl,
-            int ih_bytes, int n_table, cudaStream_t st) {
+            int ih_bytes, int n_table, bool chained, cudaStream_t st) {
     const long long N = (long long)T * B;
     const int sms = h->opt_sm_limit > 0 ? std::min(h->opt_sm_limit, h->sm_count) : h->sm_count;
     const bool fused = cell <= CELL_INT_FAST_NOTIE;
@@ -779,15 +796,19 @@ int run_reg(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out,
     if ((rc = ensure(h, h->ih, pl.ih_elements(N) * ih_bytes))) return rc;
     PreScale ps = pre_scale(h, fused);
     ps.slice = pl.U;
-    CK(cudaEventRecord(h->ev[1], st));
+    if (!chained) CK(cudaEventRecord(h->ev[1], st));
     const LinearConsts lcx = linear_consts(h, 0);
+    h->tc.pdl = chained;
+    h->tc.stamp = chained ? h->stamp(1) : nullptr;
     if ((rc = tc_gemm_launch(h->tc, x8, (N + 127) / 128 * 128, h->d_w8[0], h->w8_rows[0], h->ih.p, N, h->C, h->Ipad, h->x_uns, ih_bytes, lcx,
                              ps, lcx.fits32 && h->rs_fast[0] && h->opt_cell != 2, h->lin_notie[0] && h->opt_tie != 1, h->d_flags + 1, sms, st,
                              &h->err)))
         return rc;
     h->launches++;
-    CK(cudaEventRecord(h->ev[2], st));
+    if (!chained) CK(cudaEventRecord(h->ev[2], st));
     RecRegArgs a{};
+    a.pdl = chained;
+    a.stamp = chained ? h->stamp(2) : nullptr;
     a.T = T;
     a.B = B;
     a.H = h->H;
@@ -804,6 +825,7 @@ int run_reg(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out,
     a.abort_flag = h->d_flags + 1;
     if ((rc = rec_reg_launch(h, pl, a, cell, ih_bytes, st))) return rc;
     CK(cudaEventRecord(h->ev[3], st));
+    h->stamped[(h->ev - h->ring[0]) / 4] = chained;
     h->timing_valid = true;
     char buf[300];
     snprintf(buf, sizeof(buf), "path=int8 gemm=tcgen05_i8 rec=mma_sync_i8 r_in=registers cell=%s U=%d KS=%d KST=%d P=%d G=%d Bt=%d D=%d smem=%zu ih_bytes=%d",
@@ -858,7 +880,7 @@ int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out
         RecRegPlan &rp = h->plan_reg;
         const bool fits = rec_reg_plan(h, B, sms, bytes, cell, n_tab, &rp);
         if (!fits && h->opt_rec == 5) return fail(h, QGRU_ERR_UNSUPPORTED, "rec=reg needs H <= 1024 and room for its tables");
-        if (fits && (h->opt_rec == 5 || reg_is_faster(rp, use_gemv))) return run_reg(h, T, B, x8, out, flags, cell, rp, bytes, n_tab, st);
+        if (fits && (h->opt_rec == 5 || reg_is_faster(rp, use_gemv))) return run_reg(h, T, B, x8, out, flags, cell, rp, bytes, n_tab, h->opt_rec == 6, st);
     }
     // the fused cell needs the GEMM epilogue to pre-rescale W*x+bw: tensor-core GEMM only
     // (the one-CTA-per-row form takes it only in its branch-free shape: every scale shift-free)
@@ -909,7 +931,8 @@ int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out
     auto chunk_t0 = [&](int k) { return rev_dir ? T - (k * Tc + chunk_T(k)) : k * Tc; };
     auto chunk_ih = [&](int k) { return (void *)((char *)h->ih.p + (n_chunks > 1 ? (size_t)(k & 1) * chunk_bytes : 0)); };
 
-    CK(cudaEventRecord(h->ev[1], st));
+    const bool chained = h->opt_rec == 6 && use_gemv && h->opt_gemm != 1 && gemv_reg_ok(h, fused);
+    if (!chained) CK(cudaEventRecord(h->ev[1], st));
     const LinearConsts lcx = linear_consts(h, 0);
     bool used_tc = false;
     // the W*x GEMM of chunk k on stream `gs`
@@ -918,6 +941,8 @@ int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out
         // (the launcher also looks at how the second rescale is applied: table or shift-free scale)
         const bool gemm_fast = lcx.fits32 && h->rs_fast[0] && h->opt_cell != 2;
         const long long Nk = (long long)chunk_T(k) * B;
+        h->tc.pdl = chained;
+        h->tc.stamp = chained ? h->stamp(1) : nullptr;
         const int r = tc_gemm_launch(h->tc, x8, (N + 127) / 128 * 128, h->d_w8[0], h->w8_rows[0],
                                      chunk_ih(k), Nk, C, h->Ipad, h->x_uns, ih_bytes, lcx, ps, gemm_fast,
                                      h->lin_notie[0] && h->opt_tie != 1, h->d_flags + 1, sms, gs, &h->err,
@@ -949,7 +974,7 @@ int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out
         CK(cudaGetLastError());
         h->launches++;
     }
-    CK(cudaEventRecord(h->ev[2], st));
+    if (!chained) CK(cudaEventRecord(h->ev[2], st));
 
     const int groups = use_mma ? mp.G : pl.G;
     if (groups > h->bar_groups) {
@@ -1039,6 +1064,7 @@ int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out
         a.abort_flag = h->d_flags + 1;
         a.spin_limit = h->spin_limit;
         a.withhold_arrive = h->opt_withhold ? 1 : 0;
+        if (chained) a.stamp = h->stamp(2);
         if (use_gemv) {
             if (fused) {
                 a.tables = h->d_ftables;
@@ -1061,6 +1087,7 @@ int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out
         }
     }
     CK(cudaEventRecord(h->ev[3], st));
+    h->stamped[(h->ev - h->ring[0]) / 4] = chained;
     h->timing_valid = true;
     h->plan_text = buf;
     return QGRU_OK;
@@ -1161,7 +1188,7 @@ int forward_dir(qgru_handle *h, int T, int B, const FwdInput &in, const OutView 
     const size_t init_slot = rev ? (size_t)T : 0;
     int rc;
     h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->calls++;
+    h->stamped[h->calls++ % qgru_handle::kRing] = false;
     CK(cudaEventRecord(h->ev[0], st));
     if (use_generic(h)) {
         // dense int32 states, step by step; then to the view
@@ -1219,7 +1246,9 @@ int forward_dir(qgru_handle *h, int T, int B, const FwdInput &in, const OutView 
         x8 = (const uint8_t *)h->x8.p;
     }
     if ((rc = ensure(h, h->h8, (size_t)(2 * B + 256) * h->Hpad))) return rc;
-    if ((rc = launch_prologue(h, T, B, in, x8_shared ? nullptr : (uint8_t *)h->x8.p, (uint8_t *)h->h8.p,
+    FwdInput first = in;
+    first.stamp = h->opt_rec == 6 ? h->stamp(0) : nullptr;
+    if ((rc = launch_prologue(h, T, B, first, x8_shared ? nullptr : (uint8_t *)h->x8.p, (uint8_t *)h->h8.p,
                               with_slot0 ? out.shifted(init_slot) : OutView(), st)))
         return rc;
     if (after_prologue) CK(cudaEventRecord(after_prologue, st));
@@ -1251,7 +1280,7 @@ int qgru_forward_i32_train(qgru_handle *h, int T, int B, const int32_t *x_q, con
     cudaStream_t st = (cudaStream_t)stream;
     const long long init_slot = (flags & QGRU_FLAG_REVERSE) ? T : 0;
     h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->calls++;
+    h->stamped[h->calls++ % qgru_handle::kRing] = false;
     CK(cudaEventRecord(h->ev[0], st));
     // the step-by-step kernels keep every intermediate the training buffer wants
     OutView slot;
@@ -1339,15 +1368,29 @@ int qgru_forward_f32_host(qgru_handle *h, int T, int B, const float *x, const fl
     return qgru_synchronize(h, stream);
 }
 
+// The three times of ring slot k; a chained forward has start times on the GPU's clock in place of its middle events.
+static int slot_times(qgru_handle *h, int k, float *a, float *b, float *c) {
+    cudaEvent_t *e = h->ring[k];
+    CK(cudaEventSynchronize(e[3]));
+    CK(cudaEventElapsedTime(c, e[0], e[3]));
+    if (h->stamped[k]) {
+        unsigned long long t[3];
+        CK(cudaMemcpy(t, h->d_stamps + 3 * k, sizeof(t), cudaMemcpyDeviceToHost));
+        *a = (float)((double)(t[2] - t[1]) * 1e-6);
+        *b = std::max(0.f, *c - (float)((double)(t[2] - t[0]) * 1e-6));
+        return QGRU_OK;
+    }
+    CK(cudaEventElapsedTime(a, e[1], e[2]));
+    CK(cudaEventElapsedTime(b, e[2], e[3]));
+    return QGRU_OK;
+}
+
 int qgru_last_timing(qgru_handle *h, float *ms_input_gemm, float *ms_recurrence, float *ms_total) {
     if (!h) return QGRU_ERR_BAD_ARG;
     if (!h->timing_valid) return fail(h, QGRU_ERR_NOT_READY, "no forward has run");
     CK(cudaSetDevice(h->device));
-    CK(cudaEventSynchronize(h->ev[3]));
     float a = 0, b = 0, c = 0;
-    CK(cudaEventElapsedTime(&a, h->ev[1], h->ev[2]));
-    CK(cudaEventElapsedTime(&b, h->ev[2], h->ev[3]));
-    CK(cudaEventElapsedTime(&c, h->ev[0], h->ev[3]));
+    if (int rc = slot_times(h, (int)((h->ev - h->ring[0]) / 4), &a, &b, &c)) return rc;
     if (ms_input_gemm) *ms_input_gemm = a;
     if (ms_recurrence) *ms_recurrence = b;
     if (ms_total) *ms_total = c;
@@ -1362,12 +1405,8 @@ int qgru_timing_window(qgru_handle *h, int *n_calls, float *ms_input_gemm, float
     int n = std::min<long long>(std::min<long long>(*n_calls, qgru_handle::kRing), (long long)h->calls);
     float sa = 0, sb = 0, sc = 0;
     for (int k = 0; k < n; ++k) {
-        cudaEvent_t *e = h->ring[(h->calls - 1 - k) % qgru_handle::kRing];
-        CK(cudaEventSynchronize(e[3]));
         float a = 0, b = 0, c = 0;
-        CK(cudaEventElapsedTime(&a, e[1], e[2]));
-        CK(cudaEventElapsedTime(&b, e[2], e[3]));
-        CK(cudaEventElapsedTime(&c, e[0], e[3]));
+        if (int rc = slot_times(h, (int)((h->calls - 1 - k) % qgru_handle::kRing), &a, &b, &c)) return rc;
         sa += a; sb += b; sc += c;
     }
     *n_calls = n;
@@ -1465,7 +1504,7 @@ extern "C" int qgru_forward_i32_static(qgru_handle *h, int T, int B, const int32
     OutView out = dense_view(h, B);
     out.hq = h_q;
     h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->calls++;
+    h->stamped[h->calls++ % qgru_handle::kRing] = false;
     CK(cudaEventRecord(h->ev[0], st));
     // the array keeps what the previous call left: the state buffers' padding columns and the
     // step counters must start at zero

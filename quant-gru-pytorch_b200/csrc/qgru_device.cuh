@@ -173,6 +173,20 @@ __device__ __forceinline__ int32_t gru_cell_fused(const GateConsts &gc, const in
     return clampi((int32_t)rescale32(comb, gc.uh_to_h) + gc.zp_h, gc.h_lo, gc.h_hi);
 }
 
+// Programmatic dependent launch: a kernel lets the next one of its stream start early (its own work is not affected), and
+// the next one waits, before it reads what came before, until that has completed and is visible.  Both do
+// nothing in a launch without the attribute.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Start of this kernel's work on the GPU's clock (ns), by one thread of the grid (stamp: null or where to put it).
+__device__ __forceinline__ void put_stamp(unsigned long long *stamp) {
+    if (stamp && blockIdx.x == 0 && threadIdx.x == 0) {
+        unsigned long long t;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+        *stamp = t;
+    }
+}
+
 // 32-bit load from a shared-memory window address: table lookups stay on the shared-memory
 // path with 32-bit address arithmetic.
 __device__ __forceinline__ int32_t lds_i32(uint32_t addr) {

@@ -321,7 +321,7 @@ int fstorage_train_tail(qgru_handle *h, int T, int B, FwdInput in, float *h_out,
     uint8_t *h8 = (uint8_t *)h->h8.p;
     const size_t h8_half = (size_t)B * h->Hpad;
     h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->calls++;
+    h->stamped[h->calls++ % qgru_handle::kRing] = false;
     CK(cudaEventRecord(h->ev[0], st));
     in.x_keep = tr.m.x;
     in.h0_keep = tr.m.h0;
@@ -526,13 +526,18 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
     if ((rc = ensure(h, h->ih, (use_reg ? rp.ih_elements(N) : (size_t)N * C) * ih_bytes))) return rc;
 
     h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->calls++;
+    h->stamped[h->calls++ % qgru_handle::kRing] = false;
     CK(cudaEventRecord(h->ev[0], st));
-    if ((rc = launch_prologue(h, T, B, in, x8_shared ? nullptr : (uint8_t *)h->x8.p, h8,
+    // dependent launches (see run_reg): the register-resident forms only
+    const bool in_regs = h->opt_gemv_r != 1 && (h->Hpad == 128 || h->Hpad == 256);
+    const bool chained = h->opt_rec == 6 && h->opt_gemm != 1 && (use_reg || (small && in_regs && gemv_smem(h, n_tab) <= (size_t)h->smem_optin));
+    FwdInput first = in;
+    first.stamp = chained ? h->stamp(0) : nullptr;
+    if ((rc = launch_prologue(h, T, B, first, x8_shared ? nullptr : (uint8_t *)h->x8.p, h8,
                               with_slot0 ? out.shifted(rev ? (size_t)T : 0) : OutView(), st)))
         return rc;
     if (after_prologue) CK(cudaEventRecord(after_prologue, st));
-    CK(cudaEventRecord(h->ev[1], st));
+    if (!chained) CK(cudaEventRecord(h->ev[1], st));
     // the input projection: exact int32 sums on the tensor cores (dp4a form as fallback), float
     // requantization in the epilogue
     LinearConsts lcx = linear_consts(h, 0);
@@ -542,6 +547,8 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
     if (h->opt_gemm != 1) {
         PreScale ps{};
         ps.slice = use_reg ? rp.U : H;
+        h->tc.pdl = chained;
+        h->tc.stamp = chained ? h->stamp(1) : nullptr;
         rc = tc_gemm_launch(h->tc, x8, (N + 127) / 128 * 128, h->d_w8[0], h->w8_rows[0],
                             h->ih.p, N, C, h->Ipad, h->x_uns, ih_bytes, lcx, ps, false, false, h->d_flags + 1, sms, st,
                             &h->err);
@@ -559,7 +566,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
         }
         CK(cudaGetLastError());
     }
-    CK(cudaEventRecord(h->ev[2], st));
+    if (!chained) CK(cudaEventRecord(h->ev[2], st));
     h->launches += 1;
     char buf[256];
     RecPlan pl;
@@ -570,6 +577,8 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
                             rec_cluster_plan(H, h->Hpad, B, sms, h->smem_optin, n_tab, h->opt_r_where, h->opt_mt, h->opt_ng, h->opt_kp, &cp);
     if (use_reg) {
         RecRegArgs a{};
+        a.pdl = chained;
+        a.stamp = chained ? h->stamp(2) : nullptr;
         a.T = T; a.B = B; a.H = H; a.Hpad = h->Hpad;
         a.reverse = rev ? 1 : 0;
         a.r8 = h->d_w8[1];
@@ -629,7 +638,6 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
         a.fs_chan = chan + (size_t)3 * C;
         a.fs = fc;
         // R in registers where the form exists (Hpad 128 or 256; option gemv_r=smem: in shared memory)
-        const bool in_regs = h->opt_gemv_r != 1 && (h->Hpad == 128 || h->Hpad == 256);
         size_t smem;
         if (in_regs) {
             const size_t units = (size_t)(H + 31) / 32 * 32;
@@ -641,7 +649,18 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
                             : (ih_bytes == 1 ? (h->h_uns ? k_recurrence_gemv_reg<true, int8_t, 128, 3> : k_recurrence_gemv_reg<false, int8_t, 128, 3>)
                                              : (h->h_uns ? k_recurrence_gemv_reg<true, int16_t, 128, 3> : k_recurrence_gemv_reg<false, int16_t, 128, 3>));
             CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            kern<<<B, 2 * (int)units, smem, st>>>(h->gc_host, a);
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)B);
+            cfg.blockDim = dim3(2u * (unsigned)units);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = chained ? 1 : 0;
+            a.stamp = chained ? h->stamp(2) : nullptr;
+            CK(cudaLaunchKernelEx(&cfg, kern, (const GateConsts)h->gc_host, a));
         } else {
             auto kern = ih_bytes == 1 ? (h->h_uns ? k_recurrence_gemv<true, int8_t, 3> : k_recurrence_gemv<false, int8_t, 3>)
                                       : (h->h_uns ? k_recurrence_gemv<true, int16_t, 3> : k_recurrence_gemv<false, int16_t, 3>);
@@ -720,6 +739,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
     }
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->ev[3], st));
+    h->stamped[(h->ev - h->ring[0]) / 4] = chained;
     h->timing_valid = true;
     h->plan_text = buf;
     return QGRU_OK;

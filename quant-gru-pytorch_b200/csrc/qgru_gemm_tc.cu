@@ -172,6 +172,9 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
     __syncthreads();
     tc::tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_trigger();
+    pdl_wait();
+    put_stamp(ps.stamp);
 
     if (warp == 0) {
         if (lane == 0) {
@@ -460,7 +463,7 @@ size_t astat_smem(int) { return (size_t)STAGES_A * GN * KB + 1024 + 256 + PRE_TA
 
 template <bool XU, typename IhT, bool Fast, bool Tie>
 cudaError_t launch_f(const CUtensorMap &mw, const CUtensorMap &mx, void *ih, long long N, int C, int Kpad,
-                     LinearConsts lc, PreScale ps, int *abort_flag, int sms, int order, int x_row0, cudaStream_t st) {
+                     LinearConsts lc, PreScale ps, int *abort_flag, int sms, int order, int x_row0, bool pdl, cudaStream_t st) {
     const int m_tiles = (C + GM - 1) / GM;
     const long long n_tiles = (N + GN - 1) / GN;
     // W-stationary form (W in tensor memory): on request only (option gemm_order=w_stationary), it is
@@ -481,17 +484,26 @@ cudaError_t launch_f(const CUtensorMap &mw, const CUtensorMap &mx, void *ih, lon
     if (e != cudaSuccess) return e;
     const long long tiles = (long long)m_tiles * n_tiles;
     const unsigned grid = (unsigned)std::min<long long>(tiles, sms);   // persistent: one CTA per SM
-    kern<<<grid, GEMM_THREADS, GEMM_SMEM, st>>>(mw, mx, (IhT *)ih, N, C, Kpad, lc, ps, abort_flag, x_row0);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = GEMM_SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, mw, mx, (IhT *)ih, N, C, Kpad, lc, ps, abort_flag, x_row0);
 }
 
 template <bool XU, typename IhT>
 cudaError_t launch(const CUtensorMap &mw, const CUtensorMap &mx, void *ih, long long N, int C, int Kpad,
                    LinearConsts lc, PreScale ps, bool fast, bool notie, int *abort_flag, int sms, int order,
-                   int x_row0, cudaStream_t st) {
-    if (fast && notie) return launch_f<XU, IhT, true, false>(mw, mx, ih, N, C, Kpad, lc, ps, abort_flag, sms, order, x_row0, st);
-    return fast ? launch_f<XU, IhT, true, true>(mw, mx, ih, N, C, Kpad, lc, ps, abort_flag, sms, order, x_row0, st)
-                : launch_f<XU, IhT, false, true>(mw, mx, ih, N, C, Kpad, lc, ps, abort_flag, sms, order, x_row0, st);
+                   int x_row0, bool pdl, cudaStream_t st) {
+    if (fast && notie) return launch_f<XU, IhT, true, false>(mw, mx, ih, N, C, Kpad, lc, ps, abort_flag, sms, order, x_row0, pdl, st);
+    return fast ? launch_f<XU, IhT, true, true>(mw, mx, ih, N, C, Kpad, lc, ps, abort_flag, sms, order, x_row0, pdl, st)
+                : launch_f<XU, IhT, false, true>(mw, mx, ih, N, C, Kpad, lc, ps, abort_flag, sms, order, x_row0, pdl, st);
 }
 
 }  // namespace
@@ -500,6 +512,10 @@ int tc_gemm_launch(TcGemmState &s, const uint8_t *x8, long long x_rows_alloc, co
                    long long w_rows_alloc, void *ih, long long N, int C, int Kpad, bool x_unsigned,
                    int ih_bytes, LinearConsts lc, PreScale ps, bool fast, bool notie, int *abort_flag, int sms,
                    cudaStream_t stream, std::string *err, long long x_row0) {
+    const bool pdl = s.pdl;
+    ps.stamp = s.stamp;
+    s.pdl = false;
+    s.stamp = nullptr;
     // (token tiles that reach past the last allocated row read the tensor map's zero fill)
     if (Kpad % KB != 0 || x_row0 < 0 || x_row0 + N > x_rows_alloc || x_rows_alloc >= 0x7fffffffll ||
         (x_row0 == 0 && x_rows_alloc < (N + GN - 1) / GN * GN) || w_rows_alloc < (C + GM - 1) / GM * GM) {
@@ -530,14 +546,14 @@ int tc_gemm_launch(TcGemmState &s, const uint8_t *x8, long long x_rows_alloc, co
     fast = fast && (!ps.enabled || tab || (ps.to[0].mq != 0 && ps.to[1].mq != 0 && ps.to[2].mq != 0));
     cudaError_t e;
     if (ih_bytes == 1)
-        e = x_unsigned ? launch<true, int8_t>(mw, mx, ih, N, C, Kpad, lc, ps, fast, notie, abort_flag, sms, s.order, (int)x_row0, stream)
-                       : launch<false, int8_t>(mw, mx, ih, N, C, Kpad, lc, ps, fast, notie, abort_flag, sms, s.order, (int)x_row0, stream);
+        e = x_unsigned ? launch<true, int8_t>(mw, mx, ih, N, C, Kpad, lc, ps, fast, notie, abort_flag, sms, s.order, (int)x_row0, pdl, stream)
+                       : launch<false, int8_t>(mw, mx, ih, N, C, Kpad, lc, ps, fast, notie, abort_flag, sms, s.order, (int)x_row0, pdl, stream);
     else if (ih_bytes == 2)
-        e = x_unsigned ? launch<true, int16_t>(mw, mx, ih, N, C, Kpad, lc, ps, fast, notie, abort_flag, sms, s.order, (int)x_row0, stream)
-                       : launch<false, int16_t>(mw, mx, ih, N, C, Kpad, lc, ps, fast, notie, abort_flag, sms, s.order, (int)x_row0, stream);
+        e = x_unsigned ? launch<true, int16_t>(mw, mx, ih, N, C, Kpad, lc, ps, fast, notie, abort_flag, sms, s.order, (int)x_row0, pdl, stream)
+                       : launch<false, int16_t>(mw, mx, ih, N, C, Kpad, lc, ps, fast, notie, abort_flag, sms, s.order, (int)x_row0, pdl, stream);
     else
-        e = x_unsigned ? launch<true, int32_t>(mw, mx, ih, N, C, Kpad, lc, ps, fast, notie, abort_flag, sms, s.order, (int)x_row0, stream)
-                       : launch<false, int32_t>(mw, mx, ih, N, C, Kpad, lc, ps, fast, notie, abort_flag, sms, s.order, (int)x_row0, stream);
+        e = x_unsigned ? launch<true, int32_t>(mw, mx, ih, N, C, Kpad, lc, ps, fast, notie, abort_flag, sms, s.order, (int)x_row0, pdl, stream)
+                       : launch<false, int32_t>(mw, mx, ih, N, C, Kpad, lc, ps, fast, notie, abort_flag, sms, s.order, (int)x_row0, pdl, stream);
     if (e != cudaSuccess) {
         if (err) *err = std::string("tcgen05 GEMM launch: ") + cudaGetErrorString(e);
         return QGRU_ERR_CUDA;

@@ -99,6 +99,11 @@ struct qgru_handle {
     static constexpr int kRing = 64;
     cudaEvent_t ring[kRing][4] = {};   // per forward: start, gemm start, gemm end, recurrence end
     cudaEvent_t *ev = ring[0];          // the slot the current forward records into
+    // forwards launched as a chain of dependent launches have no events between their kernels: start times on the
+    // GPU's clock instead (prologue, product, recurrence), valid where stamped is set
+    unsigned long long *d_stamps = nullptr;   // [kRing][3]
+    bool stamped[kRing] = {};
+    unsigned long long *stamp(int k) { return d_stamps + (ev - ring[0]) / 4 * 3 + k; }
     uint64_t calls = 0;                 // forwards issued
     bool timing_valid = false;
     uint64_t launches = 0;

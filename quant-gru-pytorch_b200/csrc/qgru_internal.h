@@ -109,6 +109,7 @@ struct PreScale {
     int32_t slice;          // hidden units per slice of the stored tensor [H / slice][N][3][slice]; 0: H, i.e. [N][3H]
     Rescale to[3];
     int32_t zp_in[3];
+    unsigned long long *stamp;   // the product's start time, or null (set by the launcher)
     // optional table of that function over the clamped W*x+bw range (gate-major, n entries per
     // gate, index = value - lo); null when the range is too wide to tabulate
     const int32_t *table;

@@ -52,6 +52,7 @@ struct PrologueArgs {
     int *flags;                  // [2]
     volatile int *sticky;        // mapped host word or null: do not clear the flags
     int q_blocks;                // blocks that quantize x; the rest write the state
+    unsigned long long *stamp;   // start time, or null
 };
 
 template <int Mode>
@@ -78,6 +79,8 @@ __device__ __forceinline__ int32_t prologue_quantize(const void *src, long long 
 // multiple of 4), one 128-bit store.  Memory-bound: 51200 x 256 fp32 (cfg2) 18 us, 37 us with scalar loads.
 template <int Mode, bool Vec>
 __global__ void __launch_bounds__(256) k_prologue(const PrologueArgs a) {
+    pdl_trigger();
+    put_stamp(a.stamp);
     if (blockIdx.x == 0 && threadIdx.x == 0 && a.sticky) {
         if (a.flags[1]) *a.sticky = a.flags[1];
         a.flags[0] = 0;
@@ -314,6 +317,7 @@ struct RecArgs {
     // quantGRUForwardFP; fs_chan = [3][C] offset, bias term, scale ratio of R*h + br per channel
     const float *fs_chan = nullptr;
     FsConsts fs{};
+    unsigned long long *stamp = nullptr;   // start time (k_recurrence_gemv_reg)
 };
 
 // One CTA owns Hs hidden units (all three gates) of one group of Bt batch rows and keeps its
@@ -642,11 +646,6 @@ __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_con
     const bool j_ok = j < a.H;
 
     for (int i = tid; i < a.n_table; i += NT) tables[i] = a.tables[i];
-    for (int i = tid; i < 2 * KT; i += NT) {
-        const int at = (i / KT) * QS + (i % KT);
-        hs[at] = a.h8[(size_t)b * a.Hpad + i];      // initial state of this row (buffer 0 of h8)
-        hs[HS + at] = 0;
-    }
     if constexpr (Cell == 2) {
         for (int i = tid; i < 3 * units; i += NT) {
             const int g = i / units, u = i % units;
@@ -671,6 +670,14 @@ __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_con
             R[g][4 * c + 2] = w.z;
             R[g][4 * c + 3] = w.w;
         }
+    // (everything up to here is the handle's own and may run beside the launches before)
+    pdl_wait();
+    put_stamp(a.stamp);
+    for (int i = tid; i < 2 * KT; i += NT) {
+        const int at = (i / KT) * QS + (i % KT);
+        hs[at] = a.h8[(size_t)b * a.Hpad + i];      // initial state of this row (buffer 0 of h8)
+        hs[HS + at] = 0;
+    }
     __syncthreads();
 
     const IhT *ihp = reinterpret_cast<const IhT *>(a.ih);

@@ -123,13 +123,15 @@ int rec_reg_launch(qgru_handle *h, const RecRegPlan &pl, RecRegArgs a, RecCell c
     cfg.blockDim = dim3((unsigned)(pl.U / 16 * pl.KS * 32));
     cfg.dynamicSmemBytes = pl.smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)pl.P;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = a.pdl ? 2 : 1;
     CK(cudaLaunchKernelEx(&cfg, kern, (const GateConsts)h->gc_host, (const RecRegArgs)a));
     h->launches++;
     return QGRU_OK;

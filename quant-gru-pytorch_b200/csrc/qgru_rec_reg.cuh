@@ -42,6 +42,8 @@ struct RecRegArgs {
     FsTrainConsts tc;
     int U, P, Bt, NT, D, vec2;       // set by the launcher
     int *abort_flag;
+    bool pdl;                     // launched beside the product before it (programmatic dependent launch)
+    unsigned long long *stamp;    // start time, or null
 };
 
 typedef void (*RegKernel)(const GateConsts, const RecRegArgs);

@@ -142,6 +142,9 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
             for (int k = 0; k < 3; ++k) reinterpret_cast<float *>(consts)[k * 3 * U + i] = ok ? a.fs_chan[(size_t)k * 3 * H + g * H + j] : 0.f;
         }
     }
+    // (everything up to here is the handle's own and may run beside the launches before)
+    pdl_wait();
+    put_stamp(a.stamp);
     // initial state: the rows of the cluster, all K inputs
     for (int i = tid; i < nb * (K >> 4); i += NTH) {
         const int b = i / (K >> 4), k = (i - b * (K >> 4)) * 16;

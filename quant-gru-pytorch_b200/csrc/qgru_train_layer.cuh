@@ -219,11 +219,13 @@ int train_forward_dir(qgru_handle *h, int mode, int T, int B, const void *x, lon
     PreScale ps{};
     ps.H = H;
     ps.slice = pl.U;
+    h->tc.pdl = true;             // (dependent launches: nothing is recorded between them here)
     if ((rc = tc_gemm_launch(h->tc, x8, (N + 127) / 128 * 128, h->d_w8[0], h->w8_rows[0], h->ih.p, N, C, h->Ipad, h->x_uns, ih_bytes, lcx, ps,
                              false, false, h->d_flags + 1, sms, st, &h->err)))
         return rc;
     h->launches++;
     RecRegArgs a{};
+    a.pdl = true;
     a.T = T;
     a.B = B;
     a.H = H;
