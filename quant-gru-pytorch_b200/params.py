@@ -339,11 +339,9 @@ class GRUQuantParams:
             entry = {"dtype": ("UINT" if uns else "INT") + str(int(o.bits)),
                      "symmetric": bool(o.symmetric)}
             if n in WEIGHT_OPS:
-                sc = self.scales[n]
-                entry.update(scale=[float(s) for s in sc], zero_point=[0] * len(sc),
-                             enc_type="PER_CHANNEL",
-                             real_min=[float(s) * qmin for s in sc],
-                             real_max=[float(s) * qmax for s in sc])
+                sc = np.asarray(self.scales[n], np.float64)    # (3H values each: no Python loop over them)
+                entry.update(scale=sc.tolist(), zero_point=[0] * len(sc), enc_type="PER_CHANNEL",
+                             real_min=(sc * qmin).tolist(), real_max=(sc * qmax).tolist())
             else:
                 entry.update(scale=float(o.scale), zero_point=int(o.zero_point),
                              enc_type="PER_TENSOR",
