@@ -17,6 +17,7 @@ namespace qgru {
 namespace {
 
 constexpr int BK = 16;
+constexpr int PART_MIN = 32;   // shortest K part
 
 // One operand's BK x BT slab: thread-held values on their way from global to shared memory.
 // Trans = false: element (row, k) at src[row * K + k]; true: at src[k * rows + row].  Stored as
@@ -189,12 +190,14 @@ void launch_bt(const GemmF32 &g, int parts, long long k_part, float *ws, bool va
 
 int gemm_f32(qgru_handle *h, const GemmF32 &g, cudaStream_t st) {
     // 128 x 128 tiles where they alone (or with few K parts) fill the SMs: half the operand traffic of
-    // 64 x 64.  K is split while that leaves SMs idle, in parts of at least 128.
+    // 64 x 64.  K is split while that leaves SMs idle, in parts of two
+    // slabs or more: with two warps on an SM a slab takes about a microsecond (384 x 64 x 1600 and its two neighbours of a
+    // training step: 97 us with parts of 128, 73 with 32).
     const auto tiles = [&](int bt) { return ((g.N + bt - 1) / bt) * ((g.M + bt - 1) / bt); };
     const bool big = tiles(128) * std::max<long long>(1, g.K / 512) >= h->sm_count && g.N > 64 && g.M > 64;
     const long long t = big ? tiles(128) : tiles(64);
     const long long want = big ? 2ll * h->sm_count : 4ll * h->sm_count;
-    long long parts = std::max<long long>(1, std::min({want / std::max<long long>(1, t), g.K / 128, (long long)64}));
+    long long parts = std::max<long long>(1, std::min({want / std::max<long long>(1, t), g.K / PART_MIN, (long long)64}));
     if (t >= h->sm_count) parts = 1;
     long long k_part = ((g.K + parts - 1) / parts + BK - 1) / BK * BK;
     parts = (g.K + k_part - 1) / k_part;
