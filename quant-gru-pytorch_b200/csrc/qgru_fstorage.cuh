@@ -384,6 +384,7 @@ int fstorage_train_tail(qgru_handle *h, int T, int B, FwdInput in, float *h_out,
 // weights (chan: k_fs_channel_consts, k_train_weights), the gate tables, their training form.
 struct FsSetup {
     FsConsts fc;
+    bool tab_possible = false;  // every gate input is narrow enough to tabulate
     int n_tab = 0;              // entries of the gate tables, 0: gates are evaluated
     int n_train_tab = 0;        // the same for the training form (its outputs need the lowest mantissa bit free)
     FsChannels ch;
@@ -391,9 +392,10 @@ struct FsSetup {
     uint32_t *train_tab;
 };
 
-int fs_setup(qgru_handle *h, FsSetup &s, cudaStream_t st) {
+// The host's part: constants and table sizes, which is all that a plan needs.  Nothing is queued, so that a query may call
+// it without knowing the stream of the call that follows.
+void fs_constants(const qgru_handle *h, FsSetup &s) {
     const qgru_params &p = h->p;
-    const int C = h->C;
     FsConsts &fc = s.fc;
     // ---- constants (setRescaleParam, src/gru_forward_gpu_quant_fp.cu:821-1003): float ratios
     // of the stored scales, computed in the same float operations
@@ -432,19 +434,27 @@ int fs_setup(qgru_handle *h, FsSetup &s, cudaStream_t st) {
 
     // gate tables where every gate input has at most 10 bits (3 x 1024 floats of shared memory);
     // option cell=generic keeps the tables out of the kernels (every gate is evaluated)
-    bool tab_possible = true;
+    s.tab_possible = true;
     int tab_total = 0;
     for (int g = 0; g < 3; ++g) {
         const int n = (int)(fc.in_hi[g] - fc.in_lo[g]) + 1;
-        if (n > 1024) tab_possible = false;
+        if (n > 1024) s.tab_possible = false;
         fc.tab_off[g] = tab_total;
         tab_total += n;
     }
-    fc.tab_on = (tab_possible && h->opt_cell != 1) ? 1 : 0;
+    fc.tab_on = (s.tab_possible && h->opt_cell != 1) ? 1 : 0;
     s.n_tab = fc.tab_on ? tab_total : 0;
     s.n_train_tab = s.n_tab;
     for (int g = 0; g < 3; ++g)
         if (p.op[op_out[g]].bits > 16) s.n_train_tab = 0;
+}
+
+// The constants, and the device's part on the stream of the call that reads it.
+int fs_setup(qgru_handle *h, FsSetup &s, cudaStream_t st) {
+    fs_constants(h, s);
+    const qgru_params &p = h->p;
+    const qgru_op &ox = p.op[QGRU_OP_X], &oh = p.op[QGRU_OP_H], &oih = p.op[QGRU_OP_IH_LINEAR], &ohh = p.op[QGRU_OP_HH_LINEAR];
+    const int C = h->C;
     int rc;
     if ((rc = ensure(h, h->fs_ch, ((size_t)10 * C + 6 * 1024) * sizeof(float)))) return rc;
     float *chp = (float *)h->fs_ch.p;
@@ -464,9 +474,9 @@ int fs_setup(qgru_handle *h, FsSetup &s, cudaStream_t st) {
         }
         CK(cudaMemcpyAsync(chp, hostc.data(), hostc.size() * sizeof(float), cudaMemcpyHostToDevice, st));
         CK(cudaStreamSynchronize(st));   // hostc leaves scope
-        if (tab_possible) {
-            k_fs_tables<<<3, 256, 0, st>>>(fc, s.gate_tab);
-            k_fs_train_tables<<<3, 256, 0, st>>>(fc, s.train_tab);
+        if (s.tab_possible) {
+            k_fs_tables<<<3, 256, 0, st>>>(s.fc, s.gate_tab);
+            k_fs_train_tables<<<3, 256, 0, st>>>(s.fc, s.train_tab);
         }
         CK(cudaGetLastError());
         h->launches += 2;

@@ -312,7 +312,7 @@ int qgru_train_saved_bytes(qgru_handle *h, int mode, int T, int B, size_t *bytes
     int n_tab = h->n_ttable;
     if (mode == 1 && h->fast) {
         qgru::FsSetup fs;
-        if ((rc = qgru::fs_setup(h, fs, nullptr))) return rc;
+        qgru::fs_constants(h, fs);
         n_tab = fs.n_train_tab;
     }
     if ((rc = qgru::train_plan(h, mode, B, n_tab, &ok))) return rc;
