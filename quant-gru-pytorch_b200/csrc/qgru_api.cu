@@ -825,7 +825,7 @@ int run_reg(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out,
     a.abort_flag = h->d_flags + 1;
     if ((rc = rec_reg_launch(h, pl, a, cell, ih_bytes, st))) return rc;
     CK(cudaEventRecord(h->ev[3], st));
-    h->stamped[(h->ev - h->ring[0]) / 4] = chained;
+    h->stamped[h->slot()] = chained;
     h->timing_valid = true;
     char buf[300];
     snprintf(buf, sizeof(buf), "path=int8 gemm=tcgen05_i8 rec=mma_sync_i8 r_in=registers cell=%s U=%d KS=%d KST=%d P=%d G=%d Bt=%d D=%d smem=%zu ih_bytes=%d",
@@ -1087,7 +1087,7 @@ int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out
         }
     }
     CK(cudaEventRecord(h->ev[3], st));
-    h->stamped[(h->ev - h->ring[0]) / 4] = chained;
+    h->stamped[h->slot()] = chained;
     h->timing_valid = true;
     h->plan_text = buf;
     return QGRU_OK;
@@ -1187,8 +1187,7 @@ int forward_dir(qgru_handle *h, int T, int B, const FwdInput &in, const OutView 
     const bool rev = (flags & QGRU_FLAG_REVERSE) != 0;
     const size_t init_slot = rev ? (size_t)T : 0;
     int rc;
-    h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->stamped[h->calls++ % qgru_handle::kRing] = false;
+    take_slot(h);
     CK(cudaEventRecord(h->ev[0], st));
     if (use_generic(h)) {
         // dense int32 states, step by step; then to the view
@@ -1279,8 +1278,7 @@ int qgru_forward_i32_train(qgru_handle *h, int T, int B, const int32_t *x_q, con
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
     const long long init_slot = (flags & QGRU_FLAG_REVERSE) ? T : 0;
-    h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->stamped[h->calls++ % qgru_handle::kRing] = false;
+    take_slot(h);
     CK(cudaEventRecord(h->ev[0], st));
     // the step-by-step kernels keep every intermediate the training buffer wants
     OutView slot;
@@ -1390,7 +1388,7 @@ int qgru_last_timing(qgru_handle *h, float *ms_input_gemm, float *ms_recurrence,
     if (!h->timing_valid) return fail(h, QGRU_ERR_NOT_READY, "no forward has run");
     CK(cudaSetDevice(h->device));
     float a = 0, b = 0, c = 0;
-    if (int rc = slot_times(h, (int)((h->ev - h->ring[0]) / 4), &a, &b, &c)) return rc;
+    if (int rc = slot_times(h, h->slot(), &a, &b, &c)) return rc;
     if (ms_input_gemm) *ms_input_gemm = a;
     if (ms_recurrence) *ms_recurrence = b;
     if (ms_total) *ms_total = c;
@@ -1503,8 +1501,7 @@ extern "C" int qgru_forward_i32_static(qgru_handle *h, int T, int B, const int32
     const long long init_slot = (flags & QGRU_FLAG_REVERSE) ? T : 0;
     OutView out = dense_view(h, B);
     out.hq = h_q;
-    h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->stamped[h->calls++ % qgru_handle::kRing] = false;
+    take_slot(h);
     CK(cudaEventRecord(h->ev[0], st));
     // the array keeps what the previous call left: the state buffers' padding columns and the
     // step counters must start at zero

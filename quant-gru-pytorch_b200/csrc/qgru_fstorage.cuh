@@ -320,8 +320,7 @@ int fstorage_train_tail(qgru_handle *h, int T, int B, FwdInput in, float *h_out,
     const bool rev = flags & QGRU_FLAG_REVERSE;
     uint8_t *h8 = (uint8_t *)h->h8.p;
     const size_t h8_half = (size_t)B * h->Hpad;
-    h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->stamped[h->calls++ % qgru_handle::kRing] = false;
+    take_slot(h);
     CK(cudaEventRecord(h->ev[0], st));
     in.x_keep = tr.m.x;
     in.h0_keep = tr.m.h0;
@@ -535,8 +534,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
     }
     if ((rc = ensure(h, h->ih, (use_reg ? rp.ih_elements(N) : (size_t)N * C) * ih_bytes))) return rc;
 
-    h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->stamped[h->calls++ % qgru_handle::kRing] = false;
+    take_slot(h);
     CK(cudaEventRecord(h->ev[0], st));
     // dependent launches (see run_reg): the register-resident forms only
     const bool in_regs = h->opt_gemv_r != 1 && (h->Hpad == 128 || h->Hpad == 256);
@@ -749,7 +747,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
     }
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->ev[3], st));
-    h->stamped[(h->ev - h->ring[0]) / 4] = chained;
+    h->stamped[h->slot()] = chained;
     h->timing_valid = true;
     h->plan_text = buf;
     return QGRU_OK;

@@ -103,7 +103,8 @@ struct qgru_handle {
     // GPU's clock instead (prologue, product, recurrence), valid where stamped is set
     unsigned long long *d_stamps = nullptr;   // [kRing][3]
     bool stamped[kRing] = {};
-    unsigned long long *stamp(int k) { return d_stamps + (ev - ring[0]) / 4 * 3 + k; }
+    int slot() const { return (int)((ev - ring[0]) / 4); }
+    unsigned long long *stamp(int k) { return d_stamps + slot() * 3 + k; }
     uint64_t calls = 0;                 // forwards issued
     bool timing_valid = false;
     uint64_t launches = 0;
@@ -157,6 +158,13 @@ inline int alloc_dev(qgru_handle *h, T **p, size_t n) {
         return QGRU_ERR_NOMEM;
     }
     return QGRU_OK;
+}
+
+// The timing slot of the forward that starts.  Its middle events are what counts unless the forward says otherwise when it
+// has been queued (`stamped`).
+inline void take_slot(qgru_handle *h) {
+    h->ev = h->ring[h->calls++ % qgru_handle::kRing];
+    h->stamped[h->slot()] = false;
 }
 
 // A buffer whose size depends on the layer's sizes alone.

@@ -65,8 +65,7 @@ int qgru_forward_f32_train(qgru_handle *h, int T, int B, const float *W, const f
     if ((rc = ensure(h, h->hq32, nh * 4))) return rc;
     if ((rc = ensure(h, h->vq32, nv * 4))) return rc;
     const long long init_slot = (flags & QGRU_FLAG_REVERSE) ? T : 0;
-    h->ev = h->ring[h->calls % qgru_handle::kRing];
-    h->calls++;
+    take_slot(h);
     CK(cudaEventRecord(h->ev[0], st));
     k_quantize_f32_i32<<<grid_for(N * I, 256, h->sm_count), 256, 0, st>>>(x, x32, N * I, h->x_scale, xo.zero_point,
                                                                          op_qmin(xo), op_qmax(xo));

@@ -484,3 +484,30 @@ def test_timestep_chunks(oracle, cuda_device, shape, chunk, cfg):
         q8 = hd.forward_f32_q8(xf, hf)
         scale, zp, _ = hd.h_quant_meta()
         assert torch.equal((q8.to(torch.int32) - zp).to(torch.float32) * np.float32(scale), f), hd.describe_plan()
+
+
+def test_timing_slots_are_not_mixed_up(oracle, cuda_device):
+    """Every forward has one of 64 timing slots.  A slot that a chain of dependent launches used before (start times on
+    the GPU's clock instead of events between the kernels) must not lend them to the forward that reuses it."""
+    import torch
+    T, B, I, H = 64, 64, 512, 64
+    case = make_case(25, T, B, I, H, oracle, config_named("default"))
+    dev = cuda_device
+    want = None
+    for chained in (0, 70):
+        with gru_ops.Handle(I, H, device=dev.index or 0) as hd:
+            hd.set_option("rec", "fast")
+            hd.set_params(case.params)
+            w = [_t(a.astype(np.float32) * 0.01, dev) for a in case.wq]
+            hd.set_weights_f32(*w)
+            x = _t(case.x, dev)
+            for _ in range(chained):
+                hd.forward_f32(x[:2].contiguous(), sync=False)
+            got = []
+            for _ in range(3):
+                hd.forward_fstorage_train(*w, x, int_storage=True)
+                got.append(hd.last_timing()["input_gemm_ms"])
+        if want is None:
+            want = min(got)                       # the step-by-step path's product of 4096 rows: a hundred microseconds
+        else:
+            assert min(got) > 0.3 * want          # (the chained product of 128 rows takes a few)
