@@ -12,7 +12,9 @@
  *     initial state in slot 0 (include/gru_interface.h:389-413).
  *   - Quantized tensors crossing the boundary are int32 containers whose values are
  *     already clamped to the operator's bit width, exactly as in the reference.
- *   - `stream` is a cudaStream_t passed as void*; NULL means the legacy default stream.
+ *   - `stream` is a cudaStream_t passed as void*; NULL means the legacy default stream.  A handle has one
+ *     workspace: a call on another stream than the call before waits for that one's work on the GPU.  A call
+ *     that is captured into a graph waits for nothing; whoever launches the graph orders it.
  *     Calls are asynchronous with respect to the host unless stated otherwise.
  *   - Every function returns a qgru_status; no exception crosses this boundary.
  *   - Nothing here falls back to a CPU path: without a CUDA device the device entry

@@ -94,7 +94,7 @@ int qgru_create(qgru_handle **out, int device, int input_size, int hidden_size) 
     ok = ok && cudaMalloc(&h->d_flags, 2 * sizeof(int)) == cudaSuccess;
     ok = ok && cudaMemset(h->d_flags, 0, 2 * sizeof(int)) == cudaSuccess;
     ok = ok && cudaHostAlloc(&h->h_flags, 4 * sizeof(int), cudaHostAllocMapped) == cudaSuccess;
-    for (int r = 0; r < qgru_handle::kRing && ok; ++r)
+    for (int r = 0; r <= qgru_handle::kRing && ok; ++r)
         for (int i = 0; i < 4 && ok; ++i) ok = cudaEventCreate(&h->ring[r][i]) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
@@ -126,7 +126,8 @@ void qgru_destroy(qgru_handle *h) {
         cudaFree(h->d_wscale[i]);
         cudaFree(h->d_wq[i]);
     }
-    for (int r = 0; r < qgru_handle::kRing; ++r)
+    h->order.destroy();
+    for (int r = 0; r <= qgru_handle::kRing; ++r)
         for (int i = 0; i < 4; ++i)
             if (h->ring[r][i]) cudaEventDestroy(h->ring[r][i]);
     for (int i = 0; i < 2; ++i) {
@@ -171,7 +172,7 @@ int qgru_set_option(qgru_handle *h, const char *name, const char *value) {
         else if (v == "reg") h->opt_rec = 5;
         else if (v == "fast") {
             CK(cudaSetDevice(h->device));
-            if (int rc = alloc_once(h, &h->d_stamps, (size_t)qgru_handle::kRing * 3)) return rc;
+            if (int rc = alloc_once(h, &h->d_stamps, (size_t)(qgru_handle::kRing + 1) * 3)) return rc;
             h->opt_rec = 6;
         }
         else return fail(h, QGRU_ERR_BAD_ARG, "rec: auto|dp4a|mma|gemv|reg|fast|generic");
@@ -253,6 +254,7 @@ int qgru_set_params(qgru_handle *h, const qgru_params *p, const float *scale_W,
     // W/R/bw/br are symmetric with zp = 0 (ensureSymmetricWeightBiasConfig, src/gru_interface.cc:26-32)
     for (int k : {QGRU_OP_W, QGRU_OP_R, QGRU_OP_BW, QGRU_OP_BR})
         if (!p->op[k].symmetric) return fail(h, QGRU_ERR_UNSUPPORTED, "W/R/bw/br must be symmetric");
+    if (h->order.last) CK(cudaEventSynchronize(h->order.last));   // what is in flight reads the constants that change here
 
     h->params_set = false;
     h->weights_set = false;
@@ -550,6 +552,7 @@ int qgru_set_weights_f32(qgru_handle *h, const float *W, const float *R, const f
     if (!h->params_set) return fail(h, QGRU_ERR_NOT_READY, "set_params first");
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     const int C = h->C;
     const size_t n[4] = {(size_t)h->I * C, (size_t)h->H * C, (size_t)C, (size_t)C};
     const float *src[4] = {W, R, bw, br};
@@ -572,6 +575,7 @@ int qgru_set_weights_i32(qgru_handle *h, const int32_t *W_q, const int32_t *R_q,
     if (!h->params_set) return fail(h, QGRU_ERR_NOT_READY, "set_params first");
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     const int C = h->C;
     const size_t n[4] = {(size_t)h->I * C, (size_t)h->H * C, (size_t)C, (size_t)C};
     const int32_t *src[4] = {W_q, R_q, bw_q, br_q};
@@ -589,6 +593,7 @@ int qgru_get_weights_i32(qgru_handle *h, int32_t *W_q, int32_t *R_q, int32_t *bw
     if (!h->weights_set) return fail(h, QGRU_ERR_NOT_READY, "set_weights first");
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     const int C = h->C;
     const size_t n[4] = {(size_t)h->I * C, (size_t)h->H * C, (size_t)C, (size_t)C};
     int32_t *dst[4] = {W_q, R_q, bw_q, br_q};
@@ -825,6 +830,7 @@ int run_reg(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out,
     a.abort_flag = h->d_flags + 1;
     if ((rc = rec_reg_launch(h, pl, a, cell, ih_bytes, st))) return rc;
     CK(cudaEventRecord(h->ev[3], st));
+    h->order.tail = h->ev[3];
     h->stamped[h->slot()] = chained;
     h->timing_valid = true;
     char buf[300];
@@ -1087,6 +1093,7 @@ int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out
         }
     }
     CK(cudaEventRecord(h->ev[3], st));
+    h->order.tail = h->ev[3];
     h->stamped[h->slot()] = chained;
     h->timing_valid = true;
     h->plan_text = buf;
@@ -1113,6 +1120,7 @@ int run_wide(qgru_handle *h, int T, int B, const int32_t *x32, const int32_t *h0
     CK(cudaGetLastError());
     h->launches += 2;
     CK(cudaEventRecord(h->ev[3], st));
+    h->order.tail = h->ev[3];
     h->timing_valid = true;
     h->plan_text = "path=wide gemm=simt_i64 rec=dp4a_two_planes rows_per_cta=1";
     return QGRU_OK;
@@ -1264,6 +1272,7 @@ int qgru_forward_i32(qgru_handle *h, int T, int B, const int32_t *x_q, const int
     int rc = check_forward_args(h, T, B);
     if (rc) return rc;
     CK(cudaSetDevice(h->device));
+    USE_HANDLE(h, (cudaStream_t)stream);
     OutView out = dense_view(h, B);
     out.hq = h_q;
     return forward_dir(h, T, B, FwdInput{2, x_q, (long long)B * h->I, h->I, h0_q}, out, true, flags, (cudaStream_t)stream);
@@ -1277,6 +1286,7 @@ int qgru_forward_i32_train(qgru_handle *h, int T, int B, const int32_t *x_q, con
     if (rc) return rc;
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     const long long init_slot = (flags & QGRU_FLAG_REVERSE) ? T : 0;
     take_slot(h);
     CK(cudaEventRecord(h->ev[0], st));
@@ -1294,6 +1304,7 @@ int qgru_forward_f32(qgru_handle *h, int T, int B, const float *x, const float *
     int rc = check_forward_args(h, T, B);
     if (rc) return rc;
     CK(cudaSetDevice(h->device));
+    USE_HANDLE(h, (cudaStream_t)stream);
     OutView out = dense_view(h, B);
     out.hf = h_out;
     return forward_dir(h, T, B, FwdInput{0, x, (long long)B * h->I, h->I, h0, x_q_out}, out, true, flags, (cudaStream_t)stream);
@@ -1307,6 +1318,7 @@ int qgru_forward_f32_q8(qgru_handle *h, int T, int B, const float *x, const floa
     if (use_generic(h))
         return fail(h, QGRU_ERR_UNSUPPORTED, "the 8-bit output needs the 8-bit storage plan (x, h, W, R at most 8 bits)");
     CK(cudaSetDevice(h->device));
+    USE_HANDLE(h, (cudaStream_t)stream);
     OutView out = dense_view(h, B);
     out.h8 = h_q8;
     return forward_dir(h, T, B, FwdInput{0, x, (long long)B * h->I, h->I, h0}, out, true, flags, (cudaStream_t)stream);
@@ -1316,8 +1328,10 @@ int qgru_synchronize(qgru_handle *h, void *stream) {
     if (!h) return QGRU_ERR_BAD_ARG;
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     CK(cudaMemcpyAsync(h->h_flags, h->d_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    use_.idle();
     CK(cudaGetLastError());
     if (h->h_flags[1]) return fail(h, QGRU_ERR_TIMEOUT, "a per-step barrier wait of the recurrence kernel ran out");
     if (h->h_flags[0] & 1) return fail(h, QGRU_ERR_BAD_ARG, "quantized input outside the range its operator declares");
@@ -1331,6 +1345,7 @@ int qgru_forward_i32_host(qgru_handle *h, int T, int B, const int32_t *x_q, cons
     if (rc) return rc;
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     const size_t nx = (size_t)T * B * h->I * 4, nh = (size_t)(T + 1) * B * h->H * 4, n0 = (size_t)B * h->H * 4;
     if ((rc = ensure(h, h->stage_in, nx))) return rc;
     if ((rc = ensure(h, h->stage_out, nh))) return rc;
@@ -1352,6 +1367,7 @@ int qgru_forward_f32_host(qgru_handle *h, int T, int B, const float *x, const fl
     if (rc) return rc;
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     const size_t nx = (size_t)T * B * h->I * 4, nh = (size_t)(T + 1) * B * h->H * 4, n0 = (size_t)B * h->H * 4;
     if ((rc = ensure(h, h->stage_in, nx))) return rc;
     if ((rc = ensure(h, h->stage_out, nh))) return rc;
@@ -1385,10 +1401,10 @@ static int slot_times(qgru_handle *h, int k, float *a, float *b, float *c) {
 
 int qgru_last_timing(qgru_handle *h, float *ms_input_gemm, float *ms_recurrence, float *ms_total) {
     if (!h) return QGRU_ERR_BAD_ARG;
-    if (!h->timing_valid) return fail(h, QGRU_ERR_NOT_READY, "no forward has run");
+    if (!h->timing_valid || h->calls == 0) return fail(h, QGRU_ERR_NOT_READY, "no forward has run");
     CK(cudaSetDevice(h->device));
     float a = 0, b = 0, c = 0;
-    if (int rc = slot_times(h, h->slot(), &a, &b, &c)) return rc;
+    if (int rc = slot_times(h, (int)((h->calls - 1) % qgru_handle::kRing), &a, &b, &c)) return rc;
     if (ms_input_gemm) *ms_input_gemm = a;
     if (ms_recurrence) *ms_recurrence = b;
     if (ms_total) *ms_total = c;
@@ -1474,6 +1490,7 @@ extern "C" int qgru_forward_i32_static(qgru_handle *h, int T, int B, const int32
     if (!h->fast) return fail(h, QGRU_ERR_UNSUPPORTED, "the static-workspace forward needs the 8-bit storage plan");
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     const long long N = (long long)T * B;
     const int C = h->C;
 

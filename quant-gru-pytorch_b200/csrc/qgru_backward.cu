@@ -148,6 +148,7 @@ int qgru_backward(qgru_handle *h, int T, int B, const float *W_t, const float *R
     if (T <= 0 || B <= 0) return fail(h, QGRU_ERR_BAD_ARG, "T and B must be positive");
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     const int H = h->H, I = h->I, C = h->C;
     const long long N = (long long)T * B;
     const size_t NH = (size_t)B * H, NH3 = (size_t)B * C;

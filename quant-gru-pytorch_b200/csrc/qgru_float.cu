@@ -199,6 +199,7 @@ int qgru_forward_float(qgru_handle *h, int T, int B, const float *W, const float
     if (!h || !W || !R || !bw || !br || !x || !h_out) return QGRU_ERR_BAD_ARG;
     if (T <= 0 || B <= 0) return fail(h, QGRU_ERR_BAD_ARG, "T and B must be positive");
     CK(cudaSetDevice(h->device));
+    USE_HANDLE(h, (cudaStream_t)stream);
     return float_forward(h, T, B, W, R, bw, br, x, h0, h_out, v_out, 4, (cudaStream_t)stream);
 }
 
@@ -213,6 +214,7 @@ int qgru_calibrate_minmax(qgru_handle *h, int T, int B, const float *W, const fl
         return fail(h, QGRU_ERR_BAD_ARG, "ranges: per-channel arrays missing");
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     const int H = h->H, Cn = h->C;
     const size_t nh = (size_t)(T + 1) * B * H;
     int rc;

@@ -747,6 +747,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
     }
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->ev[3], st));
+    h->order.tail = h->ev[3];
     h->stamped[h->slot()] = chained;
     h->timing_valid = true;
     h->plan_text = buf;
@@ -764,6 +765,7 @@ int qgru_forward_fstorage(qgru_handle *h, int T, int B, const float *x, const fl
     if (!h->params_set || !h->weights_set)
         return fail(h, QGRU_ERR_NOT_READY, "set_params and set_weights first");
     CK(cudaSetDevice(h->device));
+    USE_HANDLE(h, (cudaStream_t)stream);
     OutView out = dense_view(h, B);
     out.hf = h_out;
     return qgru::fstorage_forward(h, T, B, FwdInput{1, x, (long long)B * h->I, h->I, h0, x_q_out}, out, true, flags, (cudaStream_t)stream);
@@ -789,6 +791,7 @@ int qgru_get_weights_dequantized(qgru_handle *h, float *W, float *R, float *bw, 
     if (!h->weights_set) return fail(h, QGRU_ERR_NOT_READY, "set_weights first");
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     const int C = h->C;
     const long long n[4] = {(long long)h->I * C, (long long)h->H * C, C, C};
     float *dst[4] = {W, R, bw, br};
@@ -821,6 +824,7 @@ int qgru_forward_fstorage_train(qgru_handle *h, int T, int B, const float *W, co
     if (!h->params_set || !h->weights_set)
         return fail(h, QGRU_ERR_NOT_READY, "set_params and set_weights first");
     CK(cudaSetDevice(h->device));
+    USE_HANDLE(h, (cudaStream_t)stream);
     qgru::FsTrainArgs tr{W, R, bw, br, v_out, masks ? *masks : qgru_train_masks{}};
     OutView out = dense_view(h, B);
     out.hf = h_out;

@@ -22,6 +22,68 @@ struct DevBuf {
     size_t cap = 0;
 };
 
+// Calls come on any stream, and the buffers behind a handle are one set: a call first waits, on its stream, for the call before
+// it if that came on another stream.  `last` is an event behind the work of the last call; a forward has
+// recorded one anyway (its timing slot's last event), so that calls on one stream pay for two queries of the runtime.
+struct StreamOrder {
+    cudaEvent_t own = nullptr;           // recorded by calls that have no event of their own at their end
+    cudaEvent_t last = nullptr;          // behind the last call's work; null: nothing is in flight
+    unsigned long long last_id = 0;      // the stream of that call
+    cudaEvent_t tail = nullptr;          // set by the call in progress: recorded behind everything it has queued
+    void destroy() {
+        if (own) cudaEventDestroy(own);
+        own = last = nullptr;
+    }
+};
+
+// A call's use of such a set, from begin() to the end of its scope, whichever way that is left.  A call that is being
+// captured waits for nothing and leaves nothing behind: the graph runs later, and who launches it
+// orders it with other calls.
+class StreamUse {
+  public:
+    StreamUse(StreamOrder &o, cudaStream_t st) : o_(o), st_(st) {}
+    StreamUse(const StreamUse &) = delete;
+    StreamUse &operator=(const StreamUse &) = delete;
+    // captured: the call is part of a capture that this stream has not joined yet
+    cudaError_t begin(bool captured = false) {
+        o_.tail = nullptr;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        cudaError_t e = captured ? cudaSuccess : cudaStreamIsCapturing(st_, &cap);
+        captured_ = captured || cap != cudaStreamCaptureStatusNone;
+        if (e != cudaSuccess || captured_) return e;
+        if ((e = cudaStreamGetId(st_, &id_)) != cudaSuccess) return e;
+        open_ = true;
+        return o_.last && o_.last_id != id_ ? cudaStreamWaitEvent(st_, o_.last, 0) : cudaSuccess;
+    }
+    bool captured() const { return captured_; }
+    // the host has waited for everything
+    void idle() {
+        if (open_) o_.last = nullptr;
+        open_ = false;
+    }
+    ~StreamUse() {
+        if (!open_) return;
+        if (!o_.tail) {
+            if ((!o_.own && cudaEventCreateWithFlags(&o_.own, cudaEventDisableTiming) != cudaSuccess) || cudaEventRecord(o_.own, st_) != cudaSuccess) {
+                cudaGetLastError();
+                cudaStreamSynchronize(st_);
+                o_.last = nullptr;
+                return;
+            }
+            o_.tail = o_.own;
+        }
+        o_.last = o_.tail;
+        o_.last_id = id_;
+        o_.tail = nullptr;
+    }
+
+  private:
+    StreamOrder &o_;
+    cudaStream_t st_;
+    unsigned long long id_ = 0;
+    bool open_ = false, captured_ = false;
+};
+
 struct qgru_handle {
     int device = 0, I = 0, H = 0, C = 0, Ipad = 0, Hpad = 0;
     int sm_count = 0, smem_optin = 0, coop = 0;
@@ -96,16 +158,19 @@ struct qgru_handle {
     qgru::F32RecPlan plan_fwd, plan_bwd;   // fp32 recurrences: the plan of the last batch size
     DevBuf fs_ch;                          // float-storage forward: 4 x 3H per-channel scale ratios
     bool fs_uploaded = false, fs_ready = false;   // fs_ch matches the current parameters; and the current weights
+    StreamOrder order;
+    bool captured = false;             // the call in progress is being captured into a graph
     static constexpr int kRing = 64;
-    cudaEvent_t ring[kRing][4] = {};   // per forward: start, gemm start, gemm end, recurrence end
+    // per forward: start, gemm start, gemm end, recurrence end; the last slot is for captured forwards, whose events have no times
+    cudaEvent_t ring[kRing + 1][4] = {};
     cudaEvent_t *ev = ring[0];          // the slot the current forward records into
     // forwards launched as a chain of dependent launches have no events between their kernels: start times on the
     // GPU's clock instead (prologue, product, recurrence), valid where stamped is set
-    unsigned long long *d_stamps = nullptr;   // [kRing][3]
-    bool stamped[kRing] = {};
+    unsigned long long *d_stamps = nullptr;   // [kRing + 1][3]
+    bool stamped[kRing + 1] = {};
     int slot() const { return (int)((ev - ring[0]) / 4); }
     unsigned long long *stamp(int k) { return d_stamps + slot() * 3 + k; }
-    uint64_t calls = 0;                 // forwards issued
+    uint64_t calls = 0;                 // forwards issued (captured ones not counted)
     bool timing_valid = false;
     uint64_t launches = 0;
     TcGemmState tc;
@@ -128,6 +193,12 @@ inline int fail(qgru_handle *h, int code, const std::string &msg) {
     h->err = msg;
     return code;
 }
+
+// A call's use of the handle on this stream (StreamUse).
+#define USE_HANDLE(h_, st_)              \
+    StreamUse use_(h_->order, st_);      \
+    CK(use_.begin());                    \
+    h_->captured = use_.captured()
 
 inline int ensure(qgru_handle *h, DevBuf &b, size_t bytes) {
     if (bytes <= b.cap) return QGRU_OK;
@@ -163,7 +234,7 @@ inline int alloc_dev(qgru_handle *h, T **p, size_t n) {
 // The timing slot of the forward that starts.  Its middle events are what counts unless the forward says otherwise when it
 // has been queued (`stamped`).
 inline void take_slot(qgru_handle *h) {
-    h->ev = h->ring[h->calls++ % qgru_handle::kRing];
+    h->ev = h->ring[h->captured ? qgru_handle::kRing : h->calls++ % qgru_handle::kRing];
     h->stamped[h->slot()] = false;
 }
 

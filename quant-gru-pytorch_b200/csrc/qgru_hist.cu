@@ -58,6 +58,7 @@ struct qgru_hist {
     char *d_scratch = nullptr;     // parameter derivation: per histogram an index, a search job and its result
     float *d_gather = nullptr;     // [GATHER][bins] histograms on their way to the host
     std::vector<HistMeta> meta;
+    StreamOrder order;
     bool channels_done[4] = {false, false, false, false};
     std::string err;
 };
@@ -574,6 +575,8 @@ int collect_batch(qgru_hist *hs, const std::vector<Job> &jobs, const CellSrc *ce
                   cudaStream_t st) {
     const int C = 3 * hs->H, bins = hs->bins, base_job = cell ? CELL_COUNT : 0;
     if (base_job + (int)jobs.size() > MAX_JOBS) return hfail(hs, QGRU_ERR_BAD_ARG, "too many collections in one batch");
+    StreamUse use(hs->order, st);
+    HCK(use.begin());
     k_hist_clear_keys<<<1, 2 * MAX_JOBS, 0, st>>>(hs->d_keys);
     const float tiny_range = min_scale_bins(bins) * bins;
     std::vector<float> mm;
@@ -693,6 +696,7 @@ void qgru_hist_destroy(qgru_hist *hs) {
         cudaFree(hs->own);
         cudaGetLastError();
     }
+    hs->order.destroy();
     delete hs;
 }
 
@@ -770,6 +774,7 @@ int qgru_calibrate_hist_h(qgru_handle *h, qgru_hist *hs, int T, int B, const flo
         return fail(h, QGRU_ERR_BAD_ARG, "histogram set belongs to another hidden size or device");
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     const int H = h->H, C = h->C, I = h->I;
     const long long N = (long long)T * B;
     int rc;

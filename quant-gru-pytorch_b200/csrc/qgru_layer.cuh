@@ -4,7 +4,8 @@
 //
 // A call is three launches per direction (prologue, W*x product, recurrence) and four timing events; the
 // reverse direction runs on a stream of its own beside the forward one and reads the rows the forward
-// direction has quantized where both quantize x the same way.  Device-side wait expiries of an earlier
+// direction has quantized where both quantize x the same way.  A call on another stream than the one before waits for
+// that one's work on the GPU (StreamUse): calls of one layer never overlap.  Device-side wait expiries of an earlier
 // call are reported by the next one (or by qgru_synchronize before it).
 //
 // Included at the end of qgru_api.cu, after qgru_fstorage.cuh.
@@ -18,6 +19,15 @@ bool same_x_quantization(const qgru_handle *a, const qgru_handle *b) {
     const qgru_op &p = a->p.op[QGRU_OP_X], &q = b->p.op[QGRU_OP_X];
     return a->I == b->I && a->x_scale == b->x_scale && p.zero_point == q.zero_point && op_qmin(p) == op_qmin(q) &&
            op_qmax(p) == op_qmax(q);
+}
+
+// The reverse direction's stream and the events that fork and join it.
+int layer_streams(qgru_handle *h, qgru_handle *rev) {
+    if (!rev || rev->ev_join) return QGRU_OK;
+    if (!rev->side) CK(cudaStreamCreateWithFlags(&rev->side, cudaStreamNonBlocking));
+    if (!rev->ev_split) CK(cudaEventCreateWithFlags(&rev->ev_split, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&rev->ev_join, cudaEventDisableTiming));
+    return QGRU_OK;
 }
 
 // x, h0, out, h_n: fp32 (mode 0, 1) or int32 (mode 2).
@@ -35,11 +45,11 @@ int layer_forward(qgru_handle *h, qgru_handle *rev, int mode, int T, int B, cons
     if (rev && (rev->device != h->device || rev->I != h->I || rev->H != h->H))
         return fail(h, QGRU_ERR_BAD_ARG, "the two directions differ in device or sizes");
     CK(cudaSetDevice(h->device));
-    if (rev && !rev->side) {
-        CK(cudaStreamCreateWithFlags(&rev->side, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&rev->ev_split, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&rev->ev_join, cudaEventDisableTiming));
-    }
+    if ((rc = layer_streams(h, rev))) return rc;
+    USE_HANDLE(h, st);
+    StreamUse rev_use((rev ? rev : h)->order, (rev ? rev : h)->side);
+    if (rev) CK(rev_use.begin(use_.captured()));
+    if (rev) rev->captured = use_.captured();
     const size_t BH = (size_t)B * h->H;
     // a 32-bit row offset inside a step is what the cluster recurrence has room for
     if (out_bs < 0 || out_ts < 0 || out_bs > (1ll << 25)) return fail(h, QGRU_ERR_UNSUPPORTED, "output stride too large");
@@ -70,17 +80,14 @@ int layer_forward(qgru_handle *h, qgru_handle *rev, int mode, int T, int B, cons
         const unsigned fl = d ? QGRU_FLAG_REVERSE : 0;
         rc = mode == 1 ? fstorage_forward(k, T, B, in, o, false, fl, ds, shared, after)
                        : forward_dir(k, T, B, in, o, false, fl, ds, shared, after);
-        if (rc) {
-            if (d) {
-                h->err = k->err;
-                cudaStreamWaitEvent(st, rev->ev_split, 0);
-            }
-            return rc;
-        }
-        if (d) {
+        if (rc && d) h->err = k->err;
+        if (d) {   // (a direction that failed may have queued some of its work)
             CK(cudaEventRecord(rev->ev_join, ds));
             CK(cudaStreamWaitEvent(st, rev->ev_join, 0));
+            rev->order.tail = rev->ev_join;
+            h->order.tail = nullptr;            // x8 is read until the directions have joined
         }
+        if (rc) return rc;
     }
     return QGRU_OK;
 }

@@ -43,6 +43,7 @@ int qgru_forward_f32_train(qgru_handle *h, int T, int B, const float *W, const f
     if (rc) return rc;
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
     const qgru_params &p = h->p;
     const int H = h->H, I = h->I, C = h->C;
     const long long N = (long long)T * B;

@@ -288,13 +288,8 @@ int train_check(qgru_handle *h, qgru_handle *rev, int mode, int T, int B) {
         if (mode && !d->params_set) return fail(h, QGRU_ERR_NOT_READY, "set_params first");
         if (d->H != h->H || d->I != h->I || d->device != h->device) return fail(h, QGRU_ERR_BAD_ARG, "the two directions differ in device or sizes");
     }
-    if (rev && !rev->side) {
-        CK(cudaSetDevice(h->device));
-        CK(cudaStreamCreateWithFlags(&rev->side, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&rev->ev_split, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&rev->ev_join, cudaEventDisableTiming));
-    }
-    return QGRU_OK;
+    CK(cudaSetDevice(h->device));
+    return layer_streams(h, rev);
 }
 
 }  // namespace
@@ -333,6 +328,10 @@ int qgru_train_forward(qgru_handle *h, qgru_handle *rev, int mode, int T, int B,
     if (mode == 0 && (x_bs != h->I || x_ts != (long long)B * h->I)) return fail(h, QGRU_ERR_BAD_ARG, "mode 0 needs dense x [T][B][I]");
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
+    StreamUse rev_use((rev ? rev : h)->order, (rev ? rev : h)->side);
+    if (rev) CK(rev_use.begin(use_.captured()));
+    if (rev) rev->captured = use_.captured();
     const size_t BH = (size_t)B * h->H;
     if (rev && mode == 0) CK(cudaEventRecord(rev->ev_split, st));
     for (int k = 0; k < (rev ? 2 : 1); ++k) {
@@ -352,6 +351,7 @@ int qgru_train_forward(qgru_handle *h, qgru_handle *rev, int mode, int T, int B,
         if (k) {
             CK(cudaEventRecord(rev->ev_join, ds));
             CK(cudaStreamWaitEvent(st, rev->ev_join, 0));
+            rev->order.tail = rev->ev_join;
         }
         if (rc) return rc;
     }
@@ -365,6 +365,10 @@ int qgru_train_backward(qgru_handle *h, qgru_handle *rev, int mode, int T, int B
     if ((rc = qgru::train_check(h, rev, mode, T, B))) return rc;
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
+    USE_HANDLE(h, st);
+    // the reverse direction's buffers are read on `st` last, by the product that adds its share of dx
+    StreamUse rev_use((rev ? rev : h)->order, st);
+    if (rev) CK(rev_use.begin(use_.captured()));
     const size_t BH = (size_t)B * h->H;
     const bool shared = rev && dirs[1].shares_x;
     qgru::TrainSaved s[2];

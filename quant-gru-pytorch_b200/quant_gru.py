@@ -15,7 +15,8 @@ re-quantizes weights and regenerates LUTs on every call); the reverse direction 
 same input with reversed time indexing instead of two ``flip`` copies; a quantized forward is one library
 call for both directions (they run beside each other on two CUDA streams) that reads and writes
 the module's own tensors, batch-first ones too, and does not wait for the GPU: like any torch
-operation its results are ordered on the current stream.  A device-side error of a forward is
+operation its results are ordered on the current stream.  A layer has one workspace: calls on different streams run
+one after the other on the GPU (a call captured into a graph excepted: whoever launches the graph orders it).  A device-side error of a forward is
 raised by the next forward (``forward_quantized``, which checks its input's range, waits).  Training: in train() mode with gradients enabled, forward
 runs through an autograd function whose backward is qgru_backward - the fp32 GRU in float mode,
 and with use_quantization the quantized forward in training mode (float-storage path, or the
@@ -567,6 +568,8 @@ class QuantGRU(nn.Module):
                         setattr(self, name, Histograms(self.hidden_size, device.index or 0))
                     h = st.handle.calibrate_hist(*st.weights, xd, getattr(self, name),
                                                  self._bitwidth_config.granularity_list(), h0[d], want_h=True)
+                    for w in st.weights:    # still being counted when the call returns, maybe not on the stream they were made on
+                        w.record_stream(torch.cuda.current_stream(device))
                 outs.append(torch.cat([h[1:].flip(0), h[0:1]], 0) if d == 1 else h)
             self._quant_params_dirty = True
         else:
