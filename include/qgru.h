@@ -381,7 +381,9 @@ QGRU_API int qgru_forward_f32_host(qgru_handle *h, int T, int B, const float *x,
  * waits for it).  Element (t, b, i) of x lies at t * x_ts + b * x_bs + i; element (t, b, d * H + j) of the
  * output at t * out_ts + b * out_bs + d * H + j.  h0 and h_n: [D][B][H], h0 may be NULL.  float_storage:
  * qgru_forward_fstorage's arithmetic instead of qgru_forward_f32's.  Asynchronous.  A device-side wait
- * expiry of an EARLIER layer forward that nobody has asked about is returned here (QGRU_ERR_TIMEOUT). */
+ * that has run out in an EARLIER forward of either handle, as far as the GPU has got when this is called, is
+ * returned here once (QGRU_ERR_TIMEOUT; nothing is queued), as by qgru_train_forward and
+ * qgru_train_backward; qgru_synchronize waits and so tells about every forward before it. */
 QGRU_API int qgru_layer_forward(qgru_handle *h, qgru_handle *rev, int float_storage, int T, int B,
                                 const float *x, long long x_ts, long long x_bs, const float *h0,
                                 float *out, long long out_ts, long long out_bs, float *h_n,
@@ -394,10 +396,9 @@ QGRU_API int qgru_layer_forward_i32(qgru_handle *h, qgru_handle *rev, int T, int
 /* Blocks until the work queued on `stream` by this handle is done and reports a device-side
  * bounded-wait expiry (QGRU_ERR_TIMEOUT) or CUDA error, as the reference's
  * cudaDeviceSynchronize + cudaGetLastError + throw does (src/gru_interface.cc:594-602).
- * The device-side status words belong to the handle and every forward clears them when it starts:
- * the call reports on the LAST forward queued before it.  A caller that queues several forwards
- * on one handle without synchronising in between learns the status of the last one only; call
- * this after each forward whose status matters (the host-buffer entry points do). */
+ * An expiry stays known until a call has reported it, whatever was queued after it.  The other status (integer
+ * input outside the range that its operator declares, QGRU_ERR_BAD_ARG) is cleared by every forward when it
+ * starts: a caller to whom it matters calls this after each forward (the host-buffer entry points do). */
 QGRU_API int qgru_synchronize(qgru_handle *h, void *stream);
 
 /* Timing of the two kernels of the most recent forward, measured with CUDA events on the

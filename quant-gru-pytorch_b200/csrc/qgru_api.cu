@@ -91,9 +91,12 @@ int qgru_create(qgru_handle **out, int device, int input_size, int hidden_size) 
     ok = ok && cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, device) == cudaSuccess;
     ok = ok && cudaDeviceGetAttribute(&h->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) == cudaSuccess;
     ok = ok && cudaDeviceGetAttribute(&h->coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess;
-    ok = ok && cudaMalloc(&h->d_flags, 2 * sizeof(int)) == cudaSuccess;
-    ok = ok && cudaMemset(h->d_flags, 0, 2 * sizeof(int)) == cudaSuccess;
+    void *expired = nullptr;             // the device's address of h_flags[2]
     ok = ok && cudaHostAlloc(&h->h_flags, 4 * sizeof(int), cudaHostAllocMapped) == cudaSuccess;
+    ok = ok && cudaHostGetDevicePointer(&expired, h->h_flags + 2, 0) == cudaSuccess;
+    ok = ok && cudaMalloc(&h->d_flags, 2 * sizeof(int) + sizeof(expired)) == cudaSuccess;
+    ok = ok && cudaMemset(h->d_flags, 0, 2 * sizeof(int)) == cudaSuccess;
+    ok = ok && cudaMemcpy(h->d_flags + 2, &expired, sizeof(expired), cudaMemcpyHostToDevice) == cudaSuccess;
     for (int r = 0; r <= qgru_handle::kRing && ok; ++r)
         for (int i = 0; i < 4 && ok; ++i) ok = cudaEventCreate(&h->ring[r][i]) == cudaSuccess;
     if (!ok) {
@@ -101,7 +104,7 @@ int qgru_create(qgru_handle **out, int device, int input_size, int hidden_size) 
         qgru_destroy(h);
         return QGRU_ERR_CUDA;
     }
-    h->h_flags[0] = h->h_flags[1] = h->h_flags[2] = 0;
+    for (int i = 0; i < 4; ++i) h->h_flags[i] = 0;
     *out = h;
     return QGRU_OK;
 }
@@ -740,7 +743,7 @@ int launch_prologue(qgru_handle *h, int T, int B, const FwdInput &in, uint8_t *x
     a.h_hi = op_qmax(ho);
     a.h0_keep = in.h0_keep;
     a.flags = h->d_flags;
-    a.sticky = in.mode == 2 ? nullptr : h->h_flags + 2;
+    a.clear = in.mode != 2;
     a.stamp = in.stamp;
     if (in.mode == 2) CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
     a.q_blocks = x8 ? grid_for(a.N * (h->Ipad / 16), 256, h->sm_count) : 0;
@@ -1333,7 +1336,8 @@ int qgru_synchronize(qgru_handle *h, void *stream) {
     CK(cudaStreamSynchronize(st));
     use_.idle();
     CK(cudaGetLastError());
-    if (h->h_flags[1]) return fail(h, QGRU_ERR_TIMEOUT, "a per-step barrier wait of the recurrence kernel ran out");
+    const int expired = take_expiry(h);
+    if (h->h_flags[1] || expired) return fail(h, QGRU_ERR_TIMEOUT, "a per-step barrier wait of the recurrence kernel ran out");
     if (h->h_flags[0] & 1) return fail(h, QGRU_ERR_BAD_ARG, "quantized input outside the range its operator declares");
     return QGRU_OK;
 }

@@ -187,6 +187,15 @@ __device__ __forceinline__ void put_stamp(unsigned long long *stamp) {
     }
 }
 
+// A wait inside a kernel has run out.  abort_flag is the second of the handle's two status words, which the kernels of this
+// forward look at and the next forward clears; behind the two lies the address of a word in host memory, which
+// keeps the expiry, visible at once, until a call has reported it.
+__device__ __forceinline__ void raise_abort(int *abort_flag, int bits) {
+    atomicOr(abort_flag, bits);
+    **reinterpret_cast<volatile int **>(abort_flag + 1) = bits;
+    __threadfence_system();
+}
+
 // 32-bit load from a shared-memory window address: table lookups stay on the shared-memory
 // path with 32-bit address arithmetic.
 __device__ __forceinline__ int32_t lds_i32(uint32_t addr) {

@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(256, 1) k_fs_recurrence(RecArgs a, FsRecArgs f
                 unsigned it = 0;
                 while (ld_acquire(bar) < want) {
                     if (++it > a.spin_limit || (it % 1024 == 0 && *(volatile int *)a.abort_flag)) {
-                        atomicOr(a.abort_flag, 1);
+                        raise_abort(a.abort_flag, 1);
                         break;
                     }
                 }

@@ -453,7 +453,7 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
     }
     tc::tc_fence_before_sync();
     __syncthreads();
-    if (threadIdx.x == 0 && *failed) atomicOr(abort_flag, 2);
+    if (threadIdx.x == 0 && *failed) raise_abort(abort_flag, 2);
     if (warp == 1) tc::tmem_dealloc(tmem_base, 512);
 }
 

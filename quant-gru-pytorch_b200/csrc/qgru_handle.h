@@ -142,8 +142,8 @@ struct qgru_handle {
     bool lin_fits32[2] = {false, false};      // acc + corr fits int32 (x side, h side)
     bool lin_notie[2] = {false, false};       // no channel of that layer's requantization can meet an exact tie
     bool rs_fast[2] = {false, false};   // every per-channel GEMM rescale has the shift-free form
-    int *d_flags = nullptr;                   // [0] data errors, [1] barrier abort
-    int *h_flags = nullptr;                   // pinned mirror; [2]: status of an earlier asynchronous forward (written by the GPU)
+    int *d_flags = nullptr;                   // [0] data errors, [1] a wait ran out; then the device's address of h_flags[2]
+    int *h_flags = nullptr;                   // pinned mirror of the two; [2]: a wait that ran out and has not been reported (raise_abort)
     cudaStream_t side = nullptr;              // layer forward: the reverse direction's stream
     cudaEvent_t ev_split = nullptr, ev_join = nullptr;
     unsigned *d_bar = nullptr;
@@ -229,6 +229,19 @@ inline int alloc_dev(qgru_handle *h, T **p, size_t n) {
         return QGRU_ERR_NOMEM;
     }
     return QGRU_OK;
+}
+
+// The word that a wait inside a kernel leaves when it runs out; reported once.
+inline int take_expiry(qgru_handle *h) {
+    volatile int *w = h->h_flags + 2;
+    const int v = *w;
+    if (v) *w = 0;
+    return v;
+}
+// Before a call queues anything: QGRU_ERR_TIMEOUT where a wait of a forward that has since run on the GPU ran out.
+inline int check_expiry(qgru_handle *h, qgru_handle *reverse) {
+    const int a = take_expiry(h), b = reverse ? take_expiry(reverse) : 0;
+    return a || b ? fail(h, QGRU_ERR_TIMEOUT, "a device-side wait of an earlier forward ran out: its results are not valid") : QGRU_OK;
 }
 
 // The timing slot of the forward that starts.  Its middle events are what counts unless the forward says otherwise when it

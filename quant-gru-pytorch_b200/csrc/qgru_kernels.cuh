@@ -28,10 +28,10 @@ __device__ __forceinline__ float fs_quantize_raw(float x, float scale, int32_t z
 
 // What every forward does before its first product, in ONE launch: activations to 8-bit rows padded to
 // Kpad (zeros), the initial state to its 8-bit rows and, for the slot layouts, to the outputs' first slot.
-// The status words of the call before are folded into `sticky` (host memory) and cleared.
+// The status words of the call before are cleared.
 // Mode 0: fp32 in, integer quantize; 1: fp32 in, float-storage quantize; 2: int32 containers (values
 // outside the operator's range, which the reference's quantize step would have clamped, raise bit 0
-// of flags[0]; the caller clears the flags).
+// of flags[0]; the caller clears the flags beforehand).
 struct PrologueArgs {
     const void *x;               // row n = t * B + b at x + t * x_ts + b * x_bs; null: only the state
     long long x_ts, x_bs, N;
@@ -50,7 +50,7 @@ struct PrologueArgs {
     int32_t h_zp, h_lo, h_hi;
     uint8_t *h0_keep;            // optional mask of the initial state (modes 0, 1)
     int *flags;                  // [2]
-    volatile int *sticky;        // mapped host word or null: do not clear the flags
+    int clear;                   // clear the flags
     int q_blocks;                // blocks that quantize x; the rest write the state
     unsigned long long *stamp;   // start time, or null
 };
@@ -81,8 +81,7 @@ template <int Mode, bool Vec>
 __global__ void __launch_bounds__(256) k_prologue(const PrologueArgs a) {
     pdl_trigger();
     put_stamp(a.stamp);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && a.sticky) {
-        if (a.flags[1]) *a.sticky = a.flags[1];
+    if (blockIdx.x == 0 && threadIdx.x == 0 && a.clear) {
         a.flags[0] = 0;
         a.flags[1] = 0;
     }
@@ -388,7 +387,7 @@ __global__ void __launch_bounds__(256, 1) k_recurrence_dp4a(RecArgs a) {
                 unsigned it = 0;
                 while (ld_acquire(bar) < want) {
                     if (++it > a.spin_limit || (it % 1024 == 0 && *(volatile int *)a.abort_flag)) {
-                        atomicOr(a.abort_flag, 1);
+                        raise_abort(a.abort_flag, 1);
                         break;
                     }
                 }

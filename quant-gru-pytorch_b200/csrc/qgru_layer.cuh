@@ -5,8 +5,8 @@
 // A call is three launches per direction (prologue, W*x product, recurrence) and four timing events; the
 // reverse direction runs on a stream of its own beside the forward one and reads the rows the forward
 // direction has quantized where both quantize x the same way.  A call on another stream than the one before waits for
-// that one's work on the GPU (StreamUse): calls of one layer never overlap.  Device-side wait expiries of an earlier
-// call are reported by the next one (or by qgru_synchronize before it).
+// that one's work on the GPU (StreamUse): calls of one layer never overlap.  A device-side
+// wait that runs out is known to the host at once: the first call after that reports it, or qgru_synchronize.
 //
 // Included at the end of qgru_api.cu, after qgru_fstorage.cuh.
 #pragma once
@@ -37,11 +37,8 @@ int layer_forward(qgru_handle *h, qgru_handle *rev, int mode, int T, int B, cons
     for (qgru_handle *d : {h, rev}) {
         if (!d) continue;
         if ((rc = check_forward_args(d, T, B))) return d == h ? rc : fail(h, rc, d->err);
-        if (*(volatile int *)(d->h_flags + 2)) {
-            d->h_flags[2] = 0;
-            return fail(h, QGRU_ERR_TIMEOUT, "a device-side wait of an earlier forward ran out");
-        }
     }
+    if ((rc = check_expiry(h, rev))) return rc;
     if (rev && (rev->device != h->device || rev->I != h->I || rev->H != h->H))
         return fail(h, QGRU_ERR_BAD_ARG, "the two directions differ in device or sizes");
     CK(cudaSetDevice(h->device));

@@ -192,7 +192,7 @@ k_recurrence_c64(const __grid_constant__ CUtensorMap map_r, const __grid_constan
                     STAMP(true, 2 * cw + 1);
                 }
             }
-            if (!ok) atomicOr(a.abort_flag, 1);
+            if (!ok) raise_abort(a.abort_flag, 1);
         }
     } else {
         // ---------------------------------------------------------------- epilogue warps (1 .. 16)
@@ -401,7 +401,7 @@ k_recurrence_c64(const __grid_constant__ CUtensorMap map_r, const __grid_constan
                 STAMP((warp % 15) == 1 && lane == 0, 12 + 8 * (warp / 15));
             }
         }
-        if (!ok && lane == 0) atomicOr(a.abort_flag, 1);
+        if (!ok && lane == 0) raise_abort(a.abort_flag, 1);
     }
     tc::tc_fence_before_sync();
     __syncthreads();

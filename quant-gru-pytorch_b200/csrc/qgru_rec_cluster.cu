@@ -226,7 +226,7 @@ k_recurrence_cluster(const __grid_constant__ CUtensorMap map_r, const __grid_con
             h_lo0 = (tc::smem_u32(h_tile) & 0x3FFFFu) >> 4;
             desc_hi = (uint32_t)(tc::smem_desc_sw128(0) >> 32);
             desc_lo = (uint32_t)tc::smem_desc_sw128(0);
-            if (!ok) atomicOr(a.abort_flag, 1);
+            if (!ok) raise_abort(a.abort_flag, 1);
             const uint32_t blk_bytes = (uint32_t)(a.NB * 128);           // one K-slab of the tile
             const int kb0 = part == 0 ? 0 : (KBn + 1) / 2;               // this issuer's K-slabs: [kb0, kb1)
             const int kb1 = (KP == 1 || part == 1) ? KBn : (KBn + 1) / 2;
@@ -305,7 +305,7 @@ k_recurrence_cluster(const __grid_constant__ CUtensorMap map_r, const __grid_con
                     STAMP(iw == 0, 1);
                 }
             }
-            if (!ok) atomicOr(a.abort_flag, 1);
+            if (!ok) raise_abort(a.abort_flag, 1);
         }
     } else {
         // ---------------------------------------------------------------- epilogue warps (1 .. 16)
@@ -717,7 +717,7 @@ k_recurrence_cluster(const __grid_constant__ CUtensorMap map_r, const __grid_con
             if (c_last >= 0) store_outputs(hn_last, c_last * CH, nb, out_base, s + 1 == a.T, hn_base);
             }   // sub-groups
         }
-        if (!ok && lane == 0) atomicOr(a.abort_flag, 1);
+        if (!ok && lane == 0) raise_abort(a.abort_flag, 1);
     }
     tc::tc_fence_before_sync();
     __syncthreads();

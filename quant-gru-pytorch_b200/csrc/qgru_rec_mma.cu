@@ -160,7 +160,7 @@ k_recurrence_mma(const __grid_constant__ CUtensorMap map_r, const __grid_constan
             }
             if (!ok) {
                 atomicExch(failed, 1);
-                atomicOr(a.abort_flag, 1);
+                raise_abort(a.abort_flag, 1);
             }
         }
     } else {
@@ -266,7 +266,7 @@ k_recurrence_mma(const __grid_constant__ CUtensorMap map_r, const __grid_constan
         }
         if (!ok && lane == 0) {
             atomicExch(failed, 1);
-            atomicOr(a.abort_flag, 1);
+            raise_abort(a.abort_flag, 1);
         }
     }
     tc::tc_fence_before_sync();

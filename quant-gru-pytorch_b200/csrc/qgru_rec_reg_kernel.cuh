@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
         }
         if (hf) hf += out_step;
     }
-    if (!ok && lane == 0) atomicOr(a.abort_flag, 1);
+    if (!ok && lane == 0) raise_abort(a.abort_flag, 1);
     if (Split && P > 1) {   // nobody leaves while a peer's store may be on its way
         cluster_arrive();
         cluster_wait();

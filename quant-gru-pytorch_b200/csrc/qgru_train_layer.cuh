@@ -320,11 +320,7 @@ int qgru_train_forward(qgru_handle *h, qgru_handle *rev, int mode, int T, int B,
     if (!h || !x || !dirs || !out || !h_n || mode < 0 || mode > 2) return QGRU_ERR_BAD_ARG;
     int rc;
     if ((rc = qgru::train_check(h, rev, mode, T, B))) return rc;
-    for (qgru_handle *d : {h, rev})
-        if (d && *(volatile int *)(d->h_flags + 2)) {
-            d->h_flags[2] = 0;
-            return fail(h, QGRU_ERR_TIMEOUT, "a device-side wait of an earlier forward ran out");
-        }
+    if ((rc = check_expiry(h, rev))) return rc;
     if (mode == 0 && (x_bs != h->I || x_ts != (long long)B * h->I)) return fail(h, QGRU_ERR_BAD_ARG, "mode 0 needs dense x [T][B][I]");
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
@@ -363,6 +359,7 @@ int qgru_train_backward(qgru_handle *h, qgru_handle *rev, int mode, int T, int B
     if (!h || !dout || !dirs || mode < 0 || mode > 2 || (mode == 0 && !x)) return QGRU_ERR_BAD_ARG;
     int rc;
     if ((rc = qgru::train_check(h, rev, mode, T, B))) return rc;
+    if ((rc = check_expiry(h, rev))) return rc;
     CK(cudaSetDevice(h->device));
     cudaStream_t st = (cudaStream_t)stream;
     USE_HANDLE(h, st);

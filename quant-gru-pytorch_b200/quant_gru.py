@@ -16,8 +16,10 @@ same input with reversed time indexing instead of two ``flip`` copies; a quantiz
 call for both directions (they run beside each other on two CUDA streams) that reads and writes
 the module's own tensors, batch-first ones too, and does not wait for the GPU: like any torch
 operation its results are ordered on the current stream.  A layer has one workspace: calls on different streams run
-one after the other on the GPU (a call captured into a graph excepted: whoever launches the graph orders it).  A device-side error of a forward is
-raised by the next forward (``forward_quantized``, which checks its input's range, waits).  Training: in train() mode with gradients enabled, forward
+one after the other on the GPU (a call captured into a graph excepted: whoever launches the graph orders it).  A wait inside
+a kernel that runs out is raised by the first call of the module (backward included) that begins after the GPU got
+there, or by ``synchronize()``, which waits for the module's work (as ``forward_quantized`` does, which checks its
+input's range).  Training: in train() mode with gradients enabled, forward
 runs through an autograd function whose backward is qgru_backward - the fp32 GRU in float mode,
 and with use_quantization the quantized forward in training mode (float-storage path, or the
 integer path with quant_storage_dtype="int32") with its clamp masks as straight-through
@@ -597,6 +599,12 @@ class QuantGRU(nn.Module):
         for st in self._dirs:
             st.handle.synchronize()     # values outside the operators' ranges are an error of this call
         return out
+
+    def synchronize(self):
+        """Waits for the module's work on the current stream and raises what went wrong in it on the GPU."""
+        for st in self._dirs:
+            if st.handle:
+                st.handle.synchronize()
 
     def last_plans(self):
         return [st.handle.describe_plan() if st.handle else "" for st in self._dirs]
