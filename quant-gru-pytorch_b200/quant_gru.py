@@ -109,7 +109,8 @@ class _QuantGRUFunction(torch.autograd.Function):
 class _LayerFunction(torch.autograd.Function):
     """Training of the whole layer, both directions, weights in the module's layout: one library call forward,
     one backward (qgru_train_forward / qgru_train_backward; modes as there).  Inputs: x and hx as the
-    module takes them (fp32), then w_ih, w_hh, b_ih, b_hh per direction (biases may be None)."""
+    module takes them (fp32), then w_ih, w_hh, b_ih, b_hh per direction (biases may be None).  What the backward needs
+    is in saved tensors (freed after it, hooks apply): the library's block of every direction and, in float mode, x."""
 
     @staticmethod
     def forward(ctx, module, mode, saved_bytes, x, hx, *params):
@@ -124,7 +125,7 @@ class _LayerFunction(torch.autograd.Function):
             if x.stride(-1) != 1:
                 x = x.contiguous()
             x_ts, x_bs = x.stride(t_dim), x.stride(b_dim)
-        saved = torch.empty((D, (saved_bytes + 255) // 256 * 64), dtype=torch.float32, device=x.device)
+        saved = torch.empty((D, (saved_bytes + 255) // 256 * 256), dtype=torch.uint8, device=x.device)
         dirs = (_cabi.TrainDir * D)()
         params = [p if p is None else p.contiguous() for p in params]
         for d in range(D):
@@ -137,17 +138,22 @@ class _LayerFunction(torch.autograd.Function):
         h._ck(h._lib.qgru_train_forward(h._h, handles[1]._h if D == 2 else None, mode, T, B, x.data_ptr(), x_ts, x_bs,
                                         hx.data_ptr() if hx is not None else None, dirs, out.data_ptr(), out.stride(t_dim),
                                         out.stride(b_dim), h_n.data_ptr(), gru_ops._stream(x.device)), "qgru_train_forward")
-        ctx.handles, ctx.mode, ctx.saved, ctx.dirs, ctx.batch_first = handles, mode, saved, dirs, module.batch_first
+        ctx.handles, ctx.mode, ctx.batch_first, ctx.shares_x = handles, mode, module.batch_first, [d.shares_x for d in dirs]
         ctx.shape, ctx.param_shapes = (T, B, x.shape[2], H), [None if p is None else p.shape for p in params]
         ctx.set_materialize_grads(False)
-        if mode == 0:
-            ctx.save_for_backward(x)
+        keep = [saved, x] if mode == 0 else [saved]
+        ctx.kept_as = [(t.dtype, t.shape, t.device) for t in keep]
+        ctx.save_for_backward(*keep)
         return out, h_n
 
     @staticmethod
     def backward(ctx, dout, dh_n):
+        keep = ctx.saved_tensors
+        if any((t.dtype, t.shape, t.device) != as_ for t, as_ in zip(keep, ctx.kept_as)):
+            raise RuntimeError("a saved-tensor hook has returned another type, shape or device than it was given")
+        saved, *x = [t.contiguous() for t in keep]
         T, B, I, H = ctx.shape
-        D, dev = len(ctx.handles), ctx.saved.device
+        D, dev = len(ctx.handles), saved.device
         t_dim, b_dim = (1, 0) if ctx.batch_first else (0, 1)
         if dout is None:
             dout = torch.zeros((B, T, D * H) if ctx.batch_first else (T, B, D * H), device=dev)
@@ -159,16 +165,17 @@ class _LayerFunction(torch.autograd.Function):
         dx = torch.empty((T, B, I), device=dev) if need[3] else None
         dh0 = torch.empty((D, B, H), device=dev) if need[4] else None
         grads = [torch.empty(s, device=dev) if s is not None and n else None for s, n in zip(ctx.param_shapes, need[5:])]
+        dirs = (_cabi.TrainDir * D)()
         for d in range(D):
+            dirs[d].saved, dirs[d].shares_x = saved[d].data_ptr(), ctx.shares_x[d]
             for name, g in zip(("dW", "dR", "dbw", "dbr"), grads[4 * d:4 * d + 4]):
-                setattr(ctx.dirs[d], name, g.data_ptr() if g is not None else None)
-        x = ctx.saved_tensors[0] if ctx.mode == 0 else None
+                setattr(dirs[d], name, g.data_ptr() if g is not None else None)
         h = ctx.handles[0]
         h._ck(h._lib.qgru_train_backward(h._h, ctx.handles[1]._h if D == 2 else None, ctx.mode, T, B,
-                                         x.data_ptr() if x is not None else None, dout.data_ptr(), dout.stride(t_dim),
+                                         x[0].data_ptr() if x else None, dout.data_ptr(), dout.stride(t_dim),
                                          dout.stride(b_dim), dh_n.data_ptr() if dh_n is not None else None,
                                          dx.data_ptr() if dx is not None else None, dh0.data_ptr() if dh0 is not None else None,
-                                         ctx.dirs, gru_ops._stream(dev)), "qgru_train_backward")
+                                         dirs, gru_ops._stream(dev)), "qgru_train_backward")
         if dx is not None and ctx.batch_first:
             dx = dx.transpose(0, 1)
         return (None, None, None, dx, dh0, *grads)
