@@ -499,7 +499,7 @@ def run_ours(args):
         cluster = "exchange=cluster_dsmem" in plan
         kernel = ("k_recurrence_cluster" if cluster else "k_recurrence_mma") if "rec=tcgen05" in plan \
             else ("k_recurrence_gemv" if "rec=gemv" in plan else
-                  ("k_recurrence_dp4a" if "path=int8" in plan else "k_linear_generic+k_gates_generic"))
+                  ("k_recurrence_dp4a" if "path=int8" in plan else "k_linear_rows+k_gates_generic"))
         rec_bytes = T * job_rows * (3 * H * ih_bytes + H * (4 if cluster or "rec=gemv" in plan else 5))
         per_token = profiled_traffic_per_token(kernel, args.workload)
         traffic = per_token * T * job_rows if per_token else None

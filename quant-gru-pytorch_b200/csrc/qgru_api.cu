@@ -1103,7 +1103,19 @@ int run_fast(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out
     return QGRU_OK;
 }
 
-dim3 linear_grid(long long N, int C) { return dim3((unsigned)((N + 31) / 32), (unsigned)((C + 63) / 64)); }
+// A linear layer on int32 containers.  One output per thread while all outputs are resident at once (2048 threads an SM):
+// the rows of a step, short sequences.  Tiles beyond that.  us, one output per thread / tiles: K = 512, C = 1536: one row
+// 25 / 47, 64 rows 27 / 56, 192 rows 54 / 56, 256 rows 75 / 68, 4096 rows 828 / 530; K = 128, C = 384: 512 rows 12 / 18,
+// 1024 rows 21 / 21, 4096 rows 62 / 47; K = 1024, C = 3072: 64 rows 74 / 105, 128 rows 132 / 127.
+void linear_i32(qgru_handle *h, const int32_t *wq, const int32_t *in, int32_t *out, long long N, int K, const LinearConsts &lc, uint8_t *keep,
+                cudaStream_t st) {
+    const int C = h->C;
+    if (N * C <= 2048ll * h->sm_count && N <= 65535)
+        k_linear_rows<<<dim3((unsigned)((C + 127) / 128), (unsigned)N), 128, 0, st>>>(wq, in, out, N, K, C, lc, keep);
+    else
+        k_linear_tiles<<<dim3((unsigned)((N + 31) / 32), (unsigned)((C + 63) / 64)), 256, 0, st>>>(wq, in, out, N, K, C, lc, keep);
+    h->launches++;
+}
 
 // Operands wider than 8 bits, R of 8 and states of up to 16, H <= 256: the recurrence in one launch.
 int run_wide(qgru_handle *h, int T, int B, const int32_t *x32, const int32_t *h0, const OutView &out, unsigned flags, cudaStream_t st) {
@@ -1112,7 +1124,7 @@ int run_wide(qgru_handle *h, int T, int B, const int32_t *x32, const int32_t *h0
     int rc;
     if ((rc = ensure(h, h->ih32, (size_t)N * C * 4))) return rc;
     CK(cudaEventRecord(h->ev[1], st));
-    k_linear_generic<<<linear_grid(N, C), 256, 0, st>>>(h->d_wq[0], x32, (int32_t *)h->ih32.p, N, h->I, C, linear_consts(h, 0), nullptr);
+    linear_i32(h, h->d_wq[0], x32, (int32_t *)h->ih32.p, N, h->I, linear_consts(h, 0), nullptr, st);
     CK(cudaEventRecord(h->ev[2], st));
     WideArgs a{T, B, h->H, h->Hpad, C, (flags & QGRU_FLAG_REVERSE) ? 1 : 0, h->d_w8[1], (const int32_t *)h->ih32.p, h0, out, linear_consts(h, 1),
                h->d_tables, h->n_table};
@@ -1121,7 +1133,7 @@ int run_wide(qgru_handle *h, int T, int B, const int32_t *x32, const int32_t *h0
     CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kern<<<B, 4 * ((h->H + 31) / 32 * 32), smem, st>>>(h->gc_host, a);
     CK(cudaGetLastError());
-    h->launches += 2;
+    h->launches++;
     CK(cudaEventRecord(h->ev[3], st));
     h->order.tail = h->ev[3];
     h->timing_valid = true;
@@ -1139,11 +1151,7 @@ int run_generic(qgru_handle *h, int T, int B, const int32_t *x32, int32_t *hq, i
     if ((rc = ensure(h, h->hh32, (size_t)B * C * 4))) return rc;
     CK(cudaEventRecord(h->ev[1], st));
     const LinearConsts lcx = linear_consts(h, 0), lch = linear_consts(h, 1);
-    {
-        k_linear_generic<<<linear_grid(N, C), 256, 0, st>>>(h->d_wq[0], x32, (int32_t *)h->ih32.p, N, h->I, C, lcx,
-                                                           mk ? mk->ih_linear : nullptr);
-        h->launches++;
-    }
+    linear_i32(h, h->d_wq[0], x32, (int32_t *)h->ih32.p, N, h->I, lcx, mk ? mk->ih_linear : nullptr, st);
     CK(cudaEventRecord(h->ev[2], st));
     const bool rev = flags & QGRU_FLAG_REVERSE;
     const size_t BH = (size_t)B * H;
@@ -1152,8 +1160,7 @@ int run_generic(qgru_handle *h, int T, int B, const int32_t *x32, int32_t *hq, i
         const size_t in_slot = rev ? (size_t)(T - s) : (size_t)s;
         const size_t out_slot = rev ? (size_t)(T - 1 - s) : (size_t)(s + 1);
         const size_t row = (size_t)t * B;
-        k_linear_generic<<<linear_grid(B, C), 256, 0, st>>>(h->d_wq[1], hq + in_slot * BH, (int32_t *)h->hh32.p, B, H, C, lch,
-                                             mk && mk->hh_linear ? mk->hh_linear + row * C : nullptr);
+        linear_i32(h, h->d_wq[1], hq + in_slot * BH, (int32_t *)h->hh32.p, B, H, lch, mk && mk->hh_linear ? mk->hh_linear + row * C : nullptr, st);
         dim3 g2((H + 127) / 128, B);
         if (mk)
             k_gates_train<<<g2, 128, 0, st>>>((const int32_t *)h->ih32.p + row * C, (const int32_t *)h->hh32.p,
@@ -1166,7 +1173,7 @@ int run_generic(qgru_handle *h, int T, int B, const int32_t *x32, int32_t *hq, i
                                             (const int32_t *)h->hh32.p, hq + in_slot * BH,
                                             hq + out_slot * BH, vq ? vq + (size_t)t * B * 4 * H : nullptr, B, H,
                                             h->d_gc, h->d_tables);
-        h->launches += 2;
+        h->launches++;
     }
     CK(cudaGetLastError());
     CK(cudaEventRecord(h->ev[3], st));

@@ -763,11 +763,24 @@ __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_con
 // --------------------------------------------- generic fallback (any bit width, int32 data)
 
 // out[n][m] = epilogue( sum_k W_q[k][m] * in[n][k] ) with 64-bit accumulation
-// (quantizedGemmBiasFused's arithmetic, src/gru_forward_gpu_quant.cu:110-180).  32 x 64 tiles, 2 x 4 outputs
-// per thread, K in slabs of 32 through shared memory; bound by the widening multiply-adds.
+// (quantizedGemmBiasFused's arithmetic, src/gru_forward_gpu_quant.cu:110-180), in two forms.
+// One output per thread: bound by the latency of its K dependent steps, whatever the number of outputs, until the
+// SMs' resident threads are all in use; from there on by reading W again for every row.
+// (unrolled by 4, 8 or 16 with running pointers, or with launch bounds: 3 to 70 % slower at K = 512)
+__global__ void k_linear_rows(const int32_t *__restrict__ wq, const int32_t *__restrict__ in, int32_t *__restrict__ out, long long N, int K, int C,
+                              LinearConsts lc, uint8_t *__restrict__ keep) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long n = blockIdx.y;
+    if (m >= C || n >= N) return;
+    int64_t acc = 0;
+    for (int k = 0; k < K; ++k) acc += (int64_t)wq[(size_t)k * C + m] * (int64_t)in[n * K + k];
+    out[n * C + m] = linear_epilogue(acc, lc.corr[m], lc.rs[m], lc.zp_out, lc.lo, lc.hi, keep ? keep + n * C + m : nullptr);
+}
+
+// 32 x 64 tiles, 2 x 4 outputs per thread, K in slabs of 32 through shared memory; bound by the widening multiply-adds.
 __global__ void __launch_bounds__(256)
-k_linear_generic(const int32_t *__restrict__ wq, const int32_t *__restrict__ in, int32_t *__restrict__ out, long long N, int K, int C,
-                 LinearConsts lc, uint8_t *__restrict__ keep = nullptr) {
+k_linear_tiles(const int32_t *__restrict__ wq, const int32_t *__restrict__ in, int32_t *__restrict__ out, long long N, int K, int C,
+               LinearConsts lc, uint8_t *__restrict__ keep) {
     __shared__ int32_t xs[32][33];
     __shared__ __align__(16) int32_t ws[32][64];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;

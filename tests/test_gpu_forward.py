@@ -511,3 +511,25 @@ def test_timing_slots_are_not_mixed_up(oracle, cuda_device):
             want = min(got)                       # the step-by-step path's product of 4096 rows: a hundred microseconds
         else:
             assert min(got) > 0.3 * want          # (the chained product of 128 rows takes a few)
+
+
+@pytest.mark.parametrize("cfg,I,H", [("wide16", 7, 100), ("all16_generic", 33, 43), ("wide16", 1, 1)])
+def test_int32_linear_forms_at_their_line(oracle, cuda_device, cfg, I, H):
+    """The int32 linear layer gives one output to a thread while all outputs are resident at once and goes to tiles beyond:
+    W*x on either side of that line, R*h of a step on either side of it, with the clamp masks."""
+    import torch
+    c = config_named("wide16")
+    if cfg == "all16_generic":
+        c.set_all_bitwidth(16, False)
+    line = 2048 * torch.cuda.get_device_properties(cuda_device).multi_processor_count // (3 * H)
+    for T, B in ((2, line // 2), (2, line // 2 + 1), (1, line + 1)) if H > 1 else ((3, 5),):
+        case = make_case(T + B, T, B, I, H, oracle, c)
+        want_h, want_v, want_m = oracle.forward_i32_train(T, B, I, H, case.wq, case.x_q, case.h0_q, case.params.c,
+                                                          case.params.scale_list())
+        with gru_ops.Handle(I, H, device=cuda_device.index or 0) as hd:
+            hd.set_params(case.params)
+            hd.set_weights_i32(*[_t(a, cuda_device) for a in case.wq])
+            h0 = None if case.h0_q is None else _t(case.h0_q, cuda_device)
+            h, v, m = hd.forward_i32_train(_t(case.x_q, cuda_device), h0, want_masks=True)
+        assert np.array_equal(h.cpu().numpy(), want_h) and np.array_equal(v.cpu().numpy(), want_v)
+        assert all(np.array_equal(a.cpu().numpy(), b) for a, b in zip(m, want_m))
