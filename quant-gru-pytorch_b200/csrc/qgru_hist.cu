@@ -740,6 +740,7 @@ int qgru_hist_import(qgru_hist *hs, int index, const float *counts, float min_va
                      int64_t total_count) {
     if (!hs || !counts || index < 0 || index >= hs->n || total_count < 0) return QGRU_ERR_BAD_ARG;
     HCK(cudaSetDevice(hs->device));
+    HCK(cudaDeviceSynchronize());   // counts may be on their way, on any stream, and so may the work of whoever had this memory before
     HCK(cudaMemcpy(hs->d_counts + (size_t)index * hs->bins, counts, (size_t)hs->bins * 4, cudaMemcpyHostToDevice));
     HistMeta &m = hs->meta[index];
     m = HistMeta();

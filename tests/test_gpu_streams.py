@@ -142,6 +142,31 @@ def test_calibration_on_two_streams(cuda_device, method):
     assert all(torch.equal(a, b) for a, b in zip(got, want)) and got_p == want_p
 
 
+def test_imported_counts_wait_for_what_had_the_memory_before(cuda_device):
+    """A collector's counts live in torch's cached memory: on a side stream its last owner's kernels may still be writing it."""
+    import numpy as np
+    import torch
+    Histograms = importlib.import_module(PKG_NAME + ".params").Histograms
+    H, side = 64, torch.cuda.Stream()
+    counts = np.arange(2048, dtype=np.float32)
+    busy = torch.randn(4096, 4096, device=cuda_device)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        n = Histograms(H)._storage.numel()
+        for _ in range(3):
+            for _ in range(8):
+                busy = torch.tanh(busy @ busy)
+            junk = torch.empty(n, dtype=torch.uint8, device=cuda_device)
+            at = junk.data_ptr()
+            junk.fill_(7)
+            del junk
+            hs = Histograms(H)
+            assert hs._storage.data_ptr() == at      # the very memory that the fill has not reached yet
+            hs.put(5, counts, -1.0, 2.0, float(counts.sum(dtype=np.float64)))
+            side.synchronize()
+            assert np.array_equal(np.asarray(hs.get(5)[0]), counts)
+
+
 def test_new_parameters_wait_for_what_is_in_flight(cuda_device):
     """Parameters and weights are replaced by host copies and by calls on another stream."""
     import torch
