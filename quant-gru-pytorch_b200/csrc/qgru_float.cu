@@ -3,7 +3,7 @@
 // Float mode follows hasteGRUForward / ForwardPass<float> of the reference
 // (src/gru_interface.cc:173-207, src/gru_forward_gpu.cu:23-125, 342-414): one product for W*x
 // over all timesteps, then the recurrence in one launch (qgru_rec_f32.cu; wider layers than its
-// registers hold run step by step).  Calibration runs the same forward with the gate buffer kept and
+// registers hold, and more rows than pay there, run step by step).  Calibration runs the same forward with the gate buffer kept and
 // folds the min/max of every operator in one pass over it - the reference
 // materialises five capture tensors and seven temporaries of T*B*H floats and reduces each in
 // its own pass (src/calibration_gpu.cu:1776-1953).
@@ -171,9 +171,9 @@ int float_forward(qgru_handle *h, int T, int B, const float *W, const float *R, 
     k_init_h_float<<<(unsigned)((NH + 255) / 256), 256, 0, st>>>(h0, h_out, NH);
     h->launches++;
     if ((rc = gemm_f32(h, GemmF32{x, false, W, false, wx, N, I, Cn}, st))) return rc;
-    if (float_chain_fits(h, B))
+    if (float_chain_is_faster(h, B))
         return float_chain_launch(h, FloatFwdArgs{T, B, H, R, wx, bw, br, h_out, v_out, v_stride, 0, 0, OutView()}, st);
-    // wide layers, step by step: R*h as a tiled product, then the pointwise gates
+    // wide layers and very many rows, step by step: R*h as a tiled product, then the pointwise gates
     if ((rc = ensure(h, h->f_acc2, (size_t)B * Cn * 4))) return rc;
     float *rh = (float *)h->f_acc2.p;
     dim3 grid((H + 127) / 128, (B + 1) / 2);

@@ -702,6 +702,8 @@ void make_plan(qgru_handle *h, int B, Kern kern, size_t (*floats)(int, int, int,
                 pl->Bt = Bt;
                 pl->D = D;
                 pl->G = G;
+                pl->waves = waves;
+                pl->sharing = sharing;
                 pl->smem = smem;
                 pl->ok = active0 > 0;
             }
@@ -715,6 +717,17 @@ void make_plan(qgru_handle *h, int B, Kern kern, size_t (*floats)(int, int, int,
 bool float_chain_fits(qgru_handle *h, int B) {
     make_plan(h, B, k_float_chain<false, 512>, fwd_smem_floats, &h->plan_fwd);
     return h->plan_fwd.ok;
+}
+
+// Where thousands of rows make many waves of clusters, the tiled product of a step (which reads R once for 64 or 128
+// rows) catches up.  us per step, chain / step by step: H = 512: 512 rows 60 / 66, 1024 rows 118 / 89, 4096 rows 467 / 198;
+// H = 384: 512 rows 34 / 37, 1024 rows 67 / 57; H = 256: 2048 rows 49 / 57, 4096 rows 96 / 81; H = 128: 8192 rows 55 / 57.
+// Both sides as fitted to such times (H = 32 .. 512, up to 8192 rows): on the right side at every one of the 110 sizes.
+bool float_chain_is_faster(qgru_handle *h, int B) {
+    if (!float_chain_fits(h, B)) return false;
+    const F32RecPlan &pl = h->plan_fwd;
+    const double H = h->H, chain = pl.waves * (0.7 + 0.046 * (pl.U * pl.KG / 32) * pl.Bt * pl.sharing);
+    return chain <= 34.0 + (1.48e-7 * H + 1.02e-5) * H * B;
 }
 
 // (forms of at most 384 threads have registers to spare beside R: no spills)

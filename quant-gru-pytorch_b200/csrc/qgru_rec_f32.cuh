@@ -16,6 +16,7 @@ struct F32RecPlan {
     int H = 0, B = 0, sms = 0;      // what the plan was made for
     bool ok = false;
     int P = 1, U = 32, KG = 1, Bt = 1, G = 1, D = 1;
+    int waves = 1, sharing = 1;     // clusters one after the other, CTAs on an SM at once
     size_t smem = 0;
 };
 
@@ -34,6 +35,8 @@ struct FloatFwdArgs {
 };
 // False: no plan for this shape (H > 512), the caller runs step by step.
 bool float_chain_fits(qgru_handle *h, int B);
+// Whether a step of it takes no longer than a tiled product and a pointwise launch.
+bool float_chain_is_faster(qgru_handle *h, int B);
 int float_chain_launch(qgru_handle *h, FloatFwdArgs a, cudaStream_t st);
 
 struct BwdChainArgs {

@@ -39,3 +39,22 @@ def test_float_forward_and_backward(oracle, cuda_device, T, B, I, H):
     for g, w in zip(got, want):
         g = g.cpu().numpy().reshape(w.shape)
         assert np.abs(g - w).max() <= 2e-5 * max(np.abs(w).max(), 1e-30)
+
+
+@pytest.mark.parametrize("H,few,many", [(200, 1500, 3000), (320, 500, 2500), (512, 300, 1100)])
+def test_float_forward_of_very_many_rows(cuda_device, H, few, many):
+    """Beyond some number of rows the forward goes step by step: the same states as the rows give in smaller batches."""
+    import torch
+    T, I = 3, 20
+    rng = np.random.default_rng(H)
+    w = [_t(a, cuda_device) for a in gen_weights(rng, I, H)]
+    x = _t(gen_x(rng, T, many, I), cuda_device)
+    h0 = _t((rng.standard_normal((many, H)) * 0.3).astype(np.float32), cuda_device)
+    with gru_ops.Handle(I, H, device=0) as hd:
+        launches = hd.launch_count()
+        want, want_v = hd.forward_float(*w, x[:, :few].contiguous(), h0=h0[:few], want_v=True)
+        in_one = hd.launch_count() - launches
+        got, got_v = hd.forward_float(*w, x, h0=h0, want_v=True)
+        assert hd.launch_count() - launches - in_one >= 2 * T > in_one      # step by step, and in one launch
+    # sums of H products in another order, |r|, |h| <= 1: a few ulp of values of order one
+    assert (got[:, :few] - want).abs().max() <= 2e-6 and (got_v[:, :few] - want_v).abs().max() <= 2e-5
