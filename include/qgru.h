@@ -493,7 +493,8 @@ QGRU_API double qgru_probe_last_bulk_rate(void);
  *   "probe_floor" 0 | 1                   measurement aid: the cluster recurrence runs with its MMAs and
  *                                         cells left out (results are meaningless); the recurrence time of
  *                                         qgru_last_timing is then the per-step synchronisation floor
- *   "sm_limit" n   use at most n SMs (0 = all);  "spin_limit" n   bound of the group barrier
+ *   "sm_limit" n   use at most n SMs (0 = all; quantized forwards and training: what may run beside another
+ *                  direction);  "spin_limit" n   bound of the group barrier
  *   "test_withhold_arrive" 0 | 1          failure-path test: with the dp4a recurrence on several CTAs per group,
  *                                         CTA 0 leaves out one arrival, the group's bounded wait runs out and the
  *                                         forward reports QGRU_ERR_TIMEOUT; nothing faults or hangs

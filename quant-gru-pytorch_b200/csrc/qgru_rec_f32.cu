@@ -669,8 +669,8 @@ cudaError_t launch_chain(Kern kern, const F32RecPlan &pl, Args &a, cudaStream_t 
 
 // The smallest cluster whose registers hold R: 96 values in each of at most 512 threads a CTA.
 template <typename Kern>
-void make_plan(qgru_handle *h, int B, Kern kern, size_t (*floats)(int, int, int, int, int), F32RecPlan *pl) {
-    const int H = h->H, sms = h->opt_sm_limit > 0 ? std::min(h->opt_sm_limit, h->sm_count) : h->sm_count;
+void make_plan(qgru_handle *h, int B, int sms, Kern kern, size_t (*floats)(int, int, int, int, int), F32RecPlan *pl) {
+    const int H = h->H;
     if (pl->H == H && pl->B == B && pl->sms == sms) return;
     *pl = F32RecPlan{};
     pl->H = H;
@@ -712,10 +712,13 @@ void make_plan(qgru_handle *h, int B, Kern kern, size_t (*floats)(int, int, int,
     }
 }
 
+// The SMs of a direction of a layer whose directions run side by side.
+int side_sms(const qgru_handle *h) { return h->opt_sm_limit > 0 ? std::min(h->opt_sm_limit, h->sm_count) : h->sm_count; }
+
 }  // namespace
 
 bool float_chain_fits(qgru_handle *h, int B) {
-    make_plan(h, B, k_float_chain<false, 512>, fwd_smem_floats, &h->plan_fwd);
+    make_plan(h, B, side_sms(h), k_float_chain<false, 512>, fwd_smem_floats, &h->plan_fwd);
     return h->plan_fwd.ok;
 }
 
@@ -724,8 +727,10 @@ bool float_chain_fits(qgru_handle *h, int B) {
 // H = 384: 512 rows 34 / 37, 1024 rows 67 / 57; H = 256: 2048 rows 49 / 57, 4096 rows 96 / 81; H = 128: 8192 rows 55 / 57.
 // Both sides as fitted to such times (H = 32 .. 512, up to 8192 rows): on the right side at every one of the 110 sizes.
 bool float_chain_is_faster(qgru_handle *h, int B) {
-    if (!float_chain_fits(h, B)) return false;
+    // (float inference and calibration run one direction after the other: each has the whole chip)
+    make_plan(h, B, h->sm_count, k_float_chain<false, 512>, fwd_smem_floats, &h->plan_fwd);
     const F32RecPlan &pl = h->plan_fwd;
+    if (!pl.ok) return false;
     const double H = h->H, chain = pl.waves * (0.7 + 0.046 * (pl.U * pl.KG / 32) * pl.Bt * pl.sharing);
     return chain <= 34.0 + (1.48e-7 * H + 1.02e-5) * H * B;
 }
@@ -741,7 +746,7 @@ int float_chain_launch(qgru_handle *h, FloatFwdArgs a, cudaStream_t st) {
 }
 
 bool bwd_chain_fits(qgru_handle *h, int B, int *groups) {
-    make_plan(h, B, k_bwd_chain<false, 512>, bwd_smem_floats, &h->plan_bwd);
+    make_plan(h, B, side_sms(h), k_bwd_chain<false, 512>, bwd_smem_floats, &h->plan_bwd);
     *groups = h->plan_bwd.G;
     return h->plan_bwd.ok;
 }
