@@ -1,7 +1,7 @@
 // qgru_gemm_f32.cu - fp32 matrix product on the CUDA cores: the input projection of float mode and
 // calibration, and the three products of the backward pass.
 //
-// 128 x 128 (or 64 x 64) tiles of C, 8 x 8 outputs per thread as packed pairs (fma.rn.f32x2: two IEEE
+// 128 x 128 tiles of C with 8 x 8 outputs per thread, or 64 x 64 with 4 x 4, as packed pairs (fma.rn.f32x2: two IEEE
 // fused multiply-adds per instruction, so that operand loads and the copies that duplicate A's value
 // into both halves share the issue slots the multiply-adds leave), K in slabs of 16 through two
 // shared-memory buffers, the next slab in registers while this one is multiplied.  K is split over
@@ -72,13 +72,15 @@ struct SlabLoader {
     }
 };
 
-// gridDim.z = number of K parts; part z > 1 parts write their tile to part_out[z][N * M].
-template <int BT, bool ATrans, bool BTrans, bool VecA, bool VecB>
-__global__ void __launch_bounds__((BT / 8) * (BT / 8), BT == 64 ? 8 : 2)
+// gridDim.z = number of K parts; part z > 1 parts write their tile to part_out[z][N * M].  A thread has TM x TM outputs,
+// four neighbours each way, and with TM = 8 the four half a tile further.
+template <int BT, int TM, bool ATrans, bool BTrans, bool VecA, bool VecB>
+__global__ void __launch_bounds__((BT / TM) * (BT / TM), TM == 4 ? 4 : 2)
 k_gemm_f32(const float *__restrict__ A, const float *__restrict__ Bm, float *__restrict__ C, long long N, long long K,
            int M, long long k_part, int accumulate, const uint8_t *__restrict__ mask, float *__restrict__ part_out) {
-    constexpr int THREADS = (BT / 8) * (BT / 8);
-    constexpr int TX = BT / 8;
+    static_assert(TM == 4 || TM == 8, "one or two groups of four outputs each way");
+    constexpr int THREADS = (BT / TM) * (BT / TM);
+    constexpr int TX = BT / TM;
     __shared__ __align__(16) float as[2][BK][BT + 4];
     __shared__ __align__(16) float bs[2][BK][BT + 4];
     const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
@@ -87,11 +89,11 @@ k_gemm_f32(const float *__restrict__ A, const float *__restrict__ Bm, float *__r
     const long long k_begin = (long long)blockIdx.z * k_part, k_end = min(K, k_begin + k_part);
     SlabLoader<BT, THREADS, ATrans, VecA> la;
     SlabLoader<BT, THREADS, !BTrans, VecB> lb;
-    uint64_t acc[8][4];
+    uint64_t acc[TM][TM / 2];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+        for (int j = 0; j < TM / 2; ++j) acc[i][j] = 0ull;
     la.load(A, N, K, n0, k_begin, k_end);
     lb.load(Bm, M, K, j0, k_begin, k_end);
     la.store(as[0]);
@@ -106,19 +108,29 @@ k_gemm_f32(const float *__restrict__ A, const float *__restrict__ Bm, float *__r
         }
 #pragma unroll
         for (int kk = 0; kk < BK; ++kk) {
-            // rows ty * 4 .. + 3 and BT / 2 + ty * 4 .. + 3; columns the same with tx: conflict-free 128-bit loads
+            // rows ty * 4 .. + 3 (and BT / 2 + ty * 4 .. + 3), columns the same with tx: conflict-free 128-bit loads
             const float4 a0 = *reinterpret_cast<const float4 *>(&as[buf][kk][ty * 4]);
-            const float4 a1 = *reinterpret_cast<const float4 *>(&as[buf][kk][BT / 2 + ty * 4]);
             const ulonglong2 b0 = *reinterpret_cast<const ulonglong2 *>(&bs[buf][kk][tx * 4]);
-            const ulonglong2 b1 = *reinterpret_cast<const ulonglong2 *>(&bs[buf][kk][BT / 2 + tx * 4]);
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            if constexpr (TM == 8) {
+                const float4 a1 = *reinterpret_cast<const float4 *>(&as[buf][kk][BT / 2 + ty * 4]);
+                const ulonglong2 b1 = *reinterpret_cast<const ulonglong2 *>(&bs[buf][kk][BT / 2 + tx * 4]);
+                const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint64_t aa = pack2(av[i], av[i]);
-                acc[i][0] = ffma2(aa, b0.x, acc[i][0]);
-                acc[i][1] = ffma2(aa, b0.y, acc[i][1]);
-                acc[i][2] = ffma2(aa, b1.x, acc[i][2]);
-                acc[i][3] = ffma2(aa, b1.y, acc[i][3]);
+                for (int i = 0; i < 8; ++i) {
+                    const uint64_t aa = pack2(av[i], av[i]);
+                    acc[i][0] = ffma2(aa, b0.x, acc[i][0]);
+                    acc[i][1] = ffma2(aa, b0.y, acc[i][1]);
+                    acc[i][2] = ffma2(aa, b1.x, acc[i][2]);
+                    acc[i][3] = ffma2(aa, b1.y, acc[i][3]);
+                }
+            } else {
+                const float av[4] = {a0.x, a0.y, a0.z, a0.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint64_t aa = pack2(av[i], av[i]);
+                    acc[i][0] = ffma2(aa, b0.x, acc[i][0]);
+                    acc[i][1] = ffma2(aa, b0.y, acc[i][1]);
+                }
             }
         }
         if (more) {
@@ -130,12 +142,25 @@ k_gemm_f32(const float *__restrict__ A, const float *__restrict__ Bm, float *__r
     }
     const bool split = gridDim.z > 1;
     float *out = split ? part_out + (size_t)blockIdx.z * N * M : C;
+    if ((split || (!accumulate && !mask)) && M % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < TM; ++i) {
+            const long long n = n0 + (i < 4 ? ty * 4 + i : BT / 2 + ty * 4 + i - 4);
+            if (n >= N) continue;
+#pragma unroll
+            for (int g = 0; g < TM / 4; ++g) {
+                const long long c = j0 + g * (BT / 2) + tx * 4;
+                if (c < M) *reinterpret_cast<ulonglong2 *>(out + n * M + c) = make_ulonglong2(acc[i][2 * g], acc[i][2 * g + 1]);
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
         const long long n = n0 + (i < 4 ? ty * 4 + i : BT / 2 + ty * 4 + i - 4);
         if (n >= N) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < TM / 2; ++j) {
             float v[2];
             unpack2(acc[i][j], v[0], v[1]);
 #pragma unroll
@@ -166,39 +191,40 @@ __global__ void k_gemm_f32_join(const float *__restrict__ part, float *__restric
     }
 }
 
-template <int BT, bool AT, bool BTr>
+template <int BT, int TM, bool AT, bool BTr>
 void launch(const GemmF32 &g, int parts, long long k_part, float *ws, bool va, bool vb, cudaStream_t st) {
     const dim3 grid((unsigned)((g.N + BT - 1) / BT), (unsigned)((g.M + BT - 1) / BT), (unsigned)parts);
-    const int threads = (BT / 8) * (BT / 8);
-    auto kern = va ? (vb ? k_gemm_f32<BT, AT, BTr, true, true> : k_gemm_f32<BT, AT, BTr, true, false>)
-                   : (vb ? k_gemm_f32<BT, AT, BTr, false, true> : k_gemm_f32<BT, AT, BTr, false, false>);
+    const int threads = (BT / TM) * (BT / TM);
+    auto kern = va ? (vb ? k_gemm_f32<BT, TM, AT, BTr, true, true> : k_gemm_f32<BT, TM, AT, BTr, true, false>)
+                   : (vb ? k_gemm_f32<BT, TM, AT, BTr, false, true> : k_gemm_f32<BT, TM, AT, BTr, false, false>);
     kern<<<grid, threads, 0, st>>>(g.A, g.B, g.C, g.N, g.K, g.M, k_part, g.accumulate, g.mask, ws);
 }
 
-template <int BT>
+template <int BT, int TM>
 void launch_bt(const GemmF32 &g, int parts, long long k_part, float *ws, bool va, bool vb, cudaStream_t st) {
     if (g.a_trans) {
-        if (g.b_trans) launch<BT, true, true>(g, parts, k_part, ws, va, vb, st);
-        else launch<BT, true, false>(g, parts, k_part, ws, va, vb, st);
+        if (g.b_trans) launch<BT, TM, true, true>(g, parts, k_part, ws, va, vb, st);
+        else launch<BT, TM, true, false>(g, parts, k_part, ws, va, vb, st);
     } else {
-        if (g.b_trans) launch<BT, false, true>(g, parts, k_part, ws, va, vb, st);
-        else launch<BT, false, false>(g, parts, k_part, ws, va, vb, st);
+        if (g.b_trans) launch<BT, TM, false, true>(g, parts, k_part, ws, va, vb, st);
+        else launch<BT, TM, false, false>(g, parts, k_part, ws, va, vb, st);
     }
 }
 
 }  // namespace
 
 int gemm_f32(qgru_handle *h, const GemmF32 &g, cudaStream_t st) {
-    // 128 x 128 tiles where they alone (or with few K parts) fill the SMs: half the operand traffic of
-    // 64 x 64.  K is split while that leaves SMs idle, in parts of two
-    // slabs or more: with two warps on an SM a slab takes about a microsecond (384 x 64 x 1600 and its two neighbours of a
-    // training step: 97 us with parts of 128, 73 with 32).
+    // 128 x 128 tiles where they alone (or with few K parts) fill the SMs: half the operand traffic of 64 x 64.  Those have
+    // eight warps to a tile, because a slab is latency where an SM has one tile: 4096 x 64 x 192 10 us, with two warps (8 x 8
+    // outputs a thread) 15.5; 256 x 64 x 192 6.3, with two warps and two parts 18.6.  K is split while the tiles leave SMs
+    // idle, in parts of two slabs or more (384 x 1600 x 64 15 us, with two warps 21; three such products of a training step
+    // with two warps 97 us in parts of 128 inputs, 73 in parts of 32).
     const auto tiles = [&](int bt) { return ((g.N + bt - 1) / bt) * ((g.M + bt - 1) / bt); };
     const bool big = tiles(128) * std::max<long long>(1, g.K / 512) >= h->sm_count && g.N > 64 && g.M > 64;
     const long long t = big ? tiles(128) : tiles(64);
     const long long want = big ? 2ll * h->sm_count : 4ll * h->sm_count;
     long long parts = std::max<long long>(1, std::min({want / std::max<long long>(1, t), g.K / PART_MIN, (long long)64}));
-    if (t >= h->sm_count) parts = 1;
+    if (t >= h->sm_count || g.K <= 128) parts = 1;      // (adding the parts is a launch of 4 us: as long as 128 inputs)
     long long k_part = ((g.K + parts - 1) / parts + BK - 1) / BK * BK;
     parts = (g.K + k_part - 1) / k_part;
     float *ws = nullptr;
@@ -210,8 +236,8 @@ int gemm_f32(qgru_handle *h, const GemmF32 &g, cudaStream_t st) {
     const auto al16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     const bool va = al16(g.A) && (g.a_trans ? g.N : g.K) % 4 == 0;
     const bool vb = al16(g.B) && (g.b_trans ? g.K : (long long)g.M) % 4 == 0;
-    if (big) launch_bt<128>(g, (int)parts, k_part, ws, va, vb, st);
-    else launch_bt<64>(g, (int)parts, k_part, ws, va, vb, st);
+    if (big) launch_bt<128, 8>(g, (int)parts, k_part, ws, va, vb, st);
+    else launch_bt<64, 4>(g, (int)parts, k_part, ws, va, vb, st);
     h->launches++;
     if (parts > 1) {
         const long long n = g.N * g.M;
