@@ -171,9 +171,9 @@ int float_forward(qgru_handle *h, int T, int B, const float *W, const float *R, 
     k_init_h_float<<<(unsigned)((NH + 255) / 256), 256, 0, st>>>(h0, h_out, NH);
     h->launches++;
     if ((rc = gemm_f32(h, GemmF32{x, false, W, false, wx, N, I, Cn}, st))) return rc;
-    if (float_chain_is_faster(h, B))
+    if (float_chain_is_faster(h, T, B))
         return float_chain_launch(h, FloatFwdArgs{T, B, H, R, wx, bw, br, h_out, v_out, v_stride, 0, 0, OutView()}, st);
-    // wide layers and very many rows, step by step: R*h as a tiled product, then the pointwise gates
+    // wide layers, very many rows or a step or two, step by step: R*h as a tiled product, then the pointwise gates
     if ((rc = ensure(h, h->f_acc2, (size_t)B * Cn * 4))) return rc;
     float *rh = (float *)h->f_acc2.p;
     dim3 grid((H + 127) / 128, (B + 1) / 2);

@@ -722,17 +722,18 @@ bool float_chain_fits(qgru_handle *h, int B) {
     return h->plan_fwd.ok;
 }
 
-// Where thousands of rows make many waves of clusters, the tiled product of a step (which reads R once for 64 or 128
-// rows) catches up.  us per step, chain / step by step: H = 512: 512 rows 60 / 66, 1024 rows 118 / 89, 4096 rows 467 / 198;
-// H = 384: 512 rows 34 / 37, 1024 rows 67 / 57; H = 256: 2048 rows 49 / 57, 4096 rows 96 / 81; H = 128: 8192 rows 55 / 57.
-// Both sides as fitted to such times (H = 32 .. 512, up to 8192 rows): on the right side at every one of the 110 sizes.
-bool float_chain_is_faster(qgru_handle *h, int B) {
+// Every wave of clusters loads R first, and thousands of rows make many waves, where the tiled product of a step reads R once
+// for 64 or 128 rows.  us per step, chain / step by step: H = 512: 128 rows 16 / 19, 512 rows 57 / 48, 4096 rows 460 / 176;
+// H = 384: 256 rows 16 / 19, 1024 rows 66 / 41; H = 256: 1024 rows 23 / 28, 4096 rows 93 / 69; H = 128: 4096 rows 23 / 27; and
+// calls of one step: H = 64, 64 rows 44.9 / 45.0, 4096 rows 68 / 59; H = 512, one row 57 / 48.  Both sides as fitted to
+// such times (H = 16 .. 512, up to 8192 rows): from four steps on at most 20 % off the better one at each of 120 sizes.
+bool float_chain_is_faster(qgru_handle *h, int T, int B) {
     // (float inference and calibration run one direction after the other: each has the whole chip)
     make_plan(h, B, h->sm_count, k_float_chain<false, 512>, fwd_smem_floats, &h->plan_fwd);
     const F32RecPlan &pl = h->plan_fwd;
     if (!pl.ok) return false;
     const double H = h->H, chain = pl.waves * (0.7 + 0.046 * (pl.U * pl.KG / 32) * pl.Bt * pl.sharing);
-    return chain <= 34.0 + (1.48e-7 * H + 1.02e-5) * H * B;
+    return 8.0 + 8.0 * pl.waves + T * chain <= T * (17.0 + (1.32e-7 * H + 1.0e-5) * H * B);
 }
 
 // (forms of at most 384 threads have registers to spare beside R: no spills)

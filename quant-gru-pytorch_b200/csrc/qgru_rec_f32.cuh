@@ -35,8 +35,8 @@ struct FloatFwdArgs {
 };
 // False: no plan for this shape (H > 512), the caller runs step by step.
 bool float_chain_fits(qgru_handle *h, int B);
-// Whether a step of it, with the whole chip to itself, takes no longer than a tiled product and a pointwise launch.
-bool float_chain_is_faster(qgru_handle *h, int B);
+// Whether T steps of it, with the whole chip to itself, take no longer than a tiled product and a pointwise launch a step.
+bool float_chain_is_faster(qgru_handle *h, int T, int B);
 int float_chain_launch(qgru_handle *h, FloatFwdArgs a, cudaStream_t st);
 
 struct BwdChainArgs {
