@@ -793,8 +793,10 @@ bool reg_is_faster(const RecRegPlan &pl, bool gemv) {
 }
 
 // The 8-bit path with the register-resident recurrence.  chained: the three launches of the forward as dependent launches,
-// each prepares itself (tensor maps, R to registers, tables) beside the one before; nothing may be recorded between
-// them, so that start times come from the kernels.
+// each prepares itself (tensor maps, R to registers, tables) beside the one before; a launch behind a recorded event does not
+// start early, so that start times come from the kernels instead.  (The forward direction of a bidirectional layer has
+// the event that lets the reverse direction start between its prologue and its product: that product starts when the
+// prologue is done.)
 int run_reg(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out, unsigned flags, RecCell cell, const RecRegPlan &pl,
             int ih_bytes, int n_table, bool chained, cudaStream_t st) {
     const long long N = (long long)T * B;
@@ -827,7 +829,6 @@ int run_reg(qgru_handle *h, int T, int B, const uint8_t *x8, const OutView &out,
     a.h8 = (const uint8_t *)h->h8.p;
     a.out = out;
     a.lc = linear_consts(h, 1);
-    a.gc = h->d_gc;
     a.tables = fused ? h->d_ftables : h->d_tables;
     a.n_table = n_table;
     a.abort_flag = h->d_flags + 1;

@@ -2,7 +2,8 @@
 // output (batch-first tensors, the two halves of a bidirectional output), no dense intermediate and no
 // host synchronisation.
 //
-// A call is three launches per direction (prologue, W*x product, recurrence) and four timing events; the
+// A call is three launches per direction (prologue, W*x product, recurrence) with a timing event before and behind them and,
+// where they are not dependent launches (run_reg), one on either side of the product; the
 // reverse direction runs on a stream of its own beside the forward one and reads the rows the forward
 // direction has quantized where both quantize x the same way.  A call on another stream than the one before waits for
 // that one's work on the GPU (StreamUse): calls of one layer never overlap.  A device-side

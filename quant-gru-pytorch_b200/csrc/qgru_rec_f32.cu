@@ -736,7 +736,8 @@ bool float_chain_is_faster(qgru_handle *h, int T, int B) {
     return 8.0 + 8.0 * pl.waves + T * chain <= T * (17.0 + (1.32e-7 * H + 1.0e-5) * H * B);
 }
 
-// (forms of at most 384 threads have registers to spare beside R: no spills)
+// (forms of at most 384 threads have registers to spare beside R: the backward has no spills there, the forward 40 and 68
+// bytes; with 512 threads 228 to 348 bytes)
 int float_chain_launch(qgru_handle *h, FloatFwdArgs a, cudaStream_t st) {
     const F32RecPlan &pl = h->plan_fwd;
     const bool one = pl.Bt <= std::min(pl.KG, RB), small = pl.U * pl.KG <= 384;

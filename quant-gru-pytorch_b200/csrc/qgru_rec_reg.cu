@@ -17,7 +17,8 @@
 // nothing leaves the SM and a step ends with one block barrier.  Larger layers send the new state to the
 // peers with st.async, counted on their mbarrier: no fence on the sending side.  A peer can be at most
 // one step ahead, so two state buffers are enough.
-// W*x + bw arrives by bulk copies, D steps ahead.
+// W*x + bw arrives D steps ahead: one bulk copy a step where one CTA owns the rows, 16-byte copies by every warp of what its
+// own cells read in clusters.
 #include "qgru_rec_reg_kernel.cuh"
 
 namespace qgru {

@@ -25,13 +25,12 @@ struct RecRegPlan {
 enum RecCell { CELL_INT_FAST = 0, CELL_INT_FAST_NOTIE = 1, CELL_INT_GENERIC = 2, CELL_FS = 3, CELL_INT_TRAIN = 4, CELL_FS_TRAIN = 5 };
 
 struct RecRegArgs {
-    int T, B, H, Hpad, reverse, h_unsigned;
+    int T, B, H, Hpad, reverse;
     const int8_t *r8;             // [3H][Hpad]
     const void *ih;               // [P][T*B][3][U]: W*x + bw as the cell takes it
     const uint8_t *h8;            // [B][Hpad] initial state
     OutView out;
     LinearConsts lc;              // R*h + br epilogue
-    const GateConsts *gc;         // device copy (generic cell)
     const int32_t *tables;
     int n_table;
     const float *fs_chan;         // float-storage cell: [3][C] offset, bias term, scale ratio of R*h + br

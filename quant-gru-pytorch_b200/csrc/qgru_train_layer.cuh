@@ -236,7 +236,6 @@ int train_forward_dir(qgru_handle *h, int mode, int T, int B, const void *x, lon
     a.h8 = (const uint8_t *)h->h8.p;
     a.out = out;
     a.lc = linear_consts(h, 1);
-    a.gc = h->d_gc;
     a.tables = mode == 1 ? (const int32_t *)fs.train_tab : h->d_ttables;
     a.n_table = n_tab;
     a.abort_flag = h->d_flags + 1;
