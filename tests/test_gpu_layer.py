@@ -63,3 +63,27 @@ def test_layer_forward_equals_dense_forwards(cuda_device, cfg, storage, T, B, I,
             h = m._dirs[d].handle.forward_i32(x_q.transpose(0, 1).contiguous(), reverse=d == 1)
             assert torch.equal(out_q[:, :, d * H:(d + 1) * H], (h[1:] if d == 0 else h[:T]).transpose(0, 1))
             assert torch.equal(hn_q[d], h[T] if d == 0 else h[0])
+
+
+@pytest.mark.parametrize("storage,H", [("int32", 64), ("float32", 300), ("float", 200)])
+def test_batch_sizes_that_alternate(cuda_device, storage, H):
+    """One module, batches of changing size (a last short one among them): plans, workspace and tensor maps follow."""
+    import torch
+    I, T = 20, 6
+    rng = np.random.default_rng(H)
+    xs = [torch.from_numpy(np.ascontiguousarray(gen_x(rng, b, T, I))).to(cuda_device) for b in (32, 7, 300, 31)]
+
+    def module():
+        m = _module("default", I, H, True, True, "float32" if storage == "float" else storage, xs[0], cuda_device)
+        m.use_quantization = storage != "float"
+        return m
+
+    def step(m, x):
+        out, hn = m.train()(x)
+        grads = torch.autograd.grad(out.sum() + hn.sum(), list(m.parameters()))
+        with torch.no_grad():
+            return [out.detach(), hn.detach(), *grads, *m.eval()(x)]
+    want = [step(module(), x) for x in xs]
+    m = module()
+    for i in (0, 1, 0, 2, 3, 2, 1, 0):
+        assert all(torch.equal(a, b) for a, b in zip(step(m, xs[i]), want[i])), i

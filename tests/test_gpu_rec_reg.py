@@ -68,3 +68,28 @@ def test_wide_recurrence_equals_oracle(oracle, cuda_device, cfg, T, B, H):
         assert np.array_equal(hd.forward_i32(x, h0).cpu().numpy(), want)
         assert ("path=wide" in hd.describe_plan()) == (H <= 256)
         assert torch.equal(base[0], hd.forward_i32(x, h0, reverse=True)) and torch.equal(base[1], hd.forward_f32(xf, f0))
+
+
+@pytest.mark.parametrize("H,P,rows", [(512, 4, 8), (384, 3, 8), (1024, 16, 16), (600, 10, 16)])
+def test_fast_on_either_side_of_its_line(oracle, cuda_device, H, P, rows):
+    """rec=fast takes clusters with R in registers up to so many rows a cluster (one tile of eight, two above H = 512) and
+    tcgen05 beyond; sm_limit keeps the number of clusters, and so the rows, small."""
+    import torch
+    T, I = 5, 7
+    with gru_ops.Handle(I, H, device=cuda_device.index or 0) as hd:
+        hd.set_option("rec", "fast")
+        hd.set_option("sm_limit", 2 * P)
+        seen = set()
+        for B in (rows - 1, rows, rows + 1, 2 * rows, 2 * rows + 1):
+            case = make_case(B * 31 + H, T, B, I, H, oracle, config_named("cfg2"))
+            hd.set_params(case.params)
+            hd.set_weights_i32(*[torch.from_numpy(np.ascontiguousarray(a)).to(cuda_device) for a in case.wq])
+            want = oracle.forward_i32(T, B, I, H, case.wq, case.x_q, case.h0_q, case.params.c, case.params.scale_list())
+            h0 = None if case.h0_q is None else torch.from_numpy(case.h0_q).to(cuda_device)
+            got = hd.forward_i32(torch.from_numpy(case.x_q).to(cuda_device), h0)
+            assert np.array_equal(got.cpu().numpy(), want), hd.describe_plan()
+            plan = dict(w.split("=") for w in hd.describe_plan().split() if "=" in w)
+            if plan["r_in"] == "registers":
+                assert int(plan["Bt"]) <= rows
+            seen.add((plan["r_in"] == "registers", int(plan.get("Bt", 0))))
+        assert (True, rows) in seen and any(not reg for reg, _ in seen), seen
