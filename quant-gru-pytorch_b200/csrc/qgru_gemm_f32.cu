@@ -1,5 +1,5 @@
-// qgru_gemm_f32.cu - fp32 matrix product on the CUDA cores: the input projection of float mode and
-// calibration, and the three products of the backward pass.
+// qgru_gemm_f32.cu - the fp32 matrix product: the input projection of float mode and calibration, and the three
+// products of the backward pass.  Large ones run on the tensor cores (qgru_gemm_f32_tc.cu), the others here on the CUDA cores.
 //
 // 128 x 128 tiles of C with 8 x 8 outputs per thread, or 64 x 64 with 4 x 4, as packed pairs (fma.rn.f32x2: two IEEE
 // fused multiply-adds per instruction, so that operand loads and the copies that duplicate A's value
@@ -213,7 +213,39 @@ void launch_bt(const GemmF32 &g, int parts, long long k_part, float *ws, bool va
 
 }  // namespace
 
+// the parts in h->f_split into C
+int gemm_f32_join(qgru_handle *h, const GemmF32 &g, int parts, cudaStream_t st) {
+    const long long n = g.N * g.M;
+    k_gemm_f32_join<<<grid_for(n, 256, h->sm_count), 256, 0, st>>>((const float *)h->f_split.p, g.C, n, parts, g.accumulate, g.mask);
+    h->launches++;
+    return QGRU_OK;
+}
+
 int gemm_f32(qgru_handle *h, const GemmF32 &g, cudaStream_t st) {
+    // Tensor cores where there is work for them: a slab of 32 K takes a CTA about 1.7 us there and a tile 8 us beside its slabs.
+    // us, tensor cores / fp32 pipe: 51200 x 1536 x 256 331 / 862; 12800 x 128 x 768 47 / 71; 6400 x 64 x 384 14 / 21; 384 x 3200 x 128
+    // 22 / 24; below that 384 x 1600 x 128 19 / 19, 64 x 1536 x 512 20 / 17.  A narrow C fills the tile of neither (6400 x 384 x 64
+    // 28 / 24, 12800 x 384 x 16 29 / 41); few K leave only the tile's own time (12800 x 16 x 768 31 / 18), and operands without two
+    // neighbours in one load more of it (12801 x 77 x 600 49 / 41, 12801 x 600 x 77 66 / 76).
+    const bool pairs = ((g.a_trans ? g.N : g.K) | (g.b_trans ? g.K : (long long)g.M)) % 2 == 0 &&
+                       ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 7u) == 0;
+    if (g.K >= (pairs ? 64 : 256) && (double)g.N * g.K * std::max(g.M, 64) >= (g.M <= 64 ? 2.5e8 : 1.5e8) && gemm_f32_tc_fits(g)) {
+        int width;
+        const long long t = gemm_f32_tc_tiles(g, &width);
+        long long parts = t >= h->sm_count ? 1 : std::max<long long>(1, std::min<long long>(h->sm_count / t, g.K / 64));
+        const long long k_part = ((g.K + parts - 1) / parts + 31) / 32 * 32;
+        parts = (g.K + k_part - 1) / k_part;
+        int rc;
+        if (parts > 1 && (rc = ensure(h, h->f_split, (size_t)parts * g.N * g.M * sizeof(float)))) return rc;
+        if ((rc = gemm_f32_tc_launch(h, g, (int)parts, k_part, parts > 1 ? (float *)h->f_split.p : g.C, st))) return rc;
+        h->launches++;
+        if (parts > 1) gemm_f32_join(h, g, (int)parts, st);
+        CK(cudaGetLastError());
+        return QGRU_OK;
+    }
+    const auto al16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    const bool va = al16(g.A) && (g.a_trans ? g.N : g.K) % 4 == 0;
+    const bool vb = al16(g.B) && (g.b_trans ? g.K : (long long)g.M) % 4 == 0;
     // 128 x 128 tiles where they alone (or with few K parts) fill the SMs: half the operand traffic of 64 x 64.  Those have
     // eight warps to a tile, because a slab is latency where an SM has one tile: 4096 x 64 x 192 10 us, with two warps (8 x 8
     // outputs a thread) 15.5; 256 x 64 x 192 6.3, with two warps and two parts 18.6.  K is split while the tiles leave SMs
@@ -233,17 +265,10 @@ int gemm_f32(qgru_handle *h, const GemmF32 &g, cudaStream_t st) {
         if ((rc = ensure(h, h->f_split, (size_t)parts * g.N * g.M * sizeof(float)))) return rc;
         ws = (float *)h->f_split.p;
     }
-    const auto al16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-    const bool va = al16(g.A) && (g.a_trans ? g.N : g.K) % 4 == 0;
-    const bool vb = al16(g.B) && (g.b_trans ? g.K : (long long)g.M) % 4 == 0;
     if (big) launch_bt<128, 8>(g, (int)parts, k_part, ws, va, vb, st);
     else launch_bt<64, 4>(g, (int)parts, k_part, ws, va, vb, st);
     h->launches++;
-    if (parts > 1) {
-        const long long n = g.N * g.M;
-        k_gemm_f32_join<<<grid_for(n, 256, h->sm_count), 256, 0, st>>>(ws, g.C, n, (int)parts, g.accumulate, g.mask);
-        h->launches++;
-    }
+    if (parts > 1) gemm_f32_join(h, g, (int)parts, st);
     CK(cudaGetLastError());
     return QGRU_OK;
 }

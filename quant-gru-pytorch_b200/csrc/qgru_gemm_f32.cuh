@@ -23,6 +23,13 @@ struct GemmF32 {
 };
 int gemm_f32(qgru_handle *h, const GemmF32 &g, cudaStream_t st);
 
+// The same on the tensor cores (qgru_gemm_f32_tc.cu): whether its grid and its 32-bit offsets cover the sizes; number and width of its tiles; `parts` of K into `out` (C itself with one
+// part, else [parts][N][M]), added by gemm_f32_join.
+bool gemm_f32_tc_fits(const GemmF32 &g);
+int gemm_f32_tc_tiles(const GemmF32 &g, int *width);
+int gemm_f32_join(qgru_handle *h, const GemmF32 &g, int parts, cudaStream_t st);
+int gemm_f32_tc_launch(qgru_handle *h, const GemmF32 &g, int parts, long long k_part, float *out, cudaStream_t st);
+
 // packed fp32 pairs (one register pair, element 0 in the low half)
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
     uint64_t d;
@@ -31,6 +38,16 @@ __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
 }
 __device__ __forceinline__ void unpack2(uint64_t v, float &lo, float &hi) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t fsub2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
 }
 // two independent IEEE fused multiply-adds in one instruction
 __device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {

@@ -1,0 +1,78 @@
+"""GPU tests of the fp32 product on the tensor cores (three bf16 parts per operand), at the edges of its tiles and for values
+that have no such parts."""
+import importlib
+
+import numpy as np
+import pytest
+
+from __graft_entry__ import PKG_NAME
+from tests.cases import gen_weights
+
+gru_ops = importlib.import_module(PKG_NAME + ".gru_ops")
+pytestmark = pytest.mark.gpu
+
+
+def _t(a, dev):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a)).to(dev)
+
+
+# (T * B, I, H): I and 3H at and beside tiles of 128 and 256, rows in groups of four, two and one, K with and without a rest
+@pytest.mark.parametrize("T,B,I,H", [(16, 256, 128, 128), (31, 131, 130, 86), (50, 81, 257, 43), (33, 128, 16, 171), (67, 96, 64, 256)])
+def test_products_of_the_backward(cuda_device, T, B, I, H):
+    import torch
+    rng = np.random.default_rng(I * H)
+    W, R, _, _ = gen_weights(rng, I, H)
+    v = torch.rand(T, B, 4 * H, device=cuda_device)
+    h = torch.randn(T + 1, B, H, device=cuda_device) * 0.3
+    x = torch.randn(T, B, I, device=cuda_device)
+    dh = torch.randn(T + 1, B, H, device=cuda_device)
+    with gru_ops.Handle(I, H, device=0) as hd:
+        dx, dW, dR, dbw, dbr, _ = hd.backward(_t(W, cuda_device), _t(R * 0, cuda_device), x, dh, h, v)
+    # R = 0: dp and dq of a step depend on its own gradient and what comes through the update gate; float64
+    z, r, g, q = (v[..., k * H:(k + 1) * H].double() for k in range(4))
+    carry = torch.zeros(B, H, dtype=torch.float64, device=cuda_device)
+    dp = torch.empty(T, B, 3 * H, dtype=torch.float64, device=cuda_device)
+    dq = torch.empty_like(dp)
+    for t in range(T - 1, -1, -1):
+        d = dh[t + 1].double() + carry
+        dg = (1 - g[t] ** 2) * (1 - z[t]) * d
+        dz = z[t] * (1 - z[t]) * (h[t].double() - g[t]) * d
+        dr = r[t] * (1 - r[t]) * dg * q[t]
+        dp[t], dq[t] = torch.cat([dz, dr, dg], 1), torch.cat([dz, dr, dg * r[t]], 1)
+        carry = z[t] * d
+    P, Q = dp.reshape(T * B, -1), dq.reshape(T * B, -1)
+    want = [P @ _t(W, cuda_device).double().t(), x.reshape(-1, I).double().t() @ P, h[:T].reshape(-1, H).double().t() @ Q]
+    for a, b in zip((dx, dW, dR), want):
+        # dp and dq carry a few fp32 roundings each (2^-24 of values with a spread of order one); sums over K of them less
+        a = a.double().reshape(b.shape)
+        assert (a - b).norm() <= 5e-7 * b.norm()
+        assert (a - b).abs().max() <= 1e-5 * b.abs().max()
+
+
+@pytest.mark.parametrize("value", [float("inf"), -float("inf"), float("nan"), 3.4e38])
+def test_input_projection_of_values_without_bf16_parts(cuda_device, value):
+    """A row with such a value takes the fp32 multiply-adds of its tile; the other rows are as before."""
+    import torch
+    T, B, I, H = 2, 700, 128, 300
+    rng = np.random.default_rng(3)
+    W, R, bw, br = (_t(a, cuda_device) for a in gen_weights(rng, I, H))
+    x = torch.randn(T, B, I, device=cuda_device)
+    bad = x.clone()
+    bad[0, 130, 7] = value
+    with gru_ops.Handle(I, H, device=0) as hd:
+        clean = hd.forward_float(W, R, bw, br, x)
+        got = hd.forward_float(W, R, bw, br, bad)
+    # the step in float64 for the one row (a finite product that overflows in fp32 is an infinity here too: |w| >= 2^-10)
+    pre = torch.where(W[7].abs() * abs(value) > 3.4028235e38, torch.sign(W[7]) * torch.sign(torch.tensor(value)).item() * float("inf"),
+                      (bad[0, 130].double() @ W.double())) if np.isinf(value) else bad[0, 130].double() @ W.double()
+    pre = pre + bw.double()
+    z, r = torch.sigmoid(pre[:H] + br[:H].double()), torch.sigmoid(pre[H:2 * H] + br[H:2 * H].double())
+    want = (1 - z) * torch.tanh(pre[2 * H:] + r * br[2 * H:].double())
+    row = got[1, 130].double()
+    assert torch.equal(torch.isnan(row), torch.isnan(want))
+    ok = ~torch.isnan(want)
+    assert (row - want)[ok].abs().max() <= 2e-6 if ok.any() else True
+    others = [b for b in range(B) if b != 130]
+    # (sums in another order where the tile was multiplied again)
+    assert (got[:, others] - clean[:, others]).abs().max() <= 2e-6
