@@ -11,7 +11,7 @@ _ROOT = os.path.dirname(_HERE)
 _CSRC = os.path.join(_HERE, "csrc")
 _OBJ = os.path.join(_HERE, "build")
 SOURCES = ["qgru_api.cu", "qgru_gemm_tc.cu", "qgru_rec_mma.cu", "qgru_rec_cluster.cu", "qgru_rec_c64.cu", "qgru_rec_reg.cu",
-           "qgru_rec_reg_float.cu", "qgru_float.cu", "qgru_gemm_f32.cu", "qgru_gemm_f32_tc.cu", "qgru_rec_f32.cu", "qgru_hist.cu", "qgru_backward.cu", "qgru_probe.cu", "qgru_host.cc"]
+           "qgru_rec_reg_float.cu", "qgru_float.cu", "qgru_gemm_f32.cu", "qgru_gemm_f32_tc.cu", "qgru_rec_f32.cu", "qgru_hist.cu", "qgru_backward.cu", "qgru_bwd_tc.cu", "qgru_probe.cu", "qgru_host.cc"]
 OUT = os.path.join(_HERE, "libqgru_b200.so")
 
 

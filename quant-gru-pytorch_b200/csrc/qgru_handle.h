@@ -155,7 +155,7 @@ struct qgru_handle {
     DevBuf bwd_dp, bwd_dq;                 // backward pass: gradients of W*x + bw and R*h + br, [T*B][3H] each
     DevBuf bwd_bias, bwd_pm;               // backward pass: bias sums per batch group, packed clamp masks
     DevBuf f_split;                        // fp32 matrix product: partial tiles where K is split
-    qgru::F32RecPlan plan_fwd, plan_bwd;   // fp32 recurrences: the plan of the last batch size
+    qgru::F32RecPlan plan_fwd, plan_bwd, plan_bwd_tc;   // fp32 recurrences: the plan of the last batch size
     DevBuf fs_ch;                          // float-storage forward: 4 x 3H per-channel scale ratios
     bool fs_uploaded = false, fs_ready = false;   // fs_ch matches the current parameters; and the current weights
     StreamOrder order;

@@ -753,6 +753,12 @@ bool bwd_chain_fits(qgru_handle *h, int B, int *groups) {
     return h->plan_bwd.ok;
 }
 
+// us per step in chains of 24, here / on the tensor cores: H = 96: 1 row 2.0 / 2.3, 256 rows 2.4 / 2.4; H = 112: 2.7 / 2.3, 3.3 / 2.5;
+// H = 262: 2.8 / 2.5, 9.8 / 3.7; H = 512: 3.5 / 2.8, 23.2 / 6.2.
+bool bwd_chain_tc_is_faster(qgru_handle *h, int B) {
+    return h->H > 96 && bwd_chain_tc_plan(h, B, side_sms(h), &h->plan_bwd_tc);
+}
+
 int bwd_chain_launch(qgru_handle *h, BwdChainArgs a, cudaStream_t st) {
     const F32RecPlan &pl = h->plan_bwd;
     const bool one = pl.Bt <= pl.KG, small = pl.U * pl.KG <= 384;

@@ -52,10 +52,18 @@ struct BwdChainArgs {
     const uint16_t *pm;               // packed clamp masks [T*B][H] or null
     float *dp, *dq;                   // [T*B][3H]: gradients of W*x + bw (masked) and of R*h + br
     float *bias_part;                 // [G][6][H]: sums of dp (before its mask) and of dq over the group's rows
+    const int8_t *r8;                 // where R is a quantized weight: its integers [3H][H], gates z, r, n, and the scale of each row
+    const float *r_scale;
     int U, P, KG, Bt, D;              // set by the launcher
 };
 bool bwd_chain_fits(qgru_handle *h, int B, int *groups);
 int bwd_chain_launch(qgru_handle *h, BwdChainArgs a, cudaStream_t st);
+
+// The same on the tensor cores, for a quantized R (r8, r_scale and pm are set; qgru_bwd_tc.cu).  The plan is kept in *pl for its
+// sizes; false: none.  bwd_chain_tc_is_faster plans into the handle's plan_bwd_tc.
+bool bwd_chain_tc_plan(qgru_handle *h, int B, int sms, F32RecPlan *pl);
+bool bwd_chain_tc_is_faster(qgru_handle *h, int B);
+int bwd_chain_tc_launch(qgru_handle *h, const F32RecPlan &pl, const BwdChainArgs &a, cudaStream_t st);
 
 // Bias gradients from bias_part; masks and either output may be null.
 void bwd_bias_launch(qgru_handle *h, const float *part, int G, const uint8_t *m_bw, const uint8_t *m_br, float *dbw, float *dbr, int accumulate,

@@ -27,6 +27,8 @@ struct TrainWeightsArgs {
     int64_t *corr[2];
     FastLin *fl[2];
     float *deq[2];                     // [3H][K]
+    int8_t *q8;                        // R's integers [3H][H] and scales [3H], channels z, r, n, for the backward
+    float *qscale;
     uint8_t *keep[2], *bias_keep[2];
     int K[2], Kpad[2], H;
     int32_t zp_in[2], lo[2], hi[2], b_lo[2], b_hi[2];
@@ -51,6 +53,7 @@ __global__ void __launch_bounds__(128) k_train_weights(const TrainWeightsArgs a)
             a.keep[side][(size_t)row * K + k] = (raw < lo || raw > hi) ? 0 : 1;
         }
         a.w8[side][(size_t)c * Kpad + k] = (int8_t)q;
+        if (side && k < K) a.q8[(size_t)c * K + k] = (int8_t)q;
     }
     __shared__ int red[4];
     for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
@@ -63,6 +66,7 @@ __global__ void __launch_bounds__(128) k_train_weights(const TrainWeightsArgs a)
     a.bias_keep[side][row] = (b_raw < (float)a.b_lo[side] || b_raw > (float)a.b_hi[side]) ? 0 : 1;
     a.bias_q[side][c] = bq;
     a.wsum[side][c] = sum;
+    if (side) a.qscale[c] = scale;
     const int64_t corr = rescale64((int64_t)bq, a.brs[side][c]) - (int64_t)a.zp_in[side] * (int64_t)sum;
     a.corr[side][c] = corr;
     a.fl[side][c] = make_fast_lin(a.rs[side][c], corr);
@@ -78,7 +82,8 @@ namespace {
 
 // The caller's block of one direction.
 struct TrainSaved {
-    float *h, *v, *xd, *W, *R;
+    float *h, *v, *xd, *W, *R, *r_scale;
+    int8_t *r8;
     uint16_t *pm;
     uint8_t *mx, *mh0, *mW, *mR, *mbw, *mbr;
     size_t bytes;
@@ -104,6 +109,8 @@ TrainSaved train_saved(const qgru_handle *h, int mode, int T, int B, void *base)
     s.mR = (uint8_t *)take(q * C * H);
     s.mbw = (uint8_t *)take(q * C);
     s.mbr = (uint8_t *)take(q * C);
+    s.r8 = (int8_t *)take(q * C * H);
+    s.r_scale = (float *)take(q * C * 4);
     s.bytes = at;
     return s;
 }
@@ -182,6 +189,8 @@ int train_forward_dir(qgru_handle *h, int mode, int T, int B, const void *x, lon
         w.b_hi[k] = op_qmax(bo);
     }
     w.H = H;
+    w.q8 = s.r8;
+    w.qscale = s.r_scale;
     if (mode == 1) {
         w.ch = fs.ch;
         w.chan = fs.chan;
@@ -263,14 +272,17 @@ int train_backward_dir(qgru_handle *h, int mode, int T, int B, const float *x, c
     const long long N = (long long)T * B;
     int rc, G = 0;
     if (!bwd_chain_fits(h, B, &G)) return fail(h, QGRU_ERR_UNSUPPORTED, "no one-launch recurrence for this layer");
+    const bool tc = mode != 0 && bwd_chain_tc_is_faster(h, B);
+    if (tc) G = h->plan_bwd_tc.G;
     if ((rc = ensure(h, h->bwd_dp, (size_t)N * C * 4))) return rc;
     if ((rc = ensure(h, h->bwd_dq, (size_t)N * C * 4))) return rc;
     if ((rc = ensure(h, h->bwd_bias, ((size_t)G * 2 * C + (size_t)B * H) * 4))) return rc;
     float *dp = (float *)h->bwd_dp.p, *dq = (float *)h->bwd_dq.p, *part = (float *)h->bwd_bias.p;
     if (!dh0) dh0 = part + (size_t)G * 2 * C;
-    if ((rc = bwd_chain_launch(h, BwdChainArgs{T, B, H, s.R, 1, 1, rev ? 1 : 0, s.h, s.v, dout, do_ts, do_bs, dhn, dh0, mode ? s.mh0 : nullptr,
-                                               mode ? s.pm : nullptr, dp, dq, part}, st)))
-        return rc;
+    BwdChainArgs chain{T, B, H, s.R, 1, 1, rev ? 1 : 0, s.h, s.v, dout, do_ts, do_bs, dhn, dh0, mode ? s.mh0 : nullptr, mode ? s.pm : nullptr, dp, dq, part};
+    chain.r8 = s.r8;
+    chain.r_scale = s.r_scale;
+    if ((rc = tc ? bwd_chain_tc_launch(h, h->plan_bwd_tc, chain, st) : bwd_chain_launch(h, chain, st))) return rc;
     if (d.dbw || d.dbr) bwd_bias_launch(h, part, G, mode ? s.mbw : nullptr, mode ? s.mbr : nullptr, d.dbw, d.dbr, 0, st);
     // dW[m][i] = sum_n dp[n][m] * x[n][i];  dR[m][k] = sum_n dq[n][m] * h_{t-1}[n][k]
     if (d.dW && (rc = gemm_f32(h, GemmF32{dp, true, mode ? xd : x, false, d.dW, C, N, I, 0, mode ? s.mW : nullptr}, st))) return rc;
