@@ -479,7 +479,7 @@ bool bwd_chain_tc_plan(qgru_handle *h, int B, int sms, F32RecPlan *best) {
             cudaGetLastError();
             continue;
         }
-        active = std::min(active, sms / pl.P);
+        active = std::min((int)((long long)active * sms / h->sm_count), sms / pl.P);
         if (active <= 0) continue;
         pl.waves = (B + active * most - 1) / (active * most);
         pl.Bt = (B + active * pl.waves - 1) / (active * pl.waves);

@@ -66,22 +66,22 @@ __device__ __forceinline__ void cp_async_wait_depth(int D) {
 // gate buffer of the step on its way out, the biases.
 __host__ __device__ inline size_t fwd_smem_floats(int P, int U, int KG, int Bt, int D) {
     return (size_t)(P == 1 ? 2 : 1) * Bt * P * U + (P > 1 ? (size_t)2 * Bt * U : 0) +
-           (size_t)(Bt > RB ? 2 : 1) * KG * (Bt > RB ? RB : Bt) * 3 * U + (size_t)D * Bt * 3 * U + (size_t)6 * Bt * U + (size_t)6 * U;
+           (size_t)(Bt > KG && Bt > RB ? 2 : 1) * KG * (Bt > KG && Bt > RB ? RB : Bt) * 3 * U + (size_t)D * Bt * 3 * U + (size_t)6 * Bt * U + (size_t)6 * U;
 }
 
-// One: a thread has at most one cell a step (Bt <= KG and one block of rows): its results stay in registers between the
+// One: a thread has at most one cell a step (Bt <= KG; all rows are one block): its results stay in registers between the
 // cell and the stores, and no loop, staging buffer or 64-bit index is left around them.  A step of few rows
 // is a chain of some 900 dependent instructions at about five cycles each, so their number is what counts.
 template <bool One, int MaxThreads>
 __global__ void __launch_bounds__(MaxThreads, 1) k_float_chain(const FloatFwdArgs a) {
     extern __shared__ __align__(16) float sm[];
     const int U = a.U, P = a.P, KG = a.KG, Bt = a.Bt, D = a.D, PU = P * U, H = a.H, C = 3 * H;
-    const int rb_max = min(Bt, RB), BtU = Bt * U;
+    const int rb = One ? Bt : RB, rb_max = min(Bt, rb), BtU = Bt * U;
     float *hs = sm;
     float *own = hs + (size_t)(P == 1 ? 2 : 1) * Bt * PU;
     float *part = own + (P > 1 ? 2 * BtU : 0);
     const int part_n = KG * rb_max * 3 * U;
-    float *wxs = part + (Bt > RB ? 2 : 1) * part_n;         // [D][Bt][3][U]
+    float *wxs = part + (Bt > rb ? 2 : 1) * part_n;         // [D][Bt][3][U]
     float *vst = wxs + (size_t)D * 3 * BtU;                 // [6][Bt][U]
     float *bias = vst + (size_t)6 * BtU;
 
@@ -199,8 +199,8 @@ __global__ void __launch_bounds__(MaxThreads, 1) k_float_chain(const FloatFwdArg
         const float *wxc = wxs + slot * 3 * BtU + cu;
         float *next = P > 1 ? own + ((s + 1) & 1) * BtU + cu : hs + ((s + 1) & 1) * BtU + cu;
         float o_z = 0.f, o_r = 0.f, o_g = 0.f, o_rz = 0.f, o_rr = 0.f, o_rg = 0.f, o_h = 0.f;   // One: this step's cell
-        for (int r0 = 0, pb = 0; r0 < nb; r0 += RB, pb ^= 1) {
-            const int r1 = min(nb, r0 + RB);
+        for (int r0 = 0, pb = 0; r0 < nb; r0 += rb, pb ^= 1) {
+            const int r1 = min(nb, r0 + rb);
             float *pk = part + pb * part_n + kg * rb_max * 3 * U + u;
             int b = r0;
             // (two rows at a time where there are registers for it)
@@ -667,35 +667,51 @@ cudaError_t launch_chain(Kern kern, const F32RecPlan &pl, Args &a, cudaStream_t 
     return cudaLaunchKernelEx(&cfg, kern, a);
 }
 
-// The smallest cluster whose registers hold R: 96 values in each of at most 512 threads a CTA.
-template <typename Kern>
-void make_plan(qgru_handle *h, int B, int sms, Kern kern, size_t (*floats)(int, int, int, int, int), F32RecPlan *pl) {
+// A form per cluster size whose registers hold R: 96 values in each of at most 512 threads a CTA.  `kern(threads)`: the kernel that a
+// CTA of so many threads runs.  us per step, 32 / 64 units a CTA: forward H = 256: 1 row 1.9 / 3.5, 64 rows (5 a cluster) 2.8 / 3.9,
+// 128 rows (9) 5.1 / 4.7; H = 128: 1 row 1.6 / 1.9, 256 rows (7, more than a cell a thread) 4.6 / 2.6; H = 160, 512 rows 10.8 / 7.5; backward
+// H = 256: 1 row 2.0 / 2.7, 96 rows 3.6 / 3.9, 128 rows 5.3 / 4.4.  One CTA against clusters: H = 96 1.35 / 1.7, H = 128 (512 threads)
+// 2.2 / 1.6.  The cost of a form is fitted to such times (H = 32 .. 512, 1 to 512 rows, one and two directions).
+template <typename KernOf>
+void make_plan(qgru_handle *h, int B, int sms, bool fwd, KernOf kern, size_t (*floats)(int, int, int, int, int), F32RecPlan *pl) {
     const int H = h->H;
     if (pl->H == H && pl->B == B && pl->sms == sms) return;
     *pl = F32RecPlan{};
     pl->H = H;
     pl->B = B;
     pl->sms = sms;
+    const int both = 2 * sms <= h->sm_count ? 2 : 1;      // directions side by side: as many clusters again
+    double best = 0;
     for (int P = 1; P <= 16; ++P) {
-        const int U = ((H + P - 1) / P + 31) / 32 * 32, KG = P * U / 32;
-        if (U * KG > 512 || (P - 1) * U >= H) continue;
-        // Rows per cluster: the fewest waves of clusters times the time of a step, which is a latency
-        // (two block barriers, the cell, and a cluster barrier with remote loads) plus the fp32 pipe's
-        // time per row: 96 multiply-adds in each of U * KG threads over four 32-lane pipes.
-        const int active0 = active_clusters(kern, P, U * KG, floats(P, U, KG, 1, 1) * sizeof(float));
-        double best = 0;
+        const int U = ((H + P - 1) / P + 31) / 32 * 32, KG = P * U / 32, threads = U * KG;
+        if (threads > 512 || (P - 1) * U >= H) continue;
+        const int active0 = active_clusters(kern(threads), P, threads, floats(P, U, KG, 1, 1) * sizeof(float));
+        if (active0 <= 0) continue;
+        // Cycles of a step of Bt rows: block barriers, the cell and, in a cluster, its barrier and the remote loads; spills in CTAs of
+        // more than 384 threads; the product and the partial sums of a row, where a warp of 32 units has fewer neighbours to
+        // share the row's state with.  With more than a cell a thread a row costs a block barrier's share at least.
+        const int warps = threads / 32;
+        const double base = P == 1 ? (threads <= 384 ? 2050.0 : 3500.0) : threads > 384 ? 6000.0 : U == 32 ? 2950.0 : 3100.0 + 100.0 * (P - 2);
+        const auto step = [&](int rows, int sharing) {
+            return rows <= KG ? base + (U == 32 ? 70.0 : 47.0) * warps * rows * sharing
+                   : fwd ? base + 2000.0 + std::max(750.0, (U == 32 ? 80.0 : 66.0) * warps) * rows * sharing
+                         : base + 2400.0 + (U == 32 ? std::max(540.0, 65.0 * warps) : 52.0 * warps) * rows * sharing;
+        };
         for (int Bt = 1; Bt <= MAX_ROWS && Bt <= B; ++Bt) {
             // operands three steps ahead where a step is shorter than a trip to memory
-            const int D = Bt <= RB ? 3 : 1;
+            const int D = Bt <= std::max(RB, KG) ? 3 : 1;
             const size_t smem = floats(P, U, KG, Bt, D) * sizeof(float);
             if (smem > (size_t)h->smem_optin) break;
             const int per_sm = std::max<int>(1, (int)std::min<size_t>((size_t)(active0 * P / h->sm_count), (size_t)(227 * 1024) / (smem + 1024)));
-            const int active = std::max(1, std::min(active0, sms * per_sm / P));
-            const int G = (B + Bt - 1) / Bt, waves = (G + active - 1) / active;
-            const int sharing = std::max(1, std::min(per_sm, (G * P + sms - 1) / sms));
-            const double step = (P > 1 ? 2200.0 : 900.0) + 28.0 * (U * KG / 32) * Bt * sharing;
-            if (best == 0 || waves * step < best) {
-                best = waves * step;
+            const int chip = both > 1 ? h->sm_count : sms;
+            const int active = std::max(1, std::min(active0, chip * per_sm / P));
+            const int G = (B + Bt - 1) / Bt, waves = (both * G + active - 1) / active;
+            const int sharing = std::max(1, std::min(per_sm, (both * G * P + chip - 1) / chip));
+            double cost = waves * step(Bt, sharing);
+            // One cluster too many for the chip, but with few rows: the last ones of the two directions follow one another.
+            if (both > 1 && both * G == active + 1) cost = std::min(cost, std::max(step(Bt, sharing), 2.0 * step(B - (G - 1) * Bt, sharing)));
+            if (best == 0 || cost < best) {
+                best = cost;
                 pl->P = P;
                 pl->U = U;
                 pl->KG = KG;
@@ -705,12 +721,15 @@ void make_plan(qgru_handle *h, int B, int sms, Kern kern, size_t (*floats)(int, 
                 pl->waves = waves;
                 pl->sharing = sharing;
                 pl->smem = smem;
-                pl->ok = active0 > 0;
+                pl->ok = true;
             }
         }
-        return;
     }
 }
+
+// (what a form's launch takes: float_chain_launch, bwd_chain_launch)
+auto fwd_kernel(int threads) { return threads <= 384 ? k_float_chain<false, 384> : k_float_chain<false, 512>; }
+auto bwd_kernel(int threads) { return threads <= 384 ? k_bwd_chain<false, 384> : k_bwd_chain<false, 512>; }
 
 // The SMs of a direction of a layer whose directions run side by side.
 int side_sms(const qgru_handle *h) { return h->opt_sm_limit > 0 ? std::min(h->opt_sm_limit, h->sm_count) : h->sm_count; }
@@ -718,7 +737,7 @@ int side_sms(const qgru_handle *h) { return h->opt_sm_limit > 0 ? std::min(h->op
 }  // namespace
 
 bool float_chain_fits(qgru_handle *h, int B) {
-    make_plan(h, B, side_sms(h), k_float_chain<false, 512>, fwd_smem_floats, &h->plan_fwd);
+    make_plan(h, B, side_sms(h), true, fwd_kernel, fwd_smem_floats, &h->plan_fwd);
     return h->plan_fwd.ok;
 }
 
@@ -729,7 +748,7 @@ bool float_chain_fits(qgru_handle *h, int B) {
 // such times (H = 16 .. 512, up to 8192 rows): from four steps on at most 20 % off the better one at each of 120 sizes.
 bool float_chain_is_faster(qgru_handle *h, int T, int B) {
     // (float inference and calibration run one direction after the other: each has the whole chip)
-    make_plan(h, B, h->sm_count, k_float_chain<false, 512>, fwd_smem_floats, &h->plan_fwd);
+    make_plan(h, B, h->sm_count, true, fwd_kernel, fwd_smem_floats, &h->plan_fwd);
     const F32RecPlan &pl = h->plan_fwd;
     if (!pl.ok) return false;
     const double H = h->H, chain = pl.waves * (0.7 + 0.046 * (pl.U * pl.KG / 32) * pl.Bt * pl.sharing);
@@ -740,7 +759,7 @@ bool float_chain_is_faster(qgru_handle *h, int T, int B) {
 // bytes; with 512 threads 228 to 348 bytes)
 int float_chain_launch(qgru_handle *h, FloatFwdArgs a, cudaStream_t st) {
     const F32RecPlan &pl = h->plan_fwd;
-    const bool one = pl.Bt <= std::min(pl.KG, RB), small = pl.U * pl.KG <= 384;
+    const bool one = pl.Bt <= pl.KG, small = pl.U * pl.KG <= 384;
     CK(launch_chain(one ? (small ? k_float_chain<true, 384> : k_float_chain<true, 512>)
                         : (small ? k_float_chain<false, 384> : k_float_chain<false, 512>), pl, a, st));
     h->launches++;
@@ -748,7 +767,7 @@ int float_chain_launch(qgru_handle *h, FloatFwdArgs a, cudaStream_t st) {
 }
 
 bool bwd_chain_fits(qgru_handle *h, int B, int *groups) {
-    make_plan(h, B, side_sms(h), k_bwd_chain<false, 512>, bwd_smem_floats, &h->plan_bwd);
+    make_plan(h, B, side_sms(h), false, bwd_kernel, bwd_smem_floats, &h->plan_bwd);
     *groups = h->plan_bwd.G;
     return h->plan_bwd.ok;
 }

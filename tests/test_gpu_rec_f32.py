@@ -41,6 +41,37 @@ def test_float_forward_and_backward(oracle, cuda_device, T, B, I, H):
         assert np.abs(g - w).max() <= 2e-5 * max(np.abs(w).max(), 1e-30)
 
 
+# a cell a thread with 9, 11 and 16 rows a cluster, the next number of rows, CTAs of 32 and 64 units on either side of their line
+@pytest.mark.parametrize("T,B,I,H", [(3, 130, 5, 262), (3, 75, 8, 512), (2, 112, 8, 500), (2, 119, 8, 512), (3, 96, 9, 256), (3, 128, 9, 256),
+                                     (3, 140, 6, 160), (4, 300, 5, 100), (5, 33, 4, 128)])
+def test_float_recurrences_between_their_forms(oracle, cuda_device, T, B, I, H):
+    test_float_forward_and_backward(oracle, cuda_device, T, B, I, H)
+
+
+def test_two_directions_share_an_odd_number_of_clusters(cuda_device):
+    """65 rows of 262 units in both directions: the last clusters have two rows; the same as torch.nn.GRU."""
+    import torch
+    torch.manual_seed(4)
+    QuantGRU = importlib.import_module(PKG_NAME + ".quant_gru").QuantGRU
+    T, B, I, H = 5, 65, 12, 262
+    m = QuantGRU(I, H, bidirectional=True).to(cuda_device).train()
+    m.use_quantization = False
+    ref = torch.nn.GRU(I, H, bidirectional=True).double()
+    with torch.no_grad():
+        for name, p in ref.named_parameters():
+            p.copy_(getattr(m, name).double().cpu())
+    x = torch.randn(T, B, I)
+    g = torch.randn(T, B, 2 * H)
+    xs = [x.to(cuda_device).requires_grad_(), x.double().requires_grad_()]
+    out = m(xs[0])[0]
+    want = ref(xs[1])[0]
+    assert (out.detach().cpu() - want.detach()).abs().max() <= 2e-6
+    wrt = [[xs[0]] + [getattr(m, n) for n, _ in ref.named_parameters()], [xs[1]] + [p for _, p in ref.named_parameters()]]
+    got = torch.autograd.grad(out, wrt[0], g.to(cuda_device))
+    for a, b in zip(got, torch.autograd.grad(want, wrt[1], g.double())):
+        assert (a.cpu() - b).abs().max() <= 1e-5 * b.abs().max()
+
+
 @pytest.mark.parametrize("H,few,many", [(200, 300, 3000), (320, 300, 2500), (512, 100, 1100)])
 def test_float_forward_of_very_many_rows(cuda_device, H, few, many):
     """Beyond some number of rows the forward goes step by step: the same states as the rows give in smaller batches."""
