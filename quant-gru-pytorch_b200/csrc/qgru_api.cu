@@ -660,7 +660,7 @@ bool gemv_fits(const qgru_handle *h) {
 bool gemv_reg_ok(const qgru_handle *h, bool fused) { return fused && h->opt_gemv_r != 1 && (h->Hpad == 128 || h->Hpad == 256); }
 size_t gemv_reg_smem(const qgru_handle *h, int n_table) {
     const size_t units = (size_t)(h->H + 31) / 32 * 32;
-    return (((size_t)n_table * 4 + 15) & ~size_t(15)) + (size_t)2 * 2 * (h->Hpad / 2 + 16) + 3 * units * sizeof(int) +
+    return (((size_t)n_table * 4 + 15) & ~size_t(15)) + (size_t)2 * 2 * (h->Hpad / 2 + 16) + 9 * units * sizeof(int) +
            3 * units * sizeof(FastLin);
 }
 

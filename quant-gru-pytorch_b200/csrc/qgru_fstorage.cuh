@@ -661,7 +661,7 @@ int fstorage_forward(qgru_handle *h, int T, int B, const FwdInput &in, const Out
         size_t smem;
         if (in_regs) {
             const size_t units = (size_t)(H + 31) / 32 * 32;
-            smem = (((size_t)n_tab * 4 + 15) & ~size_t(15)) + (size_t)2 * 2 * (h->Hpad / 2 + 16) + 3 * units * sizeof(int) +
+            smem = (((size_t)n_tab * 4 + 15) & ~size_t(15)) + (size_t)2 * 2 * (h->Hpad / 2 + 16) + 9 * units * sizeof(int) +
                    9 * units * sizeof(float);
             auto kern = h->Hpad == 128
                             ? (ih_bytes == 1 ? (h->h_uns ? k_recurrence_gemv_reg<true, int8_t, 64, 3> : k_recurrence_gemv_reg<false, int8_t, 64, 3>)

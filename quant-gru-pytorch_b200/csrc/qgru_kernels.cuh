@@ -621,7 +621,9 @@ __global__ void __launch_bounds__(1024, 1) k_recurrence_gemv(const __grid_consta
 // are the upper half of the CTA's warps: they hand their three partial sums over through shared
 // memory (a named barrier they only arrive on), and the lower half's warps run the cell with every
 // lane busy.  The per-unit constants of the R*h + br requantization live in shared memory (the
-// registers belong to R).
+// registers belong to R).  What is no part of the step's chain (W*x + bw of the next steps, the output of the last one) the upper
+// half does while the lower one computes the cell.
+// H = 256, one row: 0.91 -> 0.82 us a step (about 1150 cycles of dp4a, 400 of cell); H = 128: 0.52 -> 0.43.
 // Cell: 2 the tabulated integer cell, 3 the float cell of the float-storage forward (as in k_recurrence_gemv).
 template <bool HUnsigned, typename IhT, int KT, int Cell = 2, bool Tie = true>
 __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_constant__ GateConsts gc, RecArgs a) {
@@ -637,6 +639,8 @@ __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_con
     off += (size_t)2 * HS;
     int *part = reinterpret_cast<int *>(smem_raw + off);          // [3][units]: the upper K half's partial sums
     off += (size_t)3 * (NT >> 1) * sizeof(int);
+    int32_t *ring = reinterpret_cast<int32_t *>(smem_raw + off);  // [2][3][units]: W*x + bw of this and the next step
+    off += (size_t)6 * (NT >> 1) * sizeof(int);
     FastLin *fls = reinterpret_cast<FastLin *>(smem_raw + off);   // Cell 2: [3][units]
     float *fsk = reinterpret_cast<float *>(smem_raw + off);       // Cell 3: [3 gates][3 constants][units]
 
@@ -679,30 +683,10 @@ __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_con
     }
     __syncthreads();
 
-    const IhT *ihp = reinterpret_cast<const IhT *>(a.ih);
     const uint32_t tab = (uint32_t)__cvta_generic_to_shared(tables);
-    const bool worker = half == 0 && j_ok;
-    // W*x + bw of this row: loaded one step ahead, so the cell never waits for global memory
-    auto load_ih = [&](int s, int32_t (&v)[3]) {
-        const int t = a.reverse ? (a.T - 1 - s) : s;
-        const IhT *src = ihp + ((size_t)t * a.B + b) * a.C + j;
-        v[0] = (int32_t)src[0];
-        v[1] = (int32_t)src[a.H];
-        v[2] = (int32_t)src[2 * a.H];
-    };
-    // fp32 output alone, as a module asks for it: a running pointer instead of the address arithmetic of every view
-    const bool plain = a.out.hf && !a.out.hq && !a.out.h8;
-    float *hf = plain ? a.out.hf + (size_t)(a.reverse ? a.T - 1 : 1) * a.out.ts + (size_t)b * a.out.bs + j : nullptr;
-    const long long hf_step = a.reverse ? -(long long)a.out.ts : (long long)a.out.ts;
-    int32_t ihv[3] = {0, 0, 0};
-    if (worker) load_ih(0, ihv);
-    for (int s = 0; s < a.T; ++s) {
-        const unsigned char *h_cur = hs + (size_t)(s & 1) * HS;
-        unsigned char *h_nxt = hs + (size_t)((s + 1) & 1) * HS;
-        int32_t ihn[3] = {0, 0, 0};
-        if (worker && s + 1 < a.T) load_ih(s + 1, ihn);
-        int acc[3] = {0, 0, 0};
-        const uint4 *hq4 = reinterpret_cast<const uint4 *>(h_cur + half * QS);
+    const auto product = [&](const unsigned char *h, int (&acc)[3]) {
+        acc[0] = acc[1] = acc[2] = 0;
+        const uint4 *hq4 = reinterpret_cast<const uint4 *>(h);
 #pragma unroll
         for (int c = 0; c < KT / 16; ++c) {
             const uint4 hv = hq4[c];
@@ -714,48 +698,103 @@ __global__ void __launch_bounds__(512, 1) k_recurrence_gemv_reg(const __grid_con
                 acc[g] = dp4a_w<HUnsigned>((int)R[g][4 * c + 3], hv.w, acc[g]);
             }
         }
-        if (half) {
-            // hand the partial sums to the lower half's thread of the same unit; nothing to wait for here
+    };
+    // (a thread without a unit reads its neighbour's)
+    const IhT *ih_in = reinterpret_cast<const IhT *>(a.ih) + ((size_t)(a.reverse ? a.T - 1 : 0) * a.B + b) * a.C + min(j, a.H - 1);
+    const ptrdiff_t ih_step = (a.reverse ? -(ptrdiff_t)a.B : (ptrdiff_t)a.B) * a.C;
+    // fp32 output alone, as a module asks for it: a running pointer instead of the address arithmetic of every view
+    const bool plain = a.out.hf && !a.out.hq && !a.out.h8;
+    float *hf = plain ? a.out.hf + (size_t)(a.reverse ? a.T - 1 : 1) * a.out.ts + (size_t)b * a.out.bs + j : nullptr;
+    const long long hf_step = a.reverse ? -(long long)a.out.ts : (long long)a.out.ts;
+    const auto emit = [&](int s, int32_t hn) {       // state after step s of unit j
+        if (!j_ok) return;
+        if (plain) {
+            const float f = (float)(hn - gc.zp_h) * gc.h_scale;
+            *hf = f;
+            if (s + 1 == a.T && a.out.hn_f) a.out.hn_f[(size_t)b * a.H + j] = f;
+            hf += hf_step;
+        } else {
+            put_state(a.out, a.reverse ? (a.T - 1 - s) : (s + 1), b, j, a.H, s + 1 == a.T, hn, gc.zp_h, gc.h_scale);
+        }
+    };
+    if (half) {
+        // The upper half hands its partial sums to the lower half's thread of the same unit and has nothing to wait for.  While
+        // that computes the cell it stores the state of the step before and fetches W*x + bw two steps ahead, so that the lower
+        // half, whose chain of instructions is the step, has neither.  (The loads have no condition: the last steps read their own
+        // again.  Under one, what was loaded is copied, and waited for, where the branches meet.)
+        int32_t ihn[3];
+        const auto load_ih = [&]() {
+            ihn[0] = (int32_t)ih_in[0];
+            ihn[1] = (int32_t)ih_in[a.H];
+            ihn[2] = (int32_t)ih_in[2 * a.H];
+        };
+        const auto leave_ih = [&](int s) {
+#pragma unroll
+            for (int g = 0; g < 3; ++g) ring[((s & 1) * 3 + g) * units + j] = ihn[g];
+        };
+        load_ih();
+        leave_ih(0);
+        if (a.T > 1) ih_in += ih_step;
+        load_ih();
+        __syncthreads();
+        const auto state = [&](int s) {
+            const unsigned char q = hs[(size_t)(s & 1) * HS + j_at];
+            return HUnsigned ? (int32_t)q : (int32_t)(int8_t)q;
+        };
+        for (int s = 0; s < a.T; ++s) {
+            int acc[3];
+            product(hs + (size_t)(s & 1) * HS + QS, acc);
 #pragma unroll
             for (int g = 0; g < 3; ++g) part[g * units + j] = acc[g];
             asm volatile("bar.arrive 1, %0;" ::"r"(NT) : "memory");
+            leave_ih(s + 1);
+            if (s + 2 < a.T) ih_in += ih_step;
+            load_ih();
+            if (s > 0) emit(s - 1, state(s));
+            __syncthreads();
+        }
+        emit(a.T - 1, state(a.T));
+        return;
+    }
+    const unsigned char h0 = hs[j_at];
+    int32_t h_old = HUnsigned ? (int32_t)h0 : (int32_t)(int8_t)h0;      // this thread's unit, from step to step in a register
+    __syncthreads();
+    for (int s = 0; s < a.T; ++s) {
+        int acc[3];
+        product(hs + (size_t)(s & 1) * HS, acc);
+        int32_t ih[3];
+#pragma unroll
+        for (int g = 0; g < 3; ++g) ih[g] = ring[((s & 1) * 3 + g) * units + j];
+        int32_t hn;
+        if constexpr (Cell == 2) {
+            constexpr bool Ahead = KT == 64;         // (where R leaves registers: the constants ahead of the barrier)
+            FastLin f[3];
+            if constexpr (Ahead)
+#pragma unroll
+                for (int g = 0; g < 3; ++g) f[g] = fls[g * units + j];
+            asm volatile("bar.sync 1, %0;" ::"r"(NT) : "memory");
+#pragma unroll
+            for (int g = 0; g < 3; ++g) acc[g] += part[g * units + j];
+            const auto lin = [&](int g) { return lin_round<Tie>(acc[g], Ahead ? f[g] : fls[g * units + j]); };
+            const int32_t z_d = fused_gate_fast(gc, tab, ACT_Z, ih[0], lin(0));
+            const int32_t r_d = fused_gate_fast(gc, tab, ACT_R, ih[1], lin(1));
+            hn = fused_finish_fast<Tie>(gc, tab, ih[2], lin(2), z_d, r_d, h_old);
         } else {
             asm volatile("bar.sync 1, %0;" ::"r"(NT) : "memory");
 #pragma unroll
             for (int g = 0; g < 3; ++g) acc[g] += part[g * units + j];
-        }
-        if (worker) {
-            const unsigned char hb = h_cur[j_at];
-            const int32_t h_old = HUnsigned ? (int32_t)hb : (int32_t)(int8_t)hb;
-            int32_t hn;
-            if constexpr (Cell == 2) {
-                const int32_t z_d = fused_gate_fast(gc, tab, ACT_Z, ihv[0], lin_round<Tie>(acc[0], fls[j]));
-                const int32_t r_d = fused_gate_fast(gc, tab, ACT_R, ihv[1], lin_round<Tie>(acc[1], fls[units + j]));
-                hn = fused_finish_fast<Tie>(gc, tab, ihv[2], lin_round<Tie>(acc[2], fls[2 * units + j]), z_d, r_d, h_old);
-            } else {
-                const float fih[3] = {(float)ihv[0], (float)ihv[1], (float)ihv[2]};
-                float fhh[3];
+            const float fih[3] = {(float)ih[0], (float)ih[1], (float)ih[2]};
+            float fhh[3];
 #pragma unroll
-                for (int g = 0; g < 3; ++g)
-                    fhh[g] = fs_linear(acc[g], fsk[(g * 3 + 0) * units + j], fsk[(g * 3 + 1) * units + j],
-                                       fsk[(g * 3 + 2) * units + j], a.fs.zp_hh, a.fs.hh_lo, a.fs.hh_hi);
-                const float u_g = fs_sigmoid_gate_tab(a.fs, tab, 0, fih[0], fhh[0]);
-                const float r_g = fs_sigmoid_gate_tab(a.fs, tab, 1, fih[1], fhh[1]);
-                hn = (int32_t)fs_finish_tab(a.fs, tab, u_g, r_g, fih[2], fhh[2], (float)h_old);
-            }
-            h_nxt[j_at] = (unsigned char)hn;
-            if (plain) {
-                const float f = (float)(hn - gc.zp_h) * gc.h_scale;
-                *hf = f;
-                if (s + 1 == a.T && a.out.hn_f) a.out.hn_f[(size_t)b * a.H + j] = f;
-            } else {
-                put_state(a.out, a.reverse ? (a.T - 1 - s) : (s + 1), b, j, a.H, s + 1 == a.T, hn, gc.zp_h, gc.h_scale);
-            }
+            for (int g = 0; g < 3; ++g)
+                fhh[g] = fs_linear(acc[g], fsk[(g * 3 + 0) * units + j], fsk[(g * 3 + 1) * units + j],
+                                   fsk[(g * 3 + 2) * units + j], a.fs.zp_hh, a.fs.hh_lo, a.fs.hh_hi);
+            const float u_g = fs_sigmoid_gate_tab(a.fs, tab, 0, fih[0], fhh[0]);
+            const float r_g = fs_sigmoid_gate_tab(a.fs, tab, 1, fih[1], fhh[1]);
+            hn = (int32_t)fs_finish_tab(a.fs, tab, u_g, r_g, fih[2], fhh[2], (float)h_old);
         }
-        hf += hf_step;
-        ihv[0] = ihn[0];
-        ihv[1] = ihn[1];
-        ihv[2] = ihn[2];
+        h_old = hn;
+        if (j_ok) hs[(size_t)((s + 1) & 1) * HS + j_at] = (unsigned char)hn;
         __syncthreads();
     }
 }
