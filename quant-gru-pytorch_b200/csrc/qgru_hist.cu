@@ -345,23 +345,27 @@ __global__ void __launch_bounds__(128) k_channel_hist(const float *__restrict__ 
 }
 
 // ---- parameter derivation
-// Which candidates of a histogram's SQNR search can be the best: noise of every candidate, one thread each, over
+// Which candidates of a histogram's SQNR search can be the best: noise of every candidate, over
 // the histogram's occupied bins; then the candidates within `margin` of the smallest, as a bit mask.  The
 // result is defined by the host's sums, whose terms come from the C library's powf and may differ from
 // a product in the last bit.  Two fp32 sums of n such terms in the same order differ by less than
 // (2 n + 16) * 2^-24 of themselves, so with a margin of twice that the host's winner is always in the
 // mask, and where the mask holds one candidate (nearly always: the candidates' noises differ by far
 // more) nothing is left to compute.
-// One block per histogram.  3101 histograms (H = 256, per-channel weights), 101 or 357 candidates: 0.37 ms;
-// the whole derivation took 61 ms on 16 host threads.
+// (That bound does not ask for the order: a sum of n non-negative terms is within n * 2^-24 of the exact one in any.)
+// One block per histogram, as many neighbouring lanes to a candidate as 1024 threads have for all of them: an operator of 2048
+// occupied bins and 357 candidates is the longest chain (about 110 cycles a term, a division among them), and with a thread a
+// candidate, three in turn, it was the whole launch.  3101 histograms (H = 256, per-channel weights), 101 or 357
+// candidates: 128 threads 0.37 ms, 1024 threads 0.08 ms; the whole derivation took 61 ms on 16 host threads.
 constexpr int SQNR_WORDS = 12;   // at most 17 * 21 = 357 candidates
-__global__ void __launch_bounds__(128) k_sqnr_search(const float *__restrict__ counts, const int *__restrict__ index,
-                                                     const SqnrSearch *__restrict__ jobs, int bins,
-                                                     unsigned *__restrict__ mask) {
+constexpr int SQNR_THREADS = 1024;
+__global__ void __launch_bounds__(SQNR_THREADS) k_sqnr_search(const float *__restrict__ counts, const int *__restrict__ index,
+                                                              const SqnrSearch *__restrict__ jobs, int bins,
+                                                              unsigned *__restrict__ mask) {
     __shared__ float val[2048], cnt[2048];
     __shared__ float noise_s[SQNR_WORDS * 32];
     __shared__ unsigned err_s[SQNR_WORDS * 32];   // one occupied bin: the candidate's error and clip flag
-    __shared__ int warp_n[4], base;
+    __shared__ int warp_n[SQNR_THREADS / 32], base;
     __shared__ unsigned best_key;
     const SqnrSearch q = jobs[blockIdx.x];
     const float *src = counts + (size_t)index[blockIdx.x] * bins;
@@ -371,32 +375,44 @@ __global__ void __launch_bounds__(128) k_sqnr_search(const float *__restrict__ c
         best_key = 0xffffffffu;
     }
     __syncthreads();
-    for (int i0 = 0; i0 < bins; i0 += 128) {   // occupied bins, in order
+    for (int i0 = 0; i0 < bins; i0 += SQNR_THREADS) {   // occupied bins, in order
         const int i = i0 + tid;
         const float c = i < bins ? src[i] : 0.f;
         const bool on = i < bins && !(c < 1e-6f);
         const unsigned b = __ballot_sync(0xffffffffu, on);
         if (lane == 0) warp_n[warp] = __popc(b);
         __syncthreads();
-        int at = base + __popc(b & ((1u << lane) - 1u));
-        for (int w = 0; w < warp; ++w) at += warp_n[w];
+        if (warp == 0) {                                // where each warp's bins go
+            const int mine = warp_n[lane];
+            int sum = mine;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += y;
+            }
+            warp_n[lane] = base + sum - mine;
+            __syncwarp();
+            if (lane == 31) base += sum;
+        }
+        __syncthreads();
         if (on) {
+            const int at = warp_n[warp] + __popc(b & ((1u << lane) - 1u));
             val[at] = __fadd_rn(q.hmin, __fmul_rn((float)i + 0.5f, q.bw));
             cnt[at] = c;
         }
         __syncthreads();
-        if (tid == 0) base += warp_n[0] + warp_n[1] + warp_n[2] + warp_n[3];
-        __syncthreads();
     }
     const int n = base;
-    for (int c = tid; c < q.n; c += 128) {
-        float delta, offset;
-        sqnr_candidate(q, c, &delta, &offset);
-        float noise = delta > 0 ? 0.f : FLT_MAX;
+    int lanes = 32;                                     // per candidate
+    while (lanes > 1 && q.n * lanes > SQNR_THREADS) lanes >>= 1;
+    for (int c0 = 0; c0 < q.n; c0 += SQNR_THREADS / lanes) {
+        const int c = c0 + tid / lanes;
+        float delta = 0.f, offset = 0.f;
+        if (c < q.n) sqnr_candidate(q, c, &delta, &offset);
+        float noise = 0.f;
         unsigned err_bits = 0;
         if (delta > 0) {
 #pragma unroll 4
-            for (int i = 0; i < n; ++i) {
+            for (int i = tid % lanes; i < n; i += lanes) {
                 const float x = val[i];
                 float t = rintf(__fsub_rn(__fdiv_rn(x, delta), offset));
                 const bool clipped = t < 0 || t > q.steps;
@@ -408,9 +424,13 @@ __global__ void __launch_bounds__(128) k_sqnr_search(const float *__restrict__ c
                 noise = __fadd_rn(noise, __fmul_rn(err, cnt[i]));
             }
         }
-        noise_s[c] = noise;
-        err_s[c] = err_bits;
-        if (noise < FLT_MAX) atomicMin(&best_key, __float_as_uint(noise));   // non-negative: ordered as integers
+        for (int o = 1; o < lanes; o <<= 1) noise += __shfl_xor_sync(0xffffffffu, noise, o);
+        if (c < q.n && tid % lanes == 0) {
+            if (!(delta > 0)) noise = FLT_MAX;
+            noise_s[c] = noise;
+            err_s[c] = err_bits;
+            if (noise < FLT_MAX) atomicMin(&best_key, __float_as_uint(noise));   // non-negative: ordered as integers
+        }
     }
     __syncthreads();
     if (best_key == 0xffffffffu) {
@@ -418,14 +438,14 @@ __global__ void __launch_bounds__(128) k_sqnr_search(const float *__restrict__ c
         return;
     }
     const float limit = __uint_as_float(best_key) * (1.0f + (float)(4 * n + 32) * 0x1p-24f);
-    for (int c0 = warp * 32; c0 < SQNR_WORDS * 32; c0 += 128) {
-        const int c = c0 + lane;
+    if (warp < SQNR_WORDS) {
+        const int c = warp * 32 + lane;
         bool in = c < q.n && noise_s[c] <= limit;
         // a bias: one value, and the same error from candidates that are multiples of each other; the first wins
         if (in && n == 1)
             for (int k = 0; k < c && in; ++k) in = err_s[k] != err_s[c] || noise_s[k] > limit;
         const unsigned b = __ballot_sync(0xffffffffu, in);
-        if (lane == 0) mask[blockIdx.x * SQNR_WORDS + c0 / 32] = b;
+        if (lane == 0) mask[blockIdx.x * SQNR_WORDS + warp] = b;
     }
 }
 
@@ -882,7 +902,7 @@ int qgru_calc_params_from_hist(const qgru_hist *hs_c, int use_percentile, float 
         SqnrSearch *d_jobs = (SqnrSearch *)(hs->d_scratch + idx_b);
         unsigned *d_mask = (unsigned *)(hs->d_scratch + idx_b + job_b);
         HCK(cudaMemcpyAsync(d_jobs, search.data(), search.size() * sizeof(SqnrSearch), cudaMemcpyHostToDevice, 0));
-        k_sqnr_search<<<n, 128, 0, 0>>>(hs->d_counts, d_index, d_jobs, bins, d_mask);
+        k_sqnr_search<<<n, SQNR_THREADS, 0, 0>>>(hs->d_counts, d_index, d_jobs, bins, d_mask);
         HCK(cudaGetLastError());
         std::vector<unsigned> mask((size_t)n * SQNR_WORDS);
         HCK(cudaMemcpyAsync(mask.data(), d_mask, mask.size() * 4, cudaMemcpyDeviceToHost, 0));
