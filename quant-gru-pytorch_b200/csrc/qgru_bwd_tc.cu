@@ -9,14 +9,14 @@
 // three bf16 values, which lie side by side as columns of one MMA (3 x rows wide): their products are exact, each third has
 // accumulators of its own, and the sums meet in fp32.
 //
-// A step: cells (a warp per four rows and 32 units) add the P partial sums of their units and make dq; one thread a tile
+// A step: cells (a warp per two or four rows and 32 units) add the P partial sums of their units and make dq; one thread a tile
 // issues its MMAs; sixteen warps read the accumulators, 32 units each, and store them with 16-byte st.async into the
 // CTA that owns the units, counted on its mbarrier.  A cluster barrier, arrived on when a warp has read its partial sums
 // and waited for before the next ones are stored, keeps the one buffer safe; it lies behind the MMAs' time.
 //
-// H = 512, 256 rows, 200 steps: 4307 us on the fp32 pipe, 1120 here (5.6 a step, 10700 cycles: 1700 cells, 2100 MMAs, 1600 reading
-// the accumulators, 3200 until the last partial sum has come; those are 30 KB a CTA and step).  H = 256, 256 rows: 7.1 -> 3.3 us a step;
-// H = 128, 32 rows: 2.7 -> 2.3.  Pulling the partial sums with remote loads behind the barrier instead of st.async: 10900 cycles, and
+// us a step (80 steps), fp32 pipe / here: H = 512, 256 rows 21.9 / 5.3 (10700 cycles: 1700 cells, 2100 MMAs, 1600 reading the accumulators,
+// 3200 until the last partial sum has come; those are 30 KB a CTA and step), 32 rows 4.5 / 2.4; H = 256, 256 rows 6.0 / 2.9; H = 128, 32 rows
+// 1.8 / 1.5.  Pulling the partial sums with remote loads behind the barrier instead of st.async: 10900 cycles, and
 // 0.2 us a step more at H <= 256.  Operands of the cells are fetched without a condition: under one, each value was copied, and
 // waited for, where the branches meet (4700 to 7700 cycles a step).
 #include <algorithm>
@@ -94,8 +94,10 @@ __device__ __forceinline__ void split3(float x, uint32_t (&w)[3]) {
     asm("cvt.rn.bf16x2.f32 %0, %1, 0f00000000;" : "=r"(w[2]) : "f"(r));
 }
 
-template <int U>
+// RPT: rows of a cell thread.
+template <int U, int RPT>
 __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) {
+    static_assert(RPT == 2 || RPT == 4, "rows are padded to four");
     constexpr int K = 3 * U, UW = U / 32, B_GROUP = K * 128;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *ops = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = a.H, P = a.P;
     const int p = P > 1 ? (int)cluster_rank() : 0;
     const int grp = blockIdx.x / P, b0 = grp * a.Bt, nb = min(a.Bt, a.B - b0);
-    const int nq = a.rows >> 2, cell_warps = nq * UW;
+    const int cell_warps = a.rows / RPT * UW;
     const uint32_t recv_bytes = (uint32_t)(P * min(U, (H - p * U + 31) & ~31) * a.rows * 4);
     if (tid == 0) {
         tc::mbar_init(got, 1);
@@ -169,12 +171,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
     }
     tc::tc_fence_after_sync();
 
-    // cells: unit cu of this CTA's, rows r0 .. r0 + 3
+    // cells: unit cu of this CTA's, rows r0 .. r0 + RPT - 1
     const bool cells = warp < cell_warps;
-    const int r0 = warp / UW * 4, cu = warp % UW * 32 + lane, cj = p * U + cu;
-    bool act[4];
+    const int r0 = warp / UW * RPT, cu = warp % UW * 32 + lane, cj = p * U + cu;
+    bool act[RPT];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) act[e] = cells && cj < H && r0 + e < nb;
+    for (int e = 0; e < RPT; ++e) act[e] = cells && cj < H && r0 + e < nb;
     const long long dir = a.reverse ? 1 : -1, BH = dir * a.B * H;
     const size_t t_last = a.reverse ? 0 : a.T - 1, last = t_last * a.B + b0;    // first row of the last step
     const int lj = min(cj, H - 1);
@@ -191,14 +193,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
     }
     // Operands of the next step: v (4), gradient from outside, state before, masks.  The loads have no condition: a cell that does
     // not exist reads the place of one that does, so that no value waits for its load before it is used, a step later.
-    int row[4];
+    int row[RPT];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) row[e] = min(r0 + e, nb - 1);
-    float x[4][6];
-    uint32_t m[4];
+    for (int e = 0; e < RPT; ++e) row[e] = min(r0 + e, nb - 1);
+    float x[RPT][6];
+    uint32_t m[RPT];
     const auto fetch = [&]() {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
+        for (int e = 0; e < RPT; ++e) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) x[e][k] = v_in[(row[e] * 4 + k) * H];
             x[e][4] = dn_in[row[e] * a.dn_bs];
@@ -212,32 +214,41 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
         h_in += BH;
         m_in += BH;
     };
-    float zdh[4] = {}, sum[6] = {};
+    float zdh[RPT] = {}, sum[6] = {};
     fetch();
     bool ok = true;
     // what the P CTAs have sent for this thread's cells, added in their order
-    const auto carry = [&](float (&y)[4]) {
-        const float *q = recv + ((r0 >> 2) * U + cu) * 4;
+    const auto carry = [&](float (&y)[RPT]) {
+        const float *q = recv + ((r0 >> 2) * U + cu) * 4 + (r0 & 3);
         const int step = U * a.rows;
+        const auto add = [&](const float *at, float (&w)[RPT]) {
+            if constexpr (RPT == 4) {
+                const float4 v = *reinterpret_cast<const float4 *>(at);
+                w[0] = v.x;
+                w[1] = v.y;
+                w[2] = v.z;
+                w[3] = v.w;
+            } else {
+                const float2 v = *reinterpret_cast<const float2 *>(at);
+                w[0] = v.x;
+                w[1] = v.y;
+            }
+        };
         int s = 0;
         for (; s + 4 <= P; s += 4, q += 4 * step) {
-            float4 w[4];
+            float w[4][RPT];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) w[e] = *reinterpret_cast<const float4 *>(q + e * step);
+            for (int e = 0; e < 4; ++e) add(q + e * step, w[e]);
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                y[0] += w[e].x;
-                y[1] += w[e].y;
-                y[2] += w[e].z;
-                y[3] += w[e].w;
-            }
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int i = 0; i < RPT; ++i) y[i] += w[e][i];
         }
         for (; s < P; ++s, q += step) {
-            const float4 w = *reinterpret_cast<const float4 *>(q);
-            y[0] += w.x;
-            y[1] += w.y;
-            y[2] += w.z;
-            y[3] += w.w;
+            float w[RPT];
+            add(q, w);
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) y[i] += w[i];
         }
     };
     const int unit0 = tile * 128 + quad * 32;
@@ -253,11 +264,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
     const uint32_t at0 = tmem_a + (uint32_t)(mt * 8);
 
     for (int s = 0; s < a.T; ++s) {
-        float y[4] = {zdh[0], zdh[1], zdh[2], zdh[3]};
+        float y[RPT];
+#pragma unroll
+        for (int e = 0; e < RPT; ++e) y[e] = zdh[e];
         if (cells) {
             if (s == 0) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
+                for (int e = 0; e < RPT; ++e)
                     if (act[e] && a.dh_in) y[e] = a.dh_in[(size_t)(b0 + r0 + e) * H + cj];
             } else {
                 ok = ok && tc::mbar_wait(got, (uint32_t)((s - 1) & 1), WAIT_BUDGET);
@@ -266,9 +279,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
             }
         }
         if (cells) {
-            float dp[4][3], dq[4][3];
+            float dp[RPT][3], dq[RPT][3];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
+            for (int e = 0; e < RPT; ++e) {
                 const float z = x[e][0], r = x[e][1], g = x[e][2], q_g = x[e][3], h_old = x[e][5];
                 float dh = x[e][4] + y[e];
                 if (!(m[e] >> PM_H & 1)) dh *= 0.f;
@@ -300,13 +313,17 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
             }
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                uint32_t w[4][3];
+                uint32_t w[RPT][3];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) split3(dq[e][k] * scale[k], w[e]);
+                for (int e = 0; e < RPT; ++e) split3(dq[e][k] * scale[k], w[e]);
 #pragma unroll
-                for (int part = 0; part < 3; ++part)
-                    *reinterpret_cast<uint2 *>(b_ops + operand_at(part * a.rows + r0, k * U + cu, B_GROUP)) =
-                        make_uint2(__byte_perm(w[0][part], w[1][part], 0x7632), __byte_perm(w[2][part], w[3][part], 0x7632));
+                for (int part = 0; part < 3; ++part) {
+                    unsigned char *to = b_ops + operand_at(part * a.rows + r0, k * U + cu, B_GROUP);
+                    if constexpr (RPT == 4)
+                        *reinterpret_cast<uint2 *>(to) = make_uint2(__byte_perm(w[0][part], w[1][part], 0x7632), __byte_perm(w[2][part], w[3][part], 0x7632));
+                    else
+                        *reinterpret_cast<uint32_t *>(to) = __byte_perm(w[0][part], w[1][part], 0x7632);
+                }
             }
             fence_proxy_async_cta();
             tc::tc_fence_before_sync();
@@ -318,7 +335,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
             }
             // (behind the arrive, whose release would wait for them)
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
+            for (int e = 0; e < RPT; ++e)
                 if (act[e])
 #pragma unroll
                     for (int k = 0; k < 3; ++k) {
@@ -377,10 +394,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
     }
     if (cells) {
         ok = ok && tc::mbar_wait(got, (uint32_t)((a.T - 1) & 1), WAIT_BUDGET);
-        float y[4] = {zdh[0], zdh[1], zdh[2], zdh[3]};
+        float y[RPT];
+#pragma unroll
+        for (int e = 0; e < RPT; ++e) y[e] = zdh[e];
         carry(y);
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
+        for (int e = 0; e < RPT; ++e)
             if (act[e]) {
                 const size_t at = (size_t)(b0 + r0 + e) * H + cj;
                 a.dh_out[at] = a.h0_mask ? y[e] * (float)a.h0_mask[at] : y[e];
@@ -395,7 +414,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
         const int k = c / U, uu = c % U;
         if (p * U + uu >= H) continue;
         float s = 0.f;
-        for (int w = 0; w < nq; ++w) s += bsum[((w * UW + uu / 32) * 6 + k) * 32 + uu % 32];
+        for (int w = 0; w < a.rows / RPT; ++w) s += bsum[((w * UW + uu / 32) * 6 + k) * 32 + uu % 32];
         const int g = k % 3;
         a.bias_part[((size_t)grp * 6 + (k < 3 ? 0 : 3) + (a.torch && g < 2 ? 1 - g : g)) * H + p * U + uu] = s;
     }
@@ -427,7 +446,15 @@ bool fill(const F32RecPlan &pl, int H, size_t smem_optin, BwdTcArgs *a) {
     return false;
 }
 
-auto kernel_of(int U) { return U == 32 ? k_bwd_chain_tc<32> : k_bwd_chain_tc<64>; }
+// Two rows a cell thread where sixteen warps cover them: the cells are a chain of instructions at the head of the step, and twice the
+// warps have half of it each.  us a step, four rows a thread / two / one: H = 128, 32 rows 1.97 / 1.48 / 1.81; H = 256, 64 rows 2.17 / 1.82 /
+// 2.21; H = 384, 256 rows 3.7 / 3.4.  With 64 units a CTA and four tiles all warps read accumulators and four issue MMAs besides:
+// H = 512, 192 rows 4.4 / 4.7, 256 rows 5.3 / 5.3.
+auto kernel_of(int U, int rows, int tiles) {
+    const bool two = rows / 2 * (U / 32) <= WARPS && (U == 32 || tiles < 4);
+    if (U == 32) return two ? k_bwd_chain_tc<32, 2> : k_bwd_chain_tc<32, 4>;
+    return two ? k_bwd_chain_tc<64, 2> : k_bwd_chain_tc<64, 4>;
+}
 
 cudaLaunchConfig_t config(int P, int G, size_t smem, cudaStream_t st, cudaLaunchAttribute *attr) {
     cudaLaunchConfig_t cfg = {};
@@ -448,8 +475,8 @@ cudaLaunchConfig_t config(int P, int G, size_t smem, cudaStream_t st, cudaLaunch
 
 // The form for B rows.  32 units a CTA are the shorter step (half the MMAs) until a cluster has more than 20 rows: what then takes
 // longest is the H x rows partial sums that a CTA sends (14 bytes a clock), and 64 units a CTA are half the CTAs a
-// cluster, twice the clusters and half the rows.  us per step, 32 / 64 units: H = 512: 128 rows 4.8 / 5.0, 256 rows 7.0 / 6.2;
-// H = 384: 256 rows 5.5 / 4.5; H = 262: 256 rows (16 a cluster) 3.7 / 4.1.  128 units a CTA were slower everywhere.
+// cluster, twice the clusters and half the rows.  us per step (24 steps, four rows a cell thread), 32 / 64 units: H = 512: 128 rows
+// 4.8 / 5.0, 256 rows 7.0 / 6.2; H = 384: 256 rows 5.5 / 4.5; H = 262: 256 rows (16 a cluster) 3.7 / 4.1.  128 units a CTA were slower.
 bool bwd_chain_tc_plan(qgru_handle *h, int B, int sms, F32RecPlan *best) {
     const int H = h->H;
     if (best->H == H && best->B == B && best->sms == sms) return best->ok;
@@ -469,7 +496,7 @@ bool bwd_chain_tc_plan(qgru_handle *h, int B, int sms, F32RecPlan *best) {
         while (pl.Bt > 0 && !fill(pl, H, (size_t)h->smem_optin, &a)) pl.Bt -= 4;
         if (pl.Bt <= 0) continue;
         const int most = pl.Bt;
-        const auto kern = kernel_of(U);
+        const auto kern = kernel_of(U, a.rows, a.tiles);
         cudaLaunchAttribute attr[1];
         const cudaLaunchConfig_t cfg = config(pl.P, 1, (size_t)h->smem_optin, nullptr, attr);
         int active = 0;
@@ -497,7 +524,7 @@ int bwd_chain_tc_launch(qgru_handle *h, const F32RecPlan &pl, const BwdChainArgs
     static_cast<BwdChainArgs &>(a) = args;
     if (!fill(pl, h->H, (size_t)h->smem_optin, &a)) return fail(h, QGRU_ERR_UNSUPPORTED, "no plan for the chain of state gradients");
     a.abort_flag = h->d_flags + 1;
-    const auto kern = kernel_of(pl.U);
+    const auto kern = kernel_of(pl.U, a.rows, a.tiles);
     CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->smem_optin));
     CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchAttribute attr[1];

@@ -772,8 +772,8 @@ bool bwd_chain_fits(qgru_handle *h, int B, int *groups) {
     return h->plan_bwd.ok;
 }
 
-// us per step in chains of 24, here / on the tensor cores: H = 96: 1 row 2.0 / 2.3, 256 rows 2.4 / 2.4; H = 112: 2.7 / 2.3, 3.3 / 2.5;
-// H = 262: 2.8 / 2.5, 9.8 / 3.7; H = 512: 3.5 / 2.8, 23.2 / 6.2.
+// us per step in chains of 80, here / on the tensor cores: H = 100: 1 row 1.8 / 1.5, 256 rows 3.1 / 1.9; H = 256: 2.0 / 1.5, 6.0 / 2.9;
+// H = 512: 2.8 / 2.0, 21.9 / 5.3.  Up to 96 units one CTA holds R in its registers: 1.2 (H = 64) to 1.45 (H = 96).
 bool bwd_chain_tc_is_faster(qgru_handle *h, int B) {
     return h->H > 96 && bwd_chain_tc_plan(h, B, side_sms(h), &h->plan_bwd_tc);
 }
