@@ -387,22 +387,32 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm_f32_tc(const TcArgs g) {
         const int rows = (int)min((long long)TM, g.N - n0), cols = (int)min((long long)width, g.M - j0);
         const bool split = gridDim.z > 1;
         float *out = g.C + (split ? (size_t)blockIdx.z * g.N * g.M : 0) + n0 * g.M + j0;
-        if ((split || (!g.accumulate && !g.mask)) && g.M % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+        const uint8_t *mask = split || !g.mask ? nullptr : g.mask + n0 * g.M + j0;
+        const int acc = split ? 0 : g.accumulate;
+        if (g.M % 4 == 0 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(mask) * 4) & 15u) == 0) {
             const int c4 = cols >> 2;            // (M and the tile's width are multiples of four)
+#pragma unroll 4
             for (int i = tid; i < rows * c4; i += WORK) {
                 const int rr = i / c4, c = (i - rr * c4) * 4;
-                *reinterpret_cast<float4 *>(out + (long long)rr * g.M + c) = *reinterpret_cast<const float4 *>(cs + rr * C_LD + c);
+                const long long at = (long long)rr * g.M + c;
+                float4 y = *reinterpret_cast<const float4 *>(cs + rr * C_LD + c);
+                const float4 old = acc ? *reinterpret_cast<const float4 *>(out + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+                if (acc == 1) y = make_float4(y.x + old.x, y.y + old.y, y.z + old.z, y.w + old.w);
+                if (mask) {
+                    const uchar4 m = *reinterpret_cast<const uchar4 *>(mask + at);
+                    y = make_float4(y.x * (float)m.x, y.y * (float)m.y, y.z * (float)m.z, y.w * (float)m.w);
+                }
+                if (acc == 2) y = make_float4(y.x + old.x, y.y + old.y, y.z + old.z, y.w + old.w);
+                *reinterpret_cast<float4 *>(out + at) = y;
             }
         } else {
             for (int rr = warp; rr < rows; rr += WARPS)
                 for (int c = lane; c < cols; c += 32) {
                     const long long at = (long long)rr * g.M + c;
                     float y = cs[rr * C_LD + c];
-                    if (!split) {
-                        if (g.accumulate == 1) y += out[at];
-                        if (g.mask) y *= (float)g.mask[(n0 + rr) * g.M + j0 + c];
-                        if (g.accumulate == 2) y += out[at];
-                    }
+                    if (acc == 1) y += out[at];
+                    if (mask) y *= (float)mask[at];
+                    if (acc == 2) y += out[at];
                     out[at] = y;
                 }
         }

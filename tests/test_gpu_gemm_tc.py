@@ -76,3 +76,23 @@ def test_input_projection_of_values_without_bf16_parts(cuda_device, value):
     others = [b for b in range(B) if b != 130]
     # (sums in another order where the tile was multiplied again)
     assert (got[:, others] - clean[:, others]).abs().max() <= 2e-6
+
+
+@pytest.mark.parametrize("T,B,I,H", [(16, 256, 128, 128), (31, 131, 130, 86), (40, 100, 260, 44)])
+def test_masked_products_of_the_backward(cuda_device, T, B, I, H):
+    """The clamp masks of x, W and R zero their gradients' elements and change no other (rows in groups of four and single)."""
+    import torch
+    rng = np.random.default_rng(I * H)
+    W, R, _, _ = (_t(a, cuda_device) for a in gen_weights(rng, I, H))
+    rand = lambda *s: torch.randn(*s, device=cuda_device)
+    v, h, x, dh = torch.rand(T, B, 4 * H, device=cuda_device), rand(T + 1, B, H) * 0.3, rand(T, B, I), rand(T + 1, B, H)
+    shapes = {"x": (T * B, I), "h0": (B, H), "W": (I, 3 * H), "R": (H, 3 * H), "bw": (3 * H,), "br": (3 * H,),
+              "ih_linear": (T * B, 3 * H), "hh_linear": (T * B, 3 * H), "gate_input": (T * B, 3 * H),
+              "gate_output": (T * B, 3 * H), "h": (T * B, H)}
+    ones = {n: torch.ones(s, dtype=torch.uint8, device=cuda_device) for n, s in shapes.items()}
+    some = {n: (torch.rand(shapes[n], device=cuda_device) < 0.7).to(torch.uint8) for n in ("x", "W", "R")}
+    with gru_ops.Handle(I, H, device=0) as hd:
+        all_ = hd.backward(W, R, x, dh, h, v, masks=ones)
+        part = hd.backward(W, R, x, dh, h, v, masks={**ones, **some})
+    for a, b, n in zip(all_[:3], part[:3], ("x", "W", "R")):
+        assert torch.equal(a.reshape(b.shape) * some[n].reshape(b.shape), b), n
