@@ -24,12 +24,12 @@
 namespace qgru {
 namespace {
 
-RegKernel kernel_of(RecCell cell, int ih_bytes, int kst, int ks, bool hu) {
+RegKernel kernel_of(RecCell cell, int ih_bytes, int kst, int ks, bool hu, bool few) {
     switch (cell) {
-        case CELL_INT_FAST: return ih_bytes == 2 ? pick<int16_t, CELL_INT_FAST>(kst, ks, hu) : pick<int32_t, CELL_INT_FAST>(kst, ks, hu);
-        case CELL_INT_FAST_NOTIE: return ih_bytes == 2 ? pick<int16_t, CELL_INT_FAST_NOTIE>(kst, ks, hu) : pick<int32_t, CELL_INT_FAST_NOTIE>(kst, ks, hu);
-        case CELL_INT_GENERIC: return ih_bytes == 1 ? pick<int8_t, CELL_INT_GENERIC>(kst, ks, hu) : pick<int16_t, CELL_INT_GENERIC>(kst, ks, hu);
-        default: return rec_reg_float_kernel(cell, ih_bytes, kst, ks, hu);
+        case CELL_INT_FAST: return ih_bytes == 2 ? pick<int16_t, CELL_INT_FAST>(kst, ks, hu, few) : pick<int32_t, CELL_INT_FAST>(kst, ks, hu, few);
+        case CELL_INT_FAST_NOTIE: return ih_bytes == 2 ? pick<int16_t, CELL_INT_FAST_NOTIE>(kst, ks, hu, few) : pick<int32_t, CELL_INT_FAST_NOTIE>(kst, ks, hu, few);
+        case CELL_INT_GENERIC: return ih_bytes == 1 ? pick<int8_t, CELL_INT_GENERIC>(kst, ks, hu, few) : pick<int16_t, CELL_INT_GENERIC>(kst, ks, hu, few);
+        default: return rec_reg_float_kernel(cell, ih_bytes, kst, ks, hu, few);
     }
 }
 
@@ -53,7 +53,7 @@ bool rec_reg_plan(qgru_handle *h, int B, int sms, int ih_bytes, RecCell cell, in
     const int P = (groups + most - 1) / most;
     if (P > 16) return false;
     const int U = 16 * ((groups + P - 1) / P), threads = U / 16 * KS * 32;
-    const RegKernel kern = kernel_of(cell, ih_bytes, KST, KS, h->h_uns);
+    const RegKernel kern = kernel_of(cell, ih_bytes, KST, KS, h->h_uns, false);
     const int K = KS * KST * 32;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)P);
@@ -95,6 +95,18 @@ bool rec_reg_plan(qgru_handle *h, int B, int sms, int ih_bytes, RecCell cell, in
         if (Bt >= want || (pass > 0 && Bt > 0)) break;
         Bt = want;
     }
+    // Up to 128 inputs the few rows' form takes ten registers more (above, R alone fills the register file's share of a CTA):
+    // only for a last tile that gains by it, and where as many CTAs still fit.  us a step: H = 128, 592 rows 1.53 -> 1.08, float storage
+    // 2.70 -> 1.65; H = 64, 2000 rows 1.62 -> 1.06; with one row a CTA (H = 64, 592 rows) 1.04, and 1.06 in this form.
+    const int tail = (Bt - 1) % 8 + 1;
+    if (KS == 1 && KST <= 4 && tail > 1 && tail <= 4) {
+        const RegKernel other = kernel_of(cell, ih_bytes, KST, KS, h->h_uns, true);
+        int active = 0;
+        if (cudaFuncSetAttribute(other, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl->smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&active, other, &cfg) != cudaSuccess)
+            cudaGetLastError();
+        pl->few = (long long)active * sms / h->sm_count * Bt >= B;
+    }
     pl->KST = KST;
     pl->KS = KS;
     pl->U = U;
@@ -106,7 +118,7 @@ bool rec_reg_plan(qgru_handle *h, int B, int sms, int ih_bytes, RecCell cell, in
 }
 
 int rec_reg_launch(qgru_handle *h, const RecRegPlan &pl, RecRegArgs a, RecCell cell, int ih_bytes, cudaStream_t st) {
-    const RegKernel kern = kernel_of(cell, ih_bytes, pl.KST, pl.KS, h->h_uns);
+    const RegKernel kern = kernel_of(cell, ih_bytes, pl.KST, pl.KS, h->h_uns, pl.few);
     a.U = pl.U;
     a.P = pl.P;
     a.Bt = pl.Bt;

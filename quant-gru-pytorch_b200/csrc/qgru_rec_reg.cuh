@@ -15,6 +15,7 @@ struct RecRegPlan {
     int H = 0, B = 0, sms = 0, ih_bytes = 0, cell = 0, n_table = 0;      // what the plan was made for
     bool ok = false;
     int KST = 2, KS = 1, U = 16, P = 1, Bt = 1, G = 1, D = 2;
+    bool few = false;      // tiles of two to four rows take one row a thread
     size_t smem = 0;
     // W*x + bw is stored as [P][T*B][3][U]: what a CTA needs of its rows in one step is one contiguous block
     size_t ih_elements(long long N) const { return (size_t)N * 3 * P * U; }
@@ -46,7 +47,7 @@ struct RecRegArgs {
 };
 
 typedef void (*RegKernel)(const GateConsts, const RecRegArgs);
-RegKernel rec_reg_float_kernel(RecCell cell, int ih_bytes, int kst, int ks, bool hu);   // qgru_rec_reg_float.cu
+RegKernel rec_reg_float_kernel(RecCell cell, int ih_bytes, int kst, int ks, bool hu, bool few);   // qgru_rec_reg_float.cu
 
 // False where the form does not exist (H > 1024, no shared memory left).
 bool rec_reg_plan(qgru_handle *h, int B, int sms, int ih_bytes, RecCell cell, int n_table, RecRegPlan *pl);

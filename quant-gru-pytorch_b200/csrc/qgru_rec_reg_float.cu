@@ -4,11 +4,11 @@
 
 namespace qgru {
 
-RegKernel rec_reg_float_kernel(RecCell cell, int ih_bytes, int kst, int ks, bool hu) {
+RegKernel rec_reg_float_kernel(RecCell cell, int ih_bytes, int kst, int ks, bool hu, bool few) {
     switch (cell) {
-        case CELL_INT_TRAIN: return ih_bytes == 2 ? pick<int16_t, CELL_INT_TRAIN>(kst, ks, hu) : pick<int32_t, CELL_INT_TRAIN>(kst, ks, hu);
-        case CELL_FS_TRAIN: return ih_bytes == 2 ? pick<int16_t, CELL_FS_TRAIN>(kst, ks, hu) : pick<int32_t, CELL_FS_TRAIN>(kst, ks, hu);
-        default: return ih_bytes == 1 ? pick<int8_t, CELL_FS>(kst, ks, hu) : pick<int16_t, CELL_FS>(kst, ks, hu);
+        case CELL_INT_TRAIN: return ih_bytes == 2 ? pick<int16_t, CELL_INT_TRAIN>(kst, ks, hu, few) : pick<int32_t, CELL_INT_TRAIN>(kst, ks, hu, few);
+        case CELL_FS_TRAIN: return ih_bytes == 2 ? pick<int16_t, CELL_FS_TRAIN>(kst, ks, hu, few) : pick<int32_t, CELL_FS_TRAIN>(kst, ks, hu, few);
+        default: return ih_bytes == 1 ? pick<int8_t, CELL_FS>(kst, ks, hu, few) : pick<int16_t, CELL_FS>(kst, ks, hu, few);
     }
 }
 

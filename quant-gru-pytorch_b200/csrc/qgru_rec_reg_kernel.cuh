@@ -89,7 +89,7 @@ __host__ __device__ inline RegSmem reg_smem(int K, int U, int KS, int NT, int D,
     return s;
 }
 
-template <typename IhT, int KST, int Cell, bool HU, int KS>
+template <typename IhT, int KST, int Cell, bool HU, int KS, bool Few = KS == 1>
 __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ GateConsts gc, const __grid_constant__ RecRegArgs a) {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr bool Tie = Cell != CELL_INT_FAST_NOTIE, Train = Cell >= CELL_INT_TRAIN;
@@ -340,8 +340,12 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
         for (int nt = 0; nt < NT; ++nt, ih_t += Split ? RW * 48 : 24 * U) {
             const int rows = nb - nt * 8;                        // rows of this tile that exist
             if (rows <= 0) break;
+            // One CTA, two to four rows: each stands in two of the eight columns, so that a thread has one row of its two units
+            // to compute and not half of the threads two.  us a step, H = 256: 296 rows (2 a CTA) 2.12 -> 1.57, float storage 3.45 -> 2.21,
+            // 4096 rows (28, the last tile has four) 7.3 -> 7.0.
+            const bool few = Few && rows > 1 && rows <= 4;
             int32_t acc[3][4] = {};
-            const unsigned char *hb = h_cur + (nt * 8 + g8) * HS + ks * KST * 32 + q4 * 16;
+            const unsigned char *hb = h_cur + (nt * 8 + (few ? g8 >> 1 : g8)) * HS + ks * KST * 32 + q4 * 16;
 #pragma unroll
             for (int c = 0; c < KST / 2; ++c) {
                 const uint4 x = *reinterpret_cast<const uint4 *>(hb + c * 64);
@@ -363,8 +367,8 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
                 // rows compute with whatever is there (every lookup is clamped) and store nothing
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                    if (r >= rows) continue;                     // (warp-uniform: a tile of one row)
-                    const int row = 2 * q4 + r, b = nt * 8 + row;
+                    if (r >= rows || (few && r)) break;          // (warp-uniform)
+                    const int row = few ? q4 : 2 * q4 + r, b = nt * 8 + row;
                     const IhT *iv = ih_t + row * 3 * U;
                     const uint32_t hb2 = *reinterpret_cast<const uint16_t *>(h_cur + b * HS + out_j);
                     const int sums[3][2] = {{acc[0][r], acc[0][2 + r]}, {acc[1][r], acc[1][2 + r]}, {acc[2][r], acc[2][2 + r]}};
@@ -503,11 +507,11 @@ __global__ void __launch_bounds__(512, 1) k_rec_reg(const __grid_constant__ Gate
 
 // The splits of K that occur: one warp up to 256 inputs, two up to 512, four up to 1024, at most 256 each.
 template <typename IhT, int Cell, bool HU>
-RegKernel pick_shape(int kst, int ks) {
+RegKernel pick_shape(int kst, int ks, bool few) {
     if (ks == 1) {
         switch (kst) {
-            case 2: return k_rec_reg<IhT, 2, Cell, HU, 1>;
-            case 4: return k_rec_reg<IhT, 4, Cell, HU, 1>;
+            case 2: return few ? k_rec_reg<IhT, 2, Cell, HU, 1> : k_rec_reg<IhT, 2, Cell, HU, 1, false>;
+            case 4: return few ? k_rec_reg<IhT, 4, Cell, HU, 1> : k_rec_reg<IhT, 4, Cell, HU, 1, false>;
             case 6: return k_rec_reg<IhT, 6, Cell, HU, 1>;
             default: return k_rec_reg<IhT, 8, Cell, HU, 1>;
         }
@@ -516,8 +520,8 @@ RegKernel pick_shape(int kst, int ks) {
     return kst == 6 ? k_rec_reg<IhT, 6, Cell, HU, 4> : k_rec_reg<IhT, 8, Cell, HU, 4>;
 }
 template <typename IhT, int Cell>
-RegKernel pick(int kst, int ks, bool hu) {
-    return hu ? pick_shape<IhT, Cell, true>(kst, ks) : pick_shape<IhT, Cell, false>(kst, ks);
+RegKernel pick(int kst, int ks, bool hu, bool few) {
+    return hu ? pick_shape<IhT, Cell, true>(kst, ks, few) : pick_shape<IhT, Cell, false>(kst, ks, few);
 }
 
 }  // namespace

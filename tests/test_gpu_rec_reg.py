@@ -93,3 +93,36 @@ def test_fast_on_either_side_of_its_line(oracle, cuda_device, H, P, rows):
                 assert int(plan["Bt"]) <= rows
             seen.add((plan["r_in"] == "registers", int(plan.get("Bt", 0))))
         assert (True, rows) in seen and any(not reg for reg, _ in seen), seen
+
+
+@pytest.mark.parametrize("H", [33, 64, 256])
+@pytest.mark.parametrize("cfg", ["default", "cfg2", "ih16"])
+def test_tiles_of_two_to_four_rows(oracle, cuda_device, cfg, H):
+    """One CTA a row range: a tile of two to four rows puts each row in two columns of the product.  sm_limit makes the CTAs'
+    rows 1 .. 5 and 12 (a last tile of four), the last CTA's fewer; inference and training cells of both storages."""
+    import torch
+    T, I = 4, 8
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(cuda_device)
+    with gru_ops.Handle(I, H, device=cuda_device.index or 0) as hd:
+        hd.set_option("sm_limit", 3)
+        for B in (3, 5, 6, 8, 9, 11, 12, 13, 36):
+            case = make_case(B * 31 + H, T, B, I, H, oracle, config_named(cfg), with_h0=True)
+            hd.set_params(case.params)
+            w, x, h0 = [dev(a) for a in (case.W, case.R, case.bw, case.br)], dev(case.x), dev(case.h0)
+            hd.set_weights_f32(*w)
+            want = oracle.forward_i32(T, B, I, H, case.wq, case.x_q, case.h0_q, case.params.c, case.params.scale_list())
+
+            def run():
+                out = [hd.forward_f32(x, h0, reverse=True), hd.forward_fstorage(x, h0)]
+                for int_storage in (False, True):
+                    h, v, x_q, masks = hd.forward_fstorage_train(*w, x, h0, int_storage=int_storage)
+                    out += [h, v, x_q, *masks.values()]
+                return out
+
+            hd.set_option("rec", "generic")
+            base = run()
+            hd.set_option("rec", "reg")
+            assert np.array_equal(hd.forward_i32(dev(case.x_q), dev(case.h0_q)).cpu().numpy(), want), B
+            assert "r_in=registers" in hd.describe_plan()
+            for a, b in zip(base, run()):
+                assert torch.equal(a, b), (B, hd.describe_plan())
