@@ -746,9 +746,9 @@ int launch_prologue(qgru_handle *h, int T, int B, const FwdInput &in, uint8_t *x
     a.clear = in.mode != 2;
     a.stamp = in.stamp;
     if (in.mode == 2) CK(cudaMemsetAsync(h->d_flags, 0, 2 * sizeof(int), st));
-    a.q_blocks = x8 ? grid_for(a.N * (h->Ipad / 16), 256, h->sm_count) : 0;
+    const bool vec = in.mode != 2 && h->I % 4 == 0 && in.ts % 4 == 0 && in.bs % 4 == 0 && (reinterpret_cast<uintptr_t>(in.x) & 15u) == 0;
+    a.q_blocks = !x8 ? 0 : vec ? grid_for(a.N * (h->Ipad / 128), 32, h->sm_count) : grid_for(a.N * (h->Ipad / 16), 256, h->sm_count);
     const int blocks = a.q_blocks + grid_for((long long)B * h->Hpad, 256, h->sm_count);
-    const bool vec = h->I % 4 == 0 && in.ts % 4 == 0 && in.bs % 4 == 0 && (reinterpret_cast<uintptr_t>(in.x) & 15u) == 0;
     if (in.mode == 0) {
         if (vec) k_prologue<0, true><<<blocks, 256, 0, st>>>(a);
         else k_prologue<0, false><<<blocks, 256, 0, st>>>(a);

@@ -75,8 +75,56 @@ __device__ __forceinline__ int32_t prologue_quantize(const void *src, long long 
     }
 }
 
-// A thread takes 16 consecutive columns of a row: four 128-bit loads where Vec (rows and base aligned, K a
-// multiple of 4), one 128-bit store.  Memory-bound: 51200 x 256 fp32 (cfg2) 18 us, 37 us with scalar loads.
+// prologue_quantize of four values without division or conversions.  t = x * (1 / scale), in mode 1 with the zero point, differs from what
+// is rounded there by less than 2^-22 (|t| + |zp|), and the two round to different integers only if a half lies between them.  t + MAGIC
+// (in mode 0 with the zero point: a whole number) is the rounded value in the low bits of a float, where also the limits are.
+// Where a half is within 2^-21 (|t| + |zp|), or t is no number below 2^20, the four are divided: one lane in some hundreds.
+constexpr float PROLOGUE_MAGIC = 12582912.0f;        // 2^23 + 2^22
+struct PrologueNear {
+    float inv, base, zp, limit, lo, hi;
+    template <int Mode>
+    static __device__ __forceinline__ PrologueNear make(const PrologueArgs &a) {
+        PrologueNear n;
+        n.zp = (float)a.x_zp;
+        n.inv = a.x_zp > -(1 << 20) && a.x_zp < (1 << 20) ? __frcp_rn(a.x_scale) : __int_as_float(0x7fffffff);
+        n.base = PROLOGUE_MAGIC + (Mode == 0 ? n.zp : 0.f);
+        n.limit = 0.5f - (Mode == 0 ? 0.f : fabsf(n.zp) * 0x1p-21f);
+        n.lo = PROLOGUE_MAGIC + (float)a.x_lo;
+        n.hi = PROLOGUE_MAGIC + (float)a.x_hi;
+        return n;
+    }
+};
+
+// q[v] + MAGIC, clamped, in q and before the clamp in raw (different from q is all that counts)
+template <int Mode>
+__device__ __forceinline__ void prologue_quantize4(const PrologueArgs &a, const PrologueNear &n, const float4 &x, float (&q)[4], float (&raw)[4]) {
+    const float f[4] = {x.x, x.y, x.z, x.w};
+    float worst = 0.f;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        const float t = Mode == 0 ? __fmul_rn(f[v], n.inv) : __fmaf_rn(f[v], n.inv, n.zp);
+        raw[v] = __fadd_rn(t, n.base);
+        const float near = __fmaf_rn(fabsf(t), 0x1p-21f, fabsf(__fsub_rn(t, __fsub_rn(raw[v], n.base))));
+        asm("max.NaN.f32 %0, %0, %1;" : "+f"(worst) : "f"(near));
+        q[v] = fminf(fmaxf(raw[v], n.lo), n.hi);
+    }
+    if (worst < n.limit) return;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        uint8_t keep;
+        q[v] = PROLOGUE_MAGIC + (float)prologue_quantize<Mode>(f, v, a.x_scale, a.x_zp, a.x_lo, a.x_hi, keep, nullptr);
+        raw[v] = keep ? q[v] : 0.f;
+    }
+}
+
+__device__ __forceinline__ void put4(float *p, const float4 &y, bool wide) {
+    if (wide) *reinterpret_cast<float4 *>(p) = y;
+    else p[0] = y.x, p[1] = y.y, p[2] = y.z, p[3] = y.w;
+}
+
+// Vec (rows and base aligned, K a multiple of 4): a warp takes four neighbouring units of 128 columns, a lane four columns of each:
+// one 128-bit load and one store of each kind, whole lines.  Memory-bound: 409600 x 128 fp32 60 us, 51200 x 256 with the training
+// outputs 22 us (with 16 columns a thread and a division a value: 77 and 92; with conversions and no division: 77 and 26).  Else a thread takes 16 columns with scalar loads.
 template <int Mode, bool Vec>
 __global__ void __launch_bounds__(256) k_prologue(const PrologueArgs a) {
     pdl_trigger();
@@ -86,6 +134,67 @@ __global__ void __launch_bounds__(256) k_prologue(const PrologueArgs a) {
         a.flags[1] = 0;
     }
     if ((int)blockIdx.x < a.q_blocks) {
+        if constexpr (Vec) {
+            const int nch = a.Kpad >> 7, lane = threadIdx.x & 31;
+            const unsigned units = (unsigned)(a.N * nch), stride = a.q_blocks * 32u;   // (2^32 units would be 512 GB of bytes in x8)
+            const PrologueNear near = PrologueNear::make<Mode>(a);
+            const int im = __float_as_int(PROLOGUE_MAGIC);
+            const bool wide = ((reinterpret_cast<uintptr_t>(a.xq) | reinterpret_cast<uintptr_t>(a.xd) | reinterpret_cast<uintptr_t>(a.keep) * 4) & 15u) == 0;
+            for (unsigned u = (blockIdx.x * 8u + (threadIdx.x >> 5)) * 4u; u < units; u += stride) {
+                // this unit's row and columns; the next three by one step each
+                const unsigned row0 = u / (unsigned)nch, t0 = row0 / (unsigned)a.B;
+                int ch = (int)(u - row0 * nch), b = (int)(row0 - t0 * a.B);
+                unsigned row = row0;
+                const float *src = static_cast<const float *>(a.x) + t0 * a.x_ts + b * a.x_bs;
+                float4 in[4];
+                unsigned rows[4];
+                int ks[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int k = ch * 128 + lane * 4;
+                    rows[e] = row;
+                    ks[e] = u + e < units ? k : 1 << 30;
+                    in[e] = u + e < units && k < a.K ? *reinterpret_cast<const float4 *>(src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (++ch == nch) {
+                        ch = 0;
+                        ++row;
+                        src += a.x_bs;
+                        if (++b == a.B) {
+                            b = 0;
+                            src += a.x_ts - a.B * a.x_bs;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int k = ks[e];
+                    if (k >= a.Kpad) continue;
+                    uint32_t w = 0;
+                    if (k < a.K) {
+                        float q[4], raw[4];
+                        prologue_quantize4<Mode>(a, near, in[e], q, raw);
+                        w = __byte_perm(__byte_perm(__float_as_uint(q[0]), __float_as_uint(q[1]), 0x0040),
+                                        __byte_perm(__float_as_uint(q[2]), __float_as_uint(q[3]), 0x0040), 0x5410);
+                        const long long at = (long long)rows[e] * a.K + k;
+                        const int i[4] = {__float_as_int(q[0]) - im, __float_as_int(q[1]) - im, __float_as_int(q[2]) - im, __float_as_int(q[3]) - im};
+                        if (a.xq)
+                            put4(static_cast<float *>(a.xq) + at,
+                                 Mode == 1 ? make_float4((float)i[0], (float)i[1], (float)i[2], (float)i[3])
+                                           : make_float4(__int_as_float(i[0]), __int_as_float(i[1]), __int_as_float(i[2]), __int_as_float(i[3])), wide);
+                        if (a.xd)
+                            put4(a.xd + at, make_float4((float)(i[0] - a.x_zp) * a.x_scale, (float)(i[1] - a.x_zp) * a.x_scale,
+                                                        (float)(i[2] - a.x_zp) * a.x_scale, (float)(i[3] - a.x_zp) * a.x_scale), wide);
+                        if (a.keep) {
+                            const uchar4 y = make_uchar4(raw[0] == q[0], raw[1] == q[1], raw[2] == q[2], raw[3] == q[3]);
+                            if (wide) *reinterpret_cast<uchar4 *>(a.keep + at) = y;
+                            else a.keep[at] = y.x, a.keep[at + 1] = y.y, a.keep[at + 2] = y.z, a.keep[at + 3] = y.w;
+                        }
+                    }
+                    *reinterpret_cast<uint32_t *>(a.x8 + (long long)rows[e] * a.Kpad + k) = w;
+                }
+            }
+            return;
+        }
         const int kw = a.Kpad >> 4;
         const long long total = a.N * kw;
         for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += a.q_blocks * 256ll) {
@@ -93,23 +202,15 @@ __global__ void __launch_bounds__(256) k_prologue(const PrologueArgs a) {
             const int k0 = (int)(i - row * kw) * 16;
             const long long t = row / a.B, src = t * a.x_ts + (row - t * a.B) * a.x_bs;
             unsigned w[4] = {0u, 0u, 0u, 0u};
-            float4 in[4];
-            if constexpr (Vec) {
-#pragma unroll
-                for (int g = 0; g < 4; ++g)
-                    if (k0 + 4 * g < a.K) in[g] = *reinterpret_cast<const float4 *>(static_cast<const float *>(a.x) + src + k0 + 4 * g);
-            }
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
                 if (k0 + 4 * g >= a.K) continue;
-                const float f[4] = {in[g].x, in[g].y, in[g].z, in[g].w};
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const int k = k0 + 4 * g + u;
                     if (k >= a.K) continue;
                     uint8_t keep;
-                    const int32_t q = Vec ? prologue_quantize<Mode>(f, u, a.x_scale, a.x_zp, a.x_lo, a.x_hi, keep, a.flags)
-                                          : prologue_quantize<Mode>(a.x, src + k, a.x_scale, a.x_zp, a.x_lo, a.x_hi, keep, a.flags);
+                    const int32_t q = prologue_quantize<Mode>(a.x, src + k, a.x_scale, a.x_zp, a.x_lo, a.x_hi, keep, a.flags);
                     w[g] |= ((unsigned)q & 0xffu) << (8 * u);
                     if (a.xq) {
                         if constexpr (Mode == 1) static_cast<float *>(a.xq)[row * a.K + k] = (float)q;
