@@ -128,27 +128,29 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int num_kb = Kpad / KB;
     const int m_tiles = (C + GM - 1) / GM;
-    const long long n_tiles = (N + GN - 1) / GN;
-    const long long total = (long long)m_tiles * n_tiles;   // consecutive tiles share the token tile
+    const unsigned n_tiles = (unsigned)((N + GN - 1) / GN);
     const int groups = AStat ? (int)gridDim.x / m_tiles : 1;
     // accumulator buffers: all 512 columns in the streaming form; beside W in the stationary form
     const int nacc = AStat ? (num_kb > 4 ? 2 : 3) : NACC;
     const uint32_t w_col = (uint32_t)(nacc * GN);          // first tensor-memory column of W
-    // the `local`-th tile of this CTA: false when there is none
-    auto tile_of = [&](long long local, int &m0, long long &n0) -> bool {
-        if (AStat) {
-            const long long n = (long long)(blockIdx.x / m_tiles) + local * groups;
-            if (n >= n_tiles || (int)blockIdx.x >= m_tiles * groups) return false;
-            m0 = (int)(blockIdx.x % m_tiles) * GM;
-            n0 = n * GN;
-        } else {
-            const long long tile = blockIdx.x + local * gridDim.x;
-            if (tile >= total) return false;
-            m0 = (int)(tile % m_tiles) * GM;
-            n0 = (tile / m_tiles) * GN;
+    // This CTA's tiles: channel tile m of token tile n, every gridDim.x-th (consecutive tiles share the token tile), or all of one
+    // channel tile beside a stationary W.  By additions: 64-bit divisions took a quarter of all instructions (five of 22 an output;
+    // 409600 x 768, K = 128: 270 us with them, 237 without).
+    struct Tiles {
+        unsigned m, n, dm, dn, m_tiles;
+        __device__ int m0() const { return (int)m * GM; }
+        __device__ long long n0() const { return (long long)n * GN; }
+        __device__ void next() {
+            m += dm;
+            n += dn;
+            if (m >= m_tiles) {
+                m -= m_tiles;
+                ++n;
+            }
         }
-        return true;
     };
+    const Tiles first{blockIdx.x % m_tiles, AStat && (int)blockIdx.x >= m_tiles * groups ? n_tiles : blockIdx.x / m_tiles,
+                      AStat ? 0u : gridDim.x % m_tiles, AStat ? (unsigned)groups : gridDim.x / m_tiles, (unsigned)m_tiles};
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NST; ++s) {
@@ -180,8 +182,6 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
         if (lane == 0) {
             long long it = 0;   // k-slab counter across tiles: ring position and phase
             bool ok = true;
-            int m0;
-            long long n0;
 #ifdef QGRU_STAMPS
             long long dbg_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #endif
@@ -189,7 +189,7 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
                 // this CTA's slice of W, once: through the ring's slots into tensor memory, a pass of up
                 // to STAGES_A slabs at a time (every CTA takes part, with or without tiles of its own,
                 // so that the barriers below see the same sequence everywhere)
-                m0 = (int)(blockIdx.x % m_tiles) * GM;
+                const int m0 = first.m0();
                 int pass = 0;
                 for (int done = 0; done < num_kb && ok; ++pass) {
                     const int cnt = min(STAGES_A, num_kb - done);
@@ -201,7 +201,9 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
                 }
                 tc::mbar_arrive(w_done);
             }
-            for (long long local = 0; ok && tile_of(local, m0, n0); ++local) {
+            for (Tiles w = first; ok && w.n < n_tiles; w.next()) {
+                const int m0 = w.m0();
+                const long long n0 = w.n0();
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = (int)(it % NST);
                     const uint32_t ph = (uint32_t)((it / NST) & 1);
@@ -226,8 +228,6 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
         if (lane == 0) {
             const uint32_t idesc = tc::idesc_i8(GM, GN, true, !XUnsigned);
             bool ok = true;
-            int m0;
-            long long n0;
 #ifdef QGRU_STAMPS
             long long dbg_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             const long long t_start = clock64();
@@ -247,7 +247,7 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
             uint32_t ph = 0, slot_lo = ring_lo0;
             int buf = 0;
             uint32_t acc_ph = 1;   // parity to wait for on acc_empty: buffers start out free
-            for (long long local = 0; ok && tile_of(local, m0, n0); ++local) {
+            for (Tiles w = first; ok && w.n < n_tiles; w.next()) {
                 if (!WAITED(2, tc::mbar_wait(&acc_empty[buf], acc_ph, WAIT_BUDGET))) { ok = false; break; }
                 tc::tc_fence_after_sync();
                 const uint32_t d_col = tmem_base + (uint32_t)(buf * GN);
@@ -299,7 +299,7 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
 #endif
         const int part = (warp - 2) >> 2;           // which share of the token columns
         constexpr int COLS = GN / (EPI_WARPS / 4);
-        long long local = 0;
+        unsigned local = 0;
         bool ok = true;
         // per-channel constants of a tile's rows: loaded one tile ahead, so that their global-memory
         // latency is not paid at the start of every tile
@@ -309,12 +309,10 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
             FastLin fl;
             float fs_off, fs_bias, fs_ratio;   // float-storage forward (lc.fs set)
         };
-        auto load_consts = [&](long long lcl) {
+        auto load_consts = [&](const Tiles &w) {
             ChanConsts c;
-            int tm0 = 0;
-            long long tn0 = 0;
-            const bool have = tile_of(lcl, tm0, tn0);
-            const int m = tm0 + q * 32 + lane;
+            const bool have = w.n < n_tiles;
+            const int m = w.m0() + q * 32 + lane;
             const bool m_ok = have && m < C;
             c.corr = m_ok ? lc.corr[m] : 0;
             c.rs = m_ok ? lc.rs[m] : Rescale{1, 1, 0, 0, 0, 0, 0, 0};
@@ -353,26 +351,27 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
             }
         }
         const int slice = ps.slice, ld = 3 * slice;
-        ChanConsts cur = load_consts(0);
-        int m0;
-        long long n0;
-        for (; ok && tile_of(local, m0, n0); ++local) {
+        Tiles w = first;
+        ChanConsts cur = load_consts(w);
+        for (; ok && w.n < n_tiles; ++local) {
             const int buf = (int)(local % nacc);
-            const int m = m0 + q * 32 + lane;
+            const int m = w.m0() + q * 32 + lane;
+            const long long n0 = w.n0();
             const bool m_ok = m < C;
-            const ChanConsts nxt = AStat ? cur : load_consts(local + 1);
+            w.next();
+            const ChanConsts nxt = AStat ? cur : load_consts(w);
             const int64_t corr = cur.corr;
             const Rescale rs = cur.rs;
             const FastLin fl = cur.fl;
             // fused-cell mode: the channel's gate decides the second rescale (to its input scale)
-            const int gate = m_ok ? m / ps.H : 0;
+            const int gate = m_ok ? (m >= ps.H) + (m >= 2 * ps.H) : 0;
             const Rescale pre_rs = ps.to[gate];
             const int32_t pre_zp = ps.zp_in[gate];
             const int32_t c32 = (int32_t)corr;
             ok = WAITED(4, tc::mbar_wait(&acc_full[buf], (uint32_t)((local / nacc) & 1), WAIT_BUDGET));
             if (!ok) break;
             tc::tc_fence_after_sync();
-            const int unit = m - gate * ps.H, sl = unit / slice;
+            const int unit = m - gate * ps.H, sl = unit < slice ? 0 : unit / slice;
             IhT *out = ih + ((size_t)sl * N * ld + gate * slice + (unit - sl * slice));
             // this warp's COLS accumulator columns: both halves are fetched before anything is
             // computed, and the buffer goes back to the MMA warp as soon as they have arrived
