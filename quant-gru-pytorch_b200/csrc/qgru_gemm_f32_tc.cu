@@ -13,7 +13,7 @@
 // multiplies its tile again with fp32 multiply-adds, so that the result is the one they give.
 //
 // us (TFLOP/s of the fp32 product), fp32 pipe / here: 51200 x 1536 x 256 862 / 331 (122), 1536 x 51200 x 512 1860 / 448 (180),
-// 51200 x 256 x 1536 858 / 369.  The MMAs alone are 1000 cycles of a slab of 3200; bound by the eight warps' own instructions (split
+// 51200 x 256 x 1536 858 / 339 (its result masked, four columns at a time; 425 one by one).  The MMAs alone are 1000 cycles of a slab of 3200; bound by the eight warps' own instructions (split
 // 1200 cycles, sums 800, stores and loads) between which only two warps per scheduler overlap.  What did not help: sixteen
 // warps with half the sums each (112 registers: the operands in flight spill and wait); packed fp32 subtractions and sums; one
 // K order for all operands in shared memory (transposing costs 4-byte loads).

@@ -124,7 +124,8 @@ __device__ __forceinline__ void put4(float *p, const float4 &y, bool wide) {
 
 // Vec (rows and base aligned, K a multiple of 4): a warp takes four neighbouring units of 128 columns, a lane four columns of each:
 // one 128-bit load and one store of each kind, whole lines.  Memory-bound: 409600 x 128 fp32 60 us, 51200 x 256 with the training
-// outputs 22 us (with 16 columns a thread and a division a value: 77 and 92; with conversions and no division: 77 and 26).  Else a thread takes 16 columns with scalar loads.
+// outputs 22 us (16 columns a thread and a division a value: 77 and 92; conversions and no division: 77 and 26).
+// Else a thread takes 16 columns with scalar loads.
 template <int Mode, bool Vec>
 __global__ void __launch_bounds__(256) k_prologue(const PrologueArgs a) {
     pdl_trigger();
