@@ -135,7 +135,7 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
     const uint32_t w_col = (uint32_t)(nacc * GN);          // first tensor-memory column of W
     // This CTA's tiles: channel tile m of token tile n, every gridDim.x-th (consecutive tiles share the token tile), or all of one
     // channel tile beside a stationary W.  By additions: 64-bit divisions took a quarter of all instructions (five of 22 an output;
-    // 409600 x 768, K = 128: 270 us with them, 237 without).
+    // 409600 x 768, K = 128: 270 us with them, 234 without).
     struct Tiles {
         unsigned m, n, dm, dn, m_tiles;
         __device__ int m0() const { return (int)m * GM; }
@@ -402,7 +402,7 @@ k_gemm_wx_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ 
                         const int32_t t_lo = gate * ps.table_n + lc.lo - ps.lo, t_hi = t_lo + (lc.hi - lc.lo);
 #pragma unroll
                         for (int i = 0; i < 16; ++i)
-                            y[i] = lds_i32(tb + 4u * (uint32_t)min(max(lin_round<Tie>(v[i], fl) + t_c, t_lo), t_hi));
+                            y[i] = lds_table(tb + 4u * (uint32_t)min(max(lin_round<Tie>(v[i], fl) + t_c, t_lo), t_hi));
                     } else if (ps.enabled) {
 #pragma unroll
                         for (int i = 0; i < 16; ++i)
