@@ -11,8 +11,18 @@
 //
 // A step: cells (a warp per two or four rows and 32 units) add the P partial sums of their units and make dq; one thread a tile
 // issues its MMAs; sixteen warps read the accumulators, 32 units each, and store them with 16-byte st.async into the
-// CTA that owns the units, counted on its mbarrier.  A cluster barrier, arrived on when a warp has read its partial sums
-// and waited for before the next ones are stored, keeps the one buffer safe; it lies behind the MMAs' time.
+// CTA that owns the units, counted on its mbarrier.
+//
+// Every buffer is written again in every step.  What orders the next write after the last read:
+//   dq's operand     the cells wait for the MMAs of ALL tiles of the step before (b_free) before they store; that their own
+//                    partial sums have come says nothing of the tiles whose units other CTAs own.  (One barrier that every tile
+//                    commits to: a wait for each tile's acc_full in turn was 0.35 us a step at H = 512);
+//   accumulators     the MMAs of a step wait for an arrival of every warp (b_full): of a warp with cells when its share of dq is
+//                    stored, of one without at the head of the step, of both behind their reads of the step before;
+//   partial sums     a cluster barrier, arrived on when a warp has read what came for the last step and waited for before the
+//                    next ones are sent; it lies behind the MMAs' time;
+//   their mbarrier   armed for the next step by a thread that has seen the last one complete, before it arrives on that
+//                    cluster barrier.
 //
 // us a step (80 steps), fp32 pipe / here: H = 512, 256 rows 21.9 / 5.3 (10700 cycles: 1700 cells, 2100 MMAs, 1600 reading the accumulators,
 // 3200 until the last partial sum has come; those are 30 KB a CTA and step), 32 rows 4.5 / 2.4; H = 256, 256 rows 6.0 / 2.9; H = 128, 32 rows
@@ -106,8 +116,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
     float *recv = reinterpret_cast<float *>(b_ops + (3 * a.rows + 63) / 64 * B_GROUP);      // [P][rows / 4][U][4]
     float *bsum = recv + a.P * U * a.rows;                                                  // [cell warps][6][32]
     uint64_t *bars = reinterpret_cast<uint64_t *>(bsum + WARPS * 6 * 32);
-    uint64_t *got = bars, *b_full = bars + 1, *acc_full = bars + 2;                         // acc_full: one per tile
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 6);
+    uint64_t *got = bars, *b_full = bars + 1, *b_free = bars + 2, *acc_full = bars + 3;     // acc_full: one per tile
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 7);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = a.H, P = a.P;
     const int p = P > 1 ? (int)cluster_rank() : 0;
@@ -116,7 +126,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
     const uint32_t recv_bytes = (uint32_t)(P * min(U, (H - p * U + 31) & ~31) * a.rows * 4);
     if (tid == 0) {
         tc::mbar_init(got, 1);
-        tc::mbar_init(b_full, cell_warps);
+        tc::mbar_init(b_full, WARPS);
+        tc::mbar_init(b_free, (uint32_t)a.tiles);
         for (int t = 0; t < 4; ++t) tc::mbar_init(&acc_full[t], 1);
         tc::fence_barrier_init();
         tc::mbar_expect_tx(got, recv_bytes);
@@ -273,6 +284,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
                 for (int e = 0; e < RPT; ++e)
                     if (act[e] && a.dh_in) y[e] = a.dh_in[(size_t)(b0 + r0 + e) * H + cj];
             } else {
+                // (complete before the partial sums come, save where a tile's MMAs were issued late)
+                ok = ok && tc::mbar_wait(b_free, (uint32_t)((s - 1) & 1), WAIT_BUDGET);
                 ok = ok && tc::mbar_wait(got, (uint32_t)((s - 1) & 1), WAIT_BUDGET);
                 if (tid == 0) tc::mbar_expect_tx(got, recv_bytes);
                 carry(y);
@@ -344,8 +357,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
                     }
             dp_out += 3 * BH;
             dq_out += 3 * BH;
-        } else if (P > 1) {
-            cluster_arrive();
+        } else {
+            if (lane == 0) tc::mbar_arrive(b_full);     // this warp's reads of the accumulators lie behind it
+            __syncwarp();
+            if (P > 1) cluster_arrive();
         }
         if (issues) {
             if (lane == 0) {
@@ -357,6 +372,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
                     for (int k = 0; k < a.nt; ++k)
                         mma_bf16_ts(d, at0 + (uint32_t)(k * a.tiles * 8), bb + (uint32_t)((ks + k) * 2048 >> 4), idesc, (uint32_t)(ks + k));
                     tc::mma_commit(&acc_full[mt]);
+                    tc::mma_commit(b_free);
                 }
             }
             ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
@@ -383,7 +399,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
                         st_async_v4(dst + (uint32_t)(c + 4 * e) * (U * 4u), w, dst_bar);
                     }
             }
-            tc::tc_fence_before_sync();
+            tc::tc_fence_before_sync();  // (the loads are complete: tmem_ld_wait)
         }
         __syncwarp();
         // (what the next step does not wait for: while the partial sums are on their way)

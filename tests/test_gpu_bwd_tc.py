@@ -39,6 +39,39 @@ def test_chain_of_state_gradients(cuda_device, storage, cfg, B, H, bidir):
         assert (a - b).norm() <= 2e-6 * b.norm() and (a - b).abs().max() <= 2e-5 * b.abs().max()
 
 
+# 4, 16 and 28 rows a cluster; two, three and four tiles; warps that only read accumulators, and none
+@pytest.mark.parametrize("H,B,sms", [(190, 4, 8), (190, 56, 8), (257, 16, 12), (300, 56, 12), (512, 4, 24), (512, 16, 24), (512, 56, 24),
+                                     (512, 300, 0)])
+def test_long_chain_repeats_its_bits(cuda_device, H, B, sms):
+    """Operand, accumulators and partial sums are written again in each of 250 steps; sums have a fixed order, so every pass gives the
+    same bits, and the gradients of the stepwise path."""
+    import torch
+    torch.manual_seed(H + B)
+    T, I = 250, 16
+    m = QuantGRU(I, H, quant_storage_dtype="int32").to(cuda_device)
+    x = torch.randn(T, B, I, device=cuda_device)
+    m.calibrating = True
+    m(x)
+    m.calibrating = False
+    m.finalize_calibration()
+    m.use_quantization = True
+    m.train()
+    if sms:
+        m.set_option("sm_limit", sms)       # one or two clusters
+    hx = (torch.randn(1, B, H, device=cuda_device) * 0.3).requires_grad_()
+    x.requires_grad_()
+    g_out = torch.randn(T, B, H, device=cuda_device)
+    wrt = [x, hx] + list(m.parameters())
+    got = [torch.autograd.grad(m(x, hx)[0], wrt, g_out) for _ in range(4)]
+    assert m._dirs[0].handle.train_saved_bytes(2, T, B)     # (it was the one-call form)
+    for again in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], again))
+    want = torch.autograd.grad(m._forward_train_stepwise(x, hx)[0], wrt, g_out)
+    for a, b in zip(got[0], want):
+        # as above; a step's error of 2e-7 fades with the gate (z about 1/2, so two steps' worth), in sums over 250 steps of mixed sign
+        assert (a - b).norm() <= 2e-6 * b.norm() and (a - b).abs().max() <= 2e-5 * b.abs().max()
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
 def test_chain_keeps_what_is_not_finite(cuda_device, value):
     """An infinite or undefined gradient of one row reaches what it reached in fp32, and no other row."""
