@@ -1,6 +1,9 @@
-// qgru_gemm_f32_tc.cu - the fp32 matrix product on the tensor cores: every fp32 operand is the exact sum of three bf16
-// values (8 + 8 + 8 significand bits), and a product of two operands is the sum of the six partial products
+// qgru_gemm_f32_tc.cu - the fp32 matrix product on the tensor cores: every fp32 operand times 2^24 is the exact sum of three
+// bf16 values (8 + 8 + 8 significand bits), and a product of two operands is the sum of the six partial products
 // hi*hi, hi*mid, mid*hi, mid*mid, hi*lo, lo*hi; the three left out are together at most 2^-23 of it, and 2^-26 in the mean.
+// The factor is for small operands: the low part's last bit, 2^-149 of the operand at the least, stays a normal bf16 number
+// (without it the split loses bits below 2^-110, 1e-3 of a value at 2^-124, where gradients that have vanished over many steps
+// are).  The sums are multiplied by 2^-48 where they are added up.
 //
 // One CTA per 128 x (16 .. 256) tile of C and K part.  Eight warps fetch the fp32 operands a K slab of 32 ahead, split them in
 // registers and store the three parts into swizzled shared-memory tiles (three stages of 72 KB); one thread issues the
@@ -9,14 +12,16 @@
 // eight warps add the other to fp32 sums in registers, rounded to nearest.  Sums are in a fixed order.
 // Error against float64 (2-norm, operands uniform in +-0.5), here / fp32 multiply-adds: K = 32 5.5e-8 / 1.0e-7, K = 786 9.0e-8 / 5.2e-7,
 // K = 51200 in six parts 3.1e-7 / 1.7e-6.  With a sum of two slabs in tensor memory it was 3e-7 at every K.
-// Infinities, NaN and values that round to infinity in bf16 have no such parts (inf - inf); a CTA whose sums are not all finite
-// multiplies its tile again with fp32 multiply-adds, so that the result is the one they give.
+// Infinities, NaN and values that round to infinity in bf16 (from 2^104 up) have no such parts (inf - inf), and sums from 2^80
+// up overflow in tensor memory; a CTA whose sums are not all finite multiplies its tile again with fp32 multiply-adds, so
+// that the result is the one they give.
 //
-// us (TFLOP/s of the fp32 product), fp32 pipe / here: 51200 x 1536 x 256 862 / 331 (122), 1536 x 51200 x 512 1860 / 448 (180),
-// 51200 x 256 x 1536 858 / 339 (its result masked, four columns at a time; 425 one by one).  The MMAs alone are 1000 cycles of a slab of 3200; bound by the eight warps' own instructions (split
-// 1200 cycles, sums 800, stores and loads) between which only two warps per scheduler overlap.  What did not help: sixteen
-// warps with half the sums each (112 registers: the operands in flight spill and wait); packed fp32 subtractions and sums; one
-// K order for all operands in shared memory (transposing costs 4-byte loads).
+// us (TFLOP/s of the fp32 product) at N x K x M, fp32 pipe / here: 51200 x 1536 x 256 862 / 307 (131; its result masked 339, four
+// columns at a time, one by one 425), 1536 x 51200 x 512 1860 / 513 (157; 488 without the factor of 2^24).  The MMAs alone are 1000
+// cycles of a slab of 3200; bound by the eight warps' own instructions (split 1200 cycles, sums 800, stores and loads) between
+// which only two warps per scheduler overlap.  What did not help: sixteen warps with half the sums each (112 registers: the
+// operands in flight spill and wait); packed fp32 subtractions, sums and factors (the last: 51200 x 256 x 1536 428 us, 393 with
+// single ones: spills); one K order for all operands in shared memory (transposing costs 4-byte loads).
 #include <algorithm>
 #include <type_traits>
 
@@ -80,12 +85,14 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint32_t a_lo, uint32_t b_l
         : "memory");
 }
 
+constexpr float SCALE = 0x1p24f, UNSCALE = 0x1p-48f;     // of an operand, of a product
+
 // Four neighbours: their three bf16 parts, 8 bytes each.
 __device__ __forceinline__ void split4(const float (&v)[4], uint2 (&part)[3]) {
     uint32_t w[3][2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-        float x0 = v[2 * j], x1 = v[2 * j + 1];
+        float x0 = v[2 * j] * SCALE, x1 = v[2 * j + 1] * SCALE;
 #pragma unroll
         for (int p = 0; p < 3; ++p) {
             asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w[p][j]) : "f"(x1), "f"(x0));
@@ -305,7 +312,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm_f32_tc(const TcArgs g) {
 #pragma unroll
                     for (int h = 0; h < 2; ++h)
 #pragma unroll
-                        for (int e = 0; e < 16; ++e) sum[i + h][e] += __int_as_float(v[h][e]);
+                        for (int e = 0; e < 16; ++e) sum[i + h][e] = fmaf(__int_as_float(v[h][e]), UNSCALE, sum[i + h][e]);
                 }
             tc::tc_fence_before_sync();
             __syncwarp();

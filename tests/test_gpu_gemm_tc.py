@@ -17,22 +17,21 @@ def _t(a, dev):
     return torch.from_numpy(np.ascontiguousarray(a)).to(dev)
 
 
-# (T * B, I, H): I and 3H at and beside tiles of 128 and 256, rows in groups of four, two and one, K with and without a rest
-@pytest.mark.parametrize("T,B,I,H", [(16, 256, 128, 128), (31, 131, 130, 86), (50, 81, 257, 43), (33, 128, 16, 171), (67, 96, 64, 256)])
-def test_products_of_the_backward(cuda_device, T, B, I, H):
+def _backward_without_r(dev, T, B, I, H, x_scale=1.0, dh_scale=1.0):
+    """dx, dW, dR of the library (R = 0: dp and dq of a step depend on its own gradient and what comes through the update gate)
+    and the same in float64."""
     import torch
     rng = np.random.default_rng(I * H)
     W, R, _, _ = gen_weights(rng, I, H)
-    v = torch.rand(T, B, 4 * H, device=cuda_device)
-    h = torch.randn(T + 1, B, H, device=cuda_device) * 0.3
-    x = torch.randn(T, B, I, device=cuda_device)
-    dh = torch.randn(T + 1, B, H, device=cuda_device)
+    v = torch.rand(T, B, 4 * H, device=dev)
+    h = torch.randn(T + 1, B, H, device=dev) * 0.3
+    x = torch.randn(T, B, I, device=dev) * x_scale
+    dh = torch.randn(T + 1, B, H, device=dev) * dh_scale
     with gru_ops.Handle(I, H, device=0) as hd:
-        dx, dW, dR, dbw, dbr, _ = hd.backward(_t(W, cuda_device), _t(R * 0, cuda_device), x, dh, h, v)
-    # R = 0: dp and dq of a step depend on its own gradient and what comes through the update gate; float64
+        dx, dW, dR, dbw, dbr, _ = hd.backward(_t(W, dev), _t(R * 0, dev), x, dh, h, v)
     z, r, g, q = (v[..., k * H:(k + 1) * H].double() for k in range(4))
-    carry = torch.zeros(B, H, dtype=torch.float64, device=cuda_device)
-    dp = torch.empty(T, B, 3 * H, dtype=torch.float64, device=cuda_device)
+    carry = torch.zeros(B, H, dtype=torch.float64, device=dev)
+    dp = torch.empty(T, B, 3 * H, dtype=torch.float64, device=dev)
     dq = torch.empty_like(dp)
     for t in range(T - 1, -1, -1):
         d = dh[t + 1].double() + carry
@@ -42,11 +41,25 @@ def test_products_of_the_backward(cuda_device, T, B, I, H):
         dp[t], dq[t] = torch.cat([dz, dr, dg], 1), torch.cat([dz, dr, dg * r[t]], 1)
         carry = z[t] * d
     P, Q = dp.reshape(T * B, -1), dq.reshape(T * B, -1)
-    want = [P @ _t(W, cuda_device).double().t(), x.reshape(-1, I).double().t() @ P, h[:T].reshape(-1, H).double().t() @ Q]
-    for a, b in zip((dx, dW, dR), want):
+    want = [P @ _t(W, dev).double().t(), x.reshape(-1, I).double().t() @ P, h[:T].reshape(-1, H).double().t() @ Q]
+    return [a.double().reshape(b.shape) for a, b in zip((dx, dW, dR), want)], want
+
+
+# (T * B, I, H): I and 3H at and beside tiles of 128 and 256, rows in groups of four, two and one, K with and without a rest
+@pytest.mark.parametrize("T,B,I,H", [(16, 256, 128, 128), (31, 131, 130, 86), (50, 81, 257, 43), (33, 128, 16, 171), (67, 96, 64, 256)])
+def test_products_of_the_backward(cuda_device, T, B, I, H):
+    for a, b in zip(*_backward_without_r(cuda_device, T, B, I, H)):
         # dp and dq carry a few fp32 roundings each (2^-24 of values with a spread of order one); sums over K of them less
-        a = a.double().reshape(b.shape)
         assert (a - b).norm() <= 5e-7 * b.norm()
+        assert (a - b).abs().max() <= 1e-5 * b.abs().max()
+
+
+@pytest.mark.parametrize("x_scale,dh_scale", [(2.0 ** -118, 1.0), (1.0, 2.0 ** -118), (2.0 ** 50, 2.0 ** 40), (2.0 ** 105, 2.0 ** -30)])
+def test_products_of_very_small_and_large_values(cuda_device, x_scale, dh_scale):
+    """Near the ends of fp32 (2^-126, 2^128) the products are as exact as in the middle; every result here is a normal number."""
+    for a, b in zip(*_backward_without_r(cuda_device, 16, 256, 128, 128, x_scale, dh_scale)):
+        # as above, and what is below 2^-126 rounds to 2^-149: of sums near 2^-120 over 384 terms and more, 2^-150 each, less than 1e-7
+        assert (a - b).norm() <= 6e-7 * b.norm()
         assert (a - b).abs().max() <= 1e-5 * b.abs().max()
 
 
