@@ -72,6 +72,31 @@ def test_long_chain_repeats_its_bits(cuda_device, H, B, sms):
         assert (a - b).norm() <= 2e-6 * b.norm() and (a - b).abs().max() <= 2e-5 * b.abs().max()
 
 
+@pytest.mark.parametrize("scale", [2.0 ** -112, 2.0 ** -118, 2.0 ** 60, 2.0 ** 100])
+def test_chain_of_very_small_and_large_gradients(cuda_device, scale):
+    """Near the ends of fp32 (2^-126, 2^128) the chain is as exact as in the middle: gradients that were scaled by a power of two
+    come back scaled, save for what rounds below 2^-126."""
+    import torch
+    torch.manual_seed(11)
+    T, B, I, H = 4, 24, 24, 200
+    m = QuantGRU(I, H, quant_storage_dtype="float32").to(cuda_device)
+    x = torch.randn(T, B, I, device=cuda_device)
+    m.calibrating = True
+    m(x)
+    m.calibrating = False
+    m.finalize_calibration()
+    m.use_quantization = True
+    m.train()
+    hx = (torch.randn(1, B, H, device=cuda_device) * 0.3).requires_grad_()
+    g_out = torch.randn(T, B, H, device=cuda_device)
+    got = torch.autograd.grad(m(x, hx)[0], [hx, m.weight_hh_l0], g_out * scale)
+    want = torch.autograd.grad(m(x, hx)[0], [hx, m.weight_hh_l0], g_out)
+    for a, b in zip(got, want):
+        a = a.double() / scale
+        # sums of some 3H products, in four steps, of 2^-149 / 2 each at the most where a product rounds below 2^-126
+        assert (a - b).norm() <= 1e-7 * b.norm() + 2.0 ** -149 / scale * (4 * 3 * H * b.numel()) ** 0.5
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
 def test_chain_keeps_what_is_not_finite(cuda_device, value):
     """An infinite or undefined gradient of one row reaches what it reached in fp32, and no other row."""
