@@ -167,8 +167,8 @@ int qgru_backward(qgru_handle *h, int T, int B, const float *W_t, const float *R
         h->launches++;
     }
 
-    int G = 0;
-    if (bwd_chain_fits(h, B, &G)) {
+    if (bwd_chain_plan(h, B, 1)) {
+        const int G = h->plan_bwd.G;
         if ((rc = ensure(h, h->bwd_bias, (size_t)G * 2 * C * sizeof(float)))) return rc;
         float *part = (float *)h->bwd_bias.p;
         if ((rc = bwd_chain_launch(h, BwdChainArgs{T, B, H, R_t, 1, 0, 0, h_all, v, dh_new + NH, (long long)NH, H, dh, dh, m.h0, pm, dp, dq, part}, st)))

@@ -156,6 +156,7 @@ struct qgru_handle {
     DevBuf bwd_bias, bwd_pm;               // backward pass: bias sums per batch group, packed clamp masks
     DevBuf f_split;                        // fp32 matrix product: partial tiles where K is split
     qgru::F32RecPlan plan_fwd, plan_bwd, plan_bwd_tc;   // fp32 recurrences: the plan of the last batch size
+    int f32_fwd_exists = -1, f32_bwd_exists = -1;      // and whether there is a form at all (-1: not asked yet)
     DevBuf fs_ch;                          // float-storage forward: 4 x 3H per-channel scale ratios
     bool fs_uploaded = false, fs_ready = false;   // fs_ch matches the current parameters; and the current weights
     StreamOrder order;

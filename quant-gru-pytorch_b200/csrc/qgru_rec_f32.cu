@@ -673,14 +673,15 @@ cudaError_t launch_chain(Kern kern, const F32RecPlan &pl, Args &a, cudaStream_t 
 // H = 256: 1 row 2.0 / 2.7, 96 rows 3.6 / 3.9, 128 rows 5.3 / 4.4.  One CTA against clusters: H = 96 1.35 / 1.7, H = 128 (512 threads)
 // 2.2 / 1.6.  The cost of a form is fitted to such times (H = 32 .. 512, 1 to 512 rows, one and two directions).
 template <typename KernOf>
-void make_plan(qgru_handle *h, int B, int sms, bool fwd, KernOf kern, size_t (*floats)(int, int, int, int, int), F32RecPlan *pl) {
+void make_plan(qgru_handle *h, int B, int sms, int directions, bool fwd, KernOf kern, size_t (*floats)(int, int, int, int, int), F32RecPlan *pl) {
     const int H = h->H;
-    if (pl->H == H && pl->B == B && pl->sms == sms) return;
+    if (pl->H == H && pl->B == B && pl->sms == sms && pl->directions == directions) return;
     *pl = F32RecPlan{};
     pl->H = H;
     pl->B = B;
     pl->sms = sms;
-    const int both = 2 * sms <= h->sm_count ? 2 : 1;      // directions side by side: as many clusters again
+    pl->directions = directions;
+    const int chip = std::min(directions * sms, h->sm_count);   // side by side: as many clusters again, on as many SMs again
     double best = 0;
     for (int P = 1; P <= 16; ++P) {
         const int U = ((H + P - 1) / P + 31) / 32 * 32, KG = P * U / 32, threads = U * KG;
@@ -703,13 +704,12 @@ void make_plan(qgru_handle *h, int B, int sms, bool fwd, KernOf kern, size_t (*f
             const size_t smem = floats(P, U, KG, Bt, D) * sizeof(float);
             if (smem > (size_t)h->smem_optin) break;
             const int per_sm = std::max<int>(1, (int)std::min<size_t>((size_t)(active0 * P / h->sm_count), (size_t)(227 * 1024) / (smem + 1024)));
-            const int chip = both > 1 ? h->sm_count : sms;
             const int active = std::max(1, std::min(active0, chip * per_sm / P));
-            const int G = (B + Bt - 1) / Bt, waves = (both * G + active - 1) / active;
-            const int sharing = std::max(1, std::min(per_sm, (both * G * P + chip - 1) / chip));
+            const int G = (B + Bt - 1) / Bt, waves = (directions * G + active - 1) / active;
+            const int sharing = std::max(1, std::min(per_sm, (directions * G * P + chip - 1) / chip));
             double cost = waves * step(Bt, sharing);
             // One cluster too many for the chip, but with few rows: the last ones of the two directions follow one another.
-            if (both > 1 && both * G == active + 1) cost = std::min(cost, std::max(step(Bt, sharing), 2.0 * step(B - (G - 1) * Bt, sharing)));
+            if (directions > 1 && directions * G == active + 1) cost = std::min(cost, std::max(step(Bt, sharing), 2.0 * step(B - (G - 1) * Bt, sharing)));
             if (best == 0 || cost < best) {
                 best = cost;
                 pl->P = P;
@@ -731,13 +731,28 @@ void make_plan(qgru_handle *h, int B, int sms, bool fwd, KernOf kern, size_t (*f
 auto fwd_kernel(int threads) { return threads <= 384 ? k_float_chain<false, 384> : k_float_chain<false, 512>; }
 auto bwd_kernel(int threads) { return threads <= 384 ? k_bwd_chain<false, 384> : k_bwd_chain<false, 512>; }
 
-// The SMs of a direction of a layer whose directions run side by side.
+// Whether one of make_plan's forms runs at all.
+template <typename KernOf>
+bool any_form(qgru_handle *h, KernOf kern, size_t (*floats)(int, int, int, int, int), int *known) {
+    if (*known >= 0) return *known == 1;
+    *known = 0;
+    for (int P = 1; P <= 16 && *known == 0; ++P) {
+        const int U = ((h->H + P - 1) / P + 31) / 32 * 32, KG = P * U / 32, threads = U * KG;
+        const size_t smem = floats(P, U, KG, 1, 3) * sizeof(float);
+        if (threads <= 512 && (P - 1) * U < h->H && smem <= (size_t)h->smem_optin && active_clusters(kern(threads), P, threads, smem) > 0) *known = 1;
+    }
+    return *known == 1;
+}
+
+// The SMs that this handle's kernels may take.
 int side_sms(const qgru_handle *h) { return h->opt_sm_limit > 0 ? std::min(h->opt_sm_limit, h->sm_count) : h->sm_count; }
 
 }  // namespace
 
-bool float_chain_fits(qgru_handle *h, int B) {
-    make_plan(h, B, side_sms(h), true, fwd_kernel, fwd_smem_floats, &h->plan_fwd);
+bool float_chain_exists(qgru_handle *h) { return any_form(h, fwd_kernel, fwd_smem_floats, &h->f32_fwd_exists); }
+
+bool float_chain_plan(qgru_handle *h, int B, int directions) {
+    make_plan(h, B, side_sms(h), directions, true, fwd_kernel, fwd_smem_floats, &h->plan_fwd);
     return h->plan_fwd.ok;
 }
 
@@ -748,7 +763,7 @@ bool float_chain_fits(qgru_handle *h, int B) {
 // such times (H = 16 .. 512, up to 8192 rows): from four steps on at most 20 % off the better one at each of 120 sizes.
 bool float_chain_is_faster(qgru_handle *h, int T, int B) {
     // (float inference and calibration run one direction after the other: each has the whole chip)
-    make_plan(h, B, h->sm_count, true, fwd_kernel, fwd_smem_floats, &h->plan_fwd);
+    make_plan(h, B, h->sm_count, 1, true, fwd_kernel, fwd_smem_floats, &h->plan_fwd);
     const F32RecPlan &pl = h->plan_fwd;
     if (!pl.ok) return false;
     const double H = h->H, chain = pl.waves * (0.7 + 0.046 * (pl.U * pl.KG / 32) * pl.Bt * pl.sharing);
@@ -766,9 +781,10 @@ int float_chain_launch(qgru_handle *h, FloatFwdArgs a, cudaStream_t st) {
     return QGRU_OK;
 }
 
-bool bwd_chain_fits(qgru_handle *h, int B, int *groups) {
-    make_plan(h, B, side_sms(h), false, bwd_kernel, bwd_smem_floats, &h->plan_bwd);
-    *groups = h->plan_bwd.G;
+bool bwd_chain_exists(qgru_handle *h) { return any_form(h, bwd_kernel, bwd_smem_floats, &h->f32_bwd_exists); }
+
+bool bwd_chain_plan(qgru_handle *h, int B, int directions) {
+    make_plan(h, B, side_sms(h), directions, false, bwd_kernel, bwd_smem_floats, &h->plan_bwd);
     return h->plan_bwd.ok;
 }
 

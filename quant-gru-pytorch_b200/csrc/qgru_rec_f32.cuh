@@ -13,7 +13,7 @@ namespace qgru {
 // How a sequence is cut: clusters of P CTAs own Bt batch rows, each CTA U hidden units (a multiple of
 // 32); KG = P * U / 32 slices of 32 units; U * KG <= 512 threads.
 struct F32RecPlan {
-    int H = 0, B = 0, sms = 0;      // what the plan was made for
+    int H = 0, B = 0, sms = 0, directions = 0;      // what the plan was made for
     bool ok = false;
     int P = 1, U = 32, KG = 1, Bt = 1, G = 1, D = 1;
     int waves = 1, sharing = 1;     // clusters one after the other, CTAs on an SM at once
@@ -33,8 +33,11 @@ struct FloatFwdArgs {
     OutView out;                      // further copies of the states: hf, hn_f
     int U, P, KG, Bt, D;              // set by the launcher
 };
-// False: no plan for this shape (H > 512), the caller runs step by step.
-bool float_chain_fits(qgru_handle *h, int B);
+// Whether there is a form for the layer (H <= 512); else the caller runs step by step.
+bool float_chain_exists(qgru_handle *h);
+// The form for B rows, into the handle's plan_fwd; directions: 2 where another one of the same size runs beside it, each
+// within its handle's sm_limit.
+bool float_chain_plan(qgru_handle *h, int B, int directions);
 // Whether T steps of it, with the whole chip to itself, take no longer than a tiled product and a pointwise launch a step.
 bool float_chain_is_faster(qgru_handle *h, int T, int B);
 int float_chain_launch(qgru_handle *h, FloatFwdArgs a, cudaStream_t st);
@@ -56,7 +59,8 @@ struct BwdChainArgs {
     const float *r_scale;
     int U, P, KG, Bt, D;              // set by the launcher
 };
-bool bwd_chain_fits(qgru_handle *h, int B, int *groups);
+bool bwd_chain_exists(qgru_handle *h);
+bool bwd_chain_plan(qgru_handle *h, int B, int directions);     // into plan_bwd
 int bwd_chain_launch(qgru_handle *h, BwdChainArgs a, cudaStream_t st);
 
 // The same on the tensor cores, for a quantized R (r8, r_scale and pm are set; qgru_bwd_tc.cu).  The plan is kept in *pl for its

@@ -123,17 +123,17 @@ int train_ih_bytes(const qgru_handle *h) {
 
 // Whether this direction has the one-launch forms of both recurrences (mode 1 needs fs_setup's table size).
 int train_plan(qgru_handle *h, int mode, int B, int n_tab, bool *ok) {
-    int G = 0;
     const int sms = h->opt_sm_limit > 0 ? std::min(h->opt_sm_limit, h->sm_count) : h->sm_count;
-    *ok = bwd_chain_fits(h, B, &G);
-    if (mode == 0) *ok = *ok && float_chain_fits(h, B);
+    *ok = bwd_chain_exists(h);
+    if (mode == 0) *ok = *ok && float_chain_exists(h);
     else *ok = *ok && h->fast && h->opt_gemm != 1 && (h->opt_rec == 0 || h->opt_rec >= 5) &&
                rec_reg_plan(h, B, sms, train_ih_bytes(h), mode == 1 ? CELL_FS_TRAIN : CELL_INT_TRAIN, n_tab, &h->plan_train);
     return QGRU_OK;
 }
 
 int train_forward_dir(qgru_handle *h, int mode, int T, int B, const void *x, long long x_ts, long long x_bs, const float *h0,
-                      const qgru_train_dir &d, OutView out, bool rev, cudaStream_t st, const uint8_t *x8_shared, cudaEvent_t after_prologue) {
+                      const qgru_train_dir &d, OutView out, bool rev, int directions, cudaStream_t st, const uint8_t *x8_shared,
+                      cudaEvent_t after_prologue) {
     const int H = h->H, I = h->I, C = h->C;
     const long long N = (long long)T * B;
     const TrainSaved s = train_saved(h, mode, T, B, d.saved);
@@ -149,7 +149,7 @@ int train_forward_dir(qgru_handle *h, int mode, int T, int B, const void *x, lon
         if ((rc = gemm_f32(h, GemmF32{(const float *)x, false, d.W, true, (float *)h->f_wx.p, N, I, C}, st))) return rc;
         bool ok;
         if ((rc = train_plan(h, mode, B, 0, &ok))) return rc;
-        if (!ok) return fail(h, QGRU_ERR_UNSUPPORTED, "no one-launch recurrence for this layer");
+        if (!ok || !float_chain_plan(h, B, directions)) return fail(h, QGRU_ERR_UNSUPPORTED, "no one-launch recurrence for this layer");
         return float_chain_launch(h, FloatFwdArgs{T, B, H, d.R, (const float *)h->f_wx.p, d.bw, d.br, s.h, s.v, 4, 1, rev ? 1 : 0, out}, st);
     }
     const qgru_params &p = h->p;
@@ -267,13 +267,13 @@ int train_forward_dir(qgru_handle *h, int mode, int T, int B, const void *x, lon
 
 // The chain of state gradients, the bias gradients and those of W and R; dx is the caller's (two directions add up).
 int train_backward_dir(qgru_handle *h, int mode, int T, int B, const float *x, const float *dout, long long do_ts, long long do_bs,
-                       const float *dhn, float *dh0, const qgru_train_dir &d, const TrainSaved &s, const float *xd, bool rev, cudaStream_t st) {
+                       const float *dhn, float *dh0, const qgru_train_dir &d, const TrainSaved &s, const float *xd, bool rev, int directions, cudaStream_t st) {
     const int H = h->H, I = h->I, C = h->C;
     const long long N = (long long)T * B;
-    int rc, G = 0;
-    if (!bwd_chain_fits(h, B, &G)) return fail(h, QGRU_ERR_UNSUPPORTED, "no one-launch recurrence for this layer");
+    int rc;
     const bool tc = mode != 0 && bwd_chain_tc_is_faster(h, B);
-    if (tc) G = h->plan_bwd_tc.G;
+    if (!tc && !bwd_chain_plan(h, B, directions)) return fail(h, QGRU_ERR_UNSUPPORTED, "no one-launch recurrence for this layer");
+    const int G = tc ? h->plan_bwd_tc.G : h->plan_bwd.G;
     if ((rc = ensure(h, h->bwd_dp, (size_t)N * C * 4))) return rc;
     if ((rc = ensure(h, h->bwd_dq, (size_t)N * C * 4))) return rc;
     if ((rc = ensure(h, h->bwd_bias, ((size_t)G * 2 * C + (size_t)B * H) * 4))) return rc;
@@ -352,7 +352,7 @@ int qgru_train_forward(qgru_handle *h, qgru_handle *rev, int mode, int T, int B,
         if (k) CK(cudaStreamWaitEvent(ds, rev->ev_split, 0));
         dirs[k].shares_x = k && mode && qgru::same_x_quantization(h, rev);
         const uint8_t *shared = dirs[k].shares_x ? (const uint8_t *)h->x8.p : nullptr;
-        rc = qgru::train_forward_dir(d, mode, T, B, x, x_ts, x_bs, h0 ? h0 + k * BH : nullptr, dirs[k], o, k == 1, ds, shared,
+        rc = qgru::train_forward_dir(d, mode, T, B, x, x_ts, x_bs, h0 ? h0 + k * BH : nullptr, dirs[k], o, k == 1, rev ? 2 : 1, ds, shared,
                                      rev && !k && mode ? rev->ev_split : nullptr);
         if (rc && k) h->err = rev->err;
         if (k) {
@@ -392,7 +392,7 @@ int qgru_train_backward(qgru_handle *h, qgru_handle *rev, int mode, int T, int B
     for (int k = rev ? 1 : 0; k >= 0; --k) {
         qgru_handle *d = k ? rev : h;
         rc = qgru::train_backward_dir(d, mode, T, B, x, dout + k * h->H, do_ts, do_bs, dh_n ? dh_n + k * BH : nullptr, dh0 ? dh0 + k * BH : nullptr,
-                                      dirs[k], s[k], xd[k], k == 1, k ? rev->side : st);
+                                      dirs[k], s[k], xd[k], k == 1, rev ? 2 : 1, k ? rev->side : st);
         if (k) {
             if (rc) h->err = rev->err;
             rc2 = rc;

@@ -72,6 +72,50 @@ def test_two_directions_share_an_odd_number_of_clusters(cuda_device):
         assert (a.cpu() - b).abs().max() <= 1e-5 * b.abs().max()
 
 
+def _grid_of(call, name):
+    """CTAs of the launches of a kernel during the call, as the profiler saw them."""
+    import json
+    import os
+    import tempfile
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    with tempfile.TemporaryDirectory() as d:
+        p.export_chrome_trace(os.path.join(d, "t.json"))
+        with open(os.path.join(d, "t.json")) as f:
+            events = json.load(f)["traceEvents"]
+    return [e["args"]["grid"][0] for e in events if name in e.get("name", "") and "grid" in e.get("args", {})]
+
+
+@pytest.mark.parametrize("H", [256, 512])
+def test_recurrences_are_planned_within_the_sm_limit(cuda_device, H):
+    """One direction with sm_limit 20 is cut into clusters for 20 SMs (two waves of them at the most here), also where two
+    such directions would fit the chip."""
+    import torch
+    torch.manual_seed(H)
+    QuantGRU = importlib.import_module(PKG_NAME + ".quant_gru").QuantGRU
+    T, B, I = 4, 30, 16
+    x = torch.randn(T, B, I, device=cuda_device)
+
+    def step(m):
+        out = m(x)[0]
+        return out, torch.autograd.grad(out, list(m.parameters()), torch.ones_like(out))
+    m = QuantGRU(I, H).to(cuda_device).train()
+    m.use_quantization = False
+    free = step(m)
+    assert max(_grid_of(lambda: step(m), "k_float_chain")) > 2 * 20
+    m.set_option("sm_limit", 20)
+    kept = step(m)
+    for name in ("k_float_chain", "k_bwd_chain"):
+        grids = _grid_of(lambda: step(m), name)
+        assert len(grids) == 1 and grids[0] <= 2 * 20, (name, grids)
+    # other clusters, the same sums in another order
+    for a, b in zip((kept[0], *kept[1]), (free[0], *free[1])):
+        assert (a - b).abs().max() <= 1e-5 * b.abs().max()
+
+
 @pytest.mark.parametrize("H,few,many", [(200, 300, 3000), (320, 300, 2500), (512, 100, 1100)])
 def test_float_forward_of_very_many_rows(cuda_device, H, few, many):
     """Beyond some number of rows the forward goes step by step: the same states as the rows give in smaller batches."""
