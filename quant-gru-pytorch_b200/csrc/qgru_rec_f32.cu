@@ -72,10 +72,12 @@ __host__ __device__ inline size_t fwd_smem_floats(int P, int U, int KG, int Bt, 
 // One: a thread has at most one cell a step (Bt <= KG; all rows are one block): its results stay in registers between the
 // cell and the stores, and no loop, staging buffer or 64-bit index is left around them.  A step of few rows
 // is a chain of some 900 dependent instructions at about five cycles each, so their number is what counts.
-template <bool One, int MaxThreads>
+// Alone: one CTA, no cluster.  Beside R, 32 registers are left of 128 where a CTA has 512 threads (97 to 128 units in one CTA), and what the
+// cluster needs does not fit: us a step, H = 128, 300 rows 3.6 -> 2.8, 500 rows 4.4 -> 3.3 (240 bytes of spills -> 72).
+template <bool One, int MaxThreads, bool Alone>
 __global__ void __launch_bounds__(MaxThreads, 1) k_float_chain(const FloatFwdArgs a) {
     extern __shared__ __align__(16) float sm[];
-    const int U = a.U, P = a.P, KG = a.KG, Bt = a.Bt, D = a.D, PU = P * U, H = a.H, C = 3 * H;
+    const int U = a.U, P = Alone ? 1 : a.P, KG = a.KG, Bt = a.Bt, D = a.D, PU = P * U, H = a.H, C = 3 * H;
     const int rb = One ? Bt : RB, rb_max = min(Bt, rb), BtU = Bt * U;
     float *hs = sm;
     float *own = hs + (size_t)(P == 1 ? 2 : 1) * Bt * PU;
@@ -199,8 +201,9 @@ __global__ void __launch_bounds__(MaxThreads, 1) k_float_chain(const FloatFwdArg
         const float *wxc = wxs + slot * 3 * BtU + cu;
         float *next = P > 1 ? own + ((s + 1) & 1) * BtU + cu : hs + ((s + 1) & 1) * BtU + cu;
         float o_z = 0.f, o_r = 0.f, o_g = 0.f, o_rz = 0.f, o_rr = 0.f, o_rg = 0.f, o_h = 0.f;   // One: this step's cell
-        for (int r0 = 0, pb = 0; r0 < nb; r0 += rb, pb ^= 1) {
-            const int r1 = min(nb, r0 + rb);
+        int r0 = 0, pb = 0;
+        do {
+            const int r1 = One ? nb : min(nb, r0 + RB);
             float *pk = part + pb * part_n + kg * rb_max * 3 * U + u;
             int b = r0;
             // (two rows at a time where there are registers for it)
@@ -309,7 +312,10 @@ __global__ void __launch_bounds__(MaxThreads, 1) k_float_chain(const FloatFwdArg
                     }
                 }
             }
-        }
+            if constexpr (One) break;
+            r0 += RB;
+            pb ^= 1;
+        } while (r0 < nb);
         if (P > 1) cluster_arrive();
         else __syncthreads();
         // Results leave for global memory behind the arrive: a cluster barrier's release waits for
@@ -728,7 +734,7 @@ void make_plan(qgru_handle *h, int B, int sms, int directions, bool fwd, KernOf 
 }
 
 // (what a form's launch takes: float_chain_launch, bwd_chain_launch)
-auto fwd_kernel(int threads) { return threads <= 384 ? k_float_chain<false, 384> : k_float_chain<false, 512>; }
+auto fwd_kernel(int threads) { return threads <= 384 ? k_float_chain<false, 384, false> : k_float_chain<false, 512, false>; }
 auto bwd_kernel(int threads) { return threads <= 384 ? k_bwd_chain<false, 384> : k_bwd_chain<false, 512>; }
 
 // Whether one of make_plan's forms runs at all.
@@ -775,8 +781,8 @@ bool float_chain_is_faster(qgru_handle *h, int T, int B) {
 int float_chain_launch(qgru_handle *h, FloatFwdArgs a, cudaStream_t st) {
     const F32RecPlan &pl = h->plan_fwd;
     const bool one = pl.Bt <= pl.KG, small = pl.U * pl.KG <= 384;
-    CK(launch_chain(one ? (small ? k_float_chain<true, 384> : k_float_chain<true, 512>)
-                        : (small ? k_float_chain<false, 384> : k_float_chain<false, 512>), pl, a, st));
+    CK(launch_chain(one ? (small ? k_float_chain<true, 384, false> : pl.P == 1 ? k_float_chain<true, 512, true> : k_float_chain<true, 512, false>)
+                        : (small ? k_float_chain<false, 384, false> : k_float_chain<false, 512, false>), pl, a, st));
     h->launches++;
     return QGRU_OK;
 }
