@@ -201,9 +201,8 @@ __global__ void __launch_bounds__(MaxThreads, 1) k_float_chain(const FloatFwdArg
         const float *wxc = wxs + slot * 3 * BtU + cu;
         float *next = P > 1 ? own + ((s + 1) & 1) * BtU + cu : hs + ((s + 1) & 1) * BtU + cu;
         float o_z = 0.f, o_r = 0.f, o_g = 0.f, o_rz = 0.f, o_rr = 0.f, o_rg = 0.f, o_h = 0.f;   // One: this step's cell
-        int r0 = 0, pb = 0;
-        do {
-            const int r1 = One ? nb : min(nb, r0 + RB);
+        for (int r0 = 0, pb = 0; r0 < nb; r0 += rb, pb ^= 1) {
+            const int r1 = min(nb, r0 + rb);
             float *pk = part + pb * part_n + kg * rb_max * 3 * U + u;
             int b = r0;
             // (two rows at a time where there are registers for it)
@@ -312,10 +311,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) k_float_chain(const FloatFwdArg
                     }
                 }
             }
-            if constexpr (One) break;
-            r0 += RB;
-            pb ^= 1;
-        } while (r0 < nb);
+        }
         if (P > 1) cluster_arrive();
         else __syncthreads();
         // Results leave for global memory behind the arrive: a cluster barrier's release waits for
