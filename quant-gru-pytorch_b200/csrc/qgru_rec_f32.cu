@@ -17,8 +17,8 @@
 // the partial sums instead, again H values per row.  Sums are added in a fixed order.
 //
 // Measured on a B200 against the two launches per step (tiled product, pointwise kernel) that it replaces, in us
-// per step: backward H = 512, B = 256: 221 -> 21; H = 262, B = 65: 112 -> 3.1; H = 128, B = 32: 48 -> 1.85.
-// Forward with gate buffer H = 262, B = 65: 36 -> 3.0; H = 256, B = 64: 31 -> 3.8; H = 128, B = 32: 2.0.
+// per step: backward H = 512, B = 256: 221 -> 22; H = 262, B = 65: 112 -> 3.3; H = 128, B = 32: 48 -> 2.0.
+// Forward with gate buffer H = 262, B = 65: 36 -> 3.0; H = 256, B = 64: 31 -> 2.7; H = 128, B = 32: 1.6.
 #include "qgru_rec_f32.cuh"
 
 #include "qgru_cluster.cuh"
@@ -673,7 +673,10 @@ cudaError_t launch_chain(Kern kern, const F32RecPlan &pl, Args &a, cudaStream_t 
 // CTA of so many threads runs.  us per step, 32 / 64 units a CTA: forward H = 256: 1 row 1.9 / 3.5, 64 rows (5 a cluster) 2.8 / 3.9,
 // 128 rows (9) 5.1 / 4.7; H = 128: 1 row 1.6 / 1.9, 256 rows (7, more than a cell a thread) 4.6 / 2.6; H = 160, 512 rows 10.8 / 7.5; backward
 // H = 256: 1 row 2.0 / 2.7, 96 rows 3.6 / 3.9, 128 rows 5.3 / 4.4.  One CTA against clusters: H = 96 1.35 / 1.7, H = 128 (512 threads)
-// 2.2 / 1.6.  The cost of a form is fitted to such times (H = 32 .. 512, 1 to 512 rows, one and two directions).
+// 2.1 / 1.6.  The cost of a form is fitted to such times (H = 32 .. 512, 1 to 512 rows, one and two directions); that of CTAs of more
+// than 384 threads and, backward, of two CTAs of 64 units to every form of 1 to 40 rows (as fitted before, two waves of one cell
+// a thread were passed over forward: H = 480, 89 rows in two directions 24.2 us a step, now 16.9; and two CTAs taken for one
+// backward: H = 128, 512 rows in two directions 8.9, now 7.8).
 template <typename KernOf>
 void make_plan(qgru_handle *h, int B, int sms, int directions, bool fwd, KernOf kern, size_t (*floats)(int, int, int, int, int), F32RecPlan *pl) {
     const int H = h->H;
@@ -690,15 +693,21 @@ void make_plan(qgru_handle *h, int B, int sms, int directions, bool fwd, KernOf 
         if (threads > 512 || (P - 1) * U >= H) continue;
         const int active0 = active_clusters(kern(threads), P, threads, floats(P, U, KG, 1, 1) * sizeof(float));
         if (active0 <= 0) continue;
-        // Cycles of a step of Bt rows: block barriers, the cell and, in a cluster, its barrier and the remote loads; spills in CTAs of
-        // more than 384 threads; the product and the partial sums of a row, where a warp of 32 units has fewer neighbours to
-        // share the row's state with.  With more than a cell a thread a row costs a block barrier's share at least.
+        // Cycles of a step of Bt rows: block barriers, the cell and, in a cluster, its barrier and the remote loads; the product and the
+        // partial sums of a row, where a warp of 32 units has fewer neighbours to share the row's state with.  With more than a cell a
+        // thread a row costs a block barrier's share at least.  CTAs of more than 384 threads spill.
         const int warps = threads / 32;
-        const double base = P == 1 ? (threads <= 384 ? 2050.0 : 3500.0) : threads > 384 ? 6000.0 : U == 32 ? 2950.0 : 3100.0 + 100.0 * (P - 2);
+        const bool large = threads > 384;
+        const double base = P == 1 ? 2050.0 : large ? 6000.0 : U == 32 ? 2950.0 : 3100.0 + 100.0 * (P - 2);
         const auto step = [&](int rows, int sharing) {
-            return rows <= KG ? base + (U == 32 ? 70.0 : 47.0) * warps * rows * sharing
-                   : fwd ? base + 2000.0 + std::max(750.0, (U == 32 ? 80.0 : 66.0) * warps) * rows * sharing
-                         : base + 2400.0 + (U == 32 ? std::max(540.0, 65.0 * warps) : 52.0 * warps) * rows * sharing;
+            const bool one = rows <= KG;
+            if (large && P == 1) return fwd ? (one ? 3000.0 + 50.0 * warps * rows : 1500.0 + 104.0 * warps * rows)
+                                            : (one ? 3800.0 + 81.0 * warps * rows : 4950.0 + 86.0 * warps * rows);
+            if (large && fwd && one) return 5600.0 + (160.0 + 45.0 * warps) * rows;
+            if (P == 2 && U == 64 && !fwd) return one ? 3600.0 + 608.0 * rows : 4220.0 + 838.0 * rows;
+            if (one) return base + (U == 32 ? 70.0 : 47.0) * warps * rows * sharing;
+            return fwd ? base + 2000.0 + std::max(750.0, (U == 32 ? 80.0 : 66.0) * warps) * rows * sharing
+                       : base + 2400.0 + (U == 32 ? std::max(540.0, 65.0 * warps) : 52.0 * warps) * rows * sharing;
         };
         for (int Bt = 1; Bt <= MAX_ROWS && Bt <= B; ++Bt) {
             // operands three steps ahead where a step is shorter than a trip to memory
@@ -710,7 +719,9 @@ void make_plan(qgru_handle *h, int B, int sms, int directions, bool fwd, KernOf 
             const int G = (B + Bt - 1) / Bt, waves = (directions * G + active - 1) / active;
             const int sharing = std::max(1, std::min(per_sm, (directions * G * P + chip - 1) / chip));
             double cost = waves * step(Bt, sharing);
-            // One cluster too many for the chip, but with few rows: the last ones of the two directions follow one another.
+            // One cluster too many for the chip: the last one of the second direction starts when the last one of the first, which has the
+            // rest of the rows, is done.  us a step of both directions, such a plan / the best of the others: H = 262, 65 rows backward 5.4 /
+            // 7.3; H = 320, 51 rows 4.7 / 6.1 forward, 5.5 / 7.1 backward; H = 416, 43 rows 8.6 / 10.7, 7.7 / 10.4.
             if (directions > 1 && directions * G == active + 1) cost = std::min(cost, std::max(step(Bt, sharing), 2.0 * step(B - (G - 1) * Bt, sharing)));
             if (best == 0 || cost < best) {
                 best = cost;
@@ -721,7 +732,7 @@ void make_plan(qgru_handle *h, int B, int sms, int directions, bool fwd, KernOf 
                 pl->D = D;
                 pl->G = G;
                 pl->waves = waves;
-                pl->sharing = sharing;
+                pl->us = cost / 1900.0;          // (MHz under such a load)
                 pl->smem = smem;
                 pl->ok = true;
             }
@@ -729,7 +740,8 @@ void make_plan(qgru_handle *h, int B, int sms, int directions, bool fwd, KernOf 
     }
 }
 
-// (what a form's launch takes: float_chain_launch, bwd_chain_launch)
+// The kernel whose occupancy a form is planned with: the one for several cells a thread.  That for one cell has the same number of
+// registers (168, with more than 384 threads 128).
 auto fwd_kernel(int threads) { return threads <= 384 ? k_float_chain<false, 384, false> : k_float_chain<false, 512, false>; }
 auto bwd_kernel(int threads) { return threads <= 384 ? k_bwd_chain<false, 384> : k_bwd_chain<false, 512>; }
 
@@ -759,17 +771,18 @@ bool float_chain_plan(qgru_handle *h, int B, int directions) {
 }
 
 // Every wave of clusters loads R first, and thousands of rows make many waves, where the tiled product of a step reads R once
-// for 64 or 128 rows.  us per step, chain / step by step: H = 512: 128 rows 16 / 19, 512 rows 57 / 48, 4096 rows 460 / 176;
-// H = 384: 256 rows 16 / 19, 1024 rows 66 / 41; H = 256: 1024 rows 23 / 28, 4096 rows 93 / 69; H = 128: 4096 rows 23 / 27; and
-// calls of one step: H = 64, 64 rows 44.9 / 45.0, 4096 rows 68 / 59; H = 512, one row 57 / 48.  Both sides as fitted to
-// such times (H = 16 .. 512, up to 8192 rows): from four steps on at most 20 % off the better one at each of 120 sizes.
+// for 64 or 128 rows.  us per step in calls of 20, chain / step by step: H = 512: 180 rows 18.6 / 22.9, 300 rows 30.9 / 26.7; H = 384: 256
+// rows 18.3 / 20.4, 600 rows 40.6 / 29.2; H = 256: 800 rows 20.5 / 27.4, 2048 rows 47.1 / 36.1; H = 128: 4096 rows 22.3 / 32.2, 6000 rows
+// 33.4 / 31.1.  The chain as its plan costs it and 8 us a wave for R, the steps as fitted around the line between the two (far
+// beyond it the product is on the tensor cores, and the steps cost less than this says).  Over 792 calls of 2, 3, 5 and 20 steps (H = 32 ..
+// 512, 1 to 8192 rows) the choice costs 0.3 % in the mean; 15 lose more than 5 %, the worst (H = 96, 8192 rows, 3 steps) 38 %.
 bool float_chain_is_faster(qgru_handle *h, int T, int B) {
     // (float inference and calibration run one direction after the other: each has the whole chip)
     make_plan(h, B, h->sm_count, 1, true, fwd_kernel, fwd_smem_floats, &h->plan_fwd);
     const F32RecPlan &pl = h->plan_fwd;
     if (!pl.ok) return false;
-    const double H = h->H, chain = pl.waves * (0.7 + 0.046 * (pl.U * pl.KG / 32) * pl.Bt * pl.sharing);
-    return 8.0 + 8.0 * pl.waves + T * chain <= T * (17.0 + (1.32e-7 * H + 1.0e-5) * H * B);
+    const double H = h->H;
+    return 8.0 + 8.0 * pl.waves + T * pl.us <= T * (17.0 + (1.32e-7 * H + 1.0e-5) * H * B);
 }
 
 // (forms of at most 384 threads have registers to spare beside R: the backward has no spills there, the forward 40 and 68

@@ -16,7 +16,8 @@ struct F32RecPlan {
     int H = 0, B = 0, sms = 0, directions = 0;      // what the plan was made for
     bool ok = false;
     int P = 1, U = 32, KG = 1, Bt = 1, G = 1, D = 1;
-    int waves = 1, sharing = 1;     // clusters one after the other, CTAs on an SM at once
+    int waves = 1;                  // clusters one after the other
+    double us = 0;                  // estimate of a step, all waves
     size_t smem = 0;
 };
 
