@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 7);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = a.H, P = a.P;
-    const int p = P > 1 ? (int)cluster_rank() : 0;
+    const int p = (int)cluster_rank();
     const int grp = blockIdx.x / P, b0 = grp * a.Bt, nb = min(a.Bt, a.B - b0);
     const int cell_warps = a.rows / RPT * UW;
     const uint32_t recv_bytes = (uint32_t)(P * min(U, (H - p * U + 31) & ~31) * a.rows * 4);
@@ -183,12 +183,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
     }
     fence_proxy_async_cta();
     tc::tc_fence_before_sync();
-    if (P > 1) {
-        cluster_arrive();
-        cluster_wait();
-    } else {
-        __syncthreads();
-    }
+    cluster_arrive();
+    cluster_wait();
     tc::tc_fence_after_sync();
 
     // cells: unit cu of this CTA's, rows r0 .. r0 + RPT - 1
@@ -351,10 +347,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
             tc::tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(b_full);
-            if (P > 1) {
-                __syncwarp();
-                cluster_arrive();        // this warp has read what came for the last step
-            }
+            __syncwarp();
+            cluster_arrive();            // this warp has read what came for the last step
             // (behind the arrive, whose release would wait for them)
 #pragma unroll
             for (int e = 0; e < RPT; ++e)
@@ -369,7 +363,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
         } else {
             if (lane == 0) tc::mbar_arrive(b_full);     // this warp's reads of the accumulators lie behind it
             __syncwarp();
-            if (P > 1) cluster_arrive();
+            cluster_arrive();
         }
         if (issues) {
             if (lane == 0) {
@@ -391,7 +385,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
             ok = __all_sync(0xffffffffu, ok);
             tc::tc_fence_after_sync();
         }
-        if (P > 1) cluster_wait();       // every CTA has read its partial sums of the last step
+        cluster_wait();                  // every CTA has read its partial sums of the last step
         if (drains && ok) {
             for (int c = 0; c < a.rows; c += 16) {
                 int32_t v[3][16];
@@ -444,10 +438,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_bwd_chain_tc(const BwdTcArgs a) 
         a.bias_part[((size_t)grp * 6 + (k < 3 ? 0 : 3) + (a.torch && g < 2 ? 1 - g : g)) * H + p * U + uu] = s;
     }
     if (warp == WARPS - 1) tc::tmem_dealloc(tmem, 512);
-    if (P > 1) {   // nobody leaves while a peer may still store into it
-        cluster_arrive();
-        cluster_wait();
-    }
+    cluster_arrive();    // nobody leaves while a peer may still store into it
+    cluster_wait();
 }
 
 // What follows from H, U and Bt; false where it does not fit.
@@ -498,10 +490,11 @@ cudaLaunchConfig_t config(int P, int G, size_t smem, cudaStream_t st, cudaLaunch
 
 }  // namespace
 
-// The form for B rows.  32 units a CTA are the shorter step (half the MMAs) until a cluster has more than 20 rows: what then takes
-// longest is the H x rows partial sums that a CTA sends (14 bytes a clock), and 64 units a CTA are half the CTAs a
-// cluster, twice the clusters and half the rows.  us per step (24 steps, four rows a cell thread), 32 / 64 units: H = 512: 128 rows
-// 4.8 / 5.0, 256 rows 7.0 / 6.2; H = 384: 256 rows 5.5 / 4.5; H = 262: 256 rows (16 a cluster) 3.7 / 4.1.  128 units a CTA were slower.
+// The form for B rows, in clusters of two CTAs or more (H > 64).  32 units a CTA are the shorter step (half the MMAs) until a cluster
+// has more than 20 rows: what then takes longest is the H x rows partial sums that a CTA sends (14 bytes a clock), and 64 units a
+// CTA are half the CTAs a cluster, twice the clusters and half the rows.  us per step (24 steps, four rows a cell thread), 32 / 64
+// units: H = 512: 128 rows 4.8 / 5.0, 256 rows 7.0 / 6.2; H = 384: 256 rows 5.5 / 4.5; H = 262: 256 rows (16 a cluster) 3.7 / 4.1.  128 units a
+// CTA were slower.
 bool bwd_chain_tc_plan(qgru_handle *h, int B, int sms, F32RecPlan *best) {
     const int H = h->H;
     if (best->H == H && best->B == B && best->sms == sms) return best->ok;
@@ -509,7 +502,7 @@ bool bwd_chain_tc_plan(qgru_handle *h, int B, int sms, F32RecPlan *best) {
     best->H = H;
     best->B = B;
     best->sms = sms;
-    if (H > 512) return false;
+    if (H <= 64 || H > 512) return false;
     for (const int U : {32, 64}) {
         if (best->ok && best->Bt <= 20 && best->waves == 1) break;
         F32RecPlan pl = *best;
