@@ -152,6 +152,8 @@ class _LayerFunction(torch.autograd.Function):
         if any((t.dtype, t.shape, t.device) != as_ for t, as_ in zip(keep, ctx.kept_as)):
             raise RuntimeError("a saved-tensor hook has returned another type, shape or device than it was given")
         saved, *x = [t.contiguous() for t in keep]
+        if saved.data_ptr() % 256:      # (a hook's view: the library reads the block's parts as words and vectors)
+            saved = saved.clone()
         T, B, I, H = ctx.shape
         D, dev = len(ctx.handles), saved.device
         t_dim, b_dim = (1, 0) if ctx.batch_first else (0, 1)

@@ -81,6 +81,25 @@ def test_a_hook_that_returns_something_else_is_an_error(cuda_device):
 
 
 @STORAGE
+def test_a_hook_may_return_a_view_at_any_byte(cuda_device, storage):
+    """Hooks that keep every tensor as bytes of one buffer: the block comes back off its alignment."""
+    import torch
+    m = _module(storage, cuda_device, H=132)
+    x = torch.randn(9, 7, 40, device=cuda_device)
+    want = _grads(m, *m(x))
+
+    def pack(t):
+        if t.dtype != torch.uint8:
+            return t
+        flat = torch.empty(t.numel() + 3, dtype=t.dtype, device=t.device)
+        flat[3:].copy_(t.reshape(-1))
+        return flat[3:].view(t.shape)
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+        out, hn = m(x)
+    assert all(torch.equal(a, b) for a, b in zip(_grads(m, out, hn), want))
+
+
+@STORAGE
 def test_two_live_forwards_and_parameters_changed_before_the_backward(cuda_device, storage):
     """Forwards of different sizes alive at once, backwards in either order, parameters stepped in place in between."""
     import torch
