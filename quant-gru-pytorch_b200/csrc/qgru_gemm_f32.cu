@@ -226,7 +226,8 @@ int gemm_f32(qgru_handle *h, const GemmF32 &g, cudaStream_t st) {
     // us, tensor cores / fp32 pipe: 51200 x 1536 x 256 331 / 862; 12800 x 128 x 768 47 / 71; 6400 x 64 x 384 14 / 21; 384 x 3200 x 128
     // 22 / 24; below that 384 x 1600 x 128 19 / 19, 64 x 1536 x 512 20 / 17.  A narrow C fills the tile of neither (6400 x 384 x 64
     // 28 / 24, 12800 x 384 x 16 29 / 41); few K leave only the tile's own time (12800 x 16 x 768 31 / 18), and operands without two
-    // neighbours in one load more of it (12801 x 77 x 600 49 / 41, 12801 x 600 x 77 66 / 76).
+    // neighbours in one load more of it (12801 x 77 x 600 49 / 41, 12801 x 600 x 77 66 / 76).  (Before the operands' factor of 2^24, 1 to 5 %
+    // of the tensor cores' times.)
     const bool pairs = ((g.a_trans ? g.N : g.K) | (g.b_trans ? g.K : (long long)g.M)) % 2 == 0 &&
                        ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B)) & 7u) == 0;
     if (g.K >= (pairs ? 64 : 256) && (double)g.N * g.K * std::max(g.M, 64) >= (g.M <= 64 ? 2.5e8 : 1.5e8) && gemm_f32_tc_fits(g)) {

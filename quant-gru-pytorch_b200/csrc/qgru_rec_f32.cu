@@ -73,7 +73,7 @@ __host__ __device__ inline size_t fwd_smem_floats(int P, int U, int KG, int Bt, 
 // cell and the stores, and no loop, staging buffer or 64-bit index is left around them.  A step of few rows
 // is a chain of some 900 dependent instructions at about five cycles each, so their number is what counts.
 // Alone: one CTA, no cluster.  Beside R, 32 registers are left of 128 where a CTA has 512 threads (97 to 128 units in one CTA), and what the
-// cluster needs does not fit: us a step, H = 128, 300 rows 3.6 -> 2.8, 500 rows 4.4 -> 3.3 (240 bytes of spills -> 72).
+// cluster needs does not fit: us a step, H = 128, 300 rows 3.6 -> 2.8, 500 rows 4.4 -> 3.3 (240 bytes of spills -> 60).
 template <bool One, int MaxThreads, bool Alone>
 __global__ void __launch_bounds__(MaxThreads, 1) k_float_chain(const FloatFwdArgs a) {
     extern __shared__ __align__(16) float sm[];
@@ -785,8 +785,8 @@ bool float_chain_is_faster(qgru_handle *h, int T, int B) {
     return 8.0 + 8.0 * pl.waves + T * pl.us <= T * (17.0 + (1.32e-7 * H + 1.0e-5) * H * B);
 }
 
-// (forms of at most 384 threads have registers to spare beside R: the backward has no spills there, the forward 40 and 68
-// bytes; with 512 threads 228 to 348 bytes)
+// (forms of at most 384 threads have registers to spare beside R: the backward has no spills there, the forward 48 and 68
+// bytes; with 512 threads 228 to 348 bytes, without a cluster 60)
 int float_chain_launch(qgru_handle *h, FloatFwdArgs a, cudaStream_t st) {
     const F32RecPlan &pl = h->plan_fwd;
     const bool one = pl.Bt <= pl.KG, small = pl.U * pl.KG <= 384;

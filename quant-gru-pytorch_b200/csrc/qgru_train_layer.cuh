@@ -80,7 +80,8 @@ __global__ void __launch_bounds__(128) k_train_weights(const TrainWeightsArgs a)
 
 namespace {
 
-// The caller's block of one direction.
+// The caller's block of one direction.  R is in it also where the chain of state gradients reads r8: the backward takes the fp32
+// chain if the handle's sm_limit has changed to one that leaves no cluster to the other.
 struct TrainSaved {
     float *h, *v, *xd, *W, *R, *r_scale;
     int8_t *r8;
